@@ -29,6 +29,7 @@
 
 #define ENS_MAX_ATOMS 9216  // largest replica the loop takes (shared memory)
 #define ENS_MAX_CELLS 4096
+#define ENS_RANK 3          // atoms per lane of the cell sort (cells of up to 96 atoms)
 
 struct EnsArgs {
     const int* order;
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
     int* ccur = cstart + (ncell + 1);                      // [ncell]
     int* sorted = ccur + ncell;                            // [n] atoms in cell order
     __shared__ int warp_tot[THREADS / 32];
+    __shared__ int next_item;  // the list build's next cell
     const int tid = threadIdx.x, lane = tid % LPA, g = tid / LPA;
     const double dt = A.dt, hdt = 0.5 * dt, dtsq = dt * dt;
     const double c1 = R.bc1;
@@ -171,29 +173,69 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                 sorted[slot] = i;
             }
             __syncthreads();
-            for (int c = tid; c < ncell; c += THREADS) {  // insertion sort of the cell's atoms
-                const int b0 = cstart[c], b1 = cstart[c + 1];
-                for (int k = b0 + 1; k < b1; ++k) {
-                    const int v0 = sorted[k];
-                    int m = k - 1;
-                    while (m >= b0 && sorted[m] > v0) {
-                        sorted[m + 1] = sorted[m];
-                        --m;
+            // each cell's atoms into index order: a warp per cell, every
+            // lane counts the smaller indices of its (up to ENS_RANK) atoms
+            // and then places them. (A thread per cell by insertion took the
+            // whole block's time in a one-cell replica, ~n^2 / 4 dependent
+            // shared-memory moves, and kept 1 lane in 32 busy elsewhere.) In
+            // a one-cell replica the order is the identity.
+            if (ns == 0) {
+                for (int i = tid; i < n; i += THREADS) sorted[i] = i;
+            } else {
+                const int wl = tid & 31;
+                for (int c = tid >> 5; c < ncell; c += THREADS / 32) {
+                    const int b0 = cstart[c], m = cstart[c + 1] - b0;
+                    if (m <= 32 * ENS_RANK) {
+                        int v[ENS_RANK], rank[ENS_RANK];
+#pragma unroll
+                        for (int e = 0; e < ENS_RANK; ++e) {
+                            v[e] = wl + 32 * e < m ? sorted[b0 + wl + 32 * e] : 0x7fffffff;
+                            rank[e] = 0;
+                        }
+                        for (int k = 0; k < m; ++k) {
+                            const int o = sorted[b0 + k];
+#pragma unroll
+                            for (int e = 0; e < ENS_RANK; ++e) rank[e] += o < v[e];
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int e = 0; e < ENS_RANK; ++e)
+                            if (wl + 32 * e < m) sorted[b0 + rank[e]] = v[e];
+                        __syncwarp();
+                    } else if (wl == 0) {  // a collapsed cell: insertion sort
+                        for (int k = b0 + 1; k < b0 + m; ++k) {
+                            const int v0 = sorted[k];
+                            int q = k - 1;
+                            while (q >= b0 && sorted[q] > v0) {
+                                sorted[q + 1] = sorted[q];
+                                --q;
+                            }
+                            sorted[q + 1] = v0;
+                        }
                     }
-                    sorted[m + 1] = v0;
                 }
             }
+            if (tid == 0) next_item = 0;
             __syncthreads();
-            // list rows: a warp per cell, lane = one of the cell's atoms (32
-            // at a time); the stencil cells' atoms are read once per warp as
-            // shared-memory broadcasts, in stencil then index order, and each
-            // lane appends those within the list radius to its own row
+            // list rows: a warp per item, an item a cell (in a one-cell
+            // replica 32 of its atoms), taken from a shared counter; lane =
+            // one of the cell's atoms (32 at a time); the stencil cells'
+            // atoms are read once per warp as shared-memory broadcasts, in
+            // stencil then index order, and each lane appends those within
+            // the list radius to its own row. (Items on a counter, so that no
+            // warp waits for the one with the fullest cells; a one-cell
+            // replica has a warp per 32 atoms instead of one warp in all.)
             {
-                const int wid = tid >> 5, wl = tid & 31;
-                for (int c = wid; c < ncell; c += THREADS / 32) {
+                const int wl = tid & 31;
+                const int items = ns > 0 ? ncell : (n + 31) / 32;
+                for (;;) {
+                    int c = 0;
+                    if (wl == 0) c = atomicAdd(&next_item, 1);
+                    c = __shfl_sync(0xffffffffu, c, 0);
+                    if (c >= items) break;
                     const int cx = ns > 0 ? c / (nc * nc) : 0, cy = ns > 0 ? (c / nc) % nc : 0,
                               cz = ns > 0 ? c % nc : 0;
-                    const int c0 = cstart[c], c1 = cstart[c + 1];
+                    const int c0 = ns > 0 ? cstart[c] : 32 * c, c1 = ns > 0 ? cstart[c + 1] : min(n, 32 * c + 32);
                     for (int a0c = c0; a0c < c1; a0c += 32) {
                         const bool active = a0c + wl < c1;
                         const int i = active ? sorted[a0c + wl] : 0;

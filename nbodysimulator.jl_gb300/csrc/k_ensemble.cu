@@ -89,6 +89,14 @@ __device__ void ens_scan(const int* cnt, int* out, int m, int* warp_tot)
     __syncthreads();
 }
 
+// Where entry k of a row lies (16-bit units): block of 8 LPA entries, then
+// lane k % LPA, then its 8 entries in order.
+template <int LPA>
+__device__ __forceinline__ int ens_slot(int k)
+{
+    return (k & ~(8 * LPA - 1)) + (k % LPA) * 8 + (k % (8 * LPA)) / LPA;
+}
+
 template <int LPA, int POT, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, EnsArgs A)
 {
@@ -103,7 +111,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
     uint4* pos = ens_sm;                                   // [n] fixed-point x, y, z and the charge bits
     int* cstart = reinterpret_cast<int*>(pos + n);         // [ncell + 1]
     int* ccur = cstart + (ncell + 1);                      // [ncell]
-    int* sorted = ccur + ncell;                            // [n] atoms in cell order
+    uint16_t* sorted = reinterpret_cast<uint16_t*>(ccur + ncell);  // [n] atoms in cell order
+    uint16_t* cnts = sorted + n;                           // [n] list counts
     __shared__ int warp_tot[THREADS / 32];
     __shared__ int next_item;  // the list build's next cell
     const int tid = threadIdx.x, lane = tid % LPA, g = tid / LPA;
@@ -114,7 +123,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
     // the frame sink (trajectory saving), read at a save point
     const int64_t sk_every = A.save ? d.sink->every : 0;
     const int64_t sk_t0 = A.save ? d.sink->t0 : 0;
-    for (int i = tid; i < n; i += THREADS) pos[i].w = d.pfx[a0 + i].w;
+    // list rows of this loop: replica-local 16-bit indices in the list
+    // buffer's memory, 2 cap per atom (nothing else reads them: every other
+    // path builds its own lists first). Entry k of a row lies where lane
+    // k % LPA finds its 8 entries of a block of 8 LPA in one 16-byte load,
+    // four packed steps of the force loop (ens_slot).
+    uint16_t* const rows = reinterpret_cast<uint16_t*>(d.nbr);
+    for (int i = tid; i < n; i += THREADS) {
+        pos[i].w = d.pfx[a0 + i].w;
+        cnts[i] = A.reuse ? (uint16_t)min(d.nbr_count[a0 + i], cap) : (uint16_t)0;
+    }
     int since = A.reuse ? A.since[r] : -1;
 
     bool range_err = false;
@@ -227,6 +245,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
             // replica has a warp per 32 atoms instead of one warp in all.)
             {
                 const int wl = tid & 31;
+                const float rl2 = R.fx_rl2;
                 const int items = ns > 0 ? ncell : (n + 31) / 32;
                 for (;;) {
                     int c = 0;
@@ -241,7 +260,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                         const int i = active ? sorted[a0c + wl] : 0;
                         const uint4 qi = pos[i];
                         const int64_t gi = a0 + i;
-                        int* row = d.nbr + gi * d.nbr_istride;
+                        uint16_t* row = rows + gi * 2 * cap;
                         int cnt = 0;
                         for (int ox = -ns; ox <= ns; ++ox) {
                             int nx = cx + ox;
@@ -257,11 +276,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                                     nz -= nz >= nc ? nc : 0;
                                     const int cq = (nx * nc + ny) * nc + nz;
                                     const int q1 = cstart[cq + 1];
+#pragma unroll 4
                                     for (int k = cstart[cq]; k < q1; ++k) {
                                         const int j = sorted[k];
                                         float ddx, ddy, ddz;
-                                        if (active && j != i && fx_r2(qi, pos[j], ddx, ddy, ddz) < R.fx_rl2) {
-                                            if (cnt < cap) row[(int64_t)cnt * d.nbr_kstride] = (int)(a0 + j);
+                                        if (active && j != i && fx_r2(qi, pos[j], ddx, ddy, ddz) < rl2) {
+                                            if (cnt < cap) row[ens_slot<LPA>(cnt)] = (uint16_t)j;
                                             ++cnt;
                                         }
                                     }
@@ -274,6 +294,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                                 cnt = cap;
                             }
                             d.nbr_count[gi] = cnt;
+                            cnts[i] = (uint16_t)cnt;
                             A.pref[gi] = qi;
                         }
                     }
@@ -289,37 +310,49 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
         const bool lj_atoms = POT != FX_EL;
         const float lj_lo = R.fx_lj_lo, lj_hi = R.fx_lj_hi, el_lo = R.fx_el_lo, el_hi = R.fx_el_hi;
         const float sig2h = R.fx_sig2_hi, sig2l = R.fx_sig2_lo, krf = R.fx_krf;
+        const double fscale = R.fx_fscale;
         for (int i0 = 0; i0 < n; i0 += G) {
             const int i = i0 + g;
             const bool active = i < n;
             const int64_t gi = a0 + (active ? i : 0);
             const uint4 qi = pos[active ? i : 0];
-            const int cnt = active ? min(d.nbr_count[gi], cap) : 0;
+            const int cnt = active ? cnts[i] : 0;
+            const int cmax = __reduce_max_sync(0xffffffffu, cnt);  // the warp's longest row
             const float kqi =
                 POT != FX_LJ ? (float)(d.charge[gi] * R.fx_kq) : 0.0f;
-            const int* row = d.nbr + gi * d.nbr_istride;
+            // the velocity update's operands (lane k < 3: component k) are
+            // loaded ahead of the pair loop
+            const bool upd = active && lane < 3;
+            const int64_t e = 3 * gi + (lane < 3 ? lane : 0);
+            const double im = d.inv_mass[gi] * fscale;
+            const double v_in = upd ? s.v[e] : 0.0;
+            const double ao_in = upd && !A.baoab ? s.a_old[e] : 0.0;
+            const uint4* row = reinterpret_cast<const uint4*>(rows + gi * 2 * cap) + lane;
             float2 px = make_float2(0.f, 0.f), py = px, pz = px;
-            // the row entries of the next iteration are loaded before this
-            // iteration's gathers and arithmetic (one iteration ahead)
-            // (debug builds: an entry outside the replica's atoms is reported
-            // and replaced by its first atom before it indexes shared memory)
-            int jn0 = lane < cnt ? (int)a0 + dbg_index(__ldg(row + (int64_t)lane * d.nbr_kstride) - (int)a0, n, 0, d.status)
-                                 : (int)a0;
-            int jn1 = lane + LPA < cnt
-                          ? (int)a0 + dbg_index(__ldg(row + (int64_t)(lane + LPA) * d.nbr_kstride) - (int)a0, n, 0, d.status)
-                          : jn0;
-            for (int k0 = lane; k0 < cnt; k0 += 2 * LPA) {
-                const bool v1 = k0 + LPA < cnt;
-                const int j0 = jn0, j1 = jn1;
-                const int kn = k0 + 2 * LPA;
-                jn0 = kn < cnt ? (int)a0 + dbg_index(__ldg(row + (int64_t)kn * d.nbr_kstride) - (int)a0, n, 0, d.status)
-                               : (int)a0;
-                jn1 = kn + LPA < cnt
-                          ? (int)a0 + dbg_index(__ldg(row + (int64_t)(kn + LPA) * d.nbr_kstride) - (int)a0, n, 0, d.status)
-                          : jn0;
-                const uint4 q0 = pos[j0 - a0], q1 = pos[j1 - a0];
-                fx_pair2<POT>(d, s.x, gi, lj_atoms, kqi, qi, j0, j1, true, v1, q0, q1, lj_lo, lj_hi, el_lo, el_hi, sig2h,
-                              sig2l, krf, px, py, pz, range_err);
+            // one load holds the lane's entries of four packed steps; the
+            // next block's load is issued before this block's arithmetic.
+            // An entry past the row's count reads the atom itself and adds
+            // zero; steps past the warp's longest row are skipped.
+            uint4 nx = lane < cnt ? __ldcg(row) : make_uint4(0u, 0u, 0u, 0u);
+            for (int kb = 0; kb < cmax; kb += 8 * LPA) {
+                const uint4 cur = nx;
+                if (kb + 8 * LPA + lane < cnt) nx = __ldcg(row + (kb / 8 + LPA));
+                const unsigned w[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int k0 = kb + 2 * m * LPA;
+                    if (k0 >= cmax) break;
+                    const bool v0 = k0 + lane < cnt, v1 = k0 + LPA + lane < cnt;
+                    int j0 = v0 ? (int)(w[m] & 0xffffu) : (active ? i : 0);
+                    int j1 = v1 ? (int)(w[m] >> 16) : (active ? i : 0);
+                    // (debug builds: an entry outside the replica's atoms is
+                    // reported and replaced by its first atom)
+                    j0 = dbg_index(j0, n, 0, d.status);
+                    j1 = dbg_index(j1, n, 0, d.status);
+                    const uint4 q0 = pos[j0], q1 = pos[j1];
+                    fx_pair2<POT>(d, s.x, gi, lj_atoms, kqi, qi, (int)a0 + j0, (int)a0 + j1, v0, v1, q0, q1, lj_lo,
+                                  lj_hi, el_lo, el_hi, sig2h, sig2l, krf, px, py, pz, range_err);
+                }
             }
             float hx = __fadd_rn(px.x, px.y), hy = __fadd_rn(py.x, py.y), hz = __fadd_rn(pz.x, pz.y);
             float ex = 0.f, ey = 0.f, ez = 0.f;
@@ -329,30 +362,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                 fx_join(hy, ey, o, LPA);
                 fx_join(hz, ez, o, LPA);
             }
-            if (active && lane == 0) {
-                const double im = d.inv_mass[gi] * R.fx_fscale;
-                const double an[3] = {((double)hx + (double)ex) * im, ((double)hy + (double)ey) * im,
-                                      ((double)hz + (double)ez) * im};
-                if (!finite64(an[0]) || !finite64(an[1]) || !finite64(an[2])) status_set(d.status, ST_NONFINITE);
-                double* v = s.v + 3 * gi;
-                double* ao = s.a_old + 3 * gi;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    v[k] = A.baoab ? __dadd_rn(v[k], __dmul_rn(hdt, an[k])) : kick1(v[k], ao[k], an[k], dt);
-                    ao[k] = an[k];
-                    s.a_new[3 * gi + k] = an[k];
-                }
+            // every lane of the group holds the joined sums: lane k updates
+            // component k (a third of the FP64 instructions of one lane
+            // updating all three; FP64 issues at 2 lanes per clock here)
+            if (upd) {
+                const float h = lane == 0 ? hx : lane == 1 ? hy : hz, el = lane == 0 ? ex : lane == 1 ? ey : ez;
+                const double an = ((double)h + (double)el) * im;
+                if (!finite64(an)) status_set(d.status, ST_NONFINITE);
+                const double vn = A.baoab ? __dadd_rn(v_in, __dmul_rn(hdt, an)) : kick1(v_in, ao_in, an, dt);
+                s.v[e] = vn;
+                s.a_old[e] = an;
+                s.a_new[e] = an;
                 const int64_t t = step + 1 - sk_t0;  // the frame sink's index of the new state
                 if (sk_every > 0 && t % sk_every == 0) {
                     const FrameSink* sk = d.sink;
                     const int64_t slot = t / sk_every - sk->first;
                     if (slot >= 0 && slot < sk->cap) {
-                        const size_t o = (size_t)slot * 3 * d.cols + 3 * (size_t)gi;
-#pragma unroll
-                        for (int k = 0; k < 3; ++k) {
-                            sk->x[o + k] = s.x[3 * gi + k];
-                            sk->v[o + k] = v[k];
-                        }
+                        const size_t o = (size_t)slot * 3 * d.cols + (size_t)e;
+                        sk->x[o] = s.x[e];
+                        sk->v[o] = vn;
                     }
                 }
             }
@@ -424,7 +452,8 @@ bool ensemble_plan(nbg_ctx* c)
         cudaGetLastError();
         return false;
     }
-    c->ens_smem = sizeof(uint4) * (size_t)nmax + sizeof(int) * (2 * (size_t)cmax + 1 + (size_t)nmax);
+    c->ens_smem = sizeof(uint4) * (size_t)nmax + sizeof(int) * (2 * (size_t)cmax + 1) +
+                  2 * sizeof(uint16_t) * (size_t)nmax;
     ens_kernel_t k = ens_kernel(c);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->ens_smem) != cudaSuccess) {
         cudaGetLastError();

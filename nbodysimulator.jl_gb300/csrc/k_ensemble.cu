@@ -89,6 +89,17 @@ __device__ void ens_scan(const int* cnt, int* out, int m, int* warp_tot)
     __syncthreads();
 }
 
+// Distance along one axis, at least, from a candidate to any of the warp's
+// atoms, whose offsets from the reference position lie in [lo, hi]; the
+// candidate's offset as the wrapped difference, and its other image.
+__device__ __forceinline__ float ens_gap(unsigned off, float lo, float hi)
+{
+    const float o = (float)(int)off;
+    const float here = fmaxf(lo - o, o - hi);
+    const float there = o < 0.f ? o + 4294967296.f - hi : lo - (o - 4294967296.f);
+    return fmaxf(0.f, fminf(here, there));
+}
+
 // Where entry k of a row lies (16-bit units): block of 8 LPA entries, then
 // lane k % LPA, then its 8 entries in order.
 template <int LPA>
@@ -115,6 +126,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
     uint16_t* cnts = sorted + n;                           // [n] list counts
     __shared__ int warp_tot[THREADS / 32];
     __shared__ int next_item;  // the list build's next cell
+    __shared__ uint4 cand[THREADS / 32][32];  // its candidates, per warp
     const int tid = threadIdx.x, lane = tid % LPA, g = tid / LPA;
     const double dt = A.dt, hdt = 0.5 * dt, dtsq = dt * dt;
     const double c1 = R.bc1;
@@ -237,15 +249,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
             __syncthreads();
             // list rows: a warp per item, an item a cell (in a one-cell
             // replica 32 of its atoms), taken from a shared counter; lane =
-            // one of the cell's atoms (32 at a time); the stencil cells'
-            // atoms are read once per warp as shared-memory broadcasts, in
-            // stencil then index order, and each lane appends those within
-            // the list radius to its own row. (Items on a counter, so that no
-            // warp waits for the one with the fullest cells; a one-cell
-            // replica has a warp per 32 atoms instead of one warp in all.)
+            // one of the cell's atoms (32 at a time). The stencil cells'
+            // atoms pass, in stencil then index order, through a per-warp
+            // buffer that takes only those within the list radius of the box
+            // of the warp's atoms (about 3 in 4), and each lane appends those
+            // within the list radius of its own atom to its row. (Items on a
+            // counter, so that no warp waits for the one with the fullest
+            // cells; a one-cell replica has a warp per 32 atoms instead of
+            // one warp in all.)
             {
                 const int wl = tid & 31;
                 const float rl2 = R.fx_rl2;
+                uint4* const buf = cand[tid >> 5];
                 const int items = ns > 0 ? ncell : (n + 31) / 32;
                 for (;;) {
                     int c = 0;
@@ -262,6 +277,39 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                         const int64_t gi = a0 + i;
                         uint16_t* row = rows + gi * 2 * cap;
                         int cnt = 0;
+                        // the box of the warp's atoms, as offsets from the first one's position
+                        uint4 ref = qi;
+                        ref.x = __shfl_sync(0xffffffffu, qi.x, 0);
+                        ref.y = __shfl_sync(0xffffffffu, qi.y, 0);
+                        ref.z = __shfl_sync(0xffffffffu, qi.z, 0);
+                        const int rx = active ? (int)(qi.x - ref.x) : 0, ry = active ? (int)(qi.y - ref.y) : 0,
+                                  rz = active ? (int)(qi.z - ref.z) : 0;
+                        const float lox = (float)__reduce_min_sync(0xffffffffu, rx),
+                                    hix = (float)__reduce_max_sync(0xffffffffu, rx),
+                                    loy = (float)__reduce_min_sync(0xffffffffu, ry),
+                                    hiy = (float)__reduce_max_sync(0xffffffffu, ry),
+                                    loz = (float)__reduce_min_sync(0xffffffffu, rz),
+                                    hiz = (float)__reduce_max_sync(0xffffffffu, rz);
+                        int fill = 0;
+                        // the m candidates of the buffer: the tests without a
+                        // branch into a bit mask, then the lane's hits in order
+                        auto test = [&](int m) {
+                            unsigned hits = 0u;
+#pragma unroll 8
+                            for (int k = 0; k < m; ++k) {
+                                const uint4 c = buf[k];
+                                float ddx, ddy, ddz;
+                                const float r2 = fx_r2(qi, c, ddx, ddy, ddz);
+                                hits |= (r2 < rl2 && (int)c.w != i) ? 1u << k : 0u;
+                            }
+                            if (!active) hits = 0u;
+                            while (hits) {
+                                const int j = (int)buf[__ffs(hits) - 1].w;
+                                hits &= hits - 1u;
+                                if (cnt < cap) row[ens_slot<LPA>(cnt)] = (uint16_t)j;
+                                ++cnt;
+                            }
+                        };
                         for (int ox = -ns; ox <= ns; ++ox) {
                             int nx = cx + ox;
                             nx += nx < 0 ? nc : 0;
@@ -276,18 +324,40 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                                     nz -= nz >= nc ? nc : 0;
                                     const int cq = (nx * nc + ny) * nc + nz;
                                     const int q1 = cstart[cq + 1];
-#pragma unroll 4
-                                    for (int k = cstart[cq]; k < q1; ++k) {
-                                        const int j = sorted[k];
-                                        float ddx, ddy, ddz;
-                                        if (active && j != i && fx_r2(qi, pos[j], ddx, ddy, ddz) < rl2) {
-                                            if (cnt < cap) row[ens_slot<LPA>(cnt)] = (uint16_t)j;
-                                            ++cnt;
+                                    for (int kb = cstart[cq]; kb < q1; kb += 32) {
+                                        // a candidate per lane; those out of every row's reach are dropped
+                                        uint4 qc = qi;
+                                        bool keep = kb + wl < q1;
+                                        if (keep) {
+                                            const int j = sorted[kb + wl];
+                                            qc = pos[j];
+                                            qc.w = (unsigned)j;
+                                            if (ns > 0) {
+                                                const float gx = ens_gap(qc.x - ref.x, lox, hix);
+                                                const float gy = ens_gap(qc.y - ref.y, loy, hiy);
+                                                const float gz = ens_gap(qc.z - ref.z, loz, hiz);
+                                                keep = gx * gx + gy * gy + gz * gz < rl2 * 1.0002f;
+                                            }
+                                        }
+                                        const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                                        const int at = fill + __popc(bal & ((1u << wl) - 1u));
+                                        const int added = __popc(bal);
+                                        if (keep && at < 32) buf[at] = qc;
+                                        __syncwarp();
+                                        fill += added;
+                                        if (fill >= 32) {
+                                            test(32);
+                                            __syncwarp();
+                                            if (keep && at >= 32) buf[at - 32] = qc;
+                                            fill -= 32;
                                         }
                                     }
                                 }
                             }
                         }
+                        __syncwarp();
+                        test(fill);
+                        __syncwarp();  // (the buffer is free for the next chunk)
                         if (active) {
                             if (cnt > cap) {
                                 status_set(d.status, ST_NBR_OVERFLOW);

@@ -15,14 +15,19 @@
 //                    are apart by at least 1/16 of their largest |r| uses the
 //                    plain difference: its error, 2^-24 of the coordinates,
 //                    is then below 2^-19 of |r_ij|.
-//  k_allpairs        every other potential on small / unbounded systems, all
-//                    pairs through shared-memory tiles, same pair code as the
-//                    list kernel plus gravity and the magnetic dipole term.
+//  k_allpairs        every other potential on small / unbounded systems: 32
+//                    bodies a block, a warp per 128-body j-tile, the pair
+//                    arithmetic of the split-form list kernels plus gravity
+//                    and the magnetic dipole term.
 //  k_force_list      cutoff LJ + reaction-field electrostatics over a Verlet
 //                    list (one thread per atom, coalesced column-major list).
 //  k_bonded          SPC/Fw harmonic bonds and H-O-H angles, one thread per
 //                    molecule (basic_potentials.jl:367-433), FP32 terms from
 //                    FP64 intramolecular differences.
+#include <algorithm>
+#include <type_traits>
+
+#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 
 #include "nbg_internal.cuh"
@@ -458,106 +463,523 @@ int gravity_plan_chunks(nbg_ctx* c, int64_t npad) { return plan_gravity(c, npad)
 // ---------------------------------------------------------------------
 // generic all-pairs kernel
 // ---------------------------------------------------------------------
-#define AT 128
+#define AT 128        // j-tile: FP32 partials are summed in order over one tile
+#define AP_WARPS 10   // general form: j-tiles in flight per block, at most (48 KB of stages and sums)
+#define AP_SUB 32     // general form: bodies of a tile staged at a time per warp
+#define AP_COOP_TILES 16      // a tile per CTA up to 2048 bodies, then a tile per warp (an evaluation of
+                              // 1000 / 2000 / 3000 ions 12.5 / 18.6 / 31 us per CTA, 14.6 / 18.6 / 25 per warp)
+#define AP_CLUSTER_TILES 256  // most tiles whose sums a CTA holds (96 KB)
 
-__global__ void __launch_bounds__(AT) k_allpairs(Dev d, StateView s)
+// A pair that FP32 leaves open, decided (and its difference taken) in the
+// reference's FP64 arithmetic.
+struct ApExact {
+    float3 dr;
+    float r2;
+    bool lj_in, el_in, range_err;
+};
+
+static __device__ __noinline__ ApExact ap_exact(const Dev& d, const double* X, int i, int j, bool lj_pair, bool el_pair)
 {
-    __shared__ float4 sh_hi[AT];
-    __shared__ float4 sh_lo[AT];
-    __shared__ float sh_m[AT];
-    __shared__ float3 sh_mm[AT];
-    const int64_t i = blockIdx.x * (int64_t)AT + threadIdx.x;
-    const bool active = i < d.n;
-    const int64_t ii = active ? i : 0;
-    const RepDev& R = d.reps[0];
-    const PairK K(R);
-    float4 hi_i = d.phi[ii], lo_i = d.plo[ii];
-    float kqi = (d.pots & NBG_POT_EL) ? (float)(d.el_k_d * d.charge[ii]) : 0.0f;
-    float3 mi = make_float3(0.f, 0.f, 0.f);
-    if (d.pots & NBG_POT_MAG) mi = make_float3((float)d.dipole[3 * ii], (float)d.dipole[3 * ii + 1], (float)d.dipole[3 * ii + 2]);
-    Acc2 fx{0.f, 0.f}, fy{0.f, 0.f}, fz{0.f, 0.f};   // LJ + electrostatic force
-    Acc2 gx{0.f, 0.f}, gy{0.f, 0.f}, gz{0.f, 0.f};   // gravity sum m_j r / r^3
-    Acc2 mx{0.f, 0.f}, my{0.f, 0.f}, mz{0.f, 0.f};   // dipole sum
+    ApExact o{make_float3(0.f, 0.f, 0.f), 1.0f, false, false, false};
+    Dist64 q;
+    if (!distance64(X + 3 * (int64_t)i, X + 3 * (int64_t)j, d.bc, d.reps[0], q)) {
+        o.range_err = true;
+        return o;
+    }
+    o.lj_in = lj_pair && (q.r2 < d.lj_R2);
+    o.el_in = el_pair && (q.r2 < d.el_R2);
+    o.dr = make_float3((float)q.x, (float)q.y, (float)q.z);
+    o.r2 = (float)q.r2;
+    return o;
+}
+
+// 1 / x of a normal positive x, approximated as __fdividef does (a / b there
+// is a times this)
+__device__ __forceinline__ float rcp_ftz(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Bodies j staged per warp in shared memory, one array per field so that two
+// neighbouring bodies load as the two halves of a packed operand and four by
+// one load. Positions are stored negated (i - j is then an addition).
+template <int SUB>
+struct __align__(16) ApStage {
+    float f[8][SUB];  // -hi x, y, z; charge; -lo x, y, z; flags
+    __device__ __forceinline__ void put(int k, const float4& h, const float4& l)
+    {
+        f[0][k] = -h.x; f[1][k] = -h.y; f[2][k] = -h.z; f[3][k] = h.w;
+        f[4][k] = -l.x; f[5][k] = -l.y; f[6][k] = -l.z; f[7][k] = l.w;
+    }
+    // slots k .. k + 3 (k a multiple of 4) as two packed operands
+    __device__ __forceinline__ void four(int c, int k, float2 (&v)[2]) const
+    {
+        const float4 q = *reinterpret_cast<const float4*>(&f[c][k]);
+        v[0] = make_float2(q.x, q.y);
+        v[1] = make_float2(q.z, q.w);
+    }
+};
+
+// the pair constants and body i of a lane, as packed operands
+struct ApOwn {
+    float2 hx, hy, hz, lx, ly, lz, invL, Lh, Ll;
+    float kqi, lj_lo, lj_hi, el_lo, el_hi;
+    int flags;
+    __device__ __forceinline__ ApOwn(const RepDev& R, const float4& h, const float4& l, float kq)
+        : hx(make_float2(h.x, h.x)), hy(make_float2(h.y, h.y)), hz(make_float2(h.z, h.z)), lx(make_float2(l.x, l.x)),
+          ly(make_float2(l.y, l.y)), lz(make_float2(l.z, l.z)), invL(make_float2(R.invLf, R.invLf)),
+          Lh(make_float2(-R.Lh, -R.Lh)), Ll(make_float2(-R.Ll, -R.Ll)), kqi(kq), lj_lo(R.lj_lo), lj_hi(R.lj_hi),
+          el_lo(R.el_lo), el_hi(R.el_hi)
+    {
+        flags = __float_as_int(l.w);
+    }
+};
+
+// The forces on i of AP_G bodies j0 .. j0 + AP_G - 1 (staged from slot k on;
+// m of them real), in pair_cutoff's arithmetic and classification, two
+// bodies per packed instruction. One branch for the group, to the pairs that
+// FP32 does not decide: a branch per pair kept a lane's pairs from
+// overlapping. Exactly zero for a pair outside both cutoffs.
+// CUT: some cutoff is finite. SKIP: the group may hold i itself, its
+// molecule, or slots past the last body.
+#define AP_G 4
+static_assert(AP_G == 4, "a staged load holds four bodies");
+
+template <bool CUBIC, bool HAS_LJ, bool HAS_EL, bool CUT, bool WATER, bool SKIP, int SUB>
+__device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApStage<SUB>& sh, int i, int j0, int k, int m,
+                                         const double* X, float (&fx)[AP_G], float (&fy)[AP_G], float (&fz)[AP_G],
+                                         bool& range_err)
+{
+    float2 dx[AP_G / 2], dy[AP_G / 2], dz[AP_G / 2], r2[AP_G / 2], qj[AP_G / 2], fl[AP_G / 2];
+    bool lj_in[AP_G], el_in[AP_G], any = false;
+    auto at = [](float2* v, int q) -> float& { return (q & 1) ? v[q >> 1].y : v[q >> 1].x; };
+    auto pairs = [&](int q, bool& lj_pair, bool& el_pair) {
+        const int j = j0 + q;
+        const bool skip = SKIP && (q >= m || j == i);
+        lj_pair = HAS_LJ && !skip && (!WATER || (o.flags & __float_as_int(at(fl, q)) & AF_LJ) != 0);
+        el_pair = HAS_EL && !skip && !(SKIP && WATER && i / 3 == j / 3);
+    };
+    float2 jx[2], jy[2], jz[2], kx[2], ky[2], kz[2];
+    sh.four(0, k, jx);
+    sh.four(1, k, jy);
+    sh.four(2, k, jz);
+    sh.four(4, k, kx);
+    sh.four(5, k, ky);
+    sh.four(6, k, kz);
+    if (HAS_EL) sh.four(3, k, qj);
+    if (WATER) sh.four(7, k, fl);
+#pragma unroll
+    for (int h = 0; h < AP_G / 2; ++h) {
+        dx[h] = __fadd2_rn(o.hx, jx[h]);
+        dy[h] = __fadd2_rn(o.hy, jy[h]);
+        dz[h] = __fadd2_rn(o.hz, jz[h]);
+        float2 ex = __fadd2_rn(o.lx, kx[h]);
+        float2 ey = __fadd2_rn(o.ly, ky[h]);
+        float2 ez = __fadd2_rn(o.lz, kz[h]);
+        if (CUBIC) {  // split_diff's image shift
+            const float2 magic = make_float2(12582912.0f, 12582912.0f), back = make_float2(-12582912.0f, -12582912.0f);
+            const float2 sx = __fadd2_rn(__ffma2_rn(dx[h], o.invL, magic), back);
+            const float2 sy = __fadd2_rn(__ffma2_rn(dy[h], o.invL, magic), back);
+            const float2 sz = __fadd2_rn(__ffma2_rn(dz[h], o.invL, magic), back);
+            dx[h] = __ffma2_rn(sx, o.Lh, dx[h]);
+            dy[h] = __ffma2_rn(sy, o.Lh, dy[h]);
+            dz[h] = __ffma2_rn(sz, o.Lh, dz[h]);
+            ex = __ffma2_rn(sx, o.Ll, ex);
+            ey = __ffma2_rn(sy, o.Ll, ey);
+            ez = __ffma2_rn(sz, o.Ll, ez);
+        }
+        dx[h] = __fadd2_rn(dx[h], ex);
+        dy[h] = __fadd2_rn(dy[h], ey);
+        dz[h] = __fadd2_rn(dz[h], ez);
+        r2[h] = __ffma2_rn(dx[h], dx[h], __ffma2_rn(dy[h], dy[h], __fmul2_rn(dz[h], dz[h])));
+    }
+#pragma unroll
+    for (int q = 0; q < AP_G; ++q) {
+        bool lj_pair, el_pair;
+        pairs(q, lj_pair, el_pair);
+        const float r = at(r2, q);
+        lj_in[q] = lj_pair && r < (CUT ? o.lj_lo : INFINITY);
+        el_in[q] = el_pair && r < (CUT ? o.el_lo : INFINITY);
+        if (CUT) any |= (lj_pair && !lj_in[q] && r < o.lj_hi) || (el_pair && !el_in[q] && r < o.el_hi);
+        any |= !(r < INFINITY);
+    }
+    if (any) {
+#pragma unroll
+        for (int q = 0; q < AP_G; ++q) {
+            bool lj_pair, el_pair;
+            pairs(q, lj_pair, el_pair);
+            const float r = at(r2, q);
+            if (CUT && ((lj_pair && !lj_in[q] && r < o.lj_hi) || (el_pair && !el_in[q] && r < o.el_hi))) {
+                const ApExact e = ap_exact(d, X, i, j0 + q, lj_pair, el_pair);
+                lj_in[q] = e.lj_in;
+                el_in[q] = e.el_in;
+                at(dx, q) = e.dr.x;
+                at(dy, q) = e.dr.y;
+                at(dz, q) = e.dr.z;
+                at(r2, q) = e.r2;
+                range_err |= e.range_err;
+            }
+            if (!(at(r2, q) < INFINITY) && !lj_in[q] && !el_in[q]) {
+                at(dx, q) = at(dy, q) = at(dz, q) = 0.f;
+                at(r2, q) = 1.0f;
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < AP_G / 2; ++h) {
+        float2 f = make_float2(0.f, 0.f);
+        // (without cutoffs and skipped bodies every pair is in, but for those
+        // the branch above set to a difference of zero)
+        constexpr bool ALL = !CUT && !SKIP && !WATER;
+        const bool in0 = lj_in[2 * h] || el_in[2 * h], in1 = lj_in[2 * h + 1] || el_in[2 * h + 1];
+        const float2 rr = make_float2(ALL || in0 ? r2[h].x : 1.f, ALL || in1 ? r2[h].y : 1.f);
+        if (HAS_LJ) {
+            const float2 ri = make_float2(rcp_ftz(rr.x), rcp_ftz(rr.y));
+            const float2 s2 = __fmul2_rn(make_float2(d.lj_sig2, d.lj_sig2), ri);
+            const float2 s6 = __fmul2_rn(__fmul2_rn(s2, s2), s2);
+            const float2 s12 = __fmul2_rn(s6, s6);
+            const float2 t = __ffma2_rn(make_float2(2.f, 2.f), s12, make_float2(-s6.x, -s6.y));
+            const float2 g = __fmul2_rn(make_float2(d.lj_eps24, d.lj_eps24), __fmul2_rn(t, ri));
+            f = make_float2(ALL || lj_in[2 * h] ? g.x : 0.f, ALL || lj_in[2 * h + 1] ? g.y : 0.f);
+        }
+        if (HAS_EL) {
+            const float2 rb = make_float2(rsqrt_ftz(rr.x), rsqrt_ftz(rr.y));
+            const float2 t = __ffma2_rn(__fmul2_rn(rb, rb), rb, make_float2(-d.el_krf2, -d.el_krf2));
+            const float2 g = __ffma2_rn(__fmul2_rn(make_float2(o.kqi, o.kqi), qj[h]), t, f);
+            f = make_float2(ALL || el_in[2 * h] ? g.x : f.x, ALL || el_in[2 * h + 1] ? g.y : f.y);
+        }
+        const float2 vx = __fmul2_rn(f, dx[h]), vy = __fmul2_rn(f, dy[h]), vz = __fmul2_rn(f, dz[h]);
+        fx[2 * h] = vx.x; fx[2 * h + 1] = vx.y;
+        fy[2 * h] = vy.x; fy[2 * h + 1] = vy.y;
+        fz[2 * h] = vz.x; fz[2 * h + 1] = vz.y;
+    }
+}
+
+// Whether a tile may hold a body, or a molecule mate, of block b's 32 bodies
+// (a molecule can straddle two tiles), or slots past the last body.
+__device__ __forceinline__ bool ap_skips(int t, int b, int n, bool water)
+{
+    const int mine = b * 32 / AT;
+    return (t + 1) * AT > n || t == mine || (water && (t == mine - 1 || t == mine + 1));
+}
+
+// Both kernels below: every ordered pair of a system off the list path. The
+// FP32 sums of a 128-body tile run over its bodies in order and the tiles'
+// sums are folded in tile order into a compensated pair, so the result does
+// not depend on how the tiles are shared out. They replace one thread per
+// body walking every tile, which left all but n / 128 SMs idle and waited
+// ~350 cycles per pair (n = 648 water: 230 us per evaluation; 5000 ions:
+// 1.3 ms).
+
+// The cutoff potentials under infinite or cubic boundaries: a cluster of C
+// CTAs per 32 bodies i (lane = body), CTA r of it taking tiles r, r + C, ..
+// and leaving their sums in the first CTA's shared memory, which folds them
+// (the others exit: waiting for the fold held their SM's warp slots for half
+// of the kernel).
+// COOP, for systems of up to AP_COOP_TILES tiles, which are bound by
+// latency: the CTA's 8 warps evaluate 16 bodies j each of one tile into
+// shared memory, and three warps then add a component each in body order
+// (n = 648 water: 11 us against 22 with a tile per warp).
+// Otherwise a warp takes a whole tile and adds as it evaluates (bound by the
+// FP32 pipe: 22 instructions a pair and warp for the bare Coulomb force, 10
+// of them packed; an evaluation of 4000 ions 27 us, 41 with COOP; of 12000,
+// 136 us = 0.33 of the FP32 rate at 23 flop a pair).
+#define APC_WARPS 8
+
+template <bool COOP, bool CUBIC, bool HAS_LJ, bool HAS_EL, bool CUT, bool WATER>
+__global__ void __launch_bounds__(APC_WARPS * 32) k_allpairs_cut(Dev d, StateView s, int C)
+{
+    extern __shared__ float apc_sm[];
+    auto cluster = cooperative_groups::this_cluster();
+    float* const sums = cluster.map_shared_rank(apc_sm, 0);   // [tiles][3][32], the first CTA's
+    constexpr int SUB = COOP ? AT / APC_WARPS : 32;           // bodies staged at a time per warp
+    __shared__ ApStage<SUB> stage[APC_WARPS];
+    const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.x / C, rank = blockIdx.x % C;
+    const int n = (int)d.n, tiles = (n + AT - 1) / AT;
+    const int i = b * 32 + lane;
+    const bool active = i < n;
+    const int ii = active ? i : 0;
+    const float4 hi_i = d.phi[ii], lo_i = d.plo[ii];
+    const ApOwn own(d.reps[0], hi_i, lo_i, HAS_EL ? (float)(d.el_k_d * d.charge[ii]) : 0.0f);
+    ApStage<SUB>& sh = stage[w];
     bool range_err = false;
-    const bool cutpots = (d.pots & (NBG_POT_LJ | NBG_POT_EL)) != 0;
-    for (int64_t t = 0; t < d.n; t += AT) {
-        __syncthreads();
-        int64_t j = t + threadIdx.x;
-        if (j < d.n) {
-            sh_hi[threadIdx.x] = d.phi[j];
-            sh_lo[threadIdx.x] = d.plo[j];
-            sh_m[threadIdx.x] = (float)d.mass[j];
-            if (d.pots & NBG_POT_MAG)
-                sh_mm[threadIdx.x] = make_float3((float)d.dipole[3 * j], (float)d.dipole[3 * j + 1], (float)d.dipole[3 * j + 2]);
+    cluster.sync();  // every CTA runs before its shared memory is written to
+    // the m staged bodies from j0 on; put(k, the AP_G values from slot k on)
+    auto eval = [&](auto skip, int j0, int m, auto put) {
+#pragma unroll(COOP ? 4 : 2)
+        for (int k = 0; k < SUB; k += AP_G) {
+            if (k >= m) break;
+            float fx[AP_G], fy[AP_G], fz[AP_G];
+            ap_pairs<CUBIC, HAS_LJ, HAS_EL, CUT, WATER, decltype(skip)::value>(d, own, sh, ii, j0 + k, k, m - k, s.x, fx, fy,
+                                                                               fz, range_err);
+            put(k, fx, fy, fz);
         }
-        __syncthreads();
-        int m = (int)((d.n - t) < AT ? (d.n - t) : AT);
-        float px = 0.f, py = 0.f, pz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f, wx = 0.f, wy = 0.f, wz = 0.f;
-        for (int k = 0; k < m; ++k) {
-            int64_t jg = t + k;
-            if (jg == ii) continue;
-            float4 hj = sh_hi[k], lj = sh_lo[k];
-            if (cutpots) {
-                PairOut o = pair_cutoff(d, R, K, ii, jg, hi_i, lo_i, hj, lj, kqi, s.x);
-                range_err |= o.range_err;
-                px += o.fx;
-                py += o.fy;
-                pz += o.fz;
-            }
-            if (d.pots & (NBG_POT_GRAV | NBG_POT_MAG)) {
-                // plain differences: gravity and dipoles ignore the boundary
-                float3 dr = split_diff(hi_i, lo_i, hj, lj, false, R);
-                float r2 = fmaf(dr.x, dr.x, fmaf(dr.y, dr.y, dr.z * dr.z));
-                float ri = rsqrtf(r2);
-                if (d.pots & NBG_POT_GRAV) {
-                    float sg = sh_m[k] * ri * ri * ri;
-                    qx = fmaf(sg, dr.x, qx);
-                    qy = fmaf(sg, dr.y, qy);
-                    qz = fmaf(sg, dr.z, qz);
+    };
+    if constexpr (COOP) {
+        float* const val = apc_sm + tiles * 96;               // [3][AT][32]
+        for (int t = rank, ti = 0; t < tiles; t += C, ++ti) {
+            const int j0 = t * AT + w * SUB, m = min(SUB, n - j0);
+            __syncwarp();
+            if (lane < m) sh.put(lane, d.phi[j0 + lane], d.plo[j0 + lane]);
+            __syncwarp();
+            if (ti > 0) __syncthreads();  // the previous tile's values are added
+            auto put = [&](int k, const float* fx, const float* fy, const float* fz) {
+#pragma unroll
+                for (int q = 0; q < AP_G; ++q) {
+                    float* v = val + (w * SUB + k + q) * 32 + lane;
+                    v[0] = fx[q];
+                    v[AT * 32] = fy[q];
+                    v[2 * AT * 32] = fz[q];
                 }
-                if (d.pots & NBG_POT_MAG) {
-                    // (mi (mj.r) + mj (mi.r) + r (mi.mj) - 5 r (mi.r)(mj.r)) / |r|^4, r unit
-                    float3 u = make_float3(dr.x * ri, dr.y * ri, dr.z * ri);
-                    float3 mj = sh_mm[k];
-                    float mir = mi.x * u.x + mi.y * u.y + mi.z * u.z;
-                    float mjr = mj.x * u.x + mj.y * u.y + mj.z * u.z;
-                    float mimj = mi.x * mj.x + mi.y * mj.y + mi.z * mj.z;
-                    float inv4 = (ri * ri) * (ri * ri);
-                    wx += (mi.x * mjr + mj.x * mir + u.x * mimj - 5.0f * u.x * mir * mjr) * inv4;
-                    wy += (mi.y * mjr + mj.y * mir + u.y * mimj - 5.0f * u.y * mir * mjr) * inv4;
-                    wz += (mi.z * mjr + mj.z * mir + u.z * mimj - 5.0f * u.z * mir * mjr) * inv4;
+            };
+            if (ap_skips(t, b, n, WATER)) eval(std::true_type{}, j0, m, put);
+            else eval(std::false_type{}, j0, m, put);
+            __syncthreads();
+            if (w < 3) {
+                const float* v = val + w * AT * 32 + lane;
+                const int mt = min(AT, n - t * AT);
+                float p = 0.f;
+                if (mt == AT) {
+#pragma unroll 32
+                    for (int k = 0; k < AT; ++k) p = __fadd_rn(p, v[k * 32]);
+                } else {
+                    for (int k = 0; k < mt; ++k) p = __fadd_rn(p, v[k * 32]);
                 }
+                sums[(t * 3 + w) * 32 + lane] = p;
             }
         }
-        fx.add(px); fy.add(py); fz.add(pz);
-        gx.add(qx); gy.add(qy); gz.add(qz);
-        mx.add(wx); my.add(wy); mz.add(wz);
+    } else {
+        for (int ti = w; ti * C + rank < tiles; ti += W) {
+            const int t = ti * C + rank, j1 = min(n, (t + 1) * AT);
+            const bool skips = ap_skips(t, b, n, WATER);
+            float px = 0.f, py = 0.f, pz = 0.f;
+            auto put = [&](int, const float* fx, const float* fy, const float* fz) {
+#pragma unroll
+                for (int q = 0; q < AP_G; ++q) {
+                    px = __fadd_rn(px, fx[q]);
+                    py = __fadd_rn(py, fy[q]);
+                    pz = __fadd_rn(pz, fz[q]);
+                }
+            };
+            // (the next bodies are loaded before the current ones' arithmetic)
+            float4 h = hi_i, l = lo_i;
+            if (t * AT + lane < j1) {
+                h = d.phi[t * AT + lane];
+                l = d.plo[t * AT + lane];
+            }
+            for (int j0 = t * AT; j0 < j1; j0 += SUB) {
+                const int m = min(SUB, j1 - j0);
+                __syncwarp();
+                sh.put(lane, h, l);
+                __syncwarp();
+                if (j0 + SUB + lane < j1) {
+                    h = d.phi[j0 + SUB + lane];
+                    l = d.plo[j0 + SUB + lane];
+                }
+                if (skips) eval(std::true_type{}, j0, m, put);
+                else eval(std::false_type{}, j0, m, put);
+            }
+            sums[(t * 3) * 32 + lane] = px;
+            sums[(t * 3 + 1) * 32 + lane] = py;
+            sums[(t * 3 + 2) * 32 + lane] = pz;
+        }
     }
     if (range_err) status_set(d.status, ST_RANGE);
-    if (!active) return;
-    const double im = d.inv_mass[i];
-    double a[3] = {fx.value() * im, fy.value() * im, fz.value() * im};
-    if (d.pots & NBG_POT_GRAV) {
-        a[0] += -d.G * gx.value();
-        a[1] += -d.G * gy.value();
-        a[2] += -d.G * gz.value();
+    // the tiles' sums, in tile order; the other CTAs have written theirs into
+    // the first one's shared memory and leave
+    cluster.barrier_arrive();
+    if (rank != 0) return;
+    cluster.barrier_wait();
+    for (int c = w; c < 3; c += W) {
+        Acc2 a{0.f, 0.f};
+        const float* v = apc_sm + c * 32 + lane;
+#pragma unroll 8
+        for (int t = 0; t < tiles; ++t) a.add(v[t * 96]);
+        if (active) {
+            const double acc = a.value() * d.inv_mass[i];
+            if (!finite64(acc)) status_set(d.status, ST_NONFINITE);
+            s.a_new[3 * (int64_t)i + c] = acc;
+        }
     }
-    if (d.pots & NBG_POT_MAG) {
-        double cm = 3.0 * d.mu4pi / d.mass[i];
-        a[0] += cm * mx.value();
-        a[1] += cm * my.value();
-        a[2] += cm * mz.value();
+}
+
+// Every other form, and systems whose tiles' sums do not fit the cluster's
+// shared memory: a block owns 32 bodies i and each of its warps a whole tile
+// at a time; after each round of tiles their sums are folded.
+__global__ void __launch_bounds__(AP_WARPS * 32) k_allpairs(Dev d, StateView s)
+{
+    constexpr int NC = 9;  // sums: cutoff force, then gravity and dipoles
+    extern __shared__ float4 ap_sm[];
+    const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int STAGE = 3 * AP_SUB;  // float4 of one warp's stage
+    float4* const sh_hi = ap_sm + w * STAGE;
+    float4* const sh_lo = sh_hi + AP_SUB;
+    float4* const sh_mm = sh_lo + AP_SUB;                                  // dipole, mass
+    float* const part = reinterpret_cast<float*>(ap_sm + W * STAGE);       // [2][W][NC][32]
+    float* const acc = part + 2 * W * NC * 32;                             // [2][NC][32]: hi, lo
+    const int n = (int)d.n;
+    const int i = blockIdx.x * 32 + lane;
+    const bool active = i < n;
+    const int ii = active ? i : 0;
+    const RepDev& R = d.reps[0];
+    const float4 hi_i = d.phi[ii], lo_i = d.plo[ii];
+    const float kqi = (d.pots & NBG_POT_EL) ? (float)(d.el_k_d * d.charge[ii]) : 0.0f;
+    const PairK K(R);
+    float3 mi = make_float3(0.f, 0.f, 0.f);
+    if (d.pots & NBG_POT_MAG)
+        mi = make_float3((float)d.dipole[3 * ii], (float)d.dipole[3 * ii + 1], (float)d.dipole[3 * ii + 2]);
+    bool range_err = false;
+    const bool cutpots = (d.pots & (NBG_POT_LJ | NBG_POT_EL)) != 0;
+    for (int k = threadIdx.x; k < 2 * NC * 32; k += blockDim.x) acc[k] = 0.f;
+    const int tiles = (n + AT - 1) / AT;
+    const int rounds = (tiles + W - 1) / W;
+    __syncthreads();
+    for (int r = 0; r <= rounds; ++r) {
+        // the previous round's partials, folded in tile order (a warp per sum)
+        if (r > 0) {
+            const float* pp = part + ((r - 1) & 1) * W * NC * 32;
+            for (int c = w; c < NC; c += W) {
+                Acc2 a{acc[c * 32 + lane], acc[(NC + c) * 32 + lane]};
+                const int m = min(W, tiles - (r - 1) * W);
+                for (int k = 0; k < m; ++k) a.add(pp[(k * NC + c) * 32 + lane]);
+                acc[c * 32 + lane] = a.hi;
+                acc[(NC + c) * 32 + lane] = a.lo;
+            }
+        }
+        const int t = r * W + w;
+        if (r < rounds && t < tiles) {
+            float p[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) p[c] = 0.f;
+            const int j1 = min(n, (t + 1) * AT);
+            for (int j0 = t * AT; j0 < j1; j0 += AP_SUB) {
+                const int m = min(AP_SUB, j1 - j0);
+                __syncwarp();
+                if (lane < m) {
+                    sh_hi[lane] = d.phi[j0 + lane];
+                    sh_lo[lane] = d.plo[j0 + lane];
+                    float4 q = make_float4(0.f, 0.f, 0.f, (float)d.mass[j0 + lane]);
+                    if (d.pots & NBG_POT_MAG) {
+                        q.x = (float)d.dipole[3 * (j0 + lane)];
+                        q.y = (float)d.dipole[3 * (j0 + lane) + 1];
+                        q.z = (float)d.dipole[3 * (j0 + lane) + 2];
+                    }
+                    sh_mm[lane] = q;
+                }
+                __syncwarp();
+                for (int k = 0; k < m; ++k) {
+                    const int jg = j0 + k;
+                    if (jg == ii) continue;
+                    const float4 hj = sh_hi[k], lj = sh_lo[k];
+                    if (cutpots) {
+                        PairOut o = pair_cutoff(d, R, K, ii, jg, hi_i, lo_i, hj, lj, kqi, s.x);
+                        range_err |= o.range_err;
+                        p[0] += o.fx;
+                        p[1] += o.fy;
+                        p[2] += o.fz;
+                    }
+                    if (d.pots & (NBG_POT_GRAV | NBG_POT_MAG)) {
+                        // plain differences: gravity and dipoles ignore the boundary
+                        float3 dr = split_diff(hi_i, lo_i, hj, lj, false, R);
+                        float r2 = fmaf(dr.x, dr.x, fmaf(dr.y, dr.y, dr.z * dr.z));
+                        float ri = rsqrtf(r2);
+                        const float4 mj = sh_mm[k];
+                        if (d.pots & NBG_POT_GRAV) {
+                            float sg = mj.w * ri * ri * ri;
+                            p[3] = fmaf(sg, dr.x, p[3]);
+                            p[4] = fmaf(sg, dr.y, p[4]);
+                            p[5] = fmaf(sg, dr.z, p[5]);
+                        }
+                        if (d.pots & NBG_POT_MAG) {
+                            // (mi (mj.r) + mj (mi.r) + r (mi.mj) - 5 r (mi.r)(mj.r)) / |r|^4, r unit
+                            float3 u = make_float3(dr.x * ri, dr.y * ri, dr.z * ri);
+                            float mir = mi.x * u.x + mi.y * u.y + mi.z * u.z;
+                            float mjr = mj.x * u.x + mj.y * u.y + mj.z * u.z;
+                            float mimj = mi.x * mj.x + mi.y * mj.y + mi.z * mj.z;
+                            float inv4 = (ri * ri) * (ri * ri);
+                            p[6] += (mi.x * mjr + mj.x * mir + u.x * mimj - 5.0f * u.x * mir * mjr) * inv4;
+                            p[7] += (mi.y * mjr + mj.y * mir + u.y * mimj - 5.0f * u.y * mir * mjr) * inv4;
+                            p[8] += (mi.z * mjr + mj.z * mir + u.z * mimj - 5.0f * u.z * mir * mjr) * inv4;
+                        }
+                    }
+                }
+            }
+            float* pw = part + (r & 1) * W * NC * 32 + w * NC * 32;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) pw[c * 32 + lane] = p[c];
+        }
+        __syncthreads();
     }
-    for (int k = 0; k < 3; ++k) {
-        if (!finite64(a[k])) status_set(d.status, ST_NONFINITE);
-        s.a_new[3 * i + k] = a[k];
+    if (range_err) status_set(d.status, ST_RANGE);
+    // a warp per component (lane = body)
+    for (int c = w; c < 3; c += W) {
+        if (!active) continue;
+        auto value = [&](int q) { return (double)acc[q * 32 + lane] + (double)acc[(NC + q) * 32 + lane]; };
+        double a = value(c) * d.inv_mass[i];
+        if (d.pots & NBG_POT_GRAV) a += -d.G * value(3 + c);
+        if (d.pots & NBG_POT_MAG) a += 3.0 * d.mu4pi / d.mass[i] * value(6 + c);
+        if (!finite64(a)) status_set(d.status, ST_NONFINITE);
+        s.a_new[3 * (int64_t)i + c] = a;
     }
+}
+
+typedef void (*allpairs_cut_t)(Dev, StateView, int);
+
+template <bool COOP, bool CUBIC, bool CUT>
+static allpairs_cut_t ap_kernel(const Dev& d)
+{
+    if (d.kind == NBG_SYSTEM_WATER) return k_allpairs_cut<COOP, CUBIC, true, true, CUT, true>;
+    if (d.pots == NBG_POT_LJ) return k_allpairs_cut<COOP, CUBIC, true, false, CUT, false>;
+    if (d.pots == NBG_POT_EL) return k_allpairs_cut<COOP, CUBIC, false, true, CUT, false>;
+    return k_allpairs_cut<COOP, CUBIC, true, true, CUT, false>;
+}
+
+template <bool COOP>
+static allpairs_cut_t ap_kernel(const Dev& d)
+{
+    if (d.bc == NBG_BC_CUBIC) return ap_kernel<COOP, true, true>(d);
+    const bool finite = ((d.pots & NBG_POT_LJ) && isfinite(d.lj_R2)) || ((d.pots & NBG_POT_EL) && isfinite(d.el_R2));
+    return finite ? ap_kernel<COOP, false, true>(d) : ap_kernel<COOP, false, false>(d);
 }
 
 int launch_allpairs(nbg_ctx* c, const StateView& s)
 {
+    const Dev& d = c->d;
+    const int64_t tiles = (c->n + AT - 1) / AT, blocks = (c->n + 31) / 32;
+    const uint32_t cut = d.pots & (NBG_POT_LJ | NBG_POT_EL);
+    const int C = (int)std::min<int64_t>(tiles, 8);  // CTAs per cluster (8: the portable size)
+    const int64_t per = (tiles + C - 1) / C;         // tiles of a CTA
     prof_begin(c);
-    k_allpairs<<<grid_for(c->n, AT), AT, 0, c->stream>>>(c->d, s);
+    if (d.pots == cut && cut != 0 && d.bc != NBG_BC_PERIODIC && tiles <= AP_CLUSTER_TILES) {
+        const bool coop = tiles <= AP_COOP_TILES;
+        const allpairs_cut_t k = coop ? ap_kernel<true>(d) : ap_kernel<false>(d);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(blocks * C));
+        // (a tile per warp: equal rounds of at most APC_WARPS tiles)
+        const int64_t rounds = (per + APC_WARPS - 1) / APC_WARPS;
+        cfg.blockDim = dim3((unsigned)(32 * (coop ? APC_WARPS : (per + rounds - 1) / rounds)));
+        cfg.dynamicSmemBytes = sizeof(float) * 96 * (size_t)(tiles + (coop ? AT : 0));
+        cfg.stream = c->stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(float) * 96 * AP_CLUSTER_TILES);
+        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k, d, s, C);
+        if (e != cudaSuccess) return cuda_fail(c, e, "k_allpairs_cut");
+    } else {
+        // warps per block: the tiles in equal rounds of at most AP_WARPS
+        const int64_t rounds = (tiles + AP_WARPS - 1) / AP_WARPS;
+        const int W = (int)((tiles + rounds - 1) / rounds);
+        const size_t smem = sizeof(float4) * (size_t)W * 3 * AP_SUB + sizeof(float) * 32 * 9 * (2 * (size_t)W + 2);
+        k_allpairs<<<(unsigned)blocks, 32 * W, smem, c->stream>>>(d, s);
+    }
     prof_end(c);
     NBG_LAUNCH_CHECK(c, "k_allpairs");
     return NBG_OK;

@@ -14,16 +14,19 @@
 //   k_cell_sort        : each cell's atoms sorted by index (deterministic
 //                        lists), counts moved to cell_n and cleared for the
 //                        next build
-//   k_list_build_warps : (at least two cells per SM) one warp per 32 atoms of a cell; the
-//                        stencil cells' atoms (split-position hi parts moved
-//                        by the periodic shift into the cell's frame) pass
-//                        through a per-warp buffer in scan order and every
-//                        atom of the cell tests them with broadcast reads. The
+//   k_list_build_cells : (up to 25 cells per SM) blocks per cell; the stencil
+//                        cells' atoms are staged in shared memory in scan
+//                        order, and a warp per atom of the cell tests 32 of
+//                        them at a time
+//   k_list_build_warps : (more cells) one warp per 32 atoms of a cell; the
+//                        stencil cells' atoms pass through a per-warp buffer
+//                        in scan order and every atom of the cell tests them
+//                        with broadcast reads. The
 //                        list is column-major (nbr[k*n + i]) for
 //                        thread-per-atom force kernels and row-major
 //                        (nbr[i*cap + k]) for lanes-per-atom kernels.
-//   k_list_build(_lanes): (fewer cells) a thread or a group of lanes per atom
-//                        scanning its 27 cells with gathers of the split positions.
+#include <algorithm>
+
 #include "nbg_internal.cuh"
 
 struct ListCtl {
@@ -117,125 +120,235 @@ __global__ void k_cell_sort(Dev d, ListCtl L)
     }
 }
 
-// Per-atom builds, for systems with too few cells to fill the GPU one
-// warp per cell: the thread (or group of LPA lanes) of an atom scans its
-// 27 cells in the same order as the warp-per-cell build.
-__global__ void k_list_build(Dev d, ListCtl L, const double* X)
+// Blocks per cell (item (cell, c): the cell's atoms from G c in strides of
+// G chunks, so that few, full cells spread over many blocks): the stencil's
+// cells (125 or 27, or for a one-cell replica 1) are staged into shared
+// memory in scan order (cell q = ((ox+ns) w + oy+ns) w + oz+ns, then slot
+// order), and a warp per atom tests 32 candidates at a time and appends the
+// accepted ones, in order, through a ballot prefix count. Two tests, both
+// only the list's superset test (the force kernels classify every pair
+// exactly):
+//   hi parts   from two cells per SM on: the split-position hi parts, moved by
+//              the periodic shift into the cell's frame, as in
+//              k_list_build_warps
+//   SPLIT      fewer cells: the full split difference
+// The rows are those of k_list_build_warps, and of the per-atom builders that
+// SPLIT replaces (a thread or lane group per atom gathering its candidates).
+//
+// A warp per (cell, 32 atoms) with lanes as atoms leaves the chip idle where
+// cells are few: with 17 atoms a cell 15 lanes idle, and the 729 warps of
+// 12,288-atom water left three SM sub-partitions in four without one that
+// could issue. Full builds, us (this kernel / the one it replaces there):
+// water 12,288 atoms 52 / 213, 24,000 177 / 292, 98,304 478 / 579; LJ 5,000
+// 19 / 28, 11,000 25 / 62, 30,000 38 / 69, 60,000 67 / 73, 100,000 111 / 101
+// (staging a 27-cell stencil for 21 atoms then costs more than the idle
+// lanes: the line lies at 25 cells per SM).
+#define LC_WARPS 8
+#define LC_NB 125
+#define LC_BYTES 40960       // staged candidates at a time
+#define LC_MAX_PER_SM 25     // cells per SM, at most
+#define LC_SPLIT_PER_SM 2    // cells per SM below which the split difference is tested
+
+template <bool ONE, bool WATER>
+__device__ __forceinline__ bool lc_test(const float4& c, const float4& hi, int i, int mol0, float rl2, const RepDev& R)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < d.n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (!need_build(d, L, d.rep_of[i])) continue;
-        const RepDev& R = d.reps[d.rep_of[i]];
-        float4 hi = d.phi[i], lo = d.plo[i];
-        int cx = cell_coord(hi.x, R), cy = cell_coord(hi.y, R), cz = cell_coord(hi.z, R);
-        int cnt = 0;
-        const bool water = d.kind == NBG_SYSTEM_WATER;
-        const int o0 = -R.ns, o1 = R.ns;
-        for (int ox = o0; ox <= o1; ++ox) {
-            int nx = cx + ox;
-            nx += (nx < 0) ? R.nc : 0;
-            nx -= (nx >= R.nc) ? R.nc : 0;
-            for (int oy = o0; oy <= o1; ++oy) {
-                int ny = cy + oy;
-                ny += (ny < 0) ? R.nc : 0;
-                ny -= (ny >= R.nc) ? R.nc : 0;
-                for (int oz = o0; oz <= o1; ++oz) {
-                    int nz = cz + oz;
-                    nz += (nz < 0) ? R.nc : 0;
-                    nz -= (nz >= R.nc) ? R.nc : 0;
-                    int cell = R.cell0 + (nx * R.nc + ny) * R.nc + nz;
-                    int m = d.cell_n[cell];
-                    const int* atoms = d.cell_atoms + (int64_t)cell * d.cell_cap;
-                    for (int k = 0; k < m; ++k) {
-                        int j = dbg_index(atoms[k], d.n, (int)i, d.status);
-                        if (j == (int)i) continue;
-                        if (water && (j / 3 == (int)(i / 3))) continue;  // intramolecular: never a pair
-                        float4 hj = d.phi[j], lj = d.plo[j];
-                        float3 dr = split_diff(hi, lo, hj, lj, true, R);
-                        float r2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
-                        if (r2 < R.rl2) {
-                            if (cnt < d.nbr_cap) d.nbr[(int64_t)cnt * d.nbr_kstride + i * d.nbr_istride] = j;
-                            ++cnt;
-                        }
-                    }
-                }
-            }
-        }
-        if (cnt > d.nbr_cap) {
-            status_set(d.status, ST_NBR_OVERFLOW);
-            cnt = d.nbr_cap;
-        }
-        d.nbr_count[i] = cnt;
-        d.xref[3 * i] = X[3 * i];
-        d.xref[3 * i + 1] = X[3 * i + 1];
-        d.xref[3 * i + 2] = X[3 * i + 2];
+    float dx = c.x - hi.x, dy = c.y - hi.y, dz = c.z - hi.z;
+    if (ONE) {
+        // s = rint(d / L) by the 1.5 * 2^23 trick (|d / L| <= 1)
+        const float magic = 12582912.0f;
+        dx = __fmaf_rn(-__fsub_rn(__fmaf_rn(dx, R.invLf, magic), magic), R.Lh, dx);
+        dy = __fmaf_rn(-__fsub_rn(__fmaf_rn(dy, R.invLf, magic), magic), R.Lh, dy);
+        dz = __fmaf_rn(-__fsub_rn(__fmaf_rn(dz, R.invLf, magic), magic), R.Lh, dz);
     }
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const int j = __float_as_int(c.w);
+    return r2 < rl2 && j != i && (!WATER || (unsigned)(j - mol0) >= 3u);
 }
 
-// LPA lanes per atom: the group scans the 27 cells in the same order, each
-// chunk of LPA consecutive cell entries tested in parallel; accepted entries
-// keep their scan order through a ballot prefix count, so the row-major list
-// is identical to the one-thread-per-atom list.
-template <int LPA>
-__global__ void __launch_bounds__(256) k_list_build_lanes(Dev d, ListCtl L, const double* X)
+template <bool WATER>
+__device__ __forceinline__ bool lc_test_split(const float4& c, const float4& cl, const float4& hi, const float4& lo, int i,
+                                              int mol0, float rl2, const PairK& K)
 {
-    const int lane = threadIdx.x % LPA;
-    const int gbase = (threadIdx.x % 32) - lane;  // first lane of the group within the warp
-    const unsigned gmask = (LPA == 32) ? 0xffffffffu : (((1u << LPA) - 1u) << gbase);
-    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LPA;
-    if (i >= d.n) return;  // whole groups leave together
-    if (!need_build(d, L, d.rep_of[i])) return;
-    const RepDev& R = d.reps[d.rep_of[i]];
-    const float4 hi = d.phi[i], lo = d.plo[i];
-    const int cx = cell_coord(hi.x, R), cy = cell_coord(hi.y, R), cz = cell_coord(hi.z, R);
+    const float3 dr = split_diff(hi, lo, c, cl, true, K);
+    const float r2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
+    const int j = __float_as_int(c.w);
+    return r2 < rl2 && j != i && (!WATER || (unsigned)(j - mol0) >= 3u);
+}
+
+// The rows of atoms c0 .. c0 + G - 1, c0 + stride .. of a cell against the m
+// staged candidates.
+template <bool SPLIT, bool ONE, bool WATER>
+__device__ __forceinline__ void lc_rows(const Dev& d, const RepDev& R, const float4* cand, const float4* cand_lo, int m,
+                                        const int* atoms, int c0, int G, int stride, int cnt, bool first, int w, int lane)
+{
+    const float rl2 = R.rl2;
+    const PairK K(R);
+    for (int b = c0; b < cnt; b += stride)
+        for (int a = b + w; a < min(cnt, b + G); a += LC_WARPS) {
+#ifdef NBG_DEBUG
+            const int i = dbg_index(atoms[a], d.n, -1, d.status);
+            if (i < 0) continue;
+#else
+            const int i = atoms[a];
+#endif
+            const float4 hi = d.phi[i];
+            float4 lo = hi;
+            if (SPLIT) lo = d.plo[i];
+            const int mol0 = WATER ? 3 * (i / 3) : -8;  // first atom of i's molecule
+            int* const row = d.nbr + (int64_t)i * d.nbr_istride;
+            int n = first ? 0 : d.nbr_count[i];  // (a pass continues the row of the one before)
+            const unsigned below = (1u << lane) - 1u;
+            auto step = [&](int k, bool real) {
+                const float4 c = cand[k];
+                bool take;
+                if (SPLIT) take = lc_test_split<WATER>(c, cand_lo[k], hi, lo, i, mol0, rl2, K) && real;
+                else take = lc_test<ONE, WATER>(c, hi, i, mol0, rl2, R) && real;
+                const unsigned bal = __ballot_sync(0xffffffffu, take);
+                const int pos = n + __popc(bal & below);
+                if (take && pos < d.nbr_cap) row[(int64_t)pos * d.nbr_kstride] = __float_as_int(c.w);
+                n += __popc(bal);
+            };
+            int k0 = 0;
+#pragma unroll 4
+            for (; k0 + 32 <= m; k0 += 32) step(k0 + lane, true);
+            if (k0 < m) step(k0 + lane < m ? k0 + lane : 0, k0 + lane < m);
+            if (lane == 0) d.nbr_count[i] = n;
+        }
+}
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(LC_WARPS * 32) k_list_build_cells(Dev d, ListCtl L, const double* X, int G, int chunks)
+{
+    constexpr int CAP = LC_BYTES / (SPLIT ? 32 : 16);  // candidates staged at a time
+    __shared__ int nb_code[LC_NB];  // stencil cell | (shift + 1) per axis in bits 24-29
+    __shared__ int nb_off[LC_NB + 1];
+    __shared__ float4 cand[LC_BYTES / 16];
+    float4* const cand_lo = cand + (SPLIT ? CAP : 0);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool water = d.kind == NBG_SYSTEM_WATER;
-    int cnt = 0;
-    int* out = d.nbr + i * d.nbr_istride;
-    const int o0 = -R.ns, o1 = R.ns;
-    for (int ox = o0; ox <= o1; ++ox) {
-        int nx = cx + ox;
-        nx += (nx < 0) ? R.nc : 0;
-        nx -= (nx >= R.nc) ? R.nc : 0;
-        for (int oy = o0; oy <= o1; ++oy) {
-            int ny = cy + oy;
-            ny += (ny < 0) ? R.nc : 0;
-            ny -= (ny >= R.nc) ? R.nc : 0;
-            for (int oz = o0; oz <= o1; ++oz) {
-                int nz = cz + oz;
-                nz += (nz < 0) ? R.nc : 0;
-                nz -= (nz >= R.nc) ? R.nc : 0;
-                const int cell = R.cell0 + (nx * R.nc + ny) * R.nc + nz;
-                const int m = d.cell_n[cell];
-                const int* atoms = d.cell_atoms + (int64_t)cell * d.cell_cap;
-                for (int k0 = 0; k0 < m; k0 += LPA) {
-                    const int k = k0 + lane;
-                    bool take = false;
-                    int j = 0;
-                    if (k < m) {
-                        j = dbg_index(atoms[k], d.n, (int)i, d.status);
-                        if (j != (int)i && !(water && (j / 3 == (int)(i / 3)))) {
-                            float3 dr = split_diff(hi, lo, d.phi[j], d.plo[j], true, R);
-                            float r2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
-                            take = r2 < R.rl2;
+    const int64_t items = (int64_t)d.ncell_total * chunks;
+    if (d.nrep == 1 && !need_build(d, L, 0)) return;
+    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+        const int cell = (int)(it / chunks), c0 = (int)(it % chunks) * G;
+        const int rep = d.cell_rep[cell];
+        if (!need_build(d, L, rep)) continue;
+        const int cnt = min(d.cell_n[cell], d.cell_cap);
+        if (c0 >= cnt) continue;
+        const RepDev& R = d.reps[rep];
+        const int nc = R.nc;
+        const bool one = R.ns == 0;  // one cell holds the replica: minimum image per pair
+        const int sw = 2 * R.ns + 1;  // stencil width (1, 3 or 5)
+        const int nnb = sw * sw * sw;
+        const int* atoms = d.cell_atoms + (int64_t)cell * d.cell_cap;
+        __syncthreads();  // the previous item's tables are consumed
+        if (threadIdx.x < nnb) {
+            const int lc = cell - R.cell0, q = threadIdx.x;
+            const int cx = lc / (nc * nc), cy = (lc / nc) % nc, cz = lc % nc;
+            int nx = cx + q / (sw * sw) - R.ns, ny = cy + (q / sw) % sw - R.ns, nz = cz + q % sw - R.ns;
+            int sx = 1, sy = 1, sz = 1;
+            if (nx < 0) { nx += nc; sx = 0; }
+            if (nx >= nc) { nx -= nc; sx = 2; }
+            if (ny < 0) { ny += nc; sy = 0; }
+            if (ny >= nc) { ny -= nc; sy = 2; }
+            if (nz < 0) { nz += nc; sz = 0; }
+            if (nz >= nc) { nz -= nc; sz = 2; }
+            const int cq = R.cell0 + (nx * nc + ny) * nc + nz;
+            nb_code[q] = cq | (sx << 24) | (sy << 26) | (sz << 28);
+            nb_off[q + 1] = min(d.cell_n[cq], d.cell_cap);
+        }
+        __syncthreads();
+        if (w == 0) {  // inclusive sums of the counts, four per lane
+            int v[4], t = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                t += 4 * lane + e < nnb ? nb_off[4 * lane + e + 1] : 0;
+                v[e] = t;
+            }
+            int x = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (4 * lane + e < nnb) nb_off[4 * lane + e + 1] = x - t + v[e];
+            if (lane == 0) nb_off[0] = 0;
+        }
+        __syncthreads();
+        const int total = nb_off[nnb];
+        const float Lh = R.Lh;
+        for (int p0 = 0; p0 < total; p0 += CAP) {
+            if (p0 > 0) __syncthreads();  // the previous pass's candidates are tested
+            // a warp per stencil cell, four cells' loads in flight
+            for (int q0 = w; q0 < nnb; q0 += 4 * LC_WARPS) {
+                int m[4], off[4], code[4], most = 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int q = q0 + e * LC_WARPS;
+                    off[e] = q < nnb ? nb_off[q] - p0 : 0;
+                    m[e] = q < nnb ? nb_off[q + 1] - p0 - off[e] : 0;
+                    code[e] = q < nnb ? nb_code[q] : 0;
+                    if (off[e] >= CAP || off[e] + m[e] <= 0) m[e] = 0;
+                    most = max(most, m[e]);
+                }
+                for (int k0 = 0; k0 < most; k0 += 32) {
+                    int j[4];
+                    float4 h[4], l[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int k = k0 + lane, s = off[e] + k;
+                        j[e] = -1;
+                        if (k < m[e] && s >= 0 && s < CAP)
+                            j[e] = dbg_index(d.cell_atoms[(int64_t)(code[e] & 0xffffff) * d.cell_cap + k], d.n, 0, d.status);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (j[e] >= 0) {
+                            h[e] = d.phi[j[e]];
+                            if (SPLIT) l[e] = d.plo[j[e]];
+                        }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (j[e] < 0) continue;
+                        const int s = off[e] + k0 + lane;
+                        if (SPLIT) {
+                            cand[s] = make_float4(h[e].x, h[e].y, h[e].z, __int_as_float(j[e]));
+                            cand_lo[s] = l[e];
+                        } else {
+                            const float sx = (float)(((code[e] >> 24) & 3) - 1) * Lh;
+                            const float sy = (float)(((code[e] >> 26) & 3) - 1) * Lh;
+                            const float sz = (float)(((code[e] >> 28) & 3) - 1) * Lh;
+                            cand[s] = make_float4(h[e].x + sx, h[e].y + sy, h[e].z + sz, __int_as_float(j[e]));
                         }
                     }
-                    const unsigned bal = __ballot_sync(gmask, take);
-                    if (take) {
-                        const int pos = cnt + __popc(bal & gmask & ((1u << (gbase + lane)) - 1u));
-                        if (pos < d.nbr_cap) out[pos] = j;
-                    }
-                    cnt += __popc(bal & gmask);
                 }
             }
+            __syncthreads();
+            const int m = min(CAP, total - p0), stride = G * chunks;
+            const bool first = p0 == 0;
+            if (one && !SPLIT) {
+                if (water) lc_rows<SPLIT, true, true>(d, R, cand, cand_lo, m, atoms, c0, G, stride, cnt, first, w, lane);
+                else lc_rows<SPLIT, true, false>(d, R, cand, cand_lo, m, atoms, c0, G, stride, cnt, first, w, lane);
+            } else {
+                if (water) lc_rows<SPLIT, false, true>(d, R, cand, cand_lo, m, atoms, c0, G, stride, cnt, first, w, lane);
+                else lc_rows<SPLIT, false, false>(d, R, cand, cand_lo, m, atoms, c0, G, stride, cnt, first, w, lane);
+            }
         }
+        __syncthreads();  // the rows' counts
+        for (int b = c0; b < cnt; b += G * chunks)
+            if (threadIdx.x < G && b + threadIdx.x < cnt) {
+                const int i = dbg_index(atoms[b + threadIdx.x], d.n, 0, d.status);
+                if (d.nbr_count[i] > d.nbr_cap) {
+                    status_set(d.status, ST_NBR_OVERFLOW);
+                    d.nbr_count[i] = d.nbr_cap;
+                }
+                d.xref[3 * i] = X[3 * i];
+                d.xref[3 * i + 1] = X[3 * i + 1];
+                d.xref[3 * i + 2] = X[3 * i + 2];
+            }
     }
-    if (lane == 0) {
-        if (cnt > d.nbr_cap) {
-            status_set(d.status, ST_NBR_OVERFLOW);
-            cnt = d.nbr_cap;
-        }
-        d.nbr_count[i] = cnt;
-    }
-    if (lane < 3) d.xref[3 * i + lane] = X[3 * i + lane];
 }
 
 // Warp per (cell, chunk of 32 of its atoms): lane l holds atom l of the
@@ -432,25 +545,24 @@ int launch_list_build(nbg_ctx* c, const StateView& s, bool force, StepRef pos)
     const int64_t cells = c->d.ncell_total;
     k_cell_sort<<<(unsigned)std::min<int64_t>(cells, 4 * wave), 128, sizeof(int) * c->d.cell_cap, c->stream>>>(c->d, L);
     NBG_LAUNCH_CHECK(c, "k_cell_sort");
-    if (c->d.ncell_total >= 2 * c->sms) {
+    const double occ = (double)c->n / std::max<int64_t>(cells, 1);
+    if (cells <= LC_MAX_PER_SM * (int64_t)c->sms) {
+        // 32 atoms an item (4 a warp), down to 8 while the items leave an SM
+        // under 4 blocks
+        int G = 32;
+        while (G > LC_WARPS && cells * (int64_t)std::ceil(occ / G) < 4 * (int64_t)c->sms) G /= 2;
+        const int chunks = std::max(1, (int)std::ceil(occ / G));
+        const int64_t blocks = std::min<int64_t>(cells * chunks, 6 * (int64_t)c->sms);  // (cheap when idle)
+        if (cells < LC_SPLIT_PER_SM * (int64_t)c->sms)
+            k_list_build_cells<true><<<(unsigned)blocks, LC_WARPS * 32, 0, c->stream>>>(c->d, L, s.x, G, chunks);
+        else
+            k_list_build_cells<false><<<(unsigned)blocks, LC_WARPS * 32, 0, c->stream>>>(c->d, L, s.x, G, chunks);
+    } else {
         // warps per cell from the mean occupancy (with margin); fuller cells loop
-        const double occ = (double)c->n / std::max(c->d.ncell_total, 1);
         const int chunks = std::max(1, std::min((c->d.cell_cap + 31) / 32, (int)std::ceil(1.5 * occ / 32.0)));
-        const int64_t items = (int64_t)c->d.ncell_total * chunks;
+        const int64_t items = cells * chunks;
         const int64_t blocks = std::min<int64_t>((items + LW_WARPS - 1) / LW_WARPS, 1 << 20);
         k_list_build_warps<<<(unsigned)blocks, LW_WARPS * 32, 0, c->stream>>>(c->d, L, s.x, chunks);
-    } else {
-        const int lpa = c->list_lpa;
-        if (lpa <= 1) {
-            k_list_build<<<grid_for(c->n, 128), 128, 0, c->stream>>>(c->d, L, s.x);
-        } else {
-            const int per_block = 256 / lpa;
-            const int grid = (int)((c->n + per_block - 1) / per_block);
-            if (lpa == 4) k_list_build_lanes<4><<<grid, 256, 0, c->stream>>>(c->d, L, s.x);
-            else if (lpa == 8) k_list_build_lanes<8><<<grid, 256, 0, c->stream>>>(c->d, L, s.x);
-            else if (lpa == 16) k_list_build_lanes<16><<<grid, 256, 0, c->stream>>>(c->d, L, s.x);
-            else k_list_build_lanes<32><<<grid, 256, 0, c->stream>>>(c->d, L, s.x);
-        }
     }
     NBG_LAUNCH_CHECK(c, "k_list_build");
     return NBG_OK;

@@ -7,144 +7,286 @@
 // (q_j / r or q_j / R) (:321-351); bonds sum over directed bonds k d^2 / 4
 // (:353-372); angles sum k (theta - theta0)^2 / 2 (:374-397); gravity
 // -G sum_{i<j} m_i m_j / r (this project's; the reference has none).
-// Per-block partials are summed by the host in block order (deterministic).
+// Per-block partials are summed in a fixed order (deterministic).
+#include <algorithm>
+
 #include "fx_pair.cuh"
 
 #define EB 128
+#define EJ 32        // bodies j per block of k_energy_pairs
+#define EL_WARPS 8   // warps per block of k_energy_list
 
+// FP64 issues at 2 lanes per clock and SM here (a warp instruction holds its
+// SM sub-partition for 64 cycles), so these kernels are bound by their count
+// of FP64 instructions; comparisons and conversions count like any other.
+
+// The exact FP64 value of a float, by integer operations where it is normal.
+__device__ __forceinline__ double widen(float f)
+{
+    const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+    if (m - 0x00800000u >= 0x7f000000u) return (double)f;  // zero, subnormal, infinite or NaN
+    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
+// 1 / sqrt(x) to ~1 ulp: the FP32 approximation (2^-22) refined by one
+// third-order step, y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2 (error ~e^3);
+// arguments outside FP32's comfortable range take the square root and the
+// division (9 against ~40 FP64 instructions).
+__device__ __forceinline__ double rsqrt64(double x)
+{
+    const int hi = __double2hiint(x);
+    if (hi < 0x39b00000 || hi > 0x46300000) return 1.0 / sqrt(x);  // 2^-100 .. 2^100
+    const double y = widen(rsqrtf(__double2float_rn(x)));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
+// Cubic minimum image of a difference: d - L rint(d / L) (r^2 does not depend
+// on the choice at half a box). False where the image number is not a plain
+// one (beyond the reference loops' cap, or not finite).
+__device__ __forceinline__ bool nearest_image(double& d, double L, double invL)
+{
+    const double magic = 6755399441055744.0;  // 1.5 * 2^52
+    const double t = fma(d, invL, magic);
+    const int k = __double2loint(t), h = __double2hiint(t);
+    d = fma(-L, t - magic, d);
+    return (h == 0x43380000 || h == 0x4337ffff) && k >= -MINIMAGE_MAX_ITERS && k <= MINIMAGE_MAX_ITERS;
+}
+
+// x < y for non-negative doubles (NaN compares as large)
+__device__ __forceinline__ bool below(double x, double y)
+{
+    return __double_as_longlong(x) < __double_as_longlong(y);
+}
+
+// Sums over the block of up to 3 values per thread, by warps and then in
+// warp order, to out[0..K-1] by the first thread.
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double* out)
+{
+    __shared__ double sh[32][K];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < K; ++k) sh[threadIdx.x >> 5][k] = v[k];
+    __syncthreads();
+    if (threadIdx.x < K) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w][threadIdx.x];
+        out[threadIdx.x] = t;
+    }
+}
+
+// LJ, electrostatic and gravity sums over all pairs j > i: an item is 128
+// bodies i (a thread each) and 32 bodies j from shared memory. (A thread per
+// body i walking every j > i left n / 128 blocks of very uneven length:
+// 8.0 ms for 6429 gravitating bodies, 4.0 ms for 3163 ions.)
+template <int BC, bool HAS_LJ, bool HAS_EL, bool HAS_G>
 __global__ void __launch_bounds__(EB) k_energy_pairs(Dev d, const double* X, double* out /*[grid][3]*/)
 {
+    __shared__ double xj[EJ], yj[EJ], zj[EJ], qj[EJ], mj[EJ];
     const RepDev& R = d.reps[0];
-    double e_lj = 0.0, e_el = 0.0, e_g = 0.0;
-    bool range_err = false;
     const bool water = d.kind == NBG_SYSTEM_WATER;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < d.n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double* xi = X + 3 * i;
-        bool lj_i = (d.pots & NBG_POT_LJ) && (!water || i % 3 == 0);
-        double el_i = 0.0, g_i = 0.0;
-        for (int64_t j = i + 1; j < d.n; ++j) {
-            const double* xj = X + 3 * j;
-            bool lj = lj_i && (!water || j % 3 == 0);
-            bool el = (d.pots & NBG_POT_EL) && !el_excluded(d.kind, i, j);
-            if (lj || el) {
+    const int64_t jt = (d.n + EJ - 1) / EJ, items = (d.n + EB - 1) / EB * jt;
+    const double L = R.L, invL = R.invL, invR = 1.0 / d.el_R;
+    const double sR = HAS_LJ ? d.lj_sig2_d / d.lj_R2 : 0.0;  // sigma^2 / r^2 from the cutoff on
+    double e[3] = {0.0, 0.0, 0.0};
+    bool range_err = false;
+    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+        const int64_t i0 = it / jt * EB, j0 = it % jt * EJ;
+        if (j0 + EJ <= i0 + 1) continue;  // no j > i (uniform)
+        __syncthreads();
+        if (threadIdx.x < EJ && j0 + threadIdx.x < d.n) {
+            const int64_t j = j0 + threadIdx.x;
+            xj[threadIdx.x] = X[3 * j];
+            yj[threadIdx.x] = X[3 * j + 1];
+            zj[threadIdx.x] = X[3 * j + 2];
+            if (HAS_EL) qj[threadIdx.x] = d.charge[j];
+            if (HAS_G) mj[threadIdx.x] = d.mass[j];
+        }
+        __syncthreads();
+        const int64_t i = i0 + threadIdx.x;
+        if (i >= d.n) continue;
+        const double x = X[3 * i], y = X[3 * i + 1], z = X[3 * i + 2];
+        double el = 0.0, g = 0.0;
+        const int k0 = (int)max((int64_t)0, i + 1 - j0), k1 = (int)min((int64_t)EJ, d.n - j0);
+        for (int k = k0; k < k1; ++k) {
+            const int64_t j = j0 + k;
+            double dx = x - xj[k], dy = y - yj[k], dz = z - zj[k];
+            if (HAS_G) {  // (gravity ignores the boundary)
+                const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                g = fma(mj[k], rsqrt64(r2), g);
+            }
+            if (!HAS_LJ && !HAS_EL) continue;
+            const bool lj = HAS_LJ && (!water || (i % 3 == 0 && j % 3 == 0));
+            const bool ep = HAS_EL && !(water && i / 3 == j / 3);
+            if (!(lj || ep)) continue;
+            double r2;
+            bool plain = BC != NBG_BC_PERIODIC;
+            if (BC == NBG_BC_CUBIC) {
+                const bool px = nearest_image(dx, L, invL), py = nearest_image(dy, L, invL),
+                           pz = nearest_image(dz, L, invL);
+                plain = px && py && pz;
+            }
+            if (plain) {
+                r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+            } else {  // the reference's loops
                 Dist64 q;
-                if (!distance64(xi, xj, d.bc, R, q)) {
+                if (!distance64(X + 3 * i, X + 3 * j, BC, R, q)) {
                     range_err = true;
                     continue;
                 }
-                if (lj) {
-                    double r2 = q.r2;
-                    if (!(r2 < d.lj_R2)) r2 = d.lj_R2;
-                    double s6 = d.lj_sig2_d / r2;
-                    s6 = __dmul_rn(__dmul_rn(s6, s6), s6);
-                    e_lj = __dadd_rn(e_lj, __dsub_rn(__dmul_rn(s6, s6), s6));
-                }
-                if (el) {
-                    if (q.r2 < d.el_R2) {
-                        double r = sqrt(q.r2);
-                        // reaction field: 1/r + k_rf r^2 - c_rf (+ c_rf back, so eps_rf = 1 gives 1/r)
-                        double t = 1.0 / r;
-                        if (d.el_krf != 0.0) t = __dadd_rn(t, __dsub_rn(__dmul_rn(d.el_krf, q.r2), d.el_crf - 1.0 / d.el_R));
-                        el_i = __dadd_rn(el_i, __dmul_rn(d.charge[j], t));
-                    } else {
-                        el_i = __dadd_rn(el_i, d.charge[j] / d.el_R);
-                    }
-                }
+                r2 = q.r2;
             }
-            if (d.pots & NBG_POT_GRAV) {
-                double x = __dsub_rn(xi[0], xj[0]), y = __dsub_rn(xi[1], xj[1]), z = __dsub_rn(xi[2], xj[2]);
-                double r = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
-                g_i = __dadd_rn(g_i, d.mass[j] / r);
+            const double ri = rsqrt64(r2);
+            if (lj) {
+                double s6 = below(r2, d.lj_R2) ? d.lj_sig2_d * (ri * ri) : sR;
+                s6 = s6 * s6 * s6;
+                e[0] += fma(s6, s6, -s6);
+            }
+            if (ep) {
+                double t = ri;  // reaction field: 1/r + k_rf r^2 - c_rf (+ c_rf back, so eps_rf = 1 gives 1/r)
+                if (d.el_krf != 0.0) t += fma(d.el_krf, r2, -(d.el_crf - invR));
+                el = fma(qj[k], below(r2, d.el_R2) ? t : invR, el);
             }
         }
-        if (d.pots & NBG_POT_EL) e_el = __dadd_rn(e_el, __dmul_rn(el_i, d.charge[i]));
-        if (d.pots & NBG_POT_GRAV) e_g = __dadd_rn(e_g, __dmul_rn(g_i, d.mass[i]));
+        if (HAS_EL) e[1] = fma(el, d.charge[i], e[1]);
+        if (HAS_G) e[2] = fma(g, d.mass[i], e[2]);
     }
     if (range_err) status_set(d.status, ST_RANGE);
-    __shared__ double sh[3][EB];
-    sh[0][threadIdx.x] = e_lj;
-    sh[1][threadIdx.x] = e_el;
-    sh[2][threadIdx.x] = e_g;
-    __syncthreads();
-    for (int w = EB / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int k = 0; k < 3; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) out[blockIdx.x * 3 + k] = sh[k][0];
+    block_sums<3>(e, out + 3 * (int64_t)blockIdx.x);
 }
 
 // The same LJ and electrostatic sums over the Verlet list (built for X):
 // for each pair inside a cutoff, its term minus the term the reference gives
 // a pair beyond it (LJ at r = R, Coulomb q_i q_j / R); the host adds those
 // constant terms for all pairs analytically. O(N x neighbours) instead of
-// O(N^2); each pair is taken once (j > i) with the same FP64 minimum image.
-__global__ void __launch_bounds__(EB) k_energy_list(Dev d, const double* X, double* out /*[grid][2]*/)
+// O(N^2); each pair is taken once (j > i). A warp per atom reads its row,
+// keeps the entries j > i that FP32 finds within the largest cutoff (about a
+// third), and queues them by the arithmetic they need: the FP64 code then
+// runs on full warps of like pairs (14 FP64 instructions for a bare charge
+// pair, 30 for an LJ + charge pair across a face). (A thread per atom over its whole row took 1.1 ms at 12,288 atoms.)
+__global__ void __launch_bounds__(EL_WARPS * 32) k_energy_list(Dev d, const double* X, double* out /*[grid][3]*/)
 {
+    __shared__ int2 queue[EL_WARPS][4][64];
     const RepDev& R = d.reps[0];
-    double e_lj = 0.0, e_el = 0.0;
-    bool range_err = false;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool water = d.kind == NBG_SYSTEM_WATER;
+    const bool has_lj = (d.pots & NBG_POT_LJ) != 0, has_el = (d.pots & NBG_POT_EL) != 0;
+    const float reach = fmaxf(has_lj ? R.fx_lj_hi : 0.f, has_el ? R.fx_el_hi : 0.f);
+    const double L = R.L, invL = R.invL;
+    const double reach2 = 0.25 * L * L;  // (above every cutoff's square on the list path)
     double s6R = d.lj_sig2_d / d.lj_R2;
-    s6R = __dmul_rn(__dmul_rn(s6R, s6R), s6R);
-    const double ljR = __dsub_rn(__dmul_rn(s6R, s6R), s6R);
+    s6R = s6R * s6R * s6R;
+    const double ljR = fma(s6R, s6R, -s6R);
     const double invR = 1.0 / d.el_R;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < d.n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double* xi = X + 3 * i;
-        const bool lj_i = (d.pots & NBG_POT_LJ) && (!water || i % 3 == 0);
-        const int cnt = d.nbr_count[i];
-        double el_i = 0.0;
-        for (int k = 0; k < cnt; ++k) {
-            const int64_t j = dbg_index(d.nbr[(int64_t)k * d.nbr_kstride + i * d.nbr_istride], d.n, (int)i, d.status);
-            if (j <= i) continue;
-            const bool lj = lj_i && (!water || j % 3 == 0);
-            const bool el = (d.pots & NBG_POT_EL) && !el_excluded(d.kind, i, j);
-            if (!(lj || el)) continue;
-            Dist64 q;
-            if (!distance64(xi, X + 3 * j, d.bc, R, q)) {
-                range_err = true;
-                continue;
-            }
-            if (lj && q.r2 < d.lj_R2) {
-                double s6 = d.lj_sig2_d / q.r2;
-                s6 = __dmul_rn(__dmul_rn(s6, s6), s6);
-                e_lj = __dadd_rn(e_lj, __dsub_rn(__dsub_rn(__dmul_rn(s6, s6), s6), ljR));
-            }
-            if (el && q.r2 < d.el_R2) {
-                const double r = sqrt(q.r2);
-                double t = 1.0 / r;
-                if (d.el_krf != 0.0) t = __dadd_rn(t, __dsub_rn(__dmul_rn(d.el_krf, q.r2), d.el_crf - invR));
-                el_i = __dadd_rn(el_i, __dmul_rn(d.charge[j], __dsub_rn(t, invR)));
+    double e[3] = {0.0, 0.0, 0.0};
+    bool range_err = false;
+    // queues by the arithmetic their pairs need: + 1 for a pair whose bare
+    // difference is not its minimum image, + 2 for an LJ pair
+    int fill[4] = {0, 0, 0, 0};
+    auto take = [&](int2* q, int m, bool image, bool lj) {  // the first m queued pairs, one per lane
+        if (lane >= m) return;
+        const int64_t i = q[lane].x, j = q[lane].y;
+        const double x0 = X[3 * i] - X[3 * j], y0 = X[3 * i + 1] - X[3 * j + 1], z0 = X[3 * i + 2] - X[3 * j + 2];
+        double r2 = fma(x0, x0, fma(y0, y0, z0 * z0));
+        // (a pair queued as bare may still cross a face by a rounding of the
+        // fixed-point positions: its r^2 is then far above the list's)
+        if (image || !below(r2, reach2)) {
+            double dx = x0, dy = y0, dz = z0;
+            const bool px = nearest_image(dx, L, invL), py = nearest_image(dy, L, invL), pz = nearest_image(dz, L, invL);
+            r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+            if (!(px && py && pz)) {  // the reference's loops
+                Dist64 o;
+                if (!distance64(X + 3 * i, X + 3 * j, NBG_BC_CUBIC, R, o)) {
+                    range_err = true;
+                    return;
+                }
+                r2 = o.r2;
             }
         }
-        if (d.pots & NBG_POT_EL) e_el = __dadd_rn(e_el, __dmul_rn(el_i, d.charge[i]));
+        const double ri = rsqrt64(r2);
+        if (lj && below(r2, d.lj_R2)) {
+            double s6 = d.lj_sig2_d * (ri * ri);
+            s6 = s6 * s6 * s6;
+            e[0] += fma(s6, s6, -s6) - ljR;
+        }
+        if (has_el && below(r2, d.el_R2)) {
+            double t = ri - invR;
+            if (d.el_krf != 0.0) t += fma(d.el_krf, r2, -(d.el_crf - invR));
+            e[1] = fma(d.charge[i] * d.charge[j], t, e[1]);
+        }
+    };
+    const int64_t stride = (int64_t)gridDim.x * EL_WARPS;
+    for (int64_t i = blockIdx.x * (int64_t)EL_WARPS + w; i < d.n; i += stride) {
+        const bool lj_i = has_lj && (!water || fx_oxygen((int)i));
+        if (!lj_i && !has_el) continue;
+        const int cnt = min(d.nbr_count[i], d.nbr_cap);
+        const uint4 qi = d.pfx ? d.pfx[i] : make_uint4(0u, 0u, 0u, 0u);
+        const long long* im = reinterpret_cast<const long long*>(d.img) + 3 * i;
+        for (int k0 = 0; k0 < cnt; k0 += 32) {
+            const int k = k0 + lane;
+            int j = 0;
+            int cls = -1;
+            if (k < cnt) {
+                j = dbg_index(d.nbr[(int64_t)k * d.nbr_kstride + i * d.nbr_istride], d.n, (int)i, d.status);
+                const bool lj = lj_i && (!water || fx_oxygen(j));
+                if (j > (int)i && (lj || (has_el && !el_excluded(d.kind, i, j)))) {
+                    cls = lj ? 3 : 1;
+                    if (d.pfx) {
+                        const uint4 qj = d.pfx[j];
+                        float fx, fy, fz;
+                        if (fx_r2(qi, qj, fx, fy, fz) >= reach) cls = -1;
+                        // bare: the same image, and no wrap of the unsigned positions
+                        const long long* jm = reinterpret_cast<const long long*>(d.img) + 3 * (int64_t)j;
+                        if (im[0] == jm[0] && im[1] == jm[1] && im[2] == jm[2] && (qi.x >= qj.x) == ((int)(qi.x - qj.x) >= 0) &&
+                            (qi.y >= qj.y) == ((int)(qi.y - qj.y) >= 0) && (qi.z >= qj.z) == ((int)(qi.z - qj.z) >= 0))
+                            cls &= ~1;
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                int2* const q = queue[w][c];
+                const bool mine = cls == c;
+                const unsigned bal = __ballot_sync(0xffffffffu, mine);
+                if (!bal) continue;
+                if (mine) q[fill[c] + __popc(bal & ((1u << lane) - 1u))] = make_int2((int)i, j);
+                fill[c] += __popc(bal);
+                __syncwarp();
+                if (fill[c] >= 32) {
+                    take(q, 32, c & 1, c & 2);
+                    __syncwarp();
+                    if (lane < fill[c] - 32) q[lane] = q[32 + lane];
+                    fill[c] -= 32;
+                    __syncwarp();
+                }
+            }
+        }
     }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) take(queue[w][c], fill[c], c & 1, c & 2);
     if (range_err) status_set(d.status, ST_RANGE);
-    __shared__ double sh[2][EB];
-    sh[0][threadIdx.x] = e_lj;
-    sh[1][threadIdx.x] = e_el;
-    __syncthreads();
-    for (int w = EB / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int k = 0; k < 2; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 2; ++k) out[blockIdx.x * 2 + k] = sh[k][0];
+    block_sums<3>(e, out + 3 * (int64_t)blockIdx.x);
 }
 
-// kinetic sum (v.v) m/2 and m v.v (temperature), bonds and angles
+// kinetic sum (v.v) m/2 and m v.v (temperature): a thread per atom; bonds and
+// angles: a thread per molecule
 __global__ void __launch_bounds__(EB) k_energy_local(Dev d, const double* X, const double* V, double* out /*[grid][4]*/)
 {
-    double ke = 0.0, mv2 = 0.0, eb = 0.0, ea = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < d.n; i += (int64_t)gridDim.x * blockDim.x) {
+    double e[4] = {0.0, 0.0, 0.0, 0.0};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (int64_t i = t0; i < d.n; i += stride) {
         double s = __dadd_rn(__dadd_rn(__dmul_rn(V[3 * i], V[3 * i]), __dmul_rn(V[3 * i + 1], V[3 * i + 1])),
                              __dmul_rn(V[3 * i + 2], V[3 * i + 2]));
-        ke = __dadd_rn(ke, __dmul_rn(s, d.mass[i] / 2.0));
-        mv2 = __dadd_rn(mv2, __dmul_rn(d.mass[i], s));
-        if (d.kind == NBG_SYSTEM_WATER && i % 3 == 0) {
-            const double *ro = X + 3 * i, *ra = ro + 3, *rc = ro + 6;
+        e[0] = __dadd_rn(e[0], __dmul_rn(s, d.mass[i] / 2.0));
+        e[1] = __dadd_rn(e[1], __dmul_rn(d.mass[i], s));
+    }
+    if (d.kind == NBG_SYSTEM_WATER)
+        for (int64_t m = t0; m < d.n / 3; m += stride) {
+            const double *ro = X + 9 * m, *ra = ro + 3, *rc = ro + 6;
             double b1[3], b2[3];
             for (int k = 0; k < 3; ++k) {
                 b1[k] = __dsub_rn(ra[k], ro[k]);
@@ -155,89 +297,107 @@ __global__ void __launch_bounds__(EB) k_energy_local(Dev d, const double* X, con
             double d1 = __dsub_rn(n1, d.rOH), d2 = __dsub_rn(n2, d.rOH);
             // directed bonds O->H1, O->H2, H1->O, H2->O
             double t1 = __dmul_rn(__dmul_rn(d1, d1), d.kbond), t2 = __dmul_rn(__dmul_rn(d2, d2), d.kbond);
-            eb = __dadd_rn(eb, __dadd_rn(__dadd_rn(t1, t2), __dadd_rn(t1, t2)));
+            e[2] = __dadd_rn(e[2], __dadd_rn(__dadd_rn(t1, t2), __dadd_rn(t1, t2)));
             double dot = __dadd_rn(__dadd_rn(__dmul_rn(b1[0], b2[0]), __dmul_rn(b1[1], b2[1])), __dmul_rn(b1[2], b2[2]));
             double th = acos(dot / __dmul_rn(n1, n2));
             double dt = __dsub_rn(th, d.aHOH);
-            ea = __dadd_rn(ea, __dmul_rn(__dmul_rn(d.kangle, dt), dt));
+            e[3] = __dadd_rn(e[3], __dmul_rn(__dmul_rn(d.kangle, dt), dt));
         }
-    }
-    __shared__ double sh[4][EB];
-    sh[0][threadIdx.x] = ke;
-    sh[1][threadIdx.x] = mv2;
-    sh[2][threadIdx.x] = eb;
-    sh[3][threadIdx.x] = ea;
-    __syncthreads();
-    for (int w = EB / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int k = 0; k < 4; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 4; ++k) out[blockIdx.x * 4 + k] = sh[k][0];
+    block_sums<4>(e, out + 4 * (int64_t)blockIdx.x);
 }
 
-// out_host: kinetic, lj, el, bonds, angles, gravity, sum m v^2
+// The sums of the block partials in a fixed order: out[0..2] of a[na][3],
+// out[3..6] of b[nb][4]; out[7] the status word.
+__global__ void __launch_bounds__(128) k_energy_sum(const double* a, int64_t na, const double* b, int64_t nb,
+                                                     const unsigned* status, double* out)
+{
+    if (threadIdx.x == 0) out[7] = (double)*status;
+    double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int64_t k = threadIdx.x; k < na; k += blockDim.x)
+        for (int c = 0; c < 3; ++c) v[c] += a[3 * k + c];
+    for (int64_t k = threadIdx.x; k < nb; k += blockDim.x)
+        for (int c = 0; c < 4; ++c) v[3 + c] += b[4 * k + c];
+    block_sums<7>(v, out);
+}
+
+typedef void (*energy_pairs_t)(Dev, const double*, double*);
+
+template <int BC>
+static energy_pairs_t energy_pairs(const Dev& d)
+{
+    const bool lj = d.pots & NBG_POT_LJ, el = d.pots & NBG_POT_EL, g = d.pots & NBG_POT_GRAV;
+    if (g) return lj ? (el ? k_energy_pairs<BC, true, true, true> : k_energy_pairs<BC, true, false, true>)
+                     : (el ? k_energy_pairs<BC, false, true, true> : k_energy_pairs<BC, false, false, true>);
+    if (lj) return el ? k_energy_pairs<BC, true, true, false> : k_energy_pairs<BC, true, false, false>;
+    return k_energy_pairs<BC, false, true, false>;
+}
+
+// out_host: kinetic, lj, el, bonds, angles, gravity, sum m v^2, status word
 int launch_energy(nbg_ctx* c, const StateView& s, double* out_host)
 {
-    const int gp = grid_for(c->n, EB) < 1024 ? grid_for(c->n, EB) : 1024;
-    const int gl = grid_for(c->n, EB) < 256 ? grid_for(c->n, EB) : 256;
-    double* buf = nullptr;
-    size_t bytes = sizeof(double) * (3 * (size_t)gp + 4 * (size_t)gl);
-    cudaError_t e = cudaMallocAsync((void**)&buf, bytes, c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "energy scratch");
+    const Dev& d = c->d;
     const bool list = c->path == PATH_LIST && c->nrep == 1;
+    const bool any_pairs = (d.pots & (NBG_POT_LJ | NBG_POT_EL | NBG_POT_GRAV)) != 0;
+    // list: four warps per SM sub-partition (FP64 needs few), so that each
+    // fills its queue many times; all pairs: a block per item, up to 16 an SM
+    const int64_t gp = list ? std::min<int64_t>((c->n + EL_WARPS - 1) / EL_WARPS, 2 * (int64_t)c->sms)
+                       : any_pairs ? std::min<int64_t>((c->n + EB - 1) / EB * ((c->n + EJ - 1) / EJ), 16 * (int64_t)c->sms)
+                                   : 0;
+    const int64_t gl = std::min<int64_t>((c->n + EB - 1) / EB, 2 * (int64_t)c->sms);
+    // block partials, then the seven sums
+    const int64_t need = 3 * gp + 4 * gl + 8;
+    if (c->energy_cap < need) {
+        if (c->energy_buf) cudaFree(c->energy_buf);
+        c->energy_buf = nullptr;
+        c->energy_cap = 0;
+        cudaError_t e = cudaMalloc((void**)&c->energy_buf, sizeof(double) * (size_t)need);
+        if (e != cudaSuccess) {
+            c->energy_buf = nullptr;
+            return cuda_fail(c, e, "energy scratch");
+        }
+        c->energy_cap = need;
+    }
+    double* const part = c->energy_buf + 8;
     if (list) {
         // a list for exactly these positions
         int st = launch_pack(c, s);
         if (st) return st;
         if ((st = launch_list_build(c, s, true, StepRef{0, nullptr}))) return st;
-        k_energy_list<<<gp, EB, 0, c->stream>>>(c->d, s.x, buf);
+        k_energy_list<<<(unsigned)gp, EL_WARPS * 32, 0, c->stream>>>(d, s.x, part);
         NBG_LAUNCH_CHECK(c, "k_energy_list");
-    } else {
-        k_energy_pairs<<<gp, EB, 0, c->stream>>>(c->d, s.x, buf);
+    } else if (any_pairs) {
+        const energy_pairs_t k = d.bc == NBG_BC_CUBIC      ? energy_pairs<NBG_BC_CUBIC>(d)
+                                 : d.bc == NBG_BC_PERIODIC ? energy_pairs<NBG_BC_PERIODIC>(d)
+                                                           : energy_pairs<NBG_BC_INFINITE>(d);
+        k<<<(unsigned)gp, EB, 0, c->stream>>>(d, s.x, part);
         NBG_LAUNCH_CHECK(c, "k_energy_pairs");
     }
-    k_energy_local<<<gl, EB, 0, c->stream>>>(c->d, s.x, s.v, buf + 3 * gp);
+    k_energy_local<<<(unsigned)gl, EB, 0, c->stream>>>(d, s.x, s.v, part + 3 * gp);
     NBG_LAUNCH_CHECK(c, "k_energy_local");
-    std::vector<double> h(3 * (size_t)gp + 4 * (size_t)gl);
-    e = cudaMemcpyAsync(h.data(), buf, bytes, cudaMemcpyDeviceToHost, c->stream);
+    k_energy_sum<<<1, 128, 0, c->stream>>>(part, gp, part + 3 * gp, gl, d.status, c->energy_buf);
+    NBG_LAUNCH_CHECK(c, "k_energy_sum");
+    double h[8];
+    cudaError_t e = cudaMemcpyAsync(h, c->energy_buf, sizeof h, cudaMemcpyDeviceToHost, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "energy copy");
-    cudaFreeAsync(buf, c->stream);
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "energy sync");
-    double lj = 0, el = 0, g = 0, ke = 0, mv2 = 0, eb = 0, ea = 0;
+    double lj = h[0], el = h[1];
+    const double g = h[2], ke = h[3], mv2 = h[4], eb = h[5], ea = h[6];
     if (list) {
-        for (int b = 0; b < gp; ++b) {
-            lj += h[2 * b];
-            el += h[2 * b + 1];
-        }
         // every pair's beyond-cutoff term: LJ(R) per LJ pair, q_i q_j / R per charge pair
-        double s6R = c->d.lj_sig2_d / c->d.lj_R2;
+        double s6R = d.lj_sig2_d / d.lj_R2;
         s6R = s6R * s6R * s6R;
-        if (c->d.pots & NBG_POT_LJ) lj += (double)c->lj_pairs * (s6R * s6R - s6R);
-        if (c->d.pots & NBG_POT_EL) el += c->el_pair_qq / c->d.el_R;
-    } else {
-        for (int b = 0; b < gp; ++b) {
-            lj += h[3 * b];
-            el += h[3 * b + 1];
-            g += h[3 * b + 2];
-        }
-    }
-    for (int b = 0; b < gl; ++b) {
-        const double* q = h.data() + 3 * gp + 4 * b;
-        ke += q[0];
-        mv2 += q[1];
-        eb += q[2];
-        ea += q[3];
+        if (d.pots & NBG_POT_LJ) lj += (double)c->lj_pairs * (s6R * s6R - s6R);
+        if (d.pots & NBG_POT_EL) el += c->el_pair_qq / d.el_R;
     }
     out_host[0] = ke;
-    out_host[1] = (c->d.pots & NBG_POT_LJ) ? 4.0 * c->d.lj_eps * lj : 0.0;
-    out_host[2] = (c->d.pots & NBG_POT_EL) ? el * c->d.el_k_d : 0.0;
-    out_host[3] = c->d.kind == NBG_SYSTEM_WATER ? eb / 4.0 : 0.0;
-    out_host[4] = c->d.kind == NBG_SYSTEM_WATER ? ea / 2.0 : 0.0;
-    out_host[5] = (c->d.pots & NBG_POT_GRAV) ? -c->d.G * g : 0.0;
+    out_host[1] = (d.pots & NBG_POT_LJ) ? 4.0 * d.lj_eps * lj : 0.0;
+    out_host[2] = (d.pots & NBG_POT_EL) ? el * d.el_k_d : 0.0;
+    out_host[3] = d.kind == NBG_SYSTEM_WATER ? eb / 4.0 : 0.0;
+    out_host[4] = d.kind == NBG_SYSTEM_WATER ? ea / 2.0 : 0.0;
+    out_host[5] = (d.pots & NBG_POT_GRAV) ? -d.G * g : 0.0;
     out_host[6] = mv2;
+    out_host[7] = h[7];
     return NBG_OK;
 }
 

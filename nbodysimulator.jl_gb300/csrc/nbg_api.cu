@@ -750,6 +750,9 @@ static void release(nbg_ctx* c)
     if (c->frames) cudaFree(c->frames);
     c->frames = nullptr;
     c->frames_cap = 0;
+    if (c->energy_buf) cudaFree(c->energy_buf);
+    c->energy_buf = nullptr;
+    c->energy_cap = 0;
     for (void* p : c->allocs) cudaFree(p);
     c->allocs.clear();
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -1744,12 +1747,11 @@ extern "C" int nbg_energy(nbg_ctx* c, const double* u, const double* v, nbg_ener
     CK(cudaMemcpyAsync(c->ev.v, v, state_bytes(c), cudaMemcpyHostToDevice, c->stream), "v upload");
     int st;
     if (c->path == PATH_LIST) resident_dirty(c);  // the list is rebuilt for u
-    double h[7];
+    double h[8];
     for (int attempt = 0;; ++attempt) {
         if ((st = clear_status(c))) return st;
         if ((st = launch_energy(c, c->ev, h))) return st;
-        unsigned w = 0;
-        if ((st = read_status(c, &w))) return st;
+        const unsigned w = (unsigned)h[7];
         if (attempt < 6 && (w & (ST_CELL_OVERFLOW | ST_NBR_OVERFLOW)) && !(w & (ST_NONFINITE | ST_RANGE | ST_INDEX))) {
             if ((st = grow_lists(c, w))) return st;
             continue;

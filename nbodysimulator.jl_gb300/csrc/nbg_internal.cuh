@@ -318,6 +318,9 @@ struct nbg_ctx {
     float4* grav_box = nullptr;       // 2 per 128-body tile
     int64_t grav_evals = 0;           // gravity evaluations issued (the sort runs on every 8th)
     bool grav_perm_valid = false;     // the permutation belongs to the positions being evaluated
+    // block partials of nbg_energy
+    double* energy_buf = nullptr;
+    int64_t energy_cap = 0;
     // profiling of the dominant force kernel
     bool profiling = false;
     // captured step graphs (velocity Verlet / Euler-Maruyama)
@@ -432,7 +435,7 @@ int launch_save_frame(nbg_ctx* c, const StateView& s, StepRef sr);
 int launch_rhs_thermostat(nbg_ctx* c, const StateView& s);
 int gravity_plan_chunks(nbg_ctx* c, int64_t npad);
 size_t gravity_sort_bytes(int64_t n);
-int launch_energy(nbg_ctx* c, const StateView& s, double* out_host /*[8]*/);
+int launch_energy(nbg_ctx* c, const StateView& s, double* out_host /*[8], the last one the status word*/);
 int launch_pairs(nbg_ctx* c, const StateView& s, int which, int* out_j, int* out_cnt, int64_t cap_per_atom);
 
 // learned short-range model and r-RESPA (k_learned.cu)

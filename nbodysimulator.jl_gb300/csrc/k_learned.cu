@@ -28,6 +28,8 @@
 // products with tcgen05.mma into tensor memory, 128 atoms per product. Learned forces are scattered to
 // neighbours as 64-bit fixed point (2^-32 units) so the sum does not depend
 // on the order of the atomics. Training runs in FP32 on the CUDA cores.
+#include <algorithm>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -1147,107 +1149,289 @@ __global__ void __launch_bounds__(ML_TPB) k_sr_exact(Dev d, MLView m, float* e_o
 // ---------------------------------------------------------------------
 // training (FP32, CUDA cores)
 // ---------------------------------------------------------------------
-// Forward and backward of one batch: thread per sample b. X rows are raw
-// descriptors (standardised here; std != 0 uses them already standardised),
-// y raw labels. Writes x, a1, a2, g1, g2 ([B][128]) and e ([B]: dL/dout);
-// loss into *loss (atomic, FP64).
-__global__ void __launch_bounds__(64) k_train_fb(const float* __restrict__ theta, const float* __restrict__ X,
-                                                 const float* __restrict__ Y, const int* __restrict__ idx, int B,
-                                                 int standardised, float* xs, float* a1, float* a2, float* g1,
-                                                 float* g2, float* eo, double* loss)
+// One training step is three kernels: k_train_fb (forward and backward of
+// the samples), k_train_grad (weight gradients: products of the layers' inputs
+// and output gradients, summed over a slice of the batch) and k_train_step
+// (slices summed in order, loss, Adam). A thread per sample with its 41,000
+// multiply-adds in one chain and a thread per parameter walking the batch
+// took 2.2 ms for 2048 samples on 32 + 195 blocks; the three take 30 us.
+
+// Samples of one step: rows of the training set drawn by Philox (rows > 0),
+// or the batch in order.
+struct TrainBatch {
+    const float* X;    // [..][64] descriptors, raw or standardised
+    const float* Y;    // labels
+    int B;
+    int standardised;
+    int64_t rows;      // > 0: sample b is row philox(seed, b, batch) % rows
+    uint64_t seed, batch;
+};
+
+__device__ __forceinline__ int64_t train_row(const TrainBatch& t, int b)
 {
-    extern __shared__ float sw[];
-    float* W1 = sw;                  // [64][128]
-    float* W2 = W1 + ML_ND * ML_NH;  // [128][128]
-    for (int e = threadIdx.x; e < ML_ND * ML_NH; e += blockDim.x) W1[e] = theta[e];
-    for (int e = threadIdx.x; e < ML_NH * ML_NH; e += blockDim.x) W2[e] = theta[param_off_w2() + e];
+    if (t.rows <= 0) return b;
+    const uint4 w = philox(t.seed, (uint64_t)b, t.batch, 7u);
+    const uint64_t r = ((uint64_t)w.x << 32) | w.y;
+    return (int)(r % (uint64_t)t.rows);
+}
+
+// Forward and backward of TS samples per block: thread (n, h) holds column n
+// of a layer for samples 8 h .. 8 h + 7, so that a weight is loaded once for 8
+// multiply-adds and the samples' inputs come as shared-memory broadcasts. W2
+// lies in shared memory in rows of 132 floats: the forward reads it by
+// columns, the backward by rows as 16-byte vectors, both without bank
+// conflicts. The sums run in the order of one thread per sample (bound: FP32
+// issue and shared-memory reads, 41 k multiply-adds a sample).
+// Writes x, a1, a2, g1, g2 ([B][128]), e ([B]: dL/dout) and the block's sum of
+// squared errors.
+#define TS 16
+#define T_W2S 132
+
+struct TrainSmem {
+    float w2[ML_NH * T_W2S];
+    float xT[ML_ND][TS], a1T[ML_NH][TS], a2T[ML_NH][TS], g2T[ML_NH][TS];
+    float w3[ML_NH], de[TS];
+};
+
+__global__ void __launch_bounds__(256) k_train_fb(const float* __restrict__ theta, TrainBatch t, float* xs, float* a1,
+                                                  float* a2, float* g1, float* g2, float* eo, double* sq)
+{
+    extern __shared__ __align__(16) unsigned char train_sm[];
+    TrainSmem& S = *reinterpret_cast<TrainSmem*>(train_sm);
+    const int tid = threadIdx.x, n = tid & (ML_NH - 1), s0 = (tid >> 7) * 8, b0 = blockIdx.x * TS;
+    const float* W2 = theta + param_off_w2();
+    // (theta + param_off_w2() is 16-byte aligned: a multiple of 4 floats into an allocation)
+    for (int e = tid; e < ML_NH * ML_NH / 4; e += 256) {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(&S.w2[(e / 32) * T_W2S + (e % 32) * 4]);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(W2 + 4 * e) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (tid < ML_NH) S.w3[tid] = theta[param_off_w3() + tid];
+    {
+        const float* mu = theta + param_off_mu();
+        const float* sd = theta + param_off_sd();
+        const int k = tid & 63;
+        for (int s = tid >> 6; s < TS; s += 4) {
+            float x = 0.f;
+            if (b0 + s < t.B) {
+                const float v = t.X[train_row(t, b0 + s) * ML_ND + k];
+                x = t.standardised ? v : (v - mu[k]) / sd[k];
+                xs[(int64_t)(b0 + s) * ML_ND + k] = x;
+            }
+            S.xT[k][s] = x;
+        }
+    }
     __syncthreads();
-    const float* b1 = theta + param_off_b1();
-    const float* b2 = theta + param_off_b2();
-    const float* w3 = theta + param_off_w3();
-    const float b3 = theta[param_off_b3()];
-    const float* mu = theta + param_off_mu();
-    const float* sd = theta + param_off_sd();
-    const float muE = theta[param_off_muE()], sdE = theta[param_off_muE() + 1];
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const int row = idx ? idx[b] : b;
-    const float* D = X + (int64_t)row * ML_ND;
-    float* xb = xs + (int64_t)b * ML_ND;
-    for (int k = 0; k < ML_ND; ++k) xb[k] = standardised ? D[k] : (D[k] - mu[k]) / sd[k];
-    float* A1 = a1 + (int64_t)b * ML_NH;
-    float* A2 = a2 + (int64_t)b * ML_NH;
-    for (int n = 0; n < ML_NH; ++n) {
-        float z = b1[n];
-        for (int k = 0; k < ML_ND; ++k) z = fmaf(xb[k], W1[k * ML_NH + n], z);
-        A1[n] = tanhf(z);
+    float z[8];
+    auto row8 = [](const float* p, float* v) {
+        const float4 q0 = *reinterpret_cast<const float4*>(p), q1 = *reinterpret_cast<const float4*>(p + 4);
+        v[0] = q0.x; v[1] = q0.y; v[2] = q0.z; v[3] = q0.w;
+        v[4] = q1.x; v[5] = q1.y; v[6] = q1.z; v[7] = q1.w;
+    };
+    {
+        const float b = theta[param_off_b1() + n];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) z[s] = b;
+#pragma unroll 16
+        for (int k = 0; k < ML_ND; ++k) {
+            const float w = __ldg(theta + k * ML_NH + n);
+            float x[8];
+            row8(&S.xT[k][s0], x);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) z[s] = fmaf(x[s], w, z[s]);
+        }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const float v = tanhf(z[s]);
+            S.a1T[n][s0 + s] = v;
+            if (b0 + s0 + s < t.B) a1[(int64_t)(b0 + s0 + s) * ML_NH + n] = v;
+        }
     }
-    float out = b3;
-    for (int n = 0; n < ML_NH; ++n) {
-        float z = b2[n];
-        for (int k = 0; k < ML_NH; ++k) z = fmaf(A1[k], W2[k * ML_NH + n], z);
-        const float v = tanhf(z);
-        A2[n] = v;
-        out = fmaf(v, w3[n], out);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float av[8];  // a2 of column n
+    {
+        const float b = theta[param_off_b2() + n];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) z[s] = b;
+#pragma unroll 8
+        for (int k = 0; k < ML_NH; ++k) {
+            const float w = S.w2[k * T_W2S + n];
+            float x[8];
+            row8(&S.a1T[k][s0], x);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) z[s] = fmaf(x[s], w, z[s]);
+        }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            av[s] = tanhf(z[s]);
+            S.a2T[n][s0 + s] = av[s];
+            if (b0 + s0 + s < t.B) a2[(int64_t)(b0 + s0 + s) * ML_NH + n] = av[s];
+        }
     }
-    const float y = standardised ? Y[row] : (Y[row] - muE) / sdE;
-    const float err = out - y;
-    atomicAdd(loss, (double)err * (double)err / (double)B);
-    const float de = 2.f * err / (float)B;
-    eo[b] = de;
-    float* G2 = g2 + (int64_t)b * ML_NH;
-    float* G1 = g1 + (int64_t)b * ML_NH;
-    for (int n = 0; n < ML_NH; ++n) G2[n] = de * w3[n] * (1.f - A2[n] * A2[n]);
-    for (int k = 0; k < ML_NH; ++k) {
-        float s = 0.f;
-        for (int n = 0; n < ML_NH; ++n) s = fmaf(G2[n], W2[k * ML_NH + n], s);
-        G1[k] = s * (1.f - A1[k] * A1[k]);
+    __syncthreads();
+    if (tid < 32) {  // the output of a sample (lanes 16 on repeat), its error and dL/dout
+        const int s = tid % TS, b = b0 + s;
+        float out = theta[param_off_b3()];
+#pragma unroll 16
+        for (int k = 0; k < ML_NH; ++k) out = fmaf(S.a2T[k][s], S.w3[k], out);
+        float de = 0.f;
+        double e2 = 0.0;
+        if (b < t.B) {
+            const float y = t.Y[train_row(t, b)];
+            const float err = out - (t.standardised ? y : (y - theta[param_off_muE()]) / theta[param_off_muE() + 1]);
+            de = 2.f * err / (float)t.B;
+            eo[b] = de;
+            e2 = (double)err * (double)err;
+        }
+        S.de[s] = de;
+#pragma unroll
+        for (int o = TS / 2; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o, TS);
+        if (tid == 0) sq[blockIdx.x] = e2;
+    }
+    __syncthreads();
+    {
+        const float w3 = S.w3[n];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const float g = S.de[s0 + s] * w3 * (1.f - av[s] * av[s]);
+            S.g2T[n][s0 + s] = g;
+            if (b0 + s0 + s < t.B) g2[(int64_t)(b0 + s0 + s) * ML_NH + n] = g;
+        }
+    }
+    __syncthreads();
+    {
+#pragma unroll
+        for (int s = 0; s < 8; ++s) z[s] = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < ML_NH; c += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(&S.w2[n * T_W2S + c]);
+            const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float g[8];
+                row8(&S.g2T[c + e][s0], g);
+#pragma unroll
+                for (int s = 0; s < 8; ++s) z[s] = fmaf(g[s], wv[e], z[s]);
+            }
+        }
+        float a[8];
+        row8(&S.a1T[n][s0], a);
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+            if (b0 + s0 + s < t.B) g1[(int64_t)(b0 + s0 + s) * ML_NH + n] = z[s] * (1.f - a[s] * a[s]);
     }
 }
 
-// grad[p] for W1 (64x128), b1, W2 (128x128), b2, w3, b3: column sums over the
-// batch in fixed order (thread per parameter)
-__global__ void k_train_grad(int B, const float* __restrict__ xs, const float* __restrict__ a1,
-                             const float* __restrict__ a2, const float* __restrict__ g1, const float* __restrict__ g2,
-                             const float* __restrict__ eo, float* grad)
+// Weight gradients of one slice of the batch (blockIdx.y: samples s, s + 1,
+// .. of `per`) into part[slice][ML_NTRAIN]. blockIdx.x < 12: a 32 x 64 tile of
+// W1 (4 tiles) or W2 (8), 4 x 4 outputs a thread, 32 samples staged at a time;
+// the tiles of the first 32 rows also add the bias. blockIdx.x = 12: w3 and b3.
+#define TG_S 32
+
+__global__ void __launch_bounds__(128) k_train_grad(int B, int per, const float* __restrict__ xs,
+                                                    const float* __restrict__ a1, const float* __restrict__ a2,
+                                                    const float* __restrict__ g1, const float* __restrict__ g2,
+                                                    const float* __restrict__ eo, float* __restrict__ part)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nW1 = ML_ND * ML_NH, nW2 = ML_NH * ML_NH;
-    if (p >= ML_NTRAIN) return;
-    float s = 0.f;
-    if (p < nW1) {
-        const int k = p / ML_NH, n = p % ML_NH;
-        for (int b = 0; b < B; ++b) s = fmaf(xs[(int64_t)b * ML_ND + k], g1[(int64_t)b * ML_NH + n], s);
-    } else if (p < nW1 + ML_NH) {
-        const int n = p - nW1;
-        for (int b = 0; b < B; ++b) s += g1[(int64_t)b * ML_NH + n];
-    } else if (p < nW1 + ML_NH + nW2) {
-        const int q = p - nW1 - ML_NH, k = q / ML_NH, n = q % ML_NH;
-        for (int b = 0; b < B; ++b) s = fmaf(a1[(int64_t)b * ML_NH + k], g2[(int64_t)b * ML_NH + n], s);
-    } else if (p < nW1 + 2 * ML_NH + nW2) {
-        const int n = p - nW1 - ML_NH - nW2;
-        for (int b = 0; b < B; ++b) s += g2[(int64_t)b * ML_NH + n];
-    } else if (p < nW1 + 3 * ML_NH + nW2) {
-        const int n = p - nW1 - 2 * ML_NH - nW2;
-        for (int b = 0; b < B; ++b) s = fmaf(a2[(int64_t)b * ML_NH + n], eo[b], s);
-    } else {
-        for (int b = 0; b < B; ++b) s += eo[b];
+    __shared__ __align__(16) float in[TG_S][32], og[TG_S][64];
+    const int tid = threadIdx.x, s0 = blockIdx.y * per, s1 = min(B, s0 + per);
+    float* const out = part + (int64_t)blockIdx.y * ML_NTRAIN;
+    if (blockIdx.x == 12) {
+        float s = 0.f, e = 0.f;
+#pragma unroll 8
+        for (int b = s0; b < s1; ++b) {
+            s = fmaf(a2[(int64_t)b * ML_NH + tid], eo[b], s);
+            e += eo[b];
+        }
+        out[param_off_w3() + tid] = s;
+        if (tid == 0) out[param_off_b3()] = e;
+        return;
     }
-    grad[p] = s;
+    const bool second = blockIdx.x >= 4;
+    const int tile = second ? blockIdx.x - 4 : blockIdx.x;
+    const int k0 = (tile >> 1) * 32, n0 = (tile & 1) * 64, ld = second ? ML_NH : ML_ND;
+    const float* A = second ? a1 : xs;
+    const float* G = second ? g2 : g1;
+    const int tk = (tid >> 4) * 4, tn = (tid & 15) * 4;
+    float acc[4][4], bias[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int b = s0; b < s1; b += TG_S) {
+        __syncthreads();
+        // 32 samples x (8 + 16) 16-byte vectors
+        for (int e = tid; e < TG_S * 8; e += 128) {
+            const int s = e >> 3, c = (e & 7) * 4;
+            *reinterpret_cast<float4*>(&in[s][c]) =
+                b + s < s1 ? *reinterpret_cast<const float4*>(A + (int64_t)(b + s) * ld + k0 + c) : zero;
+        }
+        for (int e = tid; e < TG_S * 16; e += 128) {
+            const int s = e >> 4, c = (e & 15) * 4;
+            *reinterpret_cast<float4*>(&og[s][c]) =
+                b + s < s1 ? *reinterpret_cast<const float4*>(G + (int64_t)(b + s) * ML_NH + n0 + c) : zero;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int s = 0; s < TG_S; ++s) {
+            const float4 x = *reinterpret_cast<const float4*>(&in[s][tk]);
+            const float4 g = *reinterpret_cast<const float4*>(&og[s][tn]);
+            const float xv[4] = {x.x, x.y, x.z, x.w}, gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], gv[j], acc[i][j]);
+            if (tk == 0)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) bias[j] += gv[j];
+        }
+    }
+    float* W = out + (second ? param_off_w2() : 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j) W[(k0 + tk + i) * ML_NH + n0 + tn + j] = acc[i][j];
+    if (k0 == 0 && tk == 0)
+        for (int j = 0; j < 4; ++j) out[(second ? param_off_b2() : param_off_b1()) + n0 + tn + j] = bias[j];
 }
 
-// Adam (Kingma & Ba 2015) on the trainable parameters
-__global__ void k_adam(float* theta, const float* grad, float* m1, float* m2, int count, float lr, float b1, float b2,
-                       float eps, float c1, float c2)
+// The gradient (the slices summed in order), the batch's loss added to *loss
+// (block 0), and with ADAM (Kingma & Ba 2015) the parameters' step.
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_train_step(int B, int slices, const float* __restrict__ part,
+                                                    const double* __restrict__ sq, float* grad, double* loss, float* theta,
+                                                    float* m1, float* m2, float lr, float b1, float b2, float eps, float c1,
+                                                    float c2)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= count) return;
-    const float g = grad[p];
-    const float a = b1 * m1[p] + (1.f - b1) * g;
-    const float v = b2 * m2[p] + (1.f - b2) * g * g;
-    m1[p] = a;
-    m2[p] = v;
-    theta[p] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
+    if (p < ML_NTRAIN) {
+        float g = 0.f;
+#pragma unroll 4
+        for (int s = 0; s < slices; ++s) g += part[(int64_t)s * ML_NTRAIN + p];
+        if (ADAM) {
+            const float a = b1 * m1[p] + (1.f - b1) * g;
+            const float v = b2 * m2[p] + (1.f - b2) * g * g;
+            m1[p] = a;
+            m2[p] = v;
+            theta[p] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
+        } else {
+            grad[p] = g;
+        }
+    }
+    if (blockIdx.x != gridDim.x - 1) return;
+    // (the last block has few parameters) the blocks' squared errors, a
+    // thread's terms in order, then a tree
+    __shared__ double sh[256];
+    double e = 0.0;
+    for (int b = threadIdx.x; b < (B + TS - 1) / TS; b += blockDim.x) e += sq[b];
+    sh[threadIdx.x] = e;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss += sh[0] / (double)B;
 }
 
 // BF16 copies of W1 and W2 for inference
@@ -1306,16 +1490,6 @@ __global__ void k_ml_stats(const float* X, const float* Y, int64_t rows, float* 
             theta[param_off_muE() + 1] = (float)sd;
         }
     }
-}
-
-// random sample indices for a batch (Philox, seed and batch counter)
-__global__ void k_ml_sample(int* idx, int B, int64_t rows, uint64_t seed, uint64_t batch)
-{
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const uint4 w = philox(seed, (uint64_t)b, batch, 7u);
-    const uint64_t r = ((uint64_t)w.x << 32) | w.y;
-    idx[b] = (int)(r % (uint64_t)rows);
 }
 
 // a (=, +=, -=) F / m from the fixed-point learned forces (mode 0, 1, -1)
@@ -1600,14 +1774,21 @@ int launch_ml_stats(nbg_ctx* c, int sp)
     return NBG_OK;
 }
 
-static int train_fb_grad(nbg_ctx* c, const float* theta, const float* X, const float* Y, const int* idx, int B,
-                         bool standardised, MLTrainScratch& s)
+// forward, backward and the slices' weight gradients of one batch
+static int train_fb_grad(nbg_ctx* c, const float* theta, const TrainBatch& t, int& slices)
 {
-    const int smem = (ML_ND * ML_NH + ML_NH * ML_NH) * (int)sizeof(float);
-    k_train_fb<<<(B + 63) / 64, 64, smem, c->stream>>>(theta, X, Y, idx, B, standardised ? 1 : 0, s.xs, s.a1, s.a2,
-                                                       s.g1, s.g2, s.eo, s.loss);
+    MLTrainScratch& s = c->ml_ts;
+    if (!c->ml_attr) {
+        int st = launch_mlp_attrs(c);
+        if (st) return st;
+    }
+    k_train_fb<<<(t.B + TS - 1) / TS, 256, sizeof(TrainSmem), c->stream>>>(theta, t, s.xs, s.a1, s.a2, s.g1, s.g2, s.eo,
+                                                                           s.sq);
     NBG_LAUNCH_CHECK(c, "k_train_fb");
-    k_train_grad<<<(ML_NTRAIN + 127) / 128, 128, 0, c->stream>>>(B, s.xs, s.a1, s.a2, s.g1, s.g2, s.eo, s.grad);
+    // slices of at least 64 samples, up to ML_GRAD_SLICES (two blocks per SM)
+    const int per = std::max(64, (t.B + ML_GRAD_SLICES - 1) / ML_GRAD_SLICES);
+    slices = (t.B + per - 1) / per;
+    k_train_grad<<<dim3(13, slices), 128, 0, c->stream>>>(t.B, per, s.xs, s.a1, s.a2, s.g1, s.g2, s.eo, s.part);
     NBG_LAUNCH_CHECK(c, "k_train_grad");
     return NBG_OK;
 }
@@ -1615,29 +1796,28 @@ static int train_fb_grad(nbg_ctx* c, const float* theta, const float* X, const f
 int launch_ml_train_step(nbg_ctx* c, int sp, int B, uint64_t seed, uint64_t batch, float lr, int64_t t_adam)
 {
     MLTrainScratch& s = c->ml_ts;
-    if (!c->ml_attr) {
-        int st = launch_mlp_attrs(c);
-        if (st) return st;
-    }
-    k_ml_sample<<<(B + 255) / 256, 256, 0, c->stream>>>(s.idx, B, c->ml_rows[sp], seed, batch);
-    NBG_LAUNCH_CHECK(c, "k_ml_sample");
-    int st = train_fb_grad(c, c->ml_theta[sp], c->ml_X[sp], c->ml_Y[sp], s.idx, B, false, s);
+    int slices = 0;
+    int st = train_fb_grad(c, c->ml_theta[sp], TrainBatch{c->ml_X[sp], c->ml_Y[sp], B, 0, c->ml_rows[sp], seed, batch}, slices);
     if (st) return st;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)t_adam), c2 = 1.f - powf(b2, (float)t_adam);
-    k_adam<<<(ML_NTRAIN + 255) / 256, 256, 0, c->stream>>>(c->ml_theta[sp], s.grad, s.m1[sp], s.m2[sp], ML_NTRAIN, lr,
-                                                           b1, b2, 1e-8f, c1, c2);
-    NBG_LAUNCH_CHECK(c, "k_adam");
+    k_train_step<true><<<(ML_NTRAIN + 255) / 256, 256, 0, c->stream>>>(B, slices, s.part, s.sq, nullptr, s.loss,
+                                                                       c->ml_theta[sp], s.m1[sp], s.m2[sp], lr, b1, b2,
+                                                                       1e-8f, c1, c2);
+    NBG_LAUNCH_CHECK(c, "k_train_step");
     return NBG_OK;
 }
 
 int launch_ml_batch_grad(nbg_ctx* c, const float* theta, const float* X, const float* Y, int B)
 {
-    if (!c->ml_attr) {
-        int st = launch_mlp_attrs(c);
-        if (st) return st;
-    }
-    return train_fb_grad(c, theta, X, Y, nullptr, B, true, c->ml_ts);
+    MLTrainScratch& s = c->ml_ts;
+    int slices = 0;
+    int st = train_fb_grad(c, theta, TrainBatch{X, Y, B, 1, 0, 0, 0}, slices);
+    if (st) return st;
+    k_train_step<false><<<(ML_NTRAIN + 255) / 256, 256, 0, c->stream>>>(B, slices, s.part, s.sq, s.grad, s.loss, nullptr,
+                                                                        nullptr, nullptr, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
+    NBG_LAUNCH_CHECK(c, "k_train_step");
+    return NBG_OK;
 }
 
 int launch_mlp_attrs(nbg_ctx* c)
@@ -1646,8 +1826,7 @@ int launch_mlp_attrs(nbg_ctx* c)
     if (e != cudaSuccess) return cuda_fail(c, e, "k_mlp_bf16 shared memory");
     e = cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
     if (e != cudaSuccess) return cuda_fail(c, e, "k_mlp_tc shared memory");
-    e = cudaFuncSetAttribute(k_train_fb, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (ML_ND * ML_NH + ML_NH * ML_NH) * (int)sizeof(float));
+    e = cudaFuncSetAttribute(k_train_fb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem));
     if (e != cudaSuccess) return cuda_fail(c, e, "k_train_fb shared memory");
     c->ml_attr = true;
     return NBG_OK;

@@ -2107,24 +2107,28 @@ static int ml_scratch(nbg_ctx* c, int B)
 {
     MLTrainScratch& s = c->ml_ts;
     if (s.B >= B) return NBG_OK;
-    float** bufs[] = {&s.xs, &s.a1, &s.a2, &s.g1, &s.g2, &s.eo, &s.grad};
+    float** bufs[] = {&s.xs, &s.a1, &s.a2, &s.g1, &s.g2, &s.eo, &s.xin, &s.yin, &s.grad, &s.part};
     for (float** p : bufs) {
         if (*p) dfree(c, *p);
         *p = nullptr;
     }
-    if (s.idx) dfree(c, s.idx);
+    s.B = 0;
     if (s.loss) dfree(c, s.loss);
-    s.idx = nullptr;
+    if (s.sq) dfree(c, s.sq);
+    s.sq = nullptr;
     s.loss = nullptr;
     int st;
-    if ((st = dalloc(c, &s.idx, B))) return st;
     if ((st = dalloc(c, &s.xs, (size_t)B * 64))) return st;
     if ((st = dalloc(c, &s.a1, (size_t)B * 128))) return st;
     if ((st = dalloc(c, &s.a2, (size_t)B * 128))) return st;
     if ((st = dalloc(c, &s.g1, (size_t)B * 128))) return st;
     if ((st = dalloc(c, &s.g2, (size_t)B * 128))) return st;
     if ((st = dalloc(c, &s.eo, B))) return st;
+    if ((st = dalloc(c, &s.sq, B))) return st;
+    if ((st = dalloc(c, &s.xin, (size_t)B * 64))) return st;
+    if ((st = dalloc(c, &s.yin, B))) return st;
     if ((st = dalloc(c, &s.grad, ML_NTRAIN))) return st;
+    if ((st = dalloc(c, &s.part, (size_t)ML_GRAD_SLICES * ML_NTRAIN))) return st;
     if ((st = dalloc(c, &s.loss, 1))) return st;
     s.B = B;
     return NBG_OK;
@@ -2168,16 +2172,11 @@ extern "C" int nbg_ml_batch_gradient(nbg_ctx* c, int32_t species, const float* x
     if (st) return st;
     if ((species != 0 && species != 1) || !x || !y || !grad || B < 1) return fail(c, NBG_ERR_ARG, "bad arguments");
     if ((st = ml_scratch(c, B))) return st;
-    float *dX = nullptr, *dY = nullptr;
-    CK(cudaMallocAsync((void**)&dX, sizeof(float) * 64 * (size_t)B, c->stream), "batch alloc");
-    CK(cudaMallocAsync((void**)&dY, sizeof(float) * (size_t)B, c->stream), "batch alloc");
-    CK(cudaMemcpyAsync(dX, x, sizeof(float) * 64 * (size_t)B, cudaMemcpyHostToDevice, c->stream), "batch upload");
-    CK(cudaMemcpyAsync(dY, y, sizeof(float) * (size_t)B, cudaMemcpyHostToDevice, c->stream), "batch upload");
-    CK(cudaMemsetAsync(c->ml_ts.loss, 0, sizeof(double), c->stream), "loss clear");
-    st = launch_ml_batch_grad(c, c->ml_theta[species], dX, dY, B);
-    cudaFreeAsync(dX, c->stream);
-    cudaFreeAsync(dY, c->stream);
-    if (st) return st;
+    MLTrainScratch& s = c->ml_ts;
+    CK(cudaMemcpyAsync(s.xin, x, sizeof(float) * 64 * (size_t)B, cudaMemcpyHostToDevice, c->stream), "batch upload");
+    CK(cudaMemcpyAsync(s.yin, y, sizeof(float) * (size_t)B, cudaMemcpyHostToDevice, c->stream), "batch upload");
+    CK(cudaMemsetAsync(s.loss, 0, sizeof(double), c->stream), "loss clear");
+    if ((st = launch_ml_batch_grad(c, c->ml_theta[species], s.xin, s.yin, B))) return st;
     CK(cudaMemcpyAsync(grad, c->ml_ts.grad, sizeof(float) * ML_NTRAIN, cudaMemcpyDeviceToHost, c->stream),
        "grad download");
     double l = 0.0;

@@ -198,13 +198,14 @@ struct Dev {
 #define ML_NTRAIN (64 * 128 + 128 + 128 * 128 + 128 + 128 + 1)  // trainable parameters per species
 #define ML_NPARAM (ML_NTRAIN + 2 * 64 + 2)                      // plus mean/sd of inputs and label
 
+#define ML_GRAD_SLICES 24  // slices of a batch whose weight gradients are summed apart, at most
 struct MLTrainScratch {
-    int* idx = nullptr;
     float *xs = nullptr, *a1 = nullptr, *a2 = nullptr, *g1 = nullptr, *g2 = nullptr, *eo = nullptr;
-    float* grad = nullptr;
+    float *xin = nullptr, *yin = nullptr;  // a caller's batch
+    float *grad = nullptr, *part = nullptr;
     float* m1[2] = {nullptr, nullptr};  // Adam moments per species
     float* m2[2] = {nullptr, nullptr};
-    double* loss = nullptr;
+    double *loss = nullptr, *sq = nullptr;
     int B = 0;  // batch capacity of the scratch
 };
 

@@ -236,6 +236,226 @@ int launch_kick(nbg_ctx* c, const StateView& s, double dt, bool do_T, bool therm
     return NBG_OK;
 }
 
+// ---------------------------------------------------------------------
+// velocity Verlet inside a captured run of steps (single systems)
+// ---------------------------------------------------------------------
+// Temperature and what the next kick takes from it: red_T, the Berendsen
+// factor and the Nose-Hoover rate (thermostats.jl:76-128; the operations of
+// k_kick). They run beside the forces, on a branch of the step graph, so that
+// neither the reduction nor the FP64 divisions lie on the step's chain.
+struct ThermoAux {
+    double bfac, rate;
+};
+
+__device__ __forceinline__ void thermo_aux(const Dev& d, double T, ThermoAux* aux)
+{
+    const RepDev& R = d.reps[0];
+    if (d.therm == NBG_THERMO_BERENDSEN) {
+        const double g = 0.5 / R.tparam;
+        aux->bfac = (1.0 / T == INFINITY) ? g : __dmul_rn(g, __dsub_rn(R.T0 / T, 1.0));
+    } else {
+        const double it = 1.0 / R.tparam;
+        aux->rate = __dmul_rn(__dmul_rn(it, it), __dsub_rn(T / R.T0, (R.ndf + 1.0) / R.ndf));
+    }
+}
+
+// from a temperature already in red_T (the run's first step)
+__global__ void k_thermo_aux(Dev d, ThermoAux* aux) { thermo_aux(d, d.red_T[0], aux); }
+
+// sum m v^2 in k_kick's order: elements by thread, the block's tree, block
+// partials by the last block
+__global__ void __launch_bounds__(256) k_kick_T(Dev d, const double* __restrict__ V, double* part, unsigned* counter,
+                                                ThermoAux* aux)
+{
+    const int64_t ncomp = 3 * d.n;
+    double acc = 0.0;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ncomp; e += (int64_t)gridDim.x * blockDim.x) {
+        const double vn = V[e];
+        acc += d.mass[e / 3] * (vn * vn);
+    }
+    __shared__ double sh[256];
+    sh[threadIdx.x] = acc;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
+    }
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = sh[0];
+        __threadfence();
+        last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += ((volatile double*)part)[b];
+    sh[threadIdx.x] = t;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const double T = sh[0] / (d.kb * d.reps[0].ndf);
+        d.red_T[0] = T;
+        *counter = 0u;
+        thermo_aux(d, T, aux);
+    }
+}
+
+// The drift, packing and displacement check of a step (k_drift_pack's
+// operations); KICK: before it the kick that ends the step before (k_kick's,
+// then k_andersen's) and the saved frame of that state. A thread per component, a warp per 10
+// atoms (lane 3 a + k; lanes 30 and 31 idle): a thread per atom had three
+// components' FP64 operations in one chain, each 64 cycles of its SM
+// sub-partition, and a third of the warps. The Nose-Hoover column is moved by
+// the block after the atoms'; the other blocks read zeta from zc_in, so that
+// it may be moved meanwhile (zc_out). One launch instead of up to four per
+// step (kick, Andersen, frame, drift): 10,976 LJ atoms 45 -> 36 us a step.
+#define VV_ATOMS 40  // atoms per block of 128 threads
+
+struct VVArgs {
+    double dt, dtsq;
+    StepRef step;   // KICK: the step that ends
+    StepRef pos;    // time index of the new positions
+    int check_disp;
+    int save;       // KICK: frames are saved
+    const double* zc_in;
+    double* zc_out;
+    const ThermoAux* aux;
+};
+
+template <bool KICK>
+__global__ void __launch_bounds__(128) k_vv(Dev d, StateView s, VVArgs A)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = lane % 3;
+    const int64_t blocks = (d.n + VV_ATOMS - 1) / VV_ATOMS;
+    int64_t slot = -1;  // the frame slot of the state after the kick
+    if (KICK && A.save) {
+        const FrameSink* sink = d.sink;
+        const int64_t every = sink->every;
+        const int64_t t = step_of(A.step) + 1 - sink->t0;
+        if (every > 0 && t % every == 0) {
+            const int64_t q = t / every - sink->first;
+            if (q >= 0 && q < sink->cap) slot = q;
+        }
+    }
+    if (blockIdx.x == blocks) {  // the Nose-Hoover column (thermostats.jl:121-128): dv = 0, v[zeta] = the rate
+        if (threadIdx.x < 3) {
+            const int64_t z = 3 * d.n + threadIdx.x;
+            double x = s.x[z], v = s.v[z], a = s.a_old[z];
+            if (KICK) {
+                a = 0.0;
+                s.a_old[z] = 0.0;
+                if (threadIdx.x == 0) {
+                    v = A.aux->rate;
+                    s.v[z] = v;
+                }
+                if (slot >= 0) {
+                    d.sink->x[slot * 3 * d.cols + z] = x;
+                    d.sink->v[slot * 3 * d.cols + z] = v;
+                }
+            }
+            x = drift1(x, v, a, A.dt, A.dtsq);
+            s.x[z] = x;
+            if (threadIdx.x == 0) *A.zc_out = x;
+        }
+        return;
+    }
+    const int64_t i = blockIdx.x * (int64_t)VV_ATOMS + w * 10 + lane / 3;
+    const bool active = lane < 30 && i < d.n;
+    const int64_t e = active ? 3 * i + k : 0;
+    double x = s.x[e], v = s.v[e], a = s.a_old[e];
+    if (KICK) {
+        double an = s.a_new[e];
+        if (d.therm == NBG_THERMO_BERENDSEN) an = __dadd_rn(an, __dmul_rn(A.aux->bfac, v));
+        else if (d.therm == NBG_THERMO_NOSEHOOVER) an = __dadd_rn(an, -__dmul_rn(*A.zc_in, v));
+        if (active && !finite64(an)) status_set(d.status, ST_NONFINITE);
+        v = kick1(v, a, an, A.dt);
+        a = an;
+        if (d.therm == NBG_THERMO_ANDERSEN) {
+            const int64_t step = step_of(A.step);
+            const RepDev& R = d.reps[0];
+            if (active && philox_u53(R.seed, (uint64_t)i, (uint64_t)step) < R.tparam * A.dt) {
+                const double m = d.kind == NBG_SYSTEM_WATER ? d.mass[i] : d.mass[0];
+                const double vdev = sqrt(d.kb * R.T0 / m);
+                double z[3];
+                philox_normals3<double>(R.seed, (uint64_t)i, (uint64_t)step, z);
+                v = vdev * (k == 0 ? z[0] : k == 1 ? z[1] : z[2]);
+            }
+        }
+        if (active) {
+            s.v[e] = v;
+            s.a_old[e] = a;
+            if (slot >= 0) {
+                d.sink->x[slot * 3 * d.cols + e] = x;
+                d.sink->v[slot * 3 * d.cols + e] = v;
+            }
+        }
+    }
+    x = drift1(x, v, a, A.dt, A.dtsq);
+    const RepDev& R = d.reps[0];
+    if (active) {
+        s.x[e] = x;
+        if (d.pfx) reinterpret_cast<unsigned*>(d.pfx + i)[k] = fx_coord(x, R.fx_scale);
+        if (!d.pfx || d.split_on) {
+            float h, l;
+            if (d.img && d.bc == NBG_BC_CUBIC) split_component_image(R, x, d.img[e], h, l);
+            else split_component(d, R, x, h, l);
+            reinterpret_cast<float*>(d.phi + i)[k] = h;
+            reinterpret_cast<float*>(d.plo + i)[k] = l;
+        }
+    }
+    if (!A.check_disp) return;
+    const double dk = x - d.xref[e];
+    const double dy = __shfl_down_sync(0xffffffffu, dk, 1), dz = __shfl_down_sync(0xffffffffu, dk, 2);
+    const double dx = dk;
+    const double d2 = dx * dx + dy * dy + dz * dz;
+    if (active && k == 0 && !(d2 <= d.skin_half2)) d.rebuild_flag[(int)(step_of(A.pos) & 1)] = 1;
+}
+
+// buf: [0..1] zeta by parity of the step in the run, then the ThermoAux
+static ThermoAux* vv_aux(nbg_ctx* c) { return reinterpret_cast<ThermoAux*>(c->vv_buf + 2); }
+
+// The step kernel of a captured run: drift to the positions of time index
+// pos, after (kick) the kick that ends step sr; k: the ending step's index in
+// the run, whose parity picks the zeta copies.
+int launch_vv(nbg_ctx* c, const StateView& s, double dt, bool kick, StepRef sr, StepRef pos, int64_t k)
+{
+    VVArgs A;
+    A.dt = dt;
+    A.dtsq = dt * dt;
+    A.step = sr;
+    A.pos = pos;
+    A.check_disp = c->path == PATH_LIST ? 1 : 0;
+    A.save = c->sink_on ? 1 : 0;
+    A.zc_in = c->vv_buf + (k & 1);
+    A.zc_out = c->vv_buf + (kick ? (k + 1) & 1 : k & 1);
+    A.aux = vv_aux(c);
+    const unsigned grid = (unsigned)((c->n + VV_ATOMS - 1) / VV_ATOMS) + (c->d.therm == NBG_THERMO_NOSEHOOVER ? 1u : 0u);
+    if (kick) k_vv<true><<<grid, 128, 0, c->stream>>>(c->d, s, A);
+    else k_vv<false><<<grid, 128, 0, c->stream>>>(c->d, s, A);
+    NBG_LAUNCH_CHECK(c, "k_vv");
+    return NBG_OK;
+}
+
+// The thermostat's scalars for the next kick on `stream`: reduced from v, or
+// (reduce = false) from the temperature in red_T.
+int launch_vv_thermo(nbg_ctx* c, const double* v, bool reduce, cudaStream_t stream)
+{
+    if (reduce) {
+        const int grid = std::min(grid_for(3 * c->n, 256), c->kick_blocks);
+        k_kick_T<<<grid, 256, 0, stream>>>(c->d, v, c->kick_part, c->kick_counter, vv_aux(c));
+    } else {
+        k_thermo_aux<<<1, 1, 0, stream>>>(c->d, vv_aux(c));
+    }
+    NBG_LAUNCH_CHECK(c, "k_kick_T");
+    return NBG_OK;
+}
+
 // The thermostat part of one RHS evaluation (nbg_accel): a_new += term(v);
 // Nose-Hoover also zeroes its column and writes the rate into v.
 __global__ void k_rhs_thermostat(Dev d, StateView s)

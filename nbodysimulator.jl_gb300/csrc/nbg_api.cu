@@ -747,6 +747,12 @@ static void release(nbg_ctx* c)
     c->hw = c->hw_d = nullptr;
     if (c->pend_ev) cudaEventDestroy(c->pend_ev);
     c->pend_ev = nullptr;
+    if (c->fork_ev) cudaEventDestroy(c->fork_ev);
+    if (c->join_ev) cudaEventDestroy(c->join_ev);
+    c->fork_ev = c->join_ev = nullptr;
+    if (c->side) cudaStreamDestroy(c->side);
+    c->side = nullptr;
+    c->vv_buf = nullptr;  // (one of allocs)
     if (c->frames) cudaFree(c->frames);
     c->frames = nullptr;
     c->frames_cap = 0;
@@ -1307,6 +1313,45 @@ static int step_vv(nbg_ctx* c, double dt, StepRef sr)
     return NBG_OK;
 }
 
+// Velocity-Verlet steps 0 .. G - 1 of a capture, each kick folded into the
+// next step's drift, the thermostat's temperature reduced on a branch beside
+// the forces. The last kick is the plain one, so that the state after a
+// replay is what single steps leave.
+static int steps_vv_fused(nbg_ctx* c, double dt, int64_t G)
+{
+    int st = NBG_OK;
+    const StateView& s = c->st;
+    const bool thermo_T = c->d.therm == NBG_THERMO_BERENDSEN || c->d.therm == NBG_THERMO_NOSEHOOVER;
+    for (int64_t k = 0; k < G; ++k) {
+        const StepRef sr{k, c->d.step_dev}, pos{k + 1, c->d.step_dev};
+        const StepRef prev{k - 1, c->d.step_dev};
+        if ((st = launch_vv(c, s, dt, k > 0, prev, pos, k > 0 ? k - 1 : 0))) return st;
+        const bool branch = thermo_T && k + 1 < G;  // (the last kick reads red_T alone)
+        if (thermo_T && k > 0) {
+            CK(cudaEventRecord(c->fork_ev, c->stream), "fork");
+            CK(cudaStreamWaitEvent(c->side, c->fork_ev, 0), "fork");
+            if ((st = launch_vv_thermo(c, s.v, true, c->side))) return st;
+            CK(cudaEventRecord(c->join_ev, c->side), "join");
+        } else if (branch) {
+            CK(cudaEventRecord(c->fork_ev, c->stream), "fork");
+            CK(cudaStreamWaitEvent(c->side, c->fork_ev, 0), "fork");
+            if ((st = launch_vv_thermo(c, s.v, false, c->side))) return st;
+            CK(cudaEventRecord(c->join_ev, c->side), "join");
+        }
+        const bool force = rebuild_due(c, true);
+        if ((st = forces(c, s, force, pos))) return st;
+        c->steps_since_build = force ? 0 : c->steps_since_build + 1;
+        if (thermo_T && (k > 0 || branch)) CK(cudaStreamWaitEvent(c->stream, c->join_ev, 0), "join");
+        if (k + 1 == G) {
+            if ((st = launch_kick(c, s, dt, thermo_T))) return st;
+            c->T_valid = thermo_T;
+            if (c->d.therm == NBG_THERMO_ANDERSEN && (st = launch_andersen(c, s, dt, sr))) return st;
+            if (c->sink_on && (st = launch_save_frame(c, s, sr))) return st;
+        }
+    }
+    return NBG_OK;
+}
+
 static int step_baoab(nbg_ctx* c, double dt, StepRef sr)
 {
     int st;
@@ -1395,6 +1440,14 @@ static int capture_graph(nbg_ctx* c, double dt)
         if (st0) return st0;
         c->T_valid = true;
     }
+    const bool fuse_vv = !is_em(c) && !c->baoab && c->nrep == 1 && c->path != PATH_GRAVITY;
+    if (fuse_vv && !c->vv_buf) {
+        int st0 = dalloc(c, &c->vv_buf, 4);
+        if (st0) return st0;
+        CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking), "side stream");
+        CK(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming), "fork event");
+        CK(cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming), "join event");
+    }
     const int64_t launches0 = c->launches;
     const int64_t ssb0 = c->steps_since_build;
     cudaGraph_t g = nullptr;
@@ -1402,7 +1455,8 @@ static int capture_graph(nbg_ctx* c, double dt)
     int st = NBG_OK;
     // (BAOAB without frames: each kick folded into the next step's drift)
     const bool fuse = c->baoab && !is_em(c) && !c->sink_on;
-    for (int64_t k = 0; k < G && st == NBG_OK; ++k)
+    if (fuse_vv) st = steps_vv_fused(c, dt, G);
+    for (int64_t k = 0; k < G && st == NBG_OK && !fuse_vv; ++k)
         st = fuse ? step_baoab_fused(c, dt, StepRef{k, c->d.step_dev}, k == 0, k == G - 1)
                   : step_any(c, dt, StepRef{k, c->d.step_dev});
     if (st == NBG_OK) st = launch_step_advance(c, G);

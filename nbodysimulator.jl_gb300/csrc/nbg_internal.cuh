@@ -350,6 +350,11 @@ struct nbg_ctx {
     unsigned* kick_counter = nullptr;
     int kick_blocks = 0;
     bool T_valid = false;        // red_T holds T of the resident velocities
+    // captured runs of velocity-Verlet steps: zeta copies and the thermostat's
+    // scalars, and the branch of the step graph that reduces them
+    double* vv_buf = nullptr;
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     int sms = 0;                 // multiprocessors of the device
     // constants of the list-based energy: LJ pairs, and sum of q_i q_j over
     // all non-excluded pairs (i < j)
@@ -419,6 +424,8 @@ int fx_prepare(nbg_ctx* c);
 int launch_force_fx(nbg_ctx* c, const StateView& s);
 int launch_bonded(nbg_ctx* c, const StateView& s);
 int launch_drift(nbg_ctx* c, const StateView& s, double dt, StepRef pos);
+int launch_vv(nbg_ctx* c, const StateView& s, double dt, bool kick, StepRef sr, StepRef pos, int64_t k);
+int launch_vv_thermo(nbg_ctx* c, const double* v, bool reduce, cudaStream_t stream);
 int launch_temperature(nbg_ctx* c, const double* v);
 int launch_kick(nbg_ctx* c, const StateView& s, double dt, bool do_T, bool thermo = true);
 int launch_andersen(nbg_ctx* c, const StateView& s, double dt, StepRef step);
@@ -692,38 +699,42 @@ __device__ __forceinline__ PairOut pair_cutoff(const Dev& d, const RepDev& R, co
     return o;
 }
 
-// Split a position into (hi, lo) floats (see the layout note above).
-__device__ __forceinline__ void split_position(const Dev& d, const RepDev& R, const double* p, float* h, float* l)
+// Split a position component into (hi, lo) floats (see the layout note above).
+__device__ __forceinline__ void split_component(const Dev& d, const RepDev& R, double p, float& h, float& l)
 {
     if (d.bc == NBG_BC_CUBIC) {
-        for (int k = 0; k < 3; ++k) {
-            double w = p[k] - R.L * floor(p[k] * R.invL);
-            if (w < 0.0) w += R.L;
-            if (w >= R.L) w -= R.L;
-            double hq = rint(w * (double)R.qscale) * (double)R.qinv;
-            h[k] = (float)hq;
-            l[k] = (float)(w - hq);
-        }
+        double w = p - R.L * floor(p * R.invL);
+        if (w < 0.0) w += R.L;
+        if (w >= R.L) w -= R.L;
+        double hq = rint(w * (double)R.qscale) * (double)R.qinv;
+        h = (float)hq;
+        l = (float)(w - hq);
     } else {
-        for (int k = 0; k < 3; ++k) {
-            h[k] = (float)p[k];
-            l[k] = (float)(p[k] - (double)h[k]);
-        }
+        h = (float)p;
+        l = (float)(p - (double)h);
     }
+}
+
+__device__ __forceinline__ void split_position(const Dev& d, const RepDev& R, const double* p, float* h, float* l)
+{
+    for (int k = 0; k < 3; ++k) split_component(d, R, p[k], h[k], l[k]);
 }
 
 // Split of a position shifted by a given periodic image, w = p - L img:
 // between list builds (img fixed at the build) w stays within skin/2 of the
 // box, well inside the exact range of the hi grid (|w| < 4 L).
+__device__ __forceinline__ void split_component_image(const RepDev& R, double p, double img, float& h, float& l)
+{
+    const double w = fma(-R.L, img, p);
+    const double hq = rint(w * (double)R.qscale) * (double)R.qinv;
+    h = (float)hq;
+    l = (float)(w - hq);
+}
+
 __device__ __forceinline__ void split_position_image(const RepDev& R, const double* p, const double* img, float* h,
                                                      float* l)
 {
-    for (int k = 0; k < 3; ++k) {
-        const double w = fma(-R.L, img[k], p[k]);
-        const double hq = rint(w * (double)R.qscale) * (double)R.qinv;
-        h[k] = (float)hq;
-        l[k] = (float)(w - hq);
-    }
+    for (int k = 0; k < 3; ++k) split_component_image(R, p[k], img[k], h[k], l[k]);
 }
 
 // Fixed-point box coordinate: x / L * 2^32 rounded, modulo 2^32 (the wrap

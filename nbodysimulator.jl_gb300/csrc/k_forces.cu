@@ -138,6 +138,20 @@ __device__ __forceinline__ void grav_tile(const float4* sh_hi, const float4* sh_
     }
 }
 
+// Box of a 128-body tile from those of its four runs of 32 bodies:
+// (min x, y, z, largest |r|) and (max x, y, z, smallest |r|).
+__device__ __forceinline__ void tile_box(const float4* __restrict__ box, int64_t t, float4& lo, float4& hi)
+{
+    lo = box[8 * t];
+    hi = box[8 * t + 1];
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+        const float4 a = box[8 * t + 2 * q], b = box[8 * t + 2 * q + 1];
+        lo = make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), fmaxf(lo.w, a.w));
+        hi = make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), fminf(hi.w, b.w));
+    }
+}
+
 // Grid: (i-block, j-chunk) units; each thread owns TI bodies i (strided by
 // GB within the block) and walks the chunk's j-tiles from shared memory:
 // every lane of a warp reads the same body j (one broadcast load serves TI
@@ -182,7 +196,8 @@ __global__ void __launch_bounds__(GB, TI == 2 ? 7 : 1) k_gravity(const float4* _
     for (int k = 0; k < TI; ++k) ax[k] = ay[k] = az[k] = Acc2{0.f, 0.f};
     // boxes and radial shells of the block's TI i-tiles
     __shared__ float4 ibox_s[2 * TI];
-    if (!PLAIN && box && threadIdx.x < 2 * TI) ibox_s[threadIdx.x] = box[2 * (ib0 / GB) + threadIdx.x];
+    if (!PLAIN && box && threadIdx.x < TI)
+        tile_box(box, ib0 / GB + threadIdx.x, ibox_s[2 * threadIdx.x], ibox_s[2 * threadIdx.x + 1]);
     constexpr unsigned ALL_FAR = (1u << TI) - 1u;
     __shared__ unsigned char far_s[GB];  // per j-tile of the next GB: bit k = far from i-tile k
     for (int64_t t = t0; t < t1; ++t) {
@@ -196,7 +211,8 @@ __global__ void __launch_bounds__(GB, TI == 2 ? 7 : 1) k_gravity(const float4* _
             const int64_t tt = t + threadIdx.x;
             unsigned f = 0;
             if (tt < t1) {
-                const float4 lo4 = box[2 * tt], hi4 = box[2 * tt + 1];
+                float4 lo4, hi4;
+                tile_box(box, tt, lo4, hi4);
 #pragma unroll
                 for (int k = 0; k < TI; ++k) {
                     const float4 a = ibox_s[2 * k], b = ibox_s[2 * k + 1];  // (min x,y,z, max|r|), (max x,y,z, min|r|)
@@ -327,13 +343,39 @@ __global__ void k_grav_keys(const double* __restrict__ X, int64_t n, const unsig
     }
 }
 
-// split positions and masses in sorted order (slot s holds body perm[s])
-__global__ void k_grav_pack_sorted(const double* __restrict__ X, const double* __restrict__ mass,
-                                   const int* __restrict__ perm, int64_t n, float4* phi, float4* plo)
+// The warp's box: (min x, y, z, largest |r|), (max x, y, z, smallest |r|) of
+// 32 bodies' hi positions (a lane without a body: an inverted box)
+__device__ __forceinline__ void warp_box(bool real, float x, float y, float z, float4* box)
 {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
+    float v[8];  // minima of x, y, z, -x, -y, -z, |r|, -|r|
+    if (real) {
+        const float r = sqrtf(x * x + y * y + z * z);
+        v[0] = x; v[1] = y; v[2] = z;
+        v[3] = -x; v[4] = -y; v[5] = -z;
+        v[6] = r; v[7] = -r;
+    } else {
+        for (int k = 0; k < 8; ++k) v[k] = INFINITY;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        for (int k = 0; k < 8; ++k) v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+    if ((threadIdx.x & 31) == 0) {
+        box[0] = make_float4(v[0], v[1], v[2], -v[7]);
+        box[1] = make_float4(-v[3], -v[4], -v[5], v[6]);
+    }
+}
+
+// split positions and masses in sorted order (slot s holds body perm[s]), and
+// the boxes of each 32 slots (128 threads per block, npad a multiple of 128)
+__global__ void __launch_bounds__(GB) k_grav_pack_sorted(const double* __restrict__ X, const double* __restrict__ mass,
+                                                         const int* __restrict__ perm, int64_t n, float4* phi, float4* plo,
+                                                         float4* box)
+{
+    const int64_t s = blockIdx.x * (int64_t)GB + threadIdx.x;
+    const bool real = s < n;
+    float h[3] = {0.f, 0.f, 0.f}, l[3];
+    if (real) {
         const int64_t i = perm[s];
-        float h[3], l[3];
         for (int k = 0; k < 3; ++k) {
             const double p = X[3 * i + k];
             h[k] = (float)p;
@@ -342,35 +384,75 @@ __global__ void k_grav_pack_sorted(const double* __restrict__ X, const double* _
         phi[s] = make_float4(h[0], h[1], h[2], (float)mass[i]);
         plo[s] = make_float4(l[0], l[1], l[2], 0.f);
     }
+    warp_box(real, h[0], h[1], h[2], box + 2 * (s / 32));
 }
 
-// per 128-body tile over its real bodies: box min (x, y, z, largest |r|) and
-// box max (x, y, z, smallest |r|) (an empty tile gets an inverted box)
-__global__ void __launch_bounds__(GB) k_grav_boxes(const float4* __restrict__ phi, int64_t n, float4* box)
+// One pass over the bodies between two gravity evaluations of a captured run
+// of steps: the sum of the chunk partials (KICK; k_gravity_reduce's
+// operations) and the kick that ends step sr (k_kick's, no thermostat), the
+// saved frame of that state, the next drift (k_drift_pack's), and (PACK: the
+// next evaluation keeps the order) the sorted split positions and boxes of
+// k_grav_pack_sorted. Block: 32 slots, warp k the component k, so that small
+// systems spread their FP64 operations over the chip (1500 bodies: 47 blocks)
+// and six launches per step become two.
+struct GravStep {
+    const double* part;
+    const int* perm;  // null: slot = body
+    int jchunks;
+    double G, dt, dtsq;
+    StepRef step;     // KICK: the step that ends
+    int save;
+    float4* box;      // null: none
+};
+
+template <bool KICK, bool PACK>
+__global__ void __launch_bounds__(96) k_grav_step(Dev d, StateView s, GravStep A)
 {
-    const int64_t s = blockIdx.x * (int64_t)GB + threadIdx.x;
-    float v[8];  // minima of x, y, z, -x, -y, -z, |r|, -|r|
-    if (s < n) {
-        const float4 h = phi[s];
-        const float r = sqrtf(h.x * h.x + h.y * h.y + h.z * h.z);
-        v[0] = h.x; v[1] = h.y; v[2] = h.z;
-        v[3] = -h.x; v[4] = -h.y; v[5] = -h.z;
-        v[6] = r; v[7] = -r;
-    } else {
-        for (int k = 0; k < 8; ++k) v[k] = INFINITY;
+    __shared__ float sh[3][32];
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    const int64_t slot = blockIdx.x * (int64_t)32 + lane;
+    const bool real = slot < d.n;
+    float h = 0.f;
+    if (real) {
+        const int64_t i = A.perm ? A.perm[slot] : slot;
+        const int64_t e = 3 * i + k;
+        double x = s.x[e], v = s.v[e], a = s.a_old[e];
+        if (KICK) {
+            double t = 0.0;
+            const double* p = A.part + 3 * slot + k;
+#pragma unroll 4
+            for (int c = 0; c < A.jchunks; ++c) t += p[(int64_t)c * 3 * d.n];
+            const double an = -A.G * t;
+            if (!finite64(an)) status_set(d.status, ST_NONFINITE);
+            v = kick1(v, a, an, A.dt);
+            a = an;
+            s.a_old[e] = an;
+            s.v[e] = v;
+            if (A.save) {
+                const FrameSink* sink = d.sink;
+                const int64_t every = sink->every;
+                const int64_t f = step_of(A.step) + 1 - sink->t0;
+                if (every > 0 && f % every == 0) {
+                    const int64_t q = f / every - sink->first;
+                    if (q >= 0 && q < sink->cap) {
+                        sink->x[q * 3 * d.cols + e] = x;
+                        sink->v[q * 3 * d.cols + e] = v;
+                    }
+                }
+            }
+        }
+        x = drift1(x, v, a, A.dt, A.dtsq);
+        s.x[e] = x;
+        if (PACK) {
+            h = (float)x;
+            reinterpret_cast<float*>(d.phi + slot)[k] = h;
+            reinterpret_cast<float*>(d.plo + slot)[k] = (float)(x - (double)h);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1)
-        for (int k = 0; k < 8; ++k) v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-    __shared__ float red[GB / 32][8];
-    if ((threadIdx.x & 31) == 0)
-        for (int k = 0; k < 8; ++k) red[threadIdx.x / 32][k] = v[k];
+    if (!PACK || !A.box) return;
+    sh[k][lane] = h;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < GB / 32; ++w)
-            for (int k = 0; k < 8; ++k) v[k] = fminf(v[k], red[w][k]);
-        box[2 * blockIdx.x] = make_float4(v[0], v[1], v[2], -v[7]);
-        box[2 * blockIdx.x + 1] = make_float4(-v[3], -v[4], -v[5], v[6]);
-    }
+    if (k == 0) warp_box(real, h, sh[1][lane], sh[2][lane], A.box + 2 * (int64_t)blockIdx.x);
 }
 
 // Number of j-chunks: the smallest that makes (i-blocks x chunks) fill the
@@ -401,51 +483,109 @@ static int plan_gravity(nbg_ctx* c, int64_t npad)
     return best;
 }
 
-// Launch the gravity kernel and the chunk reduction into s.a_new. The
-// partials (grav_chunks * n * 3 doubles) live in c->grav_part.
-int launch_gravity(nbg_ctx* c, const StateView& s)
+// Whether the next gravity evaluation sorts the bodies afresh (every 8th: the
+// bodies move little in between).
+static bool grav_sorts(const nbg_ctx* c) { return c->grav_sort && (!c->grav_perm_valid || c->grav_evals % 8 == 0); }
+
+// The order and the sorted split positions and boxes of the next evaluation;
+// packed: the positions and boxes are in place for the current order.
+static int gravity_order(nbg_ctx* c, const StateView& s, bool packed)
+{
+    if (!c->grav_sort) return NBG_OK;
+    if (grav_sorts(c)) {
+        packed = false;
+        cudaError_t me = cudaMemsetAsync(c->grav_extent, 0, sizeof(unsigned), c->stream);
+        if (me != cudaSuccess) return cuda_fail(c, me, "gravity extent clear");
+        k_grav_extent<<<2 * c->sms, 256, 0, c->stream>>>(s.x, 3 * c->n, c->grav_extent);
+        NBG_LAUNCH_CHECK(c, "k_grav_extent");
+        k_grav_keys<<<grid_for(c->n, 256), 256, 0, c->stream>>>(s.x, c->n, c->grav_extent, c->grav_keys[0],
+                                                                 c->grav_vals[0]);
+        NBG_LAUNCH_CHECK(c, "k_grav_keys");
+        size_t bytes = c->grav_sort_bytes;
+        cudaError_t e = cub::DeviceRadixSort::SortPairs(c->grav_sort_tmp, bytes, c->grav_keys[0], c->grav_keys[1],
+                                                        c->grav_vals[0], c->grav_vals[1], (int)c->n, 0, 63,
+                                                        c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "gravity Morton sort");
+        c->launches += 8;  // the sort's own passes
+        c->grav_perm_valid = true;
+    }
+    ++c->grav_evals;
+    if (!packed) {
+        k_grav_pack_sorted<<<(unsigned)(c->npad / GB), GB, 0, c->stream>>>(s.x, c->d.mass, c->grav_vals[1], c->n, c->d.phi,
+                                                                           c->d.plo, c->grav_box);
+        NBG_LAUNCH_CHECK(c, "k_grav_pack_sorted");
+    }
+    return NBG_OK;
+}
+
+// the pair sums of the packed positions into c->grav_part (grav_chunks * n * 3 doubles)
+static int gravity_pairs(nbg_ctx* c)
 {
     int64_t units = (c->npad / (grav_ti(c->grav_variant) * GB)) * c->grav_chunks;
     const bool uniform = c->grav_uniform && grav_variant_packed(c->grav_variant);
     grav_kernel_t kern = grav_variant(c->d.grav_plain, c->grav_variant, uniform);
-    const int* perm = nullptr;
-    if (c->grav_sort) {
-        // Morton sort (every 8th evaluation: the bodies move little in
-        // between), sorted split positions, tile boxes
-        if (!c->grav_perm_valid || c->grav_evals % 8 == 0) {
-            cudaError_t me = cudaMemsetAsync(c->grav_extent, 0, sizeof(unsigned), c->stream);
-            if (me != cudaSuccess) return cuda_fail(c, me, "gravity extent clear");
-            k_grav_extent<<<2 * c->sms, 256, 0, c->stream>>>(s.x, 3 * c->n, c->grav_extent);
-            NBG_LAUNCH_CHECK(c, "k_grav_extent");
-            k_grav_keys<<<grid_for(c->n, 256), 256, 0, c->stream>>>(s.x, c->n, c->grav_extent, c->grav_keys[0],
-                                                                     c->grav_vals[0]);
-            NBG_LAUNCH_CHECK(c, "k_grav_keys");
-            size_t bytes = c->grav_sort_bytes;
-            cudaError_t e = cub::DeviceRadixSort::SortPairs(c->grav_sort_tmp, bytes, c->grav_keys[0], c->grav_keys[1],
-                                                            c->grav_vals[0], c->grav_vals[1], (int)c->n, 0, 63,
-                                                            c->stream);
-            if (e != cudaSuccess) return cuda_fail(c, e, "gravity Morton sort");
-            c->launches += 8;  // the sort's own passes
-            c->grav_perm_valid = true;
-        }
-        ++c->grav_evals;
-        perm = c->grav_vals[1];
-        k_grav_pack_sorted<<<grid_for(c->n, 256), 256, 0, c->stream>>>(s.x, c->d.mass, perm, c->n, c->d.phi,
-                                                                          c->d.plo);
-        NBG_LAUNCH_CHECK(c, "k_grav_pack_sorted");
-        k_grav_boxes<<<(unsigned)(c->npad / GB), GB, 0, c->stream>>>(c->d.phi, c->n, c->grav_box);
-        NBG_LAUNCH_CHECK(c, "k_grav_boxes");
-    }
     prof_begin(c);
     kern<<<(unsigned)units, GB, 0, c->stream>>>(c->d.phi, c->d.plo, c->n, c->npad, c->grav_chunks, c->grav_part,
                                                 c->grav_sort ? c->grav_box : nullptr, c->grav_far2);
     prof_end(c);
     NBG_LAUNCH_CHECK(c, "k_gravity");
-    k_gravity_reduce<<<grid_for(3 * c->n, 256), 256, 0, c->stream>>>(c->grav_part, c->n, c->grav_chunks,
-                                                                      uniform ? c->d.G * c->grav_m0 : c->d.G,
-                                                                      s.a_new, c->d.status, perm);
+    return NBG_OK;
+}
+
+static double gravity_factor(const nbg_ctx* c)
+{
+    return c->grav_uniform && grav_variant_packed(c->grav_variant) ? c->d.G * c->grav_m0 : c->d.G;
+}
+
+static int gravity_reduce(nbg_ctx* c, const StateView& s)
+{
+    k_gravity_reduce<<<grid_for(3 * c->n, 256), 256, 0, c->stream>>>(c->grav_part, c->n, c->grav_chunks, gravity_factor(c),
+                                                                      s.a_new, c->d.status,
+                                                                      c->grav_sort ? c->grav_vals[1] : nullptr);
     NBG_LAUNCH_CHECK(c, "k_gravity_reduce");
     return NBG_OK;
+}
+
+// Order, pair sums and the chunk reduction into s.a_new.
+int launch_gravity(nbg_ctx* c, const StateView& s)
+{
+    int st;
+    if ((st = gravity_order(c, s, false))) return st;
+    if ((st = gravity_pairs(c))) return st;
+    return gravity_reduce(c, s);
+}
+
+// The gravity evaluation of step k of a captured run of steps after its
+// drift: (first) the drift alone, else the previous evaluation's reduction,
+// the kick that ends step sr and the drift in one pass; (last) the reduction
+// into s.a_new follows.
+int launch_gravity_step(nbg_ctx* c, const StateView& s, double dt, StepRef sr, bool first, bool last)
+{
+    GravStep A;
+    A.part = c->grav_part;
+    A.perm = c->grav_sort ? c->grav_vals[1] : nullptr;
+    A.jchunks = c->grav_chunks;
+    A.G = gravity_factor(c);
+    A.dt = dt;
+    A.dtsq = dt * dt;
+    A.step = sr;
+    A.save = c->sink_on ? 1 : 0;
+    A.box = c->grav_sort ? c->grav_box : nullptr;
+    const bool pack = !grav_sorts(c);
+    const unsigned grid = (unsigned)(c->npad / 32);
+    if (first && !c->grav_perm_valid) A.perm = nullptr;  // (no order yet: it sorts next)
+    if (first) {
+        if (pack) k_grav_step<false, true><<<grid, 96, 0, c->stream>>>(c->d, s, A);
+        else k_grav_step<false, false><<<grid, 96, 0, c->stream>>>(c->d, s, A);
+    } else {
+        if (pack) k_grav_step<true, true><<<grid, 96, 0, c->stream>>>(c->d, s, A);
+        else k_grav_step<true, false><<<grid, 96, 0, c->stream>>>(c->d, s, A);
+    }
+    NBG_LAUNCH_CHECK(c, "k_grav_step");
+    int st;
+    if ((st = gravity_order(c, s, pack))) return st;
+    if ((st = gravity_pairs(c))) return st;
+    return last ? gravity_reduce(c, s) : NBG_OK;
 }
 
 // scratch of the Morton sort (keys, values and cub's temporary storage) and

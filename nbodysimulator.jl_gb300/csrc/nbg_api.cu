@@ -613,7 +613,7 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
             unsigned char* tmp = nullptr;
             if ((st = dalloc(c, &tmp, c->grav_sort_bytes))) return st;
             c->grav_sort_tmp = tmp;
-            if ((st = dalloc(c, &c->grav_box, 2 * (c->npad / 128)))) return st;
+            if ((st = dalloc(c, &c->grav_box, 2 * (c->npad / 32)))) return st;
             if ((st = dalloc(c, &c->grav_extent, 1))) return st;
         }
     }
@@ -1352,6 +1352,23 @@ static int steps_vv_fused(nbg_ctx* c, double dt, int64_t G)
     return NBG_OK;
 }
 
+// The same for gravity without a thermostat: a pass over the bodies and the
+// pair kernel per step.
+static int steps_gravity_fused(nbg_ctx* c, double dt, int64_t G)
+{
+    int st;
+    for (int64_t k = 0; k < G; ++k) {
+        const StepRef prev{k - 1, c->d.step_dev}, sr{k, c->d.step_dev};
+        if ((st = launch_gravity_step(c, c->st, dt, prev, k == 0, k + 1 == G))) return st;
+        c->steps_since_build += 1;
+        if (k + 1 == G) {
+            if ((st = launch_kick(c, c->st, dt, false))) return st;
+            if (c->sink_on && (st = launch_save_frame(c, c->st, sr))) return st;
+        }
+    }
+    return NBG_OK;
+}
+
 static int step_baoab(nbg_ctx* c, double dt, StepRef sr)
 {
     int st;
@@ -1455,8 +1472,12 @@ static int capture_graph(nbg_ctx* c, double dt)
     int st = NBG_OK;
     // (BAOAB without frames: each kick folded into the next step's drift)
     const bool fuse = c->baoab && !is_em(c) && !c->sink_on;
+    // (the unsorted form packs positions wrapped under cubic boundaries: not in the fused pass)
+    const bool fuse_gravity = c->path == PATH_GRAVITY && c->d.therm == NBG_THERMO_NULL &&
+                              (c->grav_sort || c->d.bc != NBG_BC_CUBIC);
     if (fuse_vv) st = steps_vv_fused(c, dt, G);
-    for (int64_t k = 0; k < G && st == NBG_OK && !fuse_vv; ++k)
+    if (fuse_gravity) st = steps_gravity_fused(c, dt, G);
+    for (int64_t k = 0; k < G && st == NBG_OK && !fuse_vv && !fuse_gravity; ++k)
         st = fuse ? step_baoab_fused(c, dt, StepRef{k, c->d.step_dev}, k == 0, k == G - 1)
                   : step_any(c, dt, StepRef{k, c->d.step_dev});
     if (st == NBG_OK) st = launch_step_advance(c, G);

@@ -316,7 +316,7 @@ struct nbg_ctx {
     int* grav_vals[2] = {nullptr, nullptr};  // [1] = the permutation (slot -> body)
     void* grav_sort_tmp = nullptr;
     size_t grav_sort_bytes = 0;
-    float4* grav_box = nullptr;       // 2 per 128-body tile
+    float4* grav_box = nullptr;       // 2 per 32 slots
     int64_t grav_evals = 0;           // gravity evaluations issued (the sort runs on every 8th)
     bool grav_perm_valid = false;     // the permutation belongs to the positions being evaluated
     // block partials of nbg_energy
@@ -403,6 +403,7 @@ struct StepRef {
 
 int launch_pack(nbg_ctx* c, const StateView& s);
 int launch_gravity(nbg_ctx* c, const StateView& s);
+int launch_gravity_step(nbg_ctx* c, const StateView& s, double dt, StepRef sr, bool first, bool last);
 bool cluster_plan(nbg_ctx* c);
 // step0: the time index of the state at the launch (for the frame sink)
 // (status: the word the launch sets its bits in; the cluster loop also

@@ -65,17 +65,6 @@ static __device__ __noinline__ FxPair fx_pair_fallback(const Dev d, const double
 // Potential kinds of the fixed-point pair kernels (compile-time forms).
 enum { FX_LJ = 1, FX_EL = 2, FX_LJEL = 3, FX_WATER = 4 };
 
-// (h, e) += the partner lane's (h, e): TwoSum of the h parts, errors into e
-__device__ __forceinline__ void fx_join(float& h, float& e, int o, int width)
-{
-    const float h2 = __shfl_xor_sync(0xffffffffu, h, o, width);
-    const float e2 = __shfl_xor_sync(0xffffffffu, e, o, width);
-    float sum, err;
-    two_sum(h, h2, sum, err);
-    h = sum;
-    e = __fadd_rn(__fadd_rn(e, e2), err);
-}
-
 // One packed pair step (entries k0 and k0 + LPA of atom row a) of the
 // fixed-point kernels: classification, FP64 fallback, LJ and reaction-field
 // factors in the units of the LJ sum, accumulated into (px, py, pz). An

@@ -94,17 +94,6 @@ __device__ __forceinline__ void bulk_copy_to_peer(unsigned dst_cluster, unsigned
 
 #define CL_WAIT_TRIES (1u << 16)
 
-// (h, e) += the partner lane's (h, e), h by TwoSum with its error into e
-__device__ __forceinline__ void cl_join(float& h, float& e, int o, int width)
-{
-    const float h2 = __shfl_xor_sync(0xffffffffu, h, o, width);
-    const float e2 = __shfl_xor_sync(0xffffffffu, e, o, width);
-    float sum, err;
-    two_sum(h, h2, sum, err);
-    h = sum;
-    e = __fadd_rn(__fadd_rn(e, e2), err);
-}
-
 // Shared memory (dynamic): split positions [parity][hi, lo][n] (float4), the
 // own atoms' positions at the last list build [per][3] (double, padded to a 16-byte end), their lists
 // [per][cap], counts [per] (int) and force partials [per][6] (float: h, e per
@@ -142,29 +131,25 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     const double dtsq = dt * dt;
     const float magic = 12582912.0f;  // 1.5 * 2^23: rint by addition
 
-    // own atom k = tid keeps its state in the registers of thread k for the
-    // whole launch
-    const int ko = tid;
-    const bool owner = tid < na;
+    // component k of own atom ko keeps its state in the registers of one
+    // thread for the whole launch: 10 atoms a warp, lane 3 a + k (a thread
+    // per atom had the three components' FP64 in one chain on two warps)
+    const int k = (tid & 31) % 3;
+    const int ko = (tid >> 5) * 10 + (tid & 31) / 3;
+    const bool owner = (tid & 31) < 30 && ko < na;
     const int io = owner ? a0 + ko : 0;
-    double x[3], v[3], a[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        x[k] = owner ? (ACCEL ? src[3 * io + k] : s.x[3 * io + k]) : 0.0;
-        v[k] = owner && !ACCEL ? s.v[3 * io + k] : 0.0;
-        a[k] = owner && !ACCEL ? s.a_old[3 * io + k] : 0.0;
-    }
+    const size_t eo = 3 * (size_t)io + k;
+    double x = owner ? (ACCEL ? src[eo] : s.x[eo]) : 0.0;
+    double v = owner && !ACCEL ? s.v[eo] : 0.0;
+    double a = owner && !ACCEL ? s.a_old[eo] : 0.0;
     const double im_o = owner ? d.inv_mass[io] : 0.0;
     if (owner && !ACCEL) {
         // the backup of the launch's start (x, v, a_old segments of 3 cols):
         // a timed-out or overflowed launch is undone from it
         const size_t seg = 3 * (size_t)d.cols;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            bk[3 * io + k] = x[k];
-            bk[seg + 3 * io + k] = v[k];
-            bk[2 * seg + 3 * io + k] = a[k];
-        }
+        bk[eo] = x;
+        bk[seg + eo] = v;
+        bk[2 * seg + eo] = a;
     }
 
     // the static w parts (charge, atom flags) of every atom in both parities
@@ -211,33 +196,22 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
         if constexpr (ACCEL) {
             if (owner && st > 0) {
                 // the right-hand side: the acceleration of the source positions
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const double an = ((double)fsum[6 * ko + 2 * k] + (double)fsum[6 * ko + 2 * k + 1]) * im_o;
-                    if (!finite64(an)) status_set(d.status, ST_NONFINITE);
-                    dst[3 * io + k] = an;
-                }
+                const double an = (widen(fsum[6 * ko + 2 * k]) + widen(fsum[6 * ko + 2 * k + 1])) * im_o;
+                if (!finite64(an)) status_set(d.status, ST_NONFINITE);
+                dst[eo] = an;
             }
         } else if (owner && st > 0) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double an = ((double)fsum[6 * ko + 2 * k] + (double)fsum[6 * ko + 2 * k + 1]) * im_o;
-                if (!finite64(an)) status_set(d.status, ST_NONFINITE);
-                v[k] = kick1(v[k], a[k], an, dt);
-                a[k] = an;
-            }
+            const double an = (widen(fsum[6 * ko + 2 * k]) + widen(fsum[6 * ko + 2 * k + 1])) * im_o;
+            if (!finite64(an)) status_set(d.status, ST_NONFINITE);
+            v = kick1(v, a, an, dt);
+            a = an;
             if (sk_every > 0 && (step0 + st - sk_t0) % sk_every == 0) {
                 const FrameSink* sk = d.sink;
                 const int64_t slot = (step0 + st - sk_t0) / sk_every - sk->first;
                 if (slot >= 0 && slot < sk->cap) {
-                    const size_t o = (size_t)slot * 3 * d.cols + 3 * (size_t)io;
-                    double* fx = sk->x;
-                    double* fv = sk->v;
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        fx[o + k] = x[k];
-                        fv[o + k] = v[k];
-                    }
+                    const size_t o = (size_t)slot * 3 * d.cols + eo;
+                    sk->x[o] = x;
+                    sk->v[o] = v;
                 }
             }
         }
@@ -247,23 +221,21 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
         float4* pl = ph + n;
         double* X = xb + (size_t)par * 3 * n;  // FP64 positions of this step
         // drift, split and displacement check of the own atoms
-        bool moved = false;
+        double dk = 0.0;
         if (owner) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (!ACCEL) x[k] = drift1(x[k], v[k], a[k], dt, dtsq);
-                X[3 * io + k] = x[k];
-            }
-            float h[3], l[3];
-            split_position(d, R, x, h, l);
-            ph[io] = make_float4(h[0], h[1], h[2], ph[io].w);
-            pl[io] = make_float4(l[0], l[1], l[2], pl[io].w);
+            if (!ACCEL) x = drift1(x, v, a, dt, dtsq);
+            X[eo] = x;
+            float h, l;
+            split_component(d, R, x, h, l);
+            reinterpret_cast<float*>(ph + io)[k] = h;
+            reinterpret_cast<float*>(pl + io)[k] = l;
             // (a launch that does not reuse lists builds at step 0, which
             // sets xref_s)
-            const double* xr = xref_s + 3 * ko;
-            const double dx = x[0] - xr[0], dy = x[1] - xr[1], dz = x[2] - xr[2];
-            moved = (st > 0 || reuse) && !(dx * dx + dy * dy + dz * dz <= d.skin_half2);
+            dk = x - xref_s[3 * ko + k];
         }
+        const double dy = __shfl_down_sync(0xffffffffu, dk, 1), dz = __shfl_down_sync(0xffffffffu, dk, 2);
+        const bool moved =
+            owner && k == 0 && (st > 0 || reuse) && !(dk * dk + dy * dy + dz * dz <= d.skin_half2);
         // the owners' generic writes become visible to the bulk-copy engine
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         const int any_moved = __syncthreads_or(moved ? 1 : 0);
@@ -356,10 +328,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
                 }
                 cnt[g] = c0;
             }
-            if (owner) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) xref_s[3 * ko + k] = x[k];
-            }
+            if (owner) xref_s[3 * ko + k] = x;
             since = 0;
             built = true;
             __syncthreads();
@@ -383,17 +352,11 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
                 py += o.fy;
                 pz += o.fz;
             }
-            float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll
-            for (int o = LPA / 2; o > 0; o >>= 1) {
-                cl_join(px, ex, o, LPA);
-                cl_join(py, ey, o, LPA);
-                cl_join(pz, ez, o, LPA);
-            }
+            const LaneSum f = lane_sums3<LPA>(px, py, pz, lane);
             if (range_err) status_set(d.status, ST_RANGE);
-            if (active && lane == 0) {
-                float* f = fsum + 6 * g;
-                f[0] = px; f[1] = ex; f[2] = py; f[3] = ey; f[4] = pz; f[5] = ez;
+            if (active && f.writer) {
+                fsum[6 * g + 2 * f.comp] = f.h;
+                fsum[6 * g + 2 * f.comp + 1] = f.e;
             }
         }
         // the next kick and drift touch only this CTA's own atoms: a block
@@ -404,13 +367,10 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     // this barrier no copy reads a CTA's shared memory any more: all may exit
     cl.sync();
     if (owner && !ACCEL) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            s.x[3 * io + k] = x[k];
-            s.v[3 * io + k] = v[k];
-            s.a_old[3 * io + k] = a[k];
-            d.xref[3 * io + k] = xref_s[3 * ko + k];
-        }
+        s.x[eo] = x;
+        s.v[eo] = v;
+        s.a_old[eo] = a;
+        d.xref[eo] = xref_s[3 * ko + k];
     }
     // the lists for the next launch, if this one built them (with their own
     // reference positions: d.xref also serves the global lists, which other

@@ -16,17 +16,7 @@
 #define EJ 32        // bodies j per block of k_energy_pairs
 #define EL_WARPS 8   // warps per block of k_energy_list
 
-// FP64 issues at 2 lanes per clock and SM here (a warp instruction holds its
-// SM sub-partition for 64 cycles), so these kernels are bound by their count
-// of FP64 instructions; comparisons and conversions count like any other.
-
-// The exact FP64 value of a float, by integer operations where it is normal.
-__device__ __forceinline__ double widen(float f)
-{
-    const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
-    if (m - 0x00800000u >= 0x7f000000u) return (double)f;  // zero, subnormal, infinite or NaN
-    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
-}
+// These kernels are bound by their count of FP64 instructions.
 
 // 1 / sqrt(x) to ~1 ulp: the FP32 approximation (2^-22) refined by one
 // third-order step, y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2 (error ~e^3);

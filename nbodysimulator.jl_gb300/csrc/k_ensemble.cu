@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                 for (int k = 0; k < 3; ++k) {
                     const double vh = fma(hdt, ao[k], v[k]);
                     const double xh = fma(hdt, vh, x[k]);
-                    const double vo = fma(c1, vh, sd * (double)z[k]);
+                    const double vo = fma(c1, vh, sd * widen(z[k]));
                     x[k] = fma(hdt, vo, xh);
                     v[k] = vo;
                 }
@@ -380,7 +380,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
         const bool lj_atoms = POT != FX_EL;
         const float lj_lo = R.fx_lj_lo, lj_hi = R.fx_lj_hi, el_lo = R.fx_el_lo, el_hi = R.fx_el_hi;
         const float sig2h = R.fx_sig2_hi, sig2l = R.fx_sig2_lo, krf = R.fx_krf;
-        const double fscale = R.fx_fscale;
         for (int i0 = 0; i0 < n; i0 += G) {
             const int i = i0 + g;
             const bool active = i < n;
@@ -390,11 +389,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
             const int cmax = __reduce_max_sync(0xffffffffu, cnt);  // the warp's longest row
             const float kqi =
                 POT != FX_LJ ? (float)(d.charge[gi] * R.fx_kq) : 0.0f;
-            // the velocity update's operands (lane k < 3: component k) are
-            // loaded ahead of the pair loop
-            const bool upd = active && lane < 3;
-            const int64_t e = 3 * gi + (lane < 3 ? lane : 0);
-            const double im = d.inv_mass[gi] * fscale;
+            // the velocity update's operands (one lane per component, as
+            // lane_sums3 leaves them) are loaded ahead of the pair loop
+            const int comp = min(lane / (LPA / 4), 2);
+            const bool upd = active && lane == comp * (LPA / 4);
+            const int64_t e = 3 * gi + comp;
+            const double im = d.inv_mass_fx[gi];
             const double v_in = upd ? s.v[e] : 0.0;
             const double ao_in = upd && !A.baoab ? s.a_old[e] : 0.0;
             const uint4* row = reinterpret_cast<const uint4*>(rows + gi * 2 * cap) + lane;
@@ -425,19 +425,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
                 }
             }
             float hx = __fadd_rn(px.x, px.y), hy = __fadd_rn(py.x, py.y), hz = __fadd_rn(pz.x, pz.y);
-            float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll
-            for (int o = LPA / 2; o > 0; o >>= 1) {
-                fx_join(hx, ex, o, LPA);
-                fx_join(hy, ey, o, LPA);
-                fx_join(hz, ez, o, LPA);
-            }
-            // every lane of the group holds the joined sums: lane k updates
-            // component k (a third of the FP64 instructions of one lane
-            // updating all three; FP64 issues at 2 lanes per clock here)
+            // a lane per component updates the velocity
+            const LaneSum f = lane_sums3<LPA>(hx, hy, hz, lane);
             if (upd) {
-                const float h = lane == 0 ? hx : lane == 1 ? hy : hz, el = lane == 0 ? ex : lane == 1 ? ey : ez;
-                const double an = ((double)h + (double)el) * im;
+                const double an = (widen(f.h) + widen(f.e)) * im;
                 if (!finite64(an)) status_set(d.status, ST_NONFINITE);
                 const double vn = A.baoab ? __dadd_rn(v_in, __dmul_rn(hdt, an)) : kick1(v_in, ao_in, an, dt);
                 s.v[e] = vn;

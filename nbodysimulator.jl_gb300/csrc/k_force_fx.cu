@@ -24,8 +24,8 @@
 // into the other of two shared-memory stages, completing on that stage's
 // mbarrier; the block meanwhile computes the current tile from its stage.
 // LPA lanes per atom take two entries per iteration (packed FP32x2 for the
-// arithmetic), keep FP32 partials, and join them by the compensated
-// butterfly of the split-form kernel; one FP64 multiply by 1/m per component.
+// arithmetic), keep FP32 partials, and join them as lane_sums3 does; one FP64
+// add and multiply for all three components.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(FX_THREADS) k_force_fx(Dev d, StateView s, con
         const int64_t ia = active ? i : 0;
         const RepDev& R = d.reps[d.rep_of[ia]];
         const uint4 qi = d.pfx[ia];
+        const double im = d.inv_mass_fx[ia];
         const int cnt = active ? min(min(d.nbr_count[ia], d.nbr_cap), s_nbox[st] * 32) : 0;
         const bool lj_i = HAS_LJ && (POT != FX_WATER || (ia % 3) == 0);
         // k q_i / (u^2 fscale): rinv^3 in box units times this is the
@@ -247,21 +248,11 @@ __global__ void __launch_bounds__(FX_THREADS) k_force_fx(Dev d, StateView s, con
         }
         // forces: the two halves, then the lanes
         float hx = __fadd_rn(px.x, px.y), hy = __fadd_rn(py.x, py.y), hz = __fadd_rn(pz.x, pz.y);
-        float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll
-        for (int o = LPA / 2; o > 0; o >>= 1) {
-            fx_join(hx, ex, o, LPA);
-            fx_join(hy, ey, o, LPA);
-            fx_join(hz, ez, o, LPA);
-        }
-        if (active && lane == 0) {
-            const double im = d.inv_mass[i] * R.fx_fscale;
-            const double a0 = ((double)hx + (double)ex) * im, a1 = ((double)hy + (double)ey) * im,
-                         a2 = ((double)hz + (double)ez) * im;
-            if (!finite64(a0) || !finite64(a1) || !finite64(a2)) status_set(d.status, ST_NONFINITE);
-            s.a_new[3 * i] = a0;
-            s.a_new[3 * i + 1] = a1;
-            s.a_new[3 * i + 2] = a2;
+        const LaneSum f = lane_sums3<LPA>(hx, hy, hz, lane);
+        const double acc = (widen(f.h) + widen(f.e)) * im;
+        if (active && f.writer) {
+            if (!finite64(acc)) status_set(d.status, ST_NONFINITE);
+            s.a_new[3 * i + f.comp] = acc;
         }
         __syncthreads();  // the stage is read; the next-but-one tile may overwrite it
     }
@@ -366,6 +357,7 @@ __global__ void __launch_bounds__(FXW_WARPS * 32, (LPA <= 4 && POT == FX_LJ) ? 4
         const int64_t ia = active ? i : 0;
         const RepDev& R = d.reps[d.rep_of[ia]];
         const uint4 qi = d.pfx[ia];
+        const double im = d.inv_mass_fx[ia];
         const int cnt = active ? min(d.nbr_count[ia], d.nbr_cap) : 0;
         const bool lj_i = HAS_LJ && (POT != FX_WATER || (ia % 3) == 0);
         const float kqi =
@@ -429,21 +421,11 @@ __global__ void __launch_bounds__(FXW_WARPS * 32, (LPA <= 4 && POT == FX_LJ) ? 4
         }
         if (timeout) break;
         float hx = __fadd_rn(px.x, px.y), hy = __fadd_rn(py.x, py.y), hz = __fadd_rn(pz.x, pz.y);
-        float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll
-        for (int o = LPA / 2; o > 0; o >>= 1) {
-            fx_join(hx, ex, o, LPA);
-            fx_join(hy, ey, o, LPA);
-            fx_join(hz, ez, o, LPA);
-        }
-        if (active && lane == 0) {
-            const double im = d.inv_mass[i] * R.fx_fscale;
-            const double a0 = ((double)hx + (double)ex) * im, a1 = ((double)hy + (double)ey) * im,
-                         a2 = ((double)hz + (double)ez) * im;
-            if (!finite64(a0) || !finite64(a1) || !finite64(a2)) status_set(d.status, ST_NONFINITE);
-            s.a_new[3 * i] = a0;
-            s.a_new[3 * i + 1] = a1;
-            s.a_new[3 * i + 2] = a2;
+        const LaneSum f = lane_sums3<LPA>(hx, hy, hz, lane);
+        const double acc = (widen(f.h) + widen(f.e)) * im;
+        if (active && f.writer) {
+            if (!finite64(acc)) status_set(d.status, ST_NONFINITE);
+            s.a_new[3 * i + f.comp] = acc;
         }
     }
     if (range_err) status_set(d.status, ST_RANGE);

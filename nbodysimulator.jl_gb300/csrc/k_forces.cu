@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(96) k_grav_step(Dev d, StateView s, GravStep A
         if (PACK) {
             h = (float)x;
             reinterpret_cast<float*>(d.phi + slot)[k] = h;
-            reinterpret_cast<float*>(d.plo + slot)[k] = (float)(x - (double)h);
+            reinterpret_cast<float*>(d.plo + slot)[k] = (float)(x - widen(h));
         }
     }
     if (!PACK || !A.box) return;
@@ -1180,17 +1180,6 @@ __global__ void __launch_bounds__(128) k_force_list(Dev d, StateView s)
     }
 }
 
-// (h, e) += the partner lane's (h, e), h by TwoSum with its error into e
-__device__ __forceinline__ void lane_join(float& h, float& e, int o, int width)
-{
-    const float h2 = __shfl_xor_sync(0xffffffffu, h, o, width);
-    const float e2 = __shfl_xor_sync(0xffffffffu, e, o, width);
-    float sum, err;
-    two_sum(h, h2, sum, err);
-    h = sum;
-    e = __fadd_rn(__fadd_rn(e, e2), err);
-}
-
 // LPA lanes per atom over a row-major list: the group reads its atom's
 // entries coalesced, each lane keeps an FP32 partial of every LPA-th entry,
 // and the partials are joined by a compensated FP32 xor butterfly of shuffles
@@ -1228,24 +1217,12 @@ __global__ void __launch_bounds__(256) k_force_list_lanes(Dev d, StateView s)
     };
     if constexpr (LPA <= 4) pair_loop(PairK(R));
     else pair_loop(R);
-    // join the lanes' partials: compensated FP32 butterfly (TwoSum; every
-    // lane ends with the same value, whatever the order of its operands)
-    float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll
-    for (int o = LPA / 2; o > 0; o >>= 1) {
-        lane_join(px, ex, o, LPA);
-        lane_join(py, ey, o, LPA);
-        lane_join(pz, ez, o, LPA);
-    }
+    const LaneSum f = lane_sums3<LPA>(px, py, pz, lane);
     if (range_err) status_set(d.status, ST_RANGE);
-    if (active && lane == 0) {
-        const double im = d.inv_mass[i];
-        const double a0 = ((double)px + (double)ex) * im, a1 = ((double)py + (double)ey) * im,
-                     a2 = ((double)pz + (double)ez) * im;
-        if (!finite64(a0) || !finite64(a1) || !finite64(a2)) status_set(d.status, ST_NONFINITE);
-        s.a_new[3 * i] = a0;
-        s.a_new[3 * i + 1] = a1;
-        s.a_new[3 * i + 2] = a2;
+    if (active && f.writer) {
+        const double acc = (widen(f.h) + widen(f.e)) * d.inv_mass[i];
+        if (!finite64(acc)) status_set(d.status, ST_NONFINITE);
+        s.a_new[3 * i + f.comp] = acc;
     }
 }
 

@@ -598,7 +598,7 @@ __global__ void k_baoab_drift(Dev d, StateView s, double dt, StepRef sr)
             const int64_t e = 3 * i + k;
             const double vh = fma(hdt, s.a_old[e], s.v[e]);
             const double x = fma(hdt, vh, s.x[e]);
-            const double vo = fma(c1, vh, sd * (double)z[k]);
+            const double vo = fma(c1, vh, sd * widen(z[k]));
             s.x[e] = fma(hdt, vo, x);
             s.v[e] = vo;
         }
@@ -636,7 +636,7 @@ __global__ void k_baoab_kick_drift(Dev d, StateView s, double dt, StepRef sr)
             s.a_old[e] = an;
             const double vh = fma(hdt, an, v);
             const double x = fma(hdt, vh, s.x[e]);
-            const double vo = fma(c1, vh, sd * (double)z[k]);
+            const double vo = fma(c1, vh, sd * widen(z[k]));
             s.x[e] = fma(hdt, vo, x);
             s.v[e] = vo;
         }

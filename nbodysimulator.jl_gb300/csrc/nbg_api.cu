@@ -314,7 +314,7 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
             R.invL = 1.0 / L;
             int e = (int)std::ceil(std::log2(L));
             int k = 22 - e;
-            R.qscale = (float)std::ldexp(1.0, k);
+            R.qmagic = std::ldexp(1.5, 52 - k);
             R.qinv = (float)std::ldexp(1.0, -k);
             double Lh = std::rint(L * std::ldexp(1.0, k)) * std::ldexp(1.0, -k);
             R.Lh = (float)Lh;
@@ -445,6 +445,13 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
         if ((st = dalloc(c, &rp, n))) return st;
         D.rsqrt_mass = rp;
         CK(cudaMemcpy(rp, rs.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "rsqrt_mass upload");
+    }
+    if (c->path == PATH_LIST && d0->bc == NBG_BC_CUBIC) {
+        std::vector<double> f(n);
+        for (int64_t i = 0; i < n; ++i) f[i] = im[i] * c->reps_h[rep_of[i]].fx_fscale;
+        if ((st = dalloc(c, &dp, n))) return st;
+        D.inv_mass_fx = dp;
+        CK(cudaMemcpy(dp, f.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "inv_mass_fx upload");
     }
     if ((st = dalloc(c, &dp, n))) return st;
     D.charge = dp;

@@ -79,7 +79,8 @@ struct RepDev {
     double box[6];      // general periodic box (lo,hi per axis)
     float Lh, Ll;       // L split on the hi grid: L = Lh + Ll
     float invLf;
-    float qscale, qinv; // 2^k and 2^-k of the hi grid
+    float qinv;         // 2^-k of the hi grid
+    double qmagic;      // 1.5 * 2^(52 - k)
     float lj_lo, lj_hi; // FP32 r^2 below lo: inside; >= hi: outside; else exact
     float el_lo, el_hi;
     float rl2;          // Verlet-list radius^2 (inflated)
@@ -147,6 +148,7 @@ struct Dev {
     const double* mass;
     const double* inv_mass;
     const double* rsqrt_mass;     // 1 / sqrt(m)
+    const double* inv_mass_fx;    // fx_fscale / m (list path, cubic; else null)
     const double* charge;
     const double* dipole;
     const int* rep_of;
@@ -524,6 +526,31 @@ __device__ __forceinline__ bool finite64(double x)
     return (__double_as_longlong(x) & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
 }
 
+// FP64 issues at 2 lanes per clock and SM here: a warp instruction holds its
+// SM sub-partition for 64 cycles whatever its mask (comparisons 98, floor and
+// rint 142, conversions to and from FP32 32 and 64). The three helpers below
+// do by integer operations what needs no FP64 arithmetic, to the same bits.
+
+// the exact FP64 value of a float
+__device__ __forceinline__ double widen(float f)
+{
+    const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+    if (m - 0x00800000u >= 0x7f000000u && m != 0u) return (double)f;  // subnormal, infinite or NaN
+    const unsigned hi = m ? (m >> 3) + 0x38000000u : 0u;
+    return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(b << 29));
+}
+
+// x / 2 (exact)
+__device__ __forceinline__ double half64(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), e = hi & 0x7ff00000u;
+    if (e - 0x00200000u >= 0x7fd00000u) return __dmul_rn(0.5, x);  // zero, small, infinite or NaN
+    return __hiloint2double((int)(hi - 0x00100000u), __double2loint(x));
+}
+
+// x < 0 (a negative zero is not)
+__device__ __forceinline__ bool negative64(double x) { return __double_as_longlong(x) > (long long)0x8000000000000000ull && __double2hiint(x) < 0; }
+
 // The reference's get_interparticle_distance in FP64, no contraction
 // (boundary_conditions.jl:111-172). Returns false when a while loop exceeded
 // MINIMAGE_MAX_ITERS (non-finite or absurdly distant coordinates).
@@ -700,19 +727,28 @@ __device__ __forceinline__ PairOut pair_cutoff(const Dev& d, const RepDev& R, co
     return o;
 }
 
+// w rounded to the hi grid of 2^-k (w + M with M = 1.5 * 2^(52-k): the sum's
+// unit is the grid's) and the remainder; the grid's integer comes from the
+// sum's low word.
+__device__ __forceinline__ void grid_split(const RepDev& R, double w, float& h, float& l)
+{
+    const double t = __dadd_rn(w, R.qmagic);
+    h = (float)__double2loint(t) * R.qinv;
+    l = (float)(w - __dsub_rn(t, R.qmagic));
+}
+
 // Split a position component into (hi, lo) floats (see the layout note above).
 __device__ __forceinline__ void split_component(const Dev& d, const RepDev& R, double p, float& h, float& l)
 {
     if (d.bc == NBG_BC_CUBIC) {
         double w = p - R.L * floor(p * R.invL);
-        if (w < 0.0) w += R.L;
-        if (w >= R.L) w -= R.L;
-        double hq = rint(w * (double)R.qscale) * (double)R.qinv;
-        h = (float)hq;
-        l = (float)(w - hq);
+        if (negative64(w)) w += R.L;
+        // (w >= 0 here, or NaN: doubles of one sign compare as integers)
+        if (__double_as_longlong(w) >= __double_as_longlong(R.L)) w -= R.L;
+        grid_split(R, w, h, l);
     } else {
         h = (float)p;
-        l = (float)(p - (double)h);
+        l = (float)(p - widen(h));
     }
 }
 
@@ -726,10 +762,7 @@ __device__ __forceinline__ void split_position(const Dev& d, const RepDev& R, co
 // box, well inside the exact range of the hi grid (|w| < 4 L).
 __device__ __forceinline__ void split_component_image(const RepDev& R, double p, double img, float& h, float& l)
 {
-    const double w = fma(-R.L, img, p);
-    const double hq = rint(w * (double)R.qscale) * (double)R.qinv;
-    h = (float)hq;
-    l = (float)(w - hq);
+    grid_split(R, fma(-R.L, img, p), h, l);
 }
 
 __device__ __forceinline__ void split_position_image(const RepDev& R, const double* p, const double* img, float* h,
@@ -779,13 +812,13 @@ __device__ __forceinline__ void pack_atom(const Dev& d, int64_t i, const double*
 // no contracted multiply-add (the reference's arithmetic).
 __device__ __forceinline__ double drift1(double u, double v, double a, double dt, double dtsq)
 {
-    return __dadd_rn(__dadd_rn(u, __dmul_rn(dt, v)), __dmul_rn(dtsq, __dmul_rn(0.5, a)));
+    return __dadd_rn(__dadd_rn(u, __dmul_rn(dt, v)), __dmul_rn(dtsq, half64(a)));
 }
 
 // Velocity-Verlet kick of one component, v' = v + dt (a/2 + a'/2).
 __device__ __forceinline__ double kick1(double v, double a, double an, double dt)
 {
-    return __dadd_rn(v, __dmul_rn(dt, __dadd_rn(__dmul_rn(0.5, a), __dmul_rn(0.5, an))));
+    return __dadd_rn(v, __dmul_rn(dt, __dadd_rn(half64(a), half64(an))));
 }
 
 // TwoSum: s + e = a + b exactly (Knuth).
@@ -794,6 +827,57 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
     s = __fadd_rn(a, b);
     float bb = __fsub_rn(s, a);
     e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+// Compensated sums over W lanes of three components: each level joins a lane's
+// (h, e) with its partner's (h by TwoSum, the errors into e, as a butterfly
+// of all three components would), but the first level leaves two components
+// on the lower half of the lanes and one on the upper, the second one
+// component per lane: 2 + 1 + 1 .. joins instead of 3 per level, and the
+// components end on different lanes, ready for FP64 arithmetic on all three
+// at once. The values equal the full butterfly's (a join does not depend on
+// its operands' order). W a power of two >= 4; lane: within the W.
+struct LaneSum {
+    float h, e;
+    int comp;     // component of this lane's sum
+    bool writer;  // one lane per component
+};
+
+__device__ __forceinline__ void lane_add(float& h, float& e, float h2, float e2)
+{
+    float s, err;
+    two_sum(h, h2, s, err);
+    h = s;
+    e = __fadd_rn(__fadd_rn(e, e2), err);
+}
+
+template <int W>
+__device__ __forceinline__ LaneSum lane_sums3(float x, float y, float z, int lane)
+{
+    static_assert(W >= 4 && W <= 32, "lanes");
+    const bool up = (lane & (W / 2)) != 0, odd = (lane & (W / 4)) != 0;
+    // the lower half keeps x and y, the upper z (its second slot is unused)
+    float a = up ? z : x, b = y, ea = 0.f, eb = 0.f;
+    const float ra = __shfl_xor_sync(0xffffffffu, up ? x : z, W / 2, W), rb = __shfl_xor_sync(0xffffffffu, y, W / 2, W);
+    lane_add(a, ea, ra, 0.f);
+    lane_add(b, eb, rb, 0.f);
+    // the lower half's lanes keep one of x and y
+    LaneSum o;
+    const bool sel = !up && odd;  // keeps y
+    o.h = sel ? b : a;
+    o.e = sel ? eb : ea;
+    const bool snd = !up && !odd;  // sends y
+    const float rh = __shfl_xor_sync(0xffffffffu, snd ? b : a, W / 4, W),
+                re = __shfl_xor_sync(0xffffffffu, snd ? eb : ea, W / 4, W);
+    lane_add(o.h, o.e, rh, re);
+#pragma unroll
+    for (int k = W / 8; k > 0; k >>= 1) {
+        const float h2 = __shfl_xor_sync(0xffffffffu, o.h, k, W), e2 = __shfl_xor_sync(0xffffffffu, o.e, k, W);
+        lane_add(o.h, o.e, h2, e2);
+    }
+    o.comp = up ? 2 : odd ? 1 : 0;
+    o.writer = lane == o.comp * (W / 4);
+    return o;
 }
 
 // Accumulator of float partials with a compensated (hi, lo) pair.
@@ -806,7 +890,7 @@ struct Acc2 {
         hi = s;
         lo = __fadd_rn(lo, e);
     }
-    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+    __device__ __forceinline__ double value() const { return widen(hi) + widen(lo); }
 };
 
 // Philox4x32-10 (Salmon et al., SC'11); counter (atom, step lo, step hi, stream)

@@ -69,15 +69,16 @@ enum { FX_LJ = 1, FX_EL = 2, FX_LJEL = 3, FX_WATER = 4 };
 // fixed-point kernels: classification, FP64 fallback, LJ and reaction-field
 // factors in the units of the LJ sum, accumulated into (px, py, pz). An
 // entry with v0 / v1 false adds exactly zero (its partner must be a valid
-// index, e.g. the atom itself).
-template <int POT>
+// index, e.g. the atom itself). LJ: some pair may be an LJ pair (false for
+// the rows of water hydrogens).
+template <int POT, bool LJ = true>
 __device__ __forceinline__ void fx_pair2(const Dev& d, const double* X, int64_t ia, bool lj_i, float kqi,
                                          const uint4& qi, int j0, int j1, bool v0, bool v1, const uint4& q0,
                                          const uint4& q1, float lj_lo, float lj_hi, float el_lo, float el_hi,
                                          float sig2h, float sig2l, float krf, float2& px, float2& py, float2& pz,
                                          bool& range_err)
 {
-    constexpr bool HAS_LJ = POT == FX_LJ || POT == FX_LJEL || POT == FX_WATER;
+    constexpr bool HAS_LJ = LJ && (POT == FX_LJ || POT == FX_LJEL || POT == FX_WATER);
     constexpr bool HAS_EL = POT == FX_EL || POT == FX_LJEL || POT == FX_WATER;
     float2 dx = make_float2(fx_diff(qi.x, q0.x), fx_diff(qi.x, q1.x));
     float2 dy = make_float2(fx_diff(qi.y, q0.y), fx_diff(qi.y, q1.y));
@@ -105,20 +106,22 @@ __device__ __forceinline__ void fx_pair2(const Dev& d, const double* X, int64_t 
             range_err |= o.range_err != 0;
         }
     }
-    const bool in0 = lj0 || el0, in1 = lj1 || el1b;
-    r2 = make_float2(in0 ? r2.x : 1.0f, in1 ? r2.y : 1.0f);
+    // (a pair outside takes a factor of zero by selection, whatever its r^2;
+    // the differences are finite)
     float2 f = make_float2(0.f, 0.f);
     if (HAS_LJ) {
-        const float2 ri = make_float2(__fdividef(1.0f, r2.x), __fdividef(1.0f, r2.y));
+        const float2 ri = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
+        // s^2 = sigma^2 / r^2 with sigma^2 / u^2 as hi + lo
         const float2 s2 = __ffma2_rn(make_float2(sig2h, sig2h), ri, __fmul2_rn(make_float2(sig2l, sig2l), ri));
         const float2 s6 = __fmul2_rn(__fmul2_rn(s2, s2), s2);
+        // (2 s^12 - s^6) / r^2 = (2 s^6 - 1) s^6 / r^2
         const float2 fl =
             __fmul2_rn(__fmul2_rn(__ffma2_rn(make_float2(2.f, 2.f), s6, make_float2(-1.f, -1.f)), s6), ri);
         f = make_float2(lj0 ? fl.x : 0.f, lj1 ? fl.y : 0.f);
     }
     if (HAS_EL) {
         const float qj0 = __int_as_float((int)q0.w), qj1 = __int_as_float((int)q1.w);
-        const float2 rb = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+        const float2 rb = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
         const float2 r3 = __fmul2_rn(__fmul2_rn(rb, rb), rb);
         const float2 fe = __fmul2_rn(make_float2(kqi * qj0, kqi * qj1), __fadd2_rn(r3, make_float2(-krf, -krf)));
         f = make_float2(el0 ? f.x + fe.x : f.x, el1b ? f.y + fe.y : f.y);
@@ -127,4 +130,3 @@ __device__ __forceinline__ void fx_pair2(const Dev& d, const double* X, int64_t 
     py = __ffma2_rn(f, dy, py);
     pz = __ffma2_rn(f, dz, pz);
 }
-

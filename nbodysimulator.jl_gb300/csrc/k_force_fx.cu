@@ -193,58 +193,8 @@ __global__ void __launch_bounds__(FX_THREADS) k_force_fx(Dev d, StateView s, con
                 qn0 = __ldg(&d.pfx[jn0]);
                 qn1 = __ldg(&d.pfx[jn1]);
             }
-            float2 dx = make_float2(fx_diff(qi.x, q0.x), fx_diff(qi.x, q1.x));
-            float2 dy = make_float2(fx_diff(qi.y, q0.y), fx_diff(qi.y, q1.y));
-            float2 dz = make_float2(fx_diff(qi.z, q0.z), fx_diff(qi.z, q1.z));
-            // the same rounding steps as fx_r2 (FFMA2 rounds each lane as FFMA)
-            float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-            const bool lp0 = HAS_LJ && lj_i && (POT != FX_WATER || fx_oxygen(j0));
-            const bool lp1 = HAS_LJ && v1 && lj_i && (POT != FX_WATER || fx_oxygen(j1));
-            const bool ep0 = HAS_EL, ep1 = HAS_EL && v1;
-            bool lj0, lj1, el0, el1b, amb0, amb1;
-            fx_classify(r2.x, lp0, ep0, lj_lo, lj_hi, el_lo, el_hi, lj0, el0, amb0);
-            fx_classify(r2.y, lp1, ep1, lj_lo, lj_hi, el_lo, el_hi, lj1, el1b, amb1);
-            if (amb0 | amb1) {
-                if (amb0) {
-                    const FxPair o = fx_pair_fallback(d, s.x, ia, j0, lp0, ep0);
-                    lj0 = o.lj_in;
-                    el0 = o.el_in;
-                    dx.x = o.dx, dy.x = o.dy, dz.x = o.dz, r2.x = o.r2;
-                    range_err |= o.range_err != 0;
-                }
-                if (amb1) {
-                    const FxPair o = fx_pair_fallback(d, s.x, ia, j1, lp1, ep1);
-                    lj1 = o.lj_in;
-                    el1b = o.el_in;
-                    dx.y = o.dx, dy.y = o.dy, dz.y = o.dz, r2.y = o.r2;
-                    range_err |= o.range_err != 0;
-                }
-            }
-            // pairs outside both cutoffs (and the masked second entry) add
-            // nothing; their r^2 is replaced so that no infinity enters
-            const bool in0 = lj0 || el0, in1 = lj1 || el1b;
-            r2 = make_float2(in0 ? r2.x : 1.0f, in1 ? r2.y : 1.0f);
-            float2 f = make_float2(0.f, 0.f);
-            if (HAS_LJ) {
-                const float2 ri = make_float2(__fdividef(1.0f, r2.x), __fdividef(1.0f, r2.y));
-                // s^2 = sigma^2 / r^2 with sigma^2 / u^2 as hi + lo
-                const float2 s2 = __ffma2_rn(make_float2(sig2h, sig2h), ri, __fmul2_rn(make_float2(sig2l, sig2l), ri));
-                const float2 s6 = __fmul2_rn(__fmul2_rn(s2, s2), s2);
-                // (2 s^12 - s^6) / r^2 = (2 s^6 - 1) s^6 / r^2
-                const float2 fl = __fmul2_rn(__fmul2_rn(__ffma2_rn(make_float2(2.f, 2.f), s6, make_float2(-1.f, -1.f)), s6),
-                                             ri);
-                f = make_float2(lj0 ? fl.x : 0.f, lj1 ? fl.y : 0.f);
-            }
-            if (HAS_EL) {
-                const float qj0 = __int_as_float((int)q0.w), qj1 = __int_as_float((int)q1.w);
-                const float2 rb = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                const float2 r3 = __fmul2_rn(__fmul2_rn(rb, rb), rb);
-                const float2 fe = __fmul2_rn(make_float2(kqi * qj0, kqi * qj1), __fadd2_rn(r3, make_float2(-krf, -krf)));
-                f = make_float2(el0 ? f.x + fe.x : f.x, el1b ? f.y + fe.y : f.y);
-            }
-            px = __ffma2_rn(f, dx, px);
-            py = __ffma2_rn(f, dy, py);
-            pz = __ffma2_rn(f, dz, pz);
+            fx_pair2<POT>(d, s.x, ia, lj_i, kqi, qi, j0, j1, true, v1, q0, q1, lj_lo, lj_hi, el_lo, el_hi, sig2h, sig2l,
+                          krf, px, py, pz, range_err);
         }
         // forces: the two halves, then the lanes
         float hx = __fadd_rn(px.x, px.y), hy = __fadd_rn(py.x, py.y), hz = __fadd_rn(pz.x, pz.y);
@@ -441,6 +391,82 @@ __global__ void __launch_bounds__(FXW_WARPS * 32, (LPA <= 4 && POT == FX_LJ) ? 4
     }
 }
 
+// A warp per atom (32 lanes, the form of the smallest systems and of the long
+// rows of water by default): the row is read as coalesced 128-byte lines,
+// two packed steps ahead, and the gathers one step ahead, with no staging and
+// no barrier: a row's lines are read once, so staging them bought nothing
+// here and a block waited for its slowest warp. The rows of hydrogens run
+// without the LJ arithmetic (warp-uniform). Latency-bound (L2 gathers):
+// 12,288-atom water 28.7 -> 18.9 us a launch; a step of 10,976 LJ atoms
+// 28.4 -> 26.
+#define FXR_WARPS 8
+
+template <int POT, bool LJ>
+__device__ __forceinline__ void fx_row(const Dev& d, const StateView& s, int64_t i, int lane, const int* row, int cap, int cnt,
+                                       int e0, int e1, const uint4& qi, float kqi, float2& px, float2& py, float2& pz,
+                                       bool& range_err)
+{
+    const RepDev& R = d.reps[d.rep_of[i]];
+    const float lj_lo = R.fx_lj_lo, lj_hi = R.fx_lj_hi, el_lo = R.fx_el_lo, el_hi = R.fx_el_hi;
+    const float sig2h = R.fx_sig2_hi, sig2l = R.fx_sig2_lo, krf = R.fx_krf;
+    // an entry past the row's count becomes the atom itself and adds zero
+    auto entry = [&](int k) { return k < cap ? __ldg(row + k) : 0; };
+    auto valid = [&](int k, int e) { return k < cnt ? dbg_index(e, d.n, (int)i, d.status) : (int)i; };
+    int j0 = valid(lane, e0), j1 = valid(lane + 32, e1);
+    uint4 q0 = __ldg(&d.pfx[j0]), q1 = __ldg(&d.pfx[j1]);
+    int n0 = 0, n1 = 0;
+    if (cnt > 64) {
+        n0 = entry(64 + lane);
+        n1 = entry(96 + lane);
+    }
+    for (int kb = 0; kb < cnt; kb += 64) {
+        const int k0 = kb + lane, k1 = k0 + 32;
+        const int c0 = j0, c1 = j1;
+        const uint4 p0 = q0, p1 = q1;
+        if (kb + 64 < cnt) {
+            j0 = valid(k0 + 64, n0);
+            j1 = valid(k1 + 64, n1);
+            q0 = __ldg(&d.pfx[j0]);
+            q1 = __ldg(&d.pfx[j1]);
+            if (kb + 128 < cnt) {
+                n0 = entry(k0 + 128);
+                n1 = entry(k1 + 128);
+            }
+        }
+        fx_pair2<POT, LJ>(d, s.x, i, LJ, kqi, qi, c0, c1, k0 < cnt, k1 < cnt, p0, p1, lj_lo, lj_hi, el_lo, el_hi, sig2h,
+                          sig2l, krf, px, py, pz, range_err);
+    }
+}
+
+template <int POT>
+__global__ void __launch_bounds__(FXR_WARPS * 32, 4) k_force_fxr(Dev d, StateView s)
+{
+    constexpr bool HAS_EL = POT == FX_EL || POT == FX_LJEL || POT == FX_WATER;
+    const int lane = threadIdx.x & 31;
+    const int64_t i = blockIdx.x * (int64_t)FXR_WARPS + (threadIdx.x >> 5);
+    if (i >= d.n) return;
+    const int cap = d.nbr_cap;
+    const int* row = d.nbr + i * d.nbr_istride;
+    // (the first entries do not wait for the count)
+    const int e0 = lane < cap ? __ldg(row + lane) : 0, e1 = lane + 32 < cap ? __ldg(row + lane + 32) : 0;
+    const int cnt = min(d.nbr_count[i], cap);
+    const uint4 qi = d.pfx[i];
+    const double im = d.inv_mass_fx[i];
+    const float kqi = HAS_EL ? (float)(d.charge[i] * d.reps[d.rep_of[i]].fx_kq) : 0.0f;
+    float2 px = make_float2(0.f, 0.f), py = px, pz = px;
+    bool range_err = false;
+    if (POT != FX_WATER || i % 3 == 0) fx_row<POT, true>(d, s, i, lane, row, cap, cnt, e0, e1, qi, kqi, px, py, pz, range_err);
+    else fx_row<POT, false>(d, s, i, lane, row, cap, cnt, e0, e1, qi, kqi, px, py, pz, range_err);
+    const LaneSum f =
+        lane_sums3<32>(__fadd_rn(px.x, px.y), __fadd_rn(py.x, py.y), __fadd_rn(pz.x, pz.y), lane);
+    const double acc = (widen(f.h) + widen(f.e)) * im;
+    if (f.writer) {
+        if (!finite64(acc)) status_set(d.status, ST_NONFINITE);
+        s.a_new[3 * i + f.comp] = acc;
+    }
+    if (range_err) status_set(d.status, ST_RANGE);
+}
+
 // ---------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------
@@ -458,9 +484,10 @@ static PFN_cuTensorMapEncodeTiled_v12000 fx_encode_fn()
     return fn;
 }
 
-// The per-warp form runs for 4, 8 and 16 lanes per atom (NBG_FX_BLOCK keeps
-// the per-block form, for comparisons), the per-block form for 32.
+// The per-warp form runs for 4, 8 and 16 lanes per atom and the warp-per-atom
+// form for 32 (NBG_FX_BLOCK keeps the per-block form, for comparisons).
 static bool fx_warp_form(const nbg_ctx* c) { return c->list_lpa <= 16 && !c->fx_block_only; }
+static bool fx_row_form(const nbg_ctx* c) { return c->list_lpa == 32 && !c->fx_block_only; }
 
 // rows (atoms) of one list box of the tensor map
 static int fx_box_rows(const nbg_ctx* c) { return fx_warp_form(c) ? 32 / c->list_lpa : FX_THREADS / c->list_lpa; }
@@ -495,6 +522,12 @@ int fx_encode_map(nbg_ctx* c)
 template <int LPA, int POT>
 static int fx_prepare_form(nbg_ctx* c)
 {
+    if (fx_row_form(c)) {
+        c->fx_grid = (int)((c->n + FXR_WARPS - 1) / FXR_WARPS);
+        c->fx_smem = 0;
+        c->fx_nbox = 0;
+        return NBG_OK;
+    }
     if constexpr (LPA <= 16) {
         if (fx_warp_form(c)) {
             const size_t smem = (size_t)FXW_WARPS * FXW_SLOTS * 1024 + 1024;
@@ -540,6 +573,10 @@ static void fx_launch(nbg_ctx* c, const StateView& s)
             k_force_fxw<LPA, POT><<<(unsigned)c->fx_grid, FXW_WARPS * 32, c->fx_smem, c->stream>>>(c->d, s, *map);
             return;
         }
+    }
+    if (fx_row_form(c)) {
+        k_force_fxr<POT><<<(unsigned)c->fx_grid, FXR_WARPS * 32, 0, c->stream>>>(c->d, s);
+        return;
     }
     k_force_fx<LPA, POT><<<(unsigned)c->fx_grid, FX_THREADS, c->fx_smem, c->stream>>>(c->d, s, *map, c->fx_nbox);
 }

@@ -35,13 +35,6 @@
 #define GB 128         // gravity block size = j-tile size
 #define GI_MAX (4 * GB)  // bodies i per block at most (TI <= 4)
 
-__device__ __forceinline__ float rsqrt_ftz(float x)
-{
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Grid: (i-block, j-chunk) units; each thread owns TI bodies i (strided by
 // GB within the block) and walks the chunk's j-tiles from shared memory:
 // every lane of a warp reads the same body j (one broadcast load serves TI
@@ -631,15 +624,6 @@ static __device__ __noinline__ ApExact ap_exact(const Dev& d, const double* X, i
     o.dr = make_float3((float)q.x, (float)q.y, (float)q.z);
     o.r2 = (float)q.r2;
     return o;
-}
-
-// 1 / x of a normal positive x, approximated as __fdividef does (a / b there
-// is a times this)
-__device__ __forceinline__ float rcp_ftz(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 
 // Bodies j staged per warp in shared memory, one array per field so that two

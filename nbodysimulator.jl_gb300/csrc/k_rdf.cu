@@ -150,15 +150,6 @@ __global__ void __launch_bounds__(256) k_rdf_pack(RdfPackArgs a)
     a.raw[t] = r;
 }
 
-// 1 / sqrt(x) by the approximate hardware instruction, subnormals flushed
-// (q^2 below 2^-126 is a self or coincident pair: bin 0 either way)
-__device__ __forceinline__ float rsqrt_ftz(float x)
-{
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // The decision on one screened pair, without branches. decided: q^2 <= lo
 // (inside half the box) and |E| < T (clear of a bin edge: E = q - 1/2 -
 // floor(q), T = 1/2 - the margin; NaN, a self pair, counts as clear). A

@@ -430,32 +430,27 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
     // gravity bodies padded to a multiple of the largest i-block (4 x 128)
     c->npad = c->path == PATH_GRAVITY ? ((n + 511) / 512) * 512 : n;
     double* dp;
-    if ((st = dalloc(c, &dp, n))) return st;
-    D.mass = dp;
-    CK(cudaMemcpy(dp, c->mass_h.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "mass upload");
-    std::vector<double> im(n);
-    for (int64_t i = 0; i < n; ++i) im[i] = 1.0 / c->mass_h[i];
-    if ((st = dalloc(c, &dp, n))) return st;
-    D.inv_mass = dp;
-    CK(cudaMemcpy(dp, im.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "inv_mass upload");
     {
-        std::vector<double> rs(n);
-        for (int64_t i = 0; i < n; ++i) rs[i] = std::sqrt(im[i]);
-        double* rp = nullptr;
-        if ((st = dalloc(c, &rp, n))) return st;
-        D.rsqrt_mass = rp;
-        CK(cudaMemcpy(rp, rs.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "rsqrt_mass upload");
+        // per-atom doubles in one allocation and one upload: mass, its inverse
+        // and root, charge, and (list path) the inverse in the fixed-point forces' units
+        const bool fx = c->path == PATH_LIST && d0->bc == NBG_BC_CUBIC;
+        std::vector<double> per((size_t)n * (fx ? 5 : 4));
+        for (int64_t i = 0; i < n; ++i) {
+            const double im = 1.0 / c->mass_h[i];
+            per[i] = c->mass_h[i];
+            per[n + i] = im;
+            per[2 * n + i] = std::sqrt(im);
+            per[3 * n + i] = c->charge_h[i];
+            if (fx) per[4 * n + i] = im * c->reps_h[rep_of[i]].fx_fscale;
+        }
+        if ((st = dalloc(c, &dp, per.size()))) return st;
+        CK(cudaMemcpy(dp, per.data(), sizeof(double) * per.size(), cudaMemcpyHostToDevice), "per-atom upload");
+        D.mass = dp;
+        D.inv_mass = dp + n;
+        D.rsqrt_mass = dp + 2 * n;
+        D.charge = dp + 3 * n;
+        D.inv_mass_fx = fx ? dp + 4 * n : nullptr;
     }
-    if (c->path == PATH_LIST && d0->bc == NBG_BC_CUBIC) {
-        std::vector<double> f(n);
-        for (int64_t i = 0; i < n; ++i) f[i] = im[i] * c->reps_h[rep_of[i]].fx_fscale;
-        if ((st = dalloc(c, &dp, n))) return st;
-        D.inv_mass_fx = dp;
-        CK(cudaMemcpy(dp, f.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "inv_mass_fx upload");
-    }
-    if ((st = dalloc(c, &dp, n))) return st;
-    D.charge = dp;
-    CK(cudaMemcpy(dp, c->charge_h.data(), sizeof(double) * n, cudaMemcpyHostToDevice), "charge upload");
     if (pots & NBG_POT_MAG) {
         if ((st = dalloc(c, &dp, 3 * n))) return st;
         D.dipole = dp;

@@ -526,6 +526,22 @@ __device__ __forceinline__ bool finite64(double x)
     return (__double_as_longlong(x) & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
 }
 
+__device__ __forceinline__ float rsqrt_ftz(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// 1 / x of a normal positive x, approximated as __fdividef does (a / b there
+// is a times this)
+__device__ __forceinline__ float rcp_ftz(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // FP64 issues at 2 lanes per clock and SM here: a warp instruction holds its
 // SM sub-partition for 64 cycles whatever its mask (comparisons 98, floor and
 // rint 142, conversions to and from FP32 32 and 64). The three helpers below

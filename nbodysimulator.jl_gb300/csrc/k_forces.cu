@@ -1233,15 +1233,6 @@ int launch_force_list(nbg_ctx* c, const StateView& s)
 // ---------------------------------------------------------------------
 // SPC/Fw bonded terms (FP64), one thread per molecule (O, H1, H2)
 // ---------------------------------------------------------------------
-__device__ __forceinline__ void cross3f(const float* a, const float* b, float* c)
-{
-    c[0] = a[1] * b[2] - a[2] * b[1];
-    c[1] = a[2] * b[0] - a[0] * b[2];
-    c[2] = a[0] * b[1] - a[1] * b[0];
-}
-
-__device__ __forceinline__ float norm3f(const float* a) { return sqrtf(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]); }
-
 // Bonds and angle of one molecule. The intramolecular differences are taken
 // in FP64 from the unwrapped positions and rounded once to FP32 (relative
 // error 2^-24); the terms themselves are FP32, like the pair forces (the bond
@@ -1259,39 +1250,13 @@ __global__ void k_bonded(Dev d, StateView s)
             r1[k] = (float)(X[3 * h1 + k] - X[3 * o + k]);
             r2[k] = (float)(X[3 * h2 + k] - X[3 * o + k]);
         }
-        // bonds (harmonic_bond_potential_acceleration!, :367-393): on O from
-        // bond O-H, -(r - rOH) k / r (r_O - r_H); on H the exact negative.
-        float fO[3] = {0.f, 0.f, 0.f}, fH1[3], fH2[3];
-        const float* hs[2] = {r1, r2};
-        float* fh[2] = {fH1, fH2};
-        for (int b = 0; b < 2; ++b) {
-            float r = norm3f(hs[b]);
-            float factor = -(r - rOH) * kb / r;
-            for (int k = 0; k < 3; ++k) {
-                float f = factor * -hs[b][k];  // rij = r_O - r_H
-                fO[k] += f;
-                fh[b][k] = -f;
-            }
-        }
-        // angle H1-O-H2 (valence_angle_potential_acceleration!, :395-433), a=H1, b=O, c=H2
-        float rcb[3] = {-r2[0], -r2[1], -r2[2]}, x[3], pa[3], pc[3];
-        cross3f(r1, r2, x);
-        cross3f(r1, x, pa);
-        cross3f(rcb, x, pc);
-        float npa = norm3f(pa), npc = norm3f(pc);
-        float nba = norm3f(r1), nbc = norm3f(r2);
-        float cosine = (r1[0] * r2[0] + r1[1] * r2[1] + r1[2] * r2[2]) / (nba * nbc);
-        cosine = fminf(1.0f, fmaxf(-1.0f, cosine));
-        float force = -ka * (acosf(cosine) - a0);
-        float sa = force / (npa * nba), sc = force / (npc * nbc);
+        float fO[3], f1[3], f2[3];
+        bonded_forces(r1, r2, rOH, kb, ka, a0, fO, f1, f2);
         const double iO = d.inv_mass[o], iH1 = d.inv_mass[h1], iH2 = d.inv_mass[h2];
         for (int k = 0; k < 3; ++k) {
-            float fa = pa[k] * sa;
-            float fc = pc[k] * sc;
-            float fb = -(fa + fc);
-            s.a_new[3 * o + k] += (double)(fO[k] + fb) * iO;
-            s.a_new[3 * h1 + k] += (double)(fH1[k] + fa) * iH1;
-            s.a_new[3 * h2 + k] += (double)(fH2[k] + fc) * iH2;
+            s.a_new[3 * o + k] = fma(widen(fO[k]), iO, s.a_new[3 * o + k]);
+            s.a_new[3 * h1 + k] = fma(widen(f1[k]), iH1, s.a_new[3 * h1 + k]);
+            s.a_new[3 * h2 + k] = fma(widen(f2[k]), iH2, s.a_new[3 * h2 + k]);
         }
     }
 }

@@ -247,25 +247,46 @@ struct ThermoAux {
     double bfac, rate;
 };
 
-__device__ __forceinline__ void thermo_aux(const Dev& d, double T, ThermoAux* aux)
+// Quotients of the thermostat's fixed parameters, taken once on the host (the
+// target temperature may change between replays: it is read from the table).
+struct ThermoK {
+    double kbndf;      // kb ndf
+    double g;          // 1 / (2 tau)
+    double it2, ndfq;  // (1 / tau)^2, (ndf + 1) / ndf
+};
+
+__device__ __forceinline__ void thermo_aux(const Dev& d, const ThermoK& K, double T, ThermoAux* aux)
 {
-    const RepDev& R = d.reps[0];
-    if (d.therm == NBG_THERMO_BERENDSEN) {
-        const double g = 0.5 / R.tparam;
-        aux->bfac = (1.0 / T == INFINITY) ? g : __dmul_rn(g, __dsub_rn(R.T0 / T, 1.0));
-    } else {
-        const double it = 1.0 / R.tparam;
-        aux->rate = __dmul_rn(__dmul_rn(it, it), __dsub_rn(T / R.T0, (R.ndf + 1.0) / R.ndf));
-    }
+    const double T0 = d.reps[0].T0;
+    if (d.therm == NBG_THERMO_BERENDSEN)  // (1 / T == Inf for 0 <= T <= 2^-1024)
+        aux->bfac = (T >= 0.0 && T <= 0x1p-1024) ? K.g : __dmul_rn(K.g, __dsub_rn(T0 / T, 1.0));
+    else
+        aux->rate = __dmul_rn(K.it2, __dsub_rn(T / T0, K.ndfq));
 }
 
 // from a temperature already in red_T (the run's first step)
-__global__ void k_thermo_aux(Dev d, ThermoAux* aux) { thermo_aux(d, d.red_T[0], aux); }
+__global__ void k_thermo_aux(Dev d, ThermoK K, ThermoAux* aux) { thermo_aux(d, K, d.red_T[0], aux); }
+
+// sh[0] of the tree sh[t] += sh[t + w], w = 128 .. 1, over 256 values (the
+// last five levels by shuffles: the same sums), in the first warp's lane 0
+__device__ __forceinline__ double tree256(double* sh, double v)
+{
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for (int w = 128; w >= 32; w >>= 1) {
+        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x >= 32) return 0.0;
+    v = sh[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
 
 // sum m v^2 in k_kick's order: elements by thread, the block's tree, block
 // partials by the last block
-__global__ void __launch_bounds__(256) k_kick_T(Dev d, const double* __restrict__ V, double* part, unsigned* counter,
-                                                ThermoAux* aux)
+__global__ void __launch_bounds__(256) k_kick_T(Dev d, ThermoK K, const double* __restrict__ V, double* part,
+                                                unsigned* counter, ThermoAux* aux)
 {
     const int64_t ncomp = 3 * d.n;
     double acc = 0.0;
@@ -274,15 +295,10 @@ __global__ void __launch_bounds__(256) k_kick_T(Dev d, const double* __restrict_
         acc += d.mass[e / 3] * (vn * vn);
     }
     __shared__ double sh[256];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
-    }
+    const double mine = tree256(sh, acc);
     __shared__ bool last;
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = sh[0];
+        part[blockIdx.x] = mine;
         __threadfence();
         last = (atomicAdd(counter, 1u) == gridDim.x - 1);
     }
@@ -291,30 +307,28 @@ __global__ void __launch_bounds__(256) k_kick_T(Dev d, const double* __restrict_
     __threadfence();
     double t = 0.0;
     for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += ((volatile double*)part)[b];
-    sh[threadIdx.x] = t;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
-    }
+    const double sum = tree256(sh, t);
     if (threadIdx.x == 0) {
-        const double T = sh[0] / (d.kb * d.reps[0].ndf);
+        const double T = sum / K.kbndf;
         d.red_T[0] = T;
         *counter = 0u;
-        thermo_aux(d, T, aux);
+        thermo_aux(d, K, T, aux);
     }
 }
 
 // The drift, packing and displacement check of a step (k_drift_pack's
 // operations); KICK: before it the kick that ends the step before (k_kick's,
-// then k_andersen's) and the saved frame of that state. A thread per component, a warp per 10
-// atoms (lane 3 a + k; lanes 30 and 31 idle): a thread per atom had three
-// components' FP64 operations in one chain, each 64 cycles of its SM
+// then k_andersen's) and the saved frame of that state. A thread per
+// component, a warp per 10 atoms (lane 3 a + k; lanes 30 and 31 idle): a
+// thread per atom had three components' FP64 operations in one chain, each 64 cycles of its SM
 // sub-partition, and a third of the warps. The Nose-Hoover column is moved by
 // the block after the atoms'; the other blocks read zeta from zc_in, so that
 // it may be moved meanwhile (zc_out). One launch instead of up to four per
 // step (kick, Andersen, frame, drift): 10,976 LJ atoms 45 -> 36 us a step.
-#define VV_ATOMS 40  // atoms per block of 128 threads
+// WATER: 3 molecules a warp (27 lanes), and the bond and angle accelerations
+// (k_bonded's) are added before the kick from the positions the lanes hold:
+// a launch and a pass over a_new less, with 4 FP64 instructions a warp
+// instead of 36.
 
 struct VVArgs {
     double dt, dtsq;
@@ -327,12 +341,13 @@ struct VVArgs {
     const ThermoAux* aux;
 };
 
-template <bool KICK>
+template <bool KICK, bool WATER>
 __global__ void __launch_bounds__(128) k_vv(Dev d, StateView s, VVArgs A)
 {
+    constexpr int PER = WATER ? 9 : 10;  // atoms per warp
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = lane % 3;
-    const int64_t blocks = (d.n + VV_ATOMS - 1) / VV_ATOMS;
+    const int64_t blocks = (d.n + 4 * PER - 1) / (4 * PER);
     int64_t slot = -1;  // the frame slot of the state after the kick
     if (KICK && A.save) {
         const FrameSink* sink = d.sink;
@@ -365,12 +380,27 @@ __global__ void __launch_bounds__(128) k_vv(Dev d, StateView s, VVArgs A)
         }
         return;
     }
-    const int64_t i = blockIdx.x * (int64_t)VV_ATOMS + w * 10 + lane / 3;
-    const bool active = lane < 30 && i < d.n;
+    const int64_t i = blockIdx.x * (int64_t)(4 * PER) + w * PER + lane / 3;
+    const bool active = lane < 3 * PER && i < d.n;
     const int64_t e = active ? 3 * i + k : 0;
     double x = s.x[e], v = s.v[e], a = s.a_old[e];
     if (KICK) {
         double an = s.a_new[e];
+        if (WATER) {
+            const int m0 = min(lane / 9, 2) * 9, site = (lane % 9) / 3;  // the molecule's first lane (O, x)
+            const float dif = (float)(x - __shfl_sync(0xffffffffu, x, m0 + k));
+            float r1[3], r2[3], fO[3], f1[3], f2[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                r1[q] = __shfl_sync(0xffffffffu, dif, m0 + 3 + q);
+                r2[q] = __shfl_sync(0xffffffffu, dif, m0 + 6 + q);
+            }
+            bonded_forces(r1, r2, (float)d.rOH, (float)d.kbond, (float)d.kangle, (float)d.aHOH, fO, f1, f2);
+            const float f = site == 0 ? (k == 0 ? fO[0] : k == 1 ? fO[1] : fO[2])
+                            : site == 1 ? (k == 0 ? f1[0] : k == 1 ? f1[1] : f1[2])
+                                        : (k == 0 ? f2[0] : k == 1 ? f2[1] : f2[2]);
+            an = fma(widen(f), d.inv_mass[active ? i : 0], an);
+        }
         if (d.therm == NBG_THERMO_BERENDSEN) an = __dadd_rn(an, __dmul_rn(A.aux->bfac, v));
         else if (d.therm == NBG_THERMO_NOSEHOOVER) an = __dadd_rn(an, -__dmul_rn(*A.zc_in, v));
         if (active && !finite64(an)) status_set(d.status, ST_NONFINITE);
@@ -435,9 +465,12 @@ int launch_vv(nbg_ctx* c, const StateView& s, double dt, bool kick, StepRef sr, 
     A.zc_in = c->vv_buf + (k & 1);
     A.zc_out = c->vv_buf + (kick ? (k + 1) & 1 : k & 1);
     A.aux = vv_aux(c);
-    const unsigned grid = (unsigned)((c->n + VV_ATOMS - 1) / VV_ATOMS) + (c->d.therm == NBG_THERMO_NOSEHOOVER ? 1u : 0u);
-    if (kick) k_vv<true><<<grid, 128, 0, c->stream>>>(c->d, s, A);
-    else k_vv<false><<<grid, 128, 0, c->stream>>>(c->d, s, A);
+    const bool water = kick && c->d.kind == NBG_SYSTEM_WATER;
+    const int64_t per = water ? 36 : 40;  // atoms per block
+    const unsigned grid = (unsigned)((c->n + per - 1) / per) + (c->d.therm == NBG_THERMO_NOSEHOOVER ? 1u : 0u);
+    if (water) k_vv<true, true><<<grid, 128, 0, c->stream>>>(c->d, s, A);
+    else if (kick) k_vv<true, false><<<grid, 128, 0, c->stream>>>(c->d, s, A);
+    else k_vv<false, false><<<grid, 128, 0, c->stream>>>(c->d, s, A);
     NBG_LAUNCH_CHECK(c, "k_vv");
     return NBG_OK;
 }
@@ -446,11 +479,14 @@ int launch_vv(nbg_ctx* c, const StateView& s, double dt, bool kick, StepRef sr, 
 // (reduce = false) from the temperature in red_T.
 int launch_vv_thermo(nbg_ctx* c, const double* v, bool reduce, cudaStream_t stream)
 {
+    const RepDev& R = c->reps_h[0];
+    const double it = 1.0 / R.tparam;
+    const ThermoK K{c->d.kb * R.ndf, 0.5 / R.tparam, it * it, (R.ndf + 1.0) / R.ndf};
     if (reduce) {
         const int grid = std::min(grid_for(3 * c->n, 256), c->kick_blocks);
-        k_kick_T<<<grid, 256, 0, stream>>>(c->d, v, c->kick_part, c->kick_counter, vv_aux(c));
+        k_kick_T<<<grid, 256, 0, stream>>>(c->d, K, v, c->kick_part, c->kick_counter, vv_aux(c));
     } else {
-        k_thermo_aux<<<1, 1, 0, stream>>>(c->d, vv_aux(c));
+        k_thermo_aux<<<1, 1, 0, stream>>>(c->d, K, vv_aux(c));
     }
     NBG_LAUNCH_CHECK(c, "k_kick_T");
     return NBG_OK;

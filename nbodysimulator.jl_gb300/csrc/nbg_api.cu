@@ -890,7 +890,8 @@ static int status_error(nbg_ctx* c, unsigned st)
 
 // Potential accelerations of state s into s.a_new (no thermostat term).
 // pos: time index of the positions in s (its parity picks the rebuild flag).
-static int forces(nbg_ctx* c, const StateView& s, bool force_build, StepRef pos)
+// bonded: the bond and angle terms of water too.
+static int forces(nbg_ctx* c, const StateView& s, bool force_build, StepRef pos, bool bonded = true)
 {
     NBG_RANGE("forces");
     int st = NBG_OK;
@@ -913,7 +914,7 @@ static int forces(nbg_ctx* c, const StateView& s, bool force_build, StepRef pos)
         st = launch_allpairs(c, s);
     }
     if (st) return st;
-    if (c->d.kind == NBG_SYSTEM_WATER) st = launch_bonded(c, s);
+    if (bonded && c->d.kind == NBG_SYSTEM_WATER) st = launch_bonded(c, s);
     return st;
 }
 
@@ -1341,7 +1342,8 @@ static int steps_vv_fused(nbg_ctx* c, double dt, int64_t G)
             CK(cudaEventRecord(c->join_ev, c->side), "join");
         }
         const bool force = rebuild_due(c, true);
-        if ((st = forces(c, s, force, pos))) return st;
+        // (the next launch_vv adds the bonded terms)
+        if ((st = forces(c, s, force, pos, k + 1 == G))) return st;
         c->steps_since_build = force ? 0 : c->steps_since_build + 1;
         if (thermo_T && (k > 0 || branch)) CK(cudaStreamWaitEvent(c->stream, c->join_ev, 0), "join");
         if (k + 1 == G) {

@@ -896,6 +896,57 @@ __device__ __forceinline__ LaneSum lane_sums3(float x, float y, float z, int lan
     return o;
 }
 
+__device__ __forceinline__ void cross3f(const float* a, const float* b, float* c)
+{
+    c[0] = a[1] * b[2] - a[2] * b[1];
+    c[1] = a[2] * b[0] - a[0] * b[2];
+    c[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+__device__ __forceinline__ float norm3f(const float* a) { return sqrtf(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]); }
+
+// SPC/Fw bond and angle forces on O, H1 and H2 from r1 = H1 - O, r2 = H2 - O.
+__device__ __forceinline__ void bonded_forces(const float* r1, const float* r2, float rOH, float kb, float ka, float a0,
+                                              float* outO, float* out1, float* out2)
+{
+    // bonds (harmonic_bond_potential_acceleration!, :367-393): on O from
+    // bond O-H, -(r - rOH) k / r (r_O - r_H); on H the exact negative.
+    float fO[3] = {0.f, 0.f, 0.f}, fH1[3], fH2[3];
+    const float* hs[2] = {r1, r2};
+    float* fh[2] = {fH1, fH2};
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        float r = norm3f(hs[b]);
+        float factor = -(r - rOH) * kb / r;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            float f = factor * -hs[b][k];  // rij = r_O - r_H
+            fO[k] += f;
+            fh[b][k] = -f;
+        }
+    }
+    // angle H1-O-H2 (valence_angle_potential_acceleration!, :395-433), a=H1, b=O, c=H2
+    float rcb[3] = {-r2[0], -r2[1], -r2[2]}, x[3], pa[3], pc[3];
+    cross3f(r1, r2, x);
+    cross3f(r1, x, pa);
+    cross3f(rcb, x, pc);
+    float npa = norm3f(pa), npc = norm3f(pc);
+    float nba = norm3f(r1), nbc = norm3f(r2);
+    float cosine = (r1[0] * r2[0] + r1[1] * r2[1] + r1[2] * r2[2]) / (nba * nbc);
+    cosine = fminf(1.0f, fmaxf(-1.0f, cosine));
+    float force = -ka * (acosf(cosine) - a0);
+    float sa = force / (npa * nba), sc = force / (npc * nbc);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float fa = pa[k] * sa;
+        float fc = pc[k] * sc;
+        float fb = -(fa + fc);
+        outO[k] = fO[k] + fb;
+        out1[k] = fH1[k] + fa;
+        out2[k] = fH2[k] + fc;
+    }
+}
+
 // Accumulator of float partials with a compensated (hi, lo) pair.
 struct Acc2 {
     float hi, lo;

@@ -34,6 +34,7 @@
 
 #define GB 128         // gravity block size = j-tile size
 #define GI_MAX (4 * GB)  // bodies i per block at most (TI <= 4)
+#define GRAV_SPREAD 2048 // largest padded system whose bodies take a thread each
 
 // Grid: (i-block, j-chunk) units; each thread owns TI bodies i (strided by
 // GB within the block) and walks the chunk's j-tiles from shared memory:
@@ -68,7 +69,7 @@ __device__ __forceinline__ void grav_tile(const float4* sh_hi, const float4* sh_
                 float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                 float ri = rsqrt_ftz(r2);
                 if (DIAG && j0 + jj == ii[k]) ri = 0.0f;
-                float sc = hj.w * ri * (ri * ri);
+                const float sc = UNIFORM ? __fmul_rn(ri, __fmul_rn(ri, ri)) : __fmul_rn(__fmul_rn(hj.w, ri), __fmul_rn(ri, ri));
                 px[k] = fmaf(sc, dx, px[k]);
                 py[k] = fmaf(sc, dy, py[k]);
                 pz[k] = fmaf(sc, dz, pz[k]);
@@ -161,7 +162,6 @@ __global__ void __launch_bounds__(GB, TI == 2 ? 7 : 1) k_gravity(const float4* _
 {
     static_assert(TI == 1 || TI == 2 || TI == 4, "TI");
     static_assert(!PACKED || TI >= 2, "packed needs pairs");
-    static_assert(PACKED || !UNIFORM, "the uniform-mass form is packed");
     __shared__ float4 sh_hi[GB];
     __shared__ float4 sh_lo[PLAIN ? 1 : GB];
     const int64_t ntile = npad / GB;
@@ -257,7 +257,7 @@ typedef void (*grav_kernel_t)(const float4*, const float4*, int64_t, int64_t, in
 
 // Kernel variants: bodies per thread (TI) x packed FP32x2; index
 // 0: TI=2 scalar, 1: TI=2 packed, 2: TI=4 scalar, 3: TI=4 packed, 4: TI=1 scalar.
-// uniform (equal masses) selects the packed forms without m_j in the loop.
+// uniform (equal masses) selects the forms without m_j in the loop (1, 3, 4).
 static grav_kernel_t grav_variant(bool plain, int v, bool uniform)
 {
     switch (v) {
@@ -266,13 +266,15 @@ static grav_kernel_t grav_variant(bool plain, int v, bool uniform)
     case 3:
         if (uniform) return plain ? k_gravity<true, 4, true, true> : k_gravity<false, 4, true, true>;
         return plain ? k_gravity<true, 4, true, false> : k_gravity<false, 4, true, false>;
-    case 4: return plain ? k_gravity<true, 1, false, false> : k_gravity<false, 1, false, false>;
+    case 4:
+        if (uniform) return plain ? k_gravity<true, 1, false, true> : k_gravity<false, 1, false, true>;
+        return plain ? k_gravity<true, 1, false, false> : k_gravity<false, 1, false, false>;
     default:
         if (uniform) return plain ? k_gravity<true, 2, true, true> : k_gravity<false, 2, true, true>;
         return plain ? k_gravity<true, 2, true, false> : k_gravity<false, 2, true, false>;
     }
 }
-static bool grav_variant_packed(int v) { return v == 1 || v == 3 || v < 0 || v > 4; }
+static bool grav_variant_uniform(int v) { return v != 0 && v != 2; }
 static int grav_ti(int v) { return v == 2 || v == 3 ? 4 : (v == 4 ? 1 : 2); }
 
 // a_i = -G sum_chunks partial_i (fixed chunk order); with a permutation the
@@ -306,34 +308,94 @@ __device__ __forceinline__ unsigned long long spread3(unsigned long long v)
 
 // Largest |coordinate| of the finite positions, rounded up to FP32, as the
 // bits of a non-negative float (which order like unsigned integers): the
-// half-width of the Morton cube. *ext must be 0 before the launch.
-__global__ void k_grav_extent(const double* __restrict__ X, int64_t m, unsigned* ext)
+// half-width of the Morton cube. *ext is 0 before (k_grav_pack_sorted clears
+// it after its use).
+__device__ __forceinline__ void extent_max(double x, unsigned* ext)
 {
-    float v = 0.f;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
-        const double a = fabs(X[e]);
-        if (isfinite(a)) v = fmaxf(v, __double2float_ru(a));
-    }
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(ext, __float_as_uint(v));
+    const unsigned v = finite64(x) ? __float_as_uint(__double2float_ru(fabs(x))) : 0u;
+    const unsigned m = __reduce_max_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(ext, m);
 }
 
-__global__ void k_grav_keys(const double* __restrict__ X, int64_t n, const unsigned* __restrict__ ext,
-                            unsigned long long* keys, int* vals)
+__global__ void __launch_bounds__(256) k_grav_extent(const double* __restrict__ X, int64_t m, unsigned* ext)
+{
+    double v = 0.0;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+        const double a = fabs(X[e]);
+        // (non-negative doubles order like integers)
+        if (finite64(a) && __double_as_longlong(a) > __double_as_longlong(v)) v = a;
+    }
+    extent_max(v, ext);
+}
+
+// vals: null where the ranks are counted (k_grav_rank)
+__global__ void __launch_bounds__(64) k_grav_keys(const double* __restrict__ X, int64_t n,
+                                                  const unsigned* __restrict__ ext, unsigned long long* keys, int* vals)
 {
     const double cells = 2097152.0;  // 2^21
-    const double S = (double)__uint_as_float(*ext) * 1.0001;
-    const double inv2S = S > 0.0 && isfinite(S) ? 0.5 / S : 0.5;
+    __shared__ double scale;         // (one FP64 division per block)
+    if (threadIdx.x == 0) {
+        const double S = (double)__uint_as_float(*ext) * 1.0001;
+        scale = S > 0.0 && isfinite(S) ? 0.5 / S : 0.5;
+    }
+    __syncthreads();
+    const double inv2S = scale;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         unsigned long long q[3];
         for (int k = 0; k < 3; ++k) {
-            double t = (X[3 * i + k] * inv2S + 0.5) * cells;
-            t = t < 0.0 ? 0.0 : (t > cells - 1.0 ? cells - 1.0 : t);
-            q[k] = isfinite(t) ? (unsigned long long)t : 0ull;
+            const double t = (X[3 * i + k] * inv2S + 0.5) * cells;
+            // clamped to [0, cells - 1]; not finite: NaN 0, +-Inf at the ends' cells
+            const long long b = __double_as_longlong(t);
+            int c = 0;
+            if (b >= __double_as_longlong(cells - 1.0)) c = t == t ? 2097151 : 0;
+            else if (b > 0) c = __double2int_rz(t);
+            q[k] = (unsigned long long)c;
         }
         keys[i] = (spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]);
-        vals[i] = (int)i;
+        if (vals) vals[i] = (int)i;
     }
+}
+
+// The stable order by counting: the rank of body i is the number of bodies j
+// with key_j < key_i, or key_j = key_i and j < i. A block ranks 32 bodies (a
+// lane each), its 8 warps count an eighth of the keys each (keys below 2^63:
+// "<=" is "< key + 1"). One launch of n^2 / 32 compares instead of a radix
+// sort's single block or chain of passes: 1500 bodies 16 -> 5.3 us. Every warp
+// reads each staged key once for its 32 bodies: shared-memory loads bound it.
+__global__ void __launch_bounds__(256) k_grav_rank(const unsigned long long* __restrict__ keys, int n, int* __restrict__ perm)
+{
+    constexpr int CH = 2048;  // keys staged at a time
+    __shared__ __align__(16) unsigned long long sk[CH];
+    __shared__ int rank[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i0 = blockIdx.x * 32, i = i0 + lane;
+    if (threadIdx.x < 32) rank[lane] = 0;
+    const unsigned long long key = i < n ? keys[i] : 0ull;
+    int cnt = 0;
+    for (int c0 = 0; c0 < n; c0 += CH) {
+        __syncthreads();
+        // (the largest key, behind the last, counts for nobody)
+        for (int k = threadIdx.x; k < CH; k += 256) sk[k] = c0 + k < n ? keys[c0 + k] : ~0ull;
+        __syncthreads();
+        const int m = min(CH, n - c0);
+        const int per = ((m + 7) / 8 + 1) & ~1;  // even: pairs of keys load as 16 bytes
+        const int b = w * per, e = min(m, b + per);
+        const int jb = c0 + b, je = c0 + e;
+        auto two = [&](int k, unsigned long long t0, unsigned long long t1) {
+            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(sk + k);
+            cnt += (q.x < t0) + (q.y < t1);
+        };
+        if (je <= i0 || jb >= i0 + 32) {  // all before the block's bodies, or all after
+            const unsigned long long t = key + (je <= i0 ? 1 : 0);
+#pragma unroll 8
+            for (int k = b; k < e; k += 2) two(k, t, t);
+        } else {
+            for (int k = b; k < e; ++k) cnt += sk[k] < key + (c0 + k < i ? 1 : 0);
+        }
+    }
+    atomicAdd(&rank[lane], cnt);
+    __syncthreads();
+    if (w == 0 && i < n) perm[rank[lane]] = i;
 }
 
 // The warp's box: (min x, y, z, largest |r|), (max x, y, z, smallest |r|) of
@@ -362,8 +424,9 @@ __device__ __forceinline__ void warp_box(bool real, float x, float y, float z, f
 // the boxes of each 32 slots (128 threads per block, npad a multiple of 128)
 __global__ void __launch_bounds__(GB) k_grav_pack_sorted(const double* __restrict__ X, const double* __restrict__ mass,
                                                          const int* __restrict__ perm, int64_t n, float4* phi, float4* plo,
-                                                         float4* box)
+                                                         float4* box, unsigned* ext)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ext = 0u;  // (ready for the next sort)
     const int64_t s = blockIdx.x * (int64_t)GB + threadIdx.x;
     const bool real = s < n;
     float h[3] = {0.f, 0.f, 0.f}, l[3];
@@ -396,6 +459,7 @@ struct GravStep {
     StepRef step;     // KICK: the step that ends
     int save;
     float4* box;      // null: none
+    unsigned* ext;    // not PACK: the extent for the sort that follows
 };
 
 template <bool KICK, bool PACK>
@@ -406,10 +470,12 @@ __global__ void __launch_bounds__(96) k_grav_step(Dev d, StateView s, GravStep A
     const int64_t slot = blockIdx.x * (int64_t)32 + lane;
     const bool real = slot < d.n;
     float h = 0.f;
+    double x = 0.0;
     if (real) {
         const int64_t i = A.perm ? A.perm[slot] : slot;
         const int64_t e = 3 * i + k;
-        double x = s.x[e], v = s.v[e], a = s.a_old[e];
+        x = s.x[e];
+        double v = s.v[e], a = s.a_old[e];
         if (KICK) {
             double t = 0.0;
             const double* p = A.part + 3 * slot + k;
@@ -442,6 +508,7 @@ __global__ void __launch_bounds__(96) k_grav_step(Dev d, StateView s, GravStep A
             reinterpret_cast<float*>(d.plo + slot)[k] = (float)(x - widen(h));
         }
     }
+    if (!PACK) extent_max(x, A.ext);
     if (!PACK || !A.box) return;
     sh[k][lane] = h;
     __syncthreads();
@@ -454,6 +521,13 @@ static int plan_gravity(nbg_ctx* c, int64_t npad)
 {
     int dev = c->device, sms = 0, occ = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // small systems: a body per thread spreads the pairs over twice the warps
+    // while even those leave SM sub-partitions without one (the packed form's
+    // arithmetic body by body, so the same bits): 1500 bodies 8.4 -> 6.5 us; a
+    // whole step, packed against spread: 2100 bodies 18.3 and 17.5 us, 3000
+    // 19.1 and 20.6.
+    // The chunks stay those of the packed form.
+    const bool spread = c->grav_variant == 1 && npad <= GRAV_SPREAD;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grav_variant(c->d.grav_plain, c->grav_variant, c->grav_uniform),
                                                   GB, 0);
     if (sms < 1) sms = 1;
@@ -473,39 +547,54 @@ static int plan_gravity(nbg_ctx* c, int64_t npad)
         }
         if (eff >= 0.97) break;
     }
+    if (spread) c->grav_variant = 4;
     return best;
 }
+
+// Up to this many bodies the order is counted (k_grav_rank), above it sorted.
+// A whole step, sorted against counted (one sort in 8 to 10 steps): 2000 bodies
+// 17.3 and 15.2 us, 8300 69 and 60, 12,000 114 and 106, 16,000 167 and 160;
+// the n^2 compares catch up with the sort soon after.
+#define GRAV_RANK_MAX 16384
+bool gravity_ranks(int64_t n) { return n <= GRAV_RANK_MAX; }
 
 // Whether the next gravity evaluation sorts the bodies afresh (every 8th: the
 // bodies move little in between).
 static bool grav_sorts(const nbg_ctx* c) { return c->grav_sort && (!c->grav_perm_valid || c->grav_evals % 8 == 0); }
 
 // The order and the sorted split positions and boxes of the next evaluation;
-// packed: the positions and boxes are in place for the current order.
-static int gravity_order(nbg_ctx* c, const StateView& s, bool packed)
+// packed: the positions and boxes are in place for the current order;
+// extent: the pass before left the extent of the positions.
+static int gravity_order(nbg_ctx* c, const StateView& s, bool packed, bool extent)
 {
     if (!c->grav_sort) return NBG_OK;
     if (grav_sorts(c)) {
         packed = false;
-        cudaError_t me = cudaMemsetAsync(c->grav_extent, 0, sizeof(unsigned), c->stream);
-        if (me != cudaSuccess) return cuda_fail(c, me, "gravity extent clear");
-        k_grav_extent<<<2 * c->sms, 256, 0, c->stream>>>(s.x, 3 * c->n, c->grav_extent);
-        NBG_LAUNCH_CHECK(c, "k_grav_extent");
-        k_grav_keys<<<grid_for(c->n, 256), 256, 0, c->stream>>>(s.x, c->n, c->grav_extent, c->grav_keys[0],
-                                                                 c->grav_vals[0]);
+        if (!extent) {
+            k_grav_extent<<<(unsigned)std::min<int64_t>(grid_for(3 * c->n, 256), 2 * c->sms), 256, 0, c->stream>>>(
+                s.x, 3 * c->n, c->grav_extent);
+            NBG_LAUNCH_CHECK(c, "k_grav_extent");
+        }
+        k_grav_keys<<<grid_for(c->n, 64), 64, 0, c->stream>>>(s.x, c->n, c->grav_extent, c->grav_keys[0],
+                                                               c->grav_vals[0]);
         NBG_LAUNCH_CHECK(c, "k_grav_keys");
-        size_t bytes = c->grav_sort_bytes;
-        cudaError_t e = cub::DeviceRadixSort::SortPairs(c->grav_sort_tmp, bytes, c->grav_keys[0], c->grav_keys[1],
-                                                        c->grav_vals[0], c->grav_vals[1], (int)c->n, 0, 63,
-                                                        c->stream);
-        if (e != cudaSuccess) return cuda_fail(c, e, "gravity Morton sort");
-        c->launches += 8;  // the sort's own passes
+        if (gravity_ranks(c->n)) {
+            k_grav_rank<<<(unsigned)((c->n + 31) / 32), 256, 0, c->stream>>>(c->grav_keys[0], (int)c->n, c->grav_vals[1]);
+            NBG_LAUNCH_CHECK(c, "k_grav_rank");
+        } else {
+            size_t bytes = c->grav_sort_bytes;
+            cudaError_t e = cub::DeviceRadixSort::SortPairs(c->grav_sort_tmp, bytes, c->grav_keys[0], c->grav_keys[1],
+                                                            c->grav_vals[0], c->grav_vals[1], (int)c->n, 0, 63,
+                                                            c->stream);
+            if (e != cudaSuccess) return cuda_fail(c, e, "gravity Morton sort");
+            c->launches += 8;  // the sort's own passes
+        }
         c->grav_perm_valid = true;
     }
     ++c->grav_evals;
     if (!packed) {
         k_grav_pack_sorted<<<(unsigned)(c->npad / GB), GB, 0, c->stream>>>(s.x, c->d.mass, c->grav_vals[1], c->n, c->d.phi,
-                                                                           c->d.plo, c->grav_box);
+                                                                           c->d.plo, c->grav_box, c->grav_extent);
         NBG_LAUNCH_CHECK(c, "k_grav_pack_sorted");
     }
     return NBG_OK;
@@ -515,7 +604,7 @@ static int gravity_order(nbg_ctx* c, const StateView& s, bool packed)
 static int gravity_pairs(nbg_ctx* c)
 {
     int64_t units = (c->npad / (grav_ti(c->grav_variant) * GB)) * c->grav_chunks;
-    const bool uniform = c->grav_uniform && grav_variant_packed(c->grav_variant);
+    const bool uniform = c->grav_uniform && grav_variant_uniform(c->grav_variant);
     grav_kernel_t kern = grav_variant(c->d.grav_plain, c->grav_variant, uniform);
     prof_begin(c);
     kern<<<(unsigned)units, GB, 0, c->stream>>>(c->d.phi, c->d.plo, c->n, c->npad, c->grav_chunks, c->grav_part,
@@ -527,7 +616,7 @@ static int gravity_pairs(nbg_ctx* c)
 
 static double gravity_factor(const nbg_ctx* c)
 {
-    return c->grav_uniform && grav_variant_packed(c->grav_variant) ? c->d.G * c->grav_m0 : c->d.G;
+    return c->grav_uniform && grav_variant_uniform(c->grav_variant) ? c->d.G * c->grav_m0 : c->d.G;
 }
 
 static int gravity_reduce(nbg_ctx* c, const StateView& s)
@@ -543,7 +632,7 @@ static int gravity_reduce(nbg_ctx* c, const StateView& s)
 int launch_gravity(nbg_ctx* c, const StateView& s)
 {
     int st;
-    if ((st = gravity_order(c, s, false))) return st;
+    if ((st = gravity_order(c, s, false, false))) return st;
     if ((st = gravity_pairs(c))) return st;
     return gravity_reduce(c, s);
 }
@@ -564,6 +653,7 @@ int launch_gravity_step(nbg_ctx* c, const StateView& s, double dt, StepRef sr, b
     A.step = sr;
     A.save = c->sink_on ? 1 : 0;
     A.box = c->grav_sort ? c->grav_box : nullptr;
+    A.ext = c->grav_extent;
     const bool pack = !grav_sorts(c);
     const unsigned grid = (unsigned)(c->npad / 32);
     if (first && !c->grav_perm_valid) A.perm = nullptr;  // (no order yet: it sorts next)
@@ -576,7 +666,7 @@ int launch_gravity_step(nbg_ctx* c, const StateView& s, double dt, StepRef sr, b
     }
     NBG_LAUNCH_CHECK(c, "k_grav_step");
     int st;
-    if ((st = gravity_order(c, s, pack))) return st;
+    if ((st = gravity_order(c, s, pack, !pack))) return st;
     if ((st = gravity_pairs(c))) return st;
     return last ? gravity_reduce(c, s) : NBG_OK;
 }

@@ -607,14 +607,16 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
         if ((st = dalloc(c, &c->grav_part, (size_t)c->grav_chunks * 3 * n))) return st;
         if (!c->d.grav_plain && !getenv("NBG_GRAVITY_NO_SORT")) {
             c->grav_sort = true;
-            for (int k = 0; k < 2; ++k) {
-                if ((st = dalloc(c, &c->grav_keys[k], n))) return st;
-                if ((st = dalloc(c, &c->grav_vals[k], n))) return st;
+            if ((st = dalloc(c, &c->grav_keys[0], n + (n & 1)))) return st;
+            if ((st = dalloc(c, &c->grav_vals[1], n))) return st;
+            if (!gravity_ranks(n)) {
+                if ((st = dalloc(c, &c->grav_keys[1], n))) return st;
+                if ((st = dalloc(c, &c->grav_vals[0], n))) return st;
+                c->grav_sort_bytes = gravity_sort_bytes(n);
+                unsigned char* tmp = nullptr;
+                if ((st = dalloc(c, &tmp, c->grav_sort_bytes))) return st;
+                c->grav_sort_tmp = tmp;
             }
-            c->grav_sort_bytes = gravity_sort_bytes(n);
-            unsigned char* tmp = nullptr;
-            if ((st = dalloc(c, &tmp, c->grav_sort_bytes))) return st;
-            c->grav_sort_tmp = tmp;
             if ((st = dalloc(c, &c->grav_box, 2 * (c->npad / 32)))) return st;
             if ((st = dalloc(c, &c->grav_extent, 1))) return st;
         }

@@ -446,6 +446,7 @@ int launch_save_frame(nbg_ctx* c, const StateView& s, StepRef sr);
 int launch_rhs_thermostat(nbg_ctx* c, const StateView& s);
 int gravity_plan_chunks(nbg_ctx* c, int64_t npad);
 size_t gravity_sort_bytes(int64_t n);
+bool gravity_ranks(int64_t n);  // the Morton order is counted, not sorted
 int launch_energy(nbg_ctx* c, const StateView& s, double* out_host /*[8], the last one the status word*/);
 int launch_pairs(nbg_ctx* c, const StateView& s, int which, int* out_j, int* out_cnt, int64_t cap_per_atom);
 

@@ -6,14 +6,15 @@
 // many steps in one launch:
 //   - CTA r owns atoms [r per, (r+1) per); its threads drift them (FP64, the
 //     reference's velocity-Verlet arithmetic) and split the new positions
-//     into its shared memory, in the buffer of the step's parity; one thread
-//     sends the contiguous range to every other CTA's same buffer as two bulk
+//     into its shared memory, in the buffer of the step's parity; a thread
+//     per peer sends the contiguous range to that CTA's same buffer as two bulk
 //     asynchronous copies (cp.async.bulk, distributed shared memory), which
-//     complete as transaction bytes on the receiver's mbarrier of that parity;
-//   - one cluster barrier per step (release/acquire) orders the rebuild flags
-//     and the FP64 copies, then every CTA waits (bounded) for its mbarrier;
-//     with two parity buffers, a copy of step s+2 can only start after the
-//     barrier of step s+1, when every CTA is done reading step s;
+//     complete as transaction bytes on the receiver's mbarrier of that parity,
+//     then arrives there (release): the arrival carries the rebuild flag and
+//     the FP64 copies. No barrier of the whole cluster: a CTA waits (bounded)
+//     for its mbarrier alone. With two parity buffers that orders the reuse
+//     too: a peer sends step s+2 after it has received this CTA's step s+1,
+//     which this CTA sends when all its threads are done reading step s;
 //   - each CTA keeps the Verlet lists of its own atoms in shared memory,
 //     rebuilt from the shared positions (all atoms scanned, the FP32 superset
 //     test of the list builders) when any atom moved more than skin/2 since
@@ -23,13 +24,20 @@
 //     state), else it builds first;
 //   - at its start a launch writes x, v, a_old of its atoms to the backup,
 //     from which the host undoes a launch that timed out or overflowed;
-//   - LPA lanes per atom evaluate the pairs (pair_cutoff: the exact pair set;
+//   - LPA lanes per atom evaluate the pairs (cl_pair: the exact pair set;
 //     the ambiguous ones read FP64 positions, which the drift also writes to
 //     a global copy of the step's parity, through L2) and join their
 //     partials (compensated FP32) into shared memory; the atom's owner thread,
 //     which keeps its x, v, a in registers for the whole launch, kicks the
 //     velocity at the start of the next step.
 // Every thread of every CTA passes the same cluster barriers (no early exit).
+//
+// Cycles per step and CTA at 1000 LJ atoms (63 per CTA, 16 lanes each), before
+// and after the cluster barrier of every step gave way to the arrivals, the
+// constants came from the constant bank and the pair lost its branches: kick
+// and drift 7100 and 4500 (FP64, two warps per SM sub-partition), exchange
+// 5100 and 4000, list build, over its ~9 steps, 4300 and 3300, forces 7200 and 5000;
+// 200 steps 2.24 ms and 1.81.
 //
 // The same kernel with ACCEL evaluates the right-hand side alone (nbg_accel):
 // the positions come from src (pinned host memory read over the CPU-GPU
@@ -73,11 +81,32 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned a, unsigned parity)
 {
     unsigned ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(a), "r"(parity)
         : "memory");
     return ok != 0;
+}
+
+// arrival on another CTA's mbarrier: this thread's writes, and those it has
+// seen through a block barrier, are visible to who waits for the phase
+__device__ __forceinline__ void mbar_arrive_peer(unsigned mbar_cluster)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mbar_cluster) : "memory");
+}
+
+// block barrier of the first `threads` threads, with an OR
+__device__ __forceinline__ bool owners_sync_or(unsigned threads, bool v)
+{
+    unsigned r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, %2, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(r)
+        : "r"((unsigned)v), "r"(threads)
+        : "memory");
+    return r != 0;
 }
 
 // bytes (a multiple of 16, 16-byte aligned ends) of this CTA's shared memory
@@ -94,12 +123,67 @@ __device__ __forceinline__ void bulk_copy_to_peer(unsigned dst_cluster, unsigned
 
 #define CL_WAIT_TRIES (1u << 16)
 
+__device__ __forceinline__ bool mbar_wait(unsigned a, unsigned parity)
+{
+    unsigned tries = 0;
+    while (!mbar_try_wait(a, parity))
+        if (++tries >= CL_WAIT_TRIES) return false;
+    return true;
+}
+
+// The force on i of listed atom j, in pair_cutoff's arithmetic and
+// classification without its branches (only a pair that FP32 does not decide
+// takes one), added to p. A potential system: every listed pair has both
+// potentials of POTS.
+template <int POTS>
+__device__ __forceinline__ void cl_pair(const Dev& d, const RepDev& R, int i, int j, const float4& hi_i, const float4& lo_i,
+                                        const float4& hi_j, const float4& lo_j, float kqi, const double* X, float (&p)[3],
+                                        bool& range_err)
+{
+    constexpr bool LJ = (POTS & NBG_POT_LJ) != 0, EL = (POTS & NBG_POT_EL) != 0;
+    float3 dr = split_diff(hi_i, lo_i, hi_j, lo_j, true, R);
+    float r2 = __fmaf_rn(dr.x, dr.x, __fmaf_rn(dr.y, dr.y, __fmul_rn(dr.z, dr.z)));
+    bool lj = LJ && r2 < R.lj_lo, el = EL && r2 < R.el_lo;
+    if ((LJ && !lj && r2 < R.lj_hi) || (EL && !el && r2 < R.el_hi)) {
+        Dist64 q;
+        if (!distance64<true>(X + 3 * i, X + 3 * j, NBG_BC_CUBIC, R, q)) {
+            range_err = true;
+            return;
+        }
+        lj = LJ && q.r2 < d.lj_R2;
+        el = EL && q.r2 < d.el_R2;
+        dr = make_float3((float)q.x, (float)q.y, (float)q.z);
+        r2 = (float)q.r2;
+    }
+    const float rr = lj || el ? r2 : 1.0f;
+    float f = 0.0f;
+    if (LJ) {
+        const float ri = rcp_ftz(rr);
+        const float s2 = __fmul_rn(d.lj_sig2, ri);
+        const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+        const float s12 = __fmul_rn(s6, s6);
+        const float g = __fmul_rn(d.lj_eps24, __fmul_rn(__fmaf_rn(2.0f, s12, -s6), ri));
+        f = lj ? g : 0.0f;
+    }
+    if (EL) {
+        const float rb = rsqrt_ftz(rr);
+        const float t = __fmaf_rn(__fmul_rn(rb, rb), rb, -d.el_krf2);
+        const float g = __fmaf_rn(__fmul_rn(kqi, hi_j.w), t, f);
+        f = el ? g : f;
+    }
+    p[0] = __fadd_rn(p[0], __fmul_rn(f, dr.x));
+    p[1] = __fadd_rn(p[1], __fmul_rn(f, dr.y));
+    p[2] = __fadd_rn(p[2], __fmul_rn(f, dr.z));
+}
+
 // Shared memory (dynamic): split positions [parity][hi, lo][n] (float4), the
 // own atoms' positions at the last list build [per][3] (double, padded to a 16-byte end), their lists
 // [per][cap], counts [per] (int) and force partials [per][6] (float: h, e per
 // component).
-template <int LPA, bool ACCEL>
-__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s, double* xb, double dt, int nsteps,
+// R: the replica's constants as a kernel argument (operands from the constant
+// bank; through d.reps every use was a load again, as the kernel stores).
+template <int LPA, bool ACCEL, int POTS>
+__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __grid_constant__ RepDev R, StateView s, double* xb, double dt, int nsteps,
                                                               int rebuild_every, int per, int cap, int* lst_g,
                                                               int* cnt_g, double* xref_g, int* since_g, int reuse,
                                                               int64_t step0, int save, int drop_step,
@@ -116,18 +200,12 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     int* cnt = lst + (size_t)per * cap;
     float* fsum = reinterpret_cast<float*>(cnt + per);
     __shared__ unsigned flag[2];  // rebuild requests of the step of each parity
-    __shared__ int build_s;
     __shared__ __align__(8) unsigned long long mbar[2];  // other CTAs' positions of each parity arrived
-    __shared__ int wait_failed;  // a bounded wait of this CTA ran out (this step)
-    __shared__ int abort_s;      // some CTA's wait ran out: every CTA leaves after the next cluster barrier
-    const RepDev& R = d.reps[0];
-    const PairK K(R);
+    __shared__ int abort_s;      // some CTA's wait ran out
     const int tid = threadIdx.x;
     const int a0 = rank * per;
     const int na = max(0, min(n - a0, per));
     const int g = tid / LPA, lane = tid % LPA;  // lane group g <-> own atom a0 + g
-    const unsigned gshift = (unsigned)((tid & 31) / LPA * LPA);
-    const unsigned gmask = (LPA == 32 ? 0xffffffffu : ((1u << LPA) - 1u));
     const double dtsq = dt * dt;
     const float magic = 12582912.0f;  // 1.5 * 2^23: rint by addition
 
@@ -137,6 +215,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     const int k = (tid & 31) % 3;
     const int ko = (tid >> 5) * 10 + (tid & 31) / 3;
     const bool owner = (tid & 31) < 30 && ko < na;
+    const int owners = (per + 9) / 10 * 32;  // threads of the warps that own atoms
     const int io = owner ? a0 + ko : 0;
     const size_t eo = 3 * (size_t)io + k;
     double x = owner ? (ACCEL ? src[eo] : s.x[eo]) : 0.0;
@@ -176,10 +255,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     }
     if (tid < 2) flag[tid] = 0u;
     if (tid == 0) {
-        wait_failed = 0;
         abort_s = 0;
-        mbar_init(smem_addr(&mbar[0]), 1);
-        mbar_init(smem_addr(&mbar[1]), 1);
+        mbar_init(smem_addr(&mbar[0]), C);  // an arrival per CTA
+        mbar_init(smem_addr(&mbar[1]), C);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // every CTA of the cluster is running (and initialised) before any
@@ -187,9 +265,18 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     cl.sync();
 
     // the frame sink (trajectory saving): state of time index step0 + st;
-    // its other fields are read at a save point
+    // its other fields are read at a save point, `unsaved` steps ahead
     const int64_t sk_every = save && owner ? d.sink->every : 0;
     const int64_t sk_t0 = save && owner ? d.sink->t0 : 0;
+    int64_t unsaved = 0;
+    if (sk_every > 0) {
+        const int64_t over = (step0 - sk_t0) % sk_every;
+        unsaved = over < 0 ? -over : sk_every - over;
+    }
+    // the FP32 sum of squares of a displacement below this is one below
+    // (skin/2)^2 in FP64 (the FP32 sum is within 5e-7 of it)
+    const float still2 = d.skin_half2 > 1e-30 ? (float)d.skin_half2 * (1.0f - 4e-6f) : 0.0f;
+    int timed_out = -1;  // the step whose wait ran out
 
     for (int st = 0; st <= nsteps; ++st) {
         // kick of the previous step with the forces its groups left in fsum
@@ -205,7 +292,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
             if (!finite64(an)) status_set(d.status, ST_NONFINITE);
             v = kick1(v, a, an, dt);
             a = an;
-            if (sk_every > 0 && (step0 + st - sk_t0) % sk_every == 0) {
+            if (sk_every > 0 && --unsaved == 0) {
+                unsaved = sk_every;
                 const FrameSink* sk = d.sink;
                 const int64_t slot = (step0 + st - sk_t0) / sk_every - sk->first;
                 if (slot >= 0 && slot < sk->cap) {
@@ -220,113 +308,110 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
         float4* ph = cl_pos + (2 * par) * (size_t)n;
         float4* pl = ph + n;
         double* X = xb + (size_t)par * 3 * n;  // FP64 positions of this step
+        const unsigned mb = smem_addr(&mbar[par]);
         // drift, split and displacement check of the own atoms
-        double dk = 0.0;
-        if (owner) {
-            if (!ACCEL) x = drift1(x, v, a, dt, dtsq);
-            X[eo] = x;
-            float h, l;
-            split_component(d, R, x, h, l);
-            reinterpret_cast<float*>(ph + io)[k] = h;
-            reinterpret_cast<float*>(pl + io)[k] = l;
-            // (a launch that does not reuse lists builds at step 0, which
-            // sets xref_s)
-            dk = x - xref_s[3 * ko + k];
-        }
-        const double dy = __shfl_down_sync(0xffffffffu, dk, 1), dz = __shfl_down_sync(0xffffffffu, dk, 2);
-        const bool moved =
-            owner && k == 0 && (st > 0 || reuse) && !(dk * dk + dy * dy + dz * dz <= d.skin_half2);
-        // the owners' generic writes become visible to the bulk-copy engine
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const int any_moved = __syncthreads_or(moved ? 1 : 0);
-        // the own atoms' split positions (contiguous hi and lo ranges) go to
-        // every other CTA as two bulk copies each, completing on its mbarrier
-        // of this parity; this CTA expects the other (n - na) atoms' 32 bytes
-        if (tid == 0) {
-            const unsigned mb = smem_addr(&mbar[par]);
-            mbar_arrive_expect_tx(mb, (unsigned)(n - na) * 32u);
-            // (drop_step: a host-set test of the timeout path; no CTA sends
-            // that step's positions, so its waits run out with nothing in flight)
-            if (na > 0 && st != drop_step) {
-                const unsigned sh = smem_addr(ph + a0), sl = smem_addr(pl + a0), bytes = (unsigned)na * 16u;
-                for (int r = 0; r < C; ++r) {
-                    if (r == rank) continue;
-                    const unsigned rmb = cluster_addr(mb, r);
-                    bulk_copy_to_peer(cluster_addr(sh, r), sh, bytes, rmb);
-                    bulk_copy_to_peer(cluster_addr(sl, r), sl, bytes, rmb);
+        if (tid < owners) {
+            double dk = 0.0;
+            if (owner) {
+                if (!ACCEL) x = drift1(x, v, a, dt, dtsq);
+                X[eo] = x;
+                float h, l;
+                split_component(d, R, x, h, l);
+                reinterpret_cast<float*>(ph + io)[k] = h;
+                reinterpret_cast<float*>(pl + io)[k] = l;
+                // (a launch that does not reuse lists builds at step 0, which
+                // sets xref_s)
+                dk = x - xref_s[3 * ko + k];
+            }
+            const float fk = (float)dk, fk2 = fk * fk;
+            const float f2 = fk2 + __shfl_down_sync(0xffffffffu, fk2, 1) + __shfl_down_sync(0xffffffffu, fk2, 2);
+            bool moved = owner && k == 0 && (st > 0 || reuse) && !(f2 < still2);
+            if (__any_sync(0xffffffffu, moved)) {
+                const double dy = __shfl_down_sync(0xffffffffu, dk, 1), dz = __shfl_down_sync(0xffffffffu, dk, 2);
+                moved = moved && !(dk * dk + dy * dy + dz * dz <= d.skin_half2);
+            }
+            // the owners' generic writes become visible to the bulk-copy engine
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            const bool any_moved = owners_sync_or((unsigned)owners, moved);
+            // the own atoms' split positions (contiguous hi and lo ranges) go to
+            // every other CTA as two bulk copies each, completing on its mbarrier
+            // of this parity; this CTA expects the other (n - na) atoms' 32 bytes
+            if (tid < 32) {
+                // every thread has read the last step's flag; peers write it
+                // again only after the arrivals below
+                if (tid == 0) flag[par ^ 1] = 0u;
+                __syncwarp();
+                if (tid < C) {
+                    if (any_moved) *cl.map_shared_rank(&flag[par], tid) = 1u;
+                    if (tid == rank) {
+                        mbar_arrive_expect_tx(mb, (unsigned)(n - na) * 32u);
+                    } else {
+                        const unsigned rmb = cluster_addr(mb, tid);
+                        // (drop_step: a host-set test of the timeout path; no CTA sends
+                        // that step's positions, so its waits run out with nothing in flight)
+                        if (na > 0 && st != drop_step) {
+                            const unsigned sh = smem_addr(ph + a0), sl = smem_addr(pl + a0), bytes = (unsigned)na * 16u;
+                            bulk_copy_to_peer(cluster_addr(sh, tid), sh, bytes, rmb);
+                            bulk_copy_to_peer(cluster_addr(sl, tid), sl, bytes, rmb);
+                        }
+                        mbar_arrive_peer(rmb);
+                    }
                 }
             }
-        }
-        if (any_moved && tid < C) *cl.map_shared_rank(&flag[par], tid) = 1u;
-        // arrive (release) / wait (acquire) at cluster scope: the rebuild
-        // flags, the FP64 copies X and an abort raised in the previous step
-        // are visible past it
-        cl.sync();
-        const unsigned mb_cur = smem_addr(&mbar[par]), phase_cur = (unsigned)((st >> 1) & 1);
-        if (abort_s) {
-            // every CTA saw the same flag after the same barrier: leave the
-            // step loop together, once this step's incoming copies (sent
-            // before the barrier) have landed (bounded)
-            unsigned tries = 0;
-            while (!mbar_try_wait(mb_cur, phase_cur) && ++tries < CL_WAIT_TRIES) {
-            }
-            break;
         }
         // the other CTAs' positions of this step: the k-th use of mbar[par]
-        // completes phase k (bounded wait; a timeout is reported as
-        // ST_TIMEOUT and ends the launch at the next cluster barrier)
-        {
-            unsigned tries = 0;
-            while (!mbar_try_wait(mb_cur, phase_cur)) {
-                if (++tries >= CL_WAIT_TRIES) {
-                    wait_failed = 1;
-                    break;
-                }
-            }
+        // completes phase k. A wait that ran out ends this CTA's loop (and, as
+        // it sends no further step, the others' at their next wait)
+        if (__syncthreads_or(mbar_wait(mb, (unsigned)((st >> 1) & 1)) ? 0 : 1)) {
+            if (tid == 0) status_set(d.status, ST_TIMEOUT);
+            if (tid < C) *cl.map_shared_rank(&abort_s, tid) = 1;
+            timed_out = st;
+            break;
         }
-        __syncthreads();
-        if (tid == 0 && wait_failed) {
-            status_set(d.status, ST_TIMEOUT);
-            for (int r = 0; r < C; ++r) *cl.map_shared_rank(&abort_s, r) = 1;
-        }
-        if (tid == 0) {
-            build_s = ((st == 0 && !reuse) || flag[par] != 0u || (rebuild_every > 0 && since >= rebuild_every)) ? 1 : 0;
-            // the next writes to flag[par] come at step st + 2, after the
-            // barrier of step st + 1, which this CTA passes only later
-            flag[par] = 0u;
-        }
-        __syncthreads();
-        if (build_s) {
-            // lists of the own atoms: group g scans every atom j (lane-strided),
-            // entries in j order (ballot-compacted)
-            const bool active = g < na;
-            const int i = active ? a0 + g : 0;
-            const float4 hi = ph[i];
-            int c0 = 0;
-            for (int jb = 0; jb < n; jb += LPA) {
-                const int j = jb + lane;
-                bool take = false;
-                if (active && j < n && j != i) {
-                    const float4 hj = ph[j];
-                    float dx = hj.x - hi.x, dy = hj.y - hi.y, dz = hj.z - hi.z;
-                    dx = __fmaf_rn(-__fsub_rn(__fmaf_rn(dx, R.invLf, magic), magic), R.Lh, dx);
-                    dy = __fmaf_rn(-__fsub_rn(__fmaf_rn(dy, R.invLf, magic), magic), R.Lh, dy);
-                    dz = __fmaf_rn(-__fsub_rn(__fmaf_rn(dz, R.invLf, magic), magic), R.Lh, dz);
-                    take = dx * dx + dy * dy + dz * dz < R.rl2;
+        const bool build = (st == 0 && !reuse) || *(volatile unsigned*)&flag[par] != 0u ||
+                           (rebuild_every > 0 && since >= rebuild_every);
+        if (build) {
+            // lists of the own atoms, entries in j order (ballot-compacted): a
+            // warp tests 32 atoms j at a time against the atoms of its groups
+            constexpr int A = 32 / LPA;
+            const int ga = (tid >> 5) * A, ln = tid & 31;
+            if (ga < na) {
+                float hx[A], hy[A], hz[A];
+                int c0[A];
+#pragma unroll
+                for (int q = 0; q < A; ++q) {
+                    const float4 h = ph[a0 + min(ga + q, na - 1)];
+                    hx[q] = h.x;
+                    hy[q] = h.y;
+                    hz[q] = h.z;
+                    c0[q] = 0;
                 }
-                const unsigned m = (__ballot_sync(0xffffffffu, take) >> gshift) & gmask;
-                if (take) {
-                    const int q = c0 + __popc(m & ((1u << lane) - 1u));
-                    if (q < cap) lst[g * cap + q] = j;
+                for (int jb = 0; jb < n; jb += 32) {
+                    const int j = jb + ln;
+                    const float4 hj = ph[min(j, n - 1)];
+#pragma unroll
+                    for (int q = 0; q < A; ++q) {
+                        float dx = hj.x - hx[q], dy = hj.y - hy[q], dz = hj.z - hz[q];
+                        dx = __fmaf_rn(-__fsub_rn(__fmaf_rn(dx, R.invLf, magic), magic), R.Lh, dx);
+                        dy = __fmaf_rn(-__fsub_rn(__fmaf_rn(dy, R.invLf, magic), magic), R.Lh, dy);
+                        dz = __fmaf_rn(-__fsub_rn(__fmaf_rn(dz, R.invLf, magic), magic), R.Lh, dz);
+                        const bool take = j < n && j != a0 + ga + q && dx * dx + dy * dy + dz * dz < R.rl2;
+                        const unsigned m = __ballot_sync(0xffffffffu, take);
+                        const int t = c0[q] + __popc(m & ((1u << ln) - 1u));
+                        if (take && t < cap && ga + q < na) lst[(ga + q) * cap + t] = j;
+                        c0[q] += __popc(m);
+                    }
                 }
-                c0 += __popc(m);
-            }
-            if (active && lane == 0) {
-                if (c0 > cap) {
-                    status_set(d.status, ST_NBR_OVERFLOW);
-                    c0 = cap;
+#pragma unroll
+                for (int q = 0; q < A; ++q) {
+                    if (ln == 0 && ga + q < na) {
+                        if (c0[q] > cap) {
+                            status_set(d.status, ST_NBR_OVERFLOW);
+                            c0[q] = cap;
+                        }
+                        cnt[ga + q] = c0[q];
+                    }
                 }
-                cnt[g] = c0;
             }
             if (owner) xref_s[3 * ko + k] = x;
             since = 0;
@@ -340,19 +425,16 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
             const bool active = g < na;
             const int i = active ? a0 + g : 0;
             const float4 hi_i = ph[i], lo_i = pl[i];
-            const float kqi = (d.pots & NBG_POT_EL) ? (float)(d.el_k_d * d.charge[i]) : 0.0f;
+            const float kqi = (POTS & NBG_POT_EL) ? (float)(d.el_k_d * d.charge[i]) : 0.0f;
             const int c = active ? cnt[g] : 0;
-            float px = 0.f, py = 0.f, pz = 0.f;
+            float p[3] = {0.f, 0.f, 0.f};
             bool range_err = false;
+#pragma unroll 2
             for (int k = lane; k < c; k += LPA) {
                 const int j = dbg_index(lst[g * cap + k], d.n, i, d.status);
-                const PairOut o = pair_cutoff<true>(d, R, K, i, j, hi_i, lo_i, ph[j], pl[j], kqi, X);
-                range_err |= o.range_err;
-                px += o.fx;
-                py += o.fy;
-                pz += o.fz;
+                cl_pair<POTS>(d, R, i, j, hi_i, lo_i, ph[j], pl[j], kqi, X, p, range_err);
             }
-            const LaneSum f = lane_sums3<LPA>(px, py, pz, lane);
+            const LaneSum f = lane_sums3<LPA>(p[0], p[1], p[2], lane);
             if (range_err) status_set(d.status, ST_RANGE);
             if (active && f.writer) {
                 fsum[6 * g + 2 * f.comp] = f.h;
@@ -364,8 +446,17 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
         __syncthreads();
     }
     // every CTA has waited for all copies into its shared memory, so after
-    // this barrier no copy reads a CTA's shared memory any more: all may exit
+    // this barrier no copy reads a CTA's shared memory any more: all may exit.
+    // After a timeout (every CTA sees it past the barrier) copies of the step
+    // that it broke off at and of the next may still be on their way: one more
+    // bounded wait for each
     cl.sync();
+    if (abort_s) {
+        if (timed_out >= 0) {
+            for (int q = timed_out; q < timed_out + 2; ++q) mbar_wait(smem_addr(&mbar[q & 1]), (unsigned)((q >> 1) & 1));
+        }
+        cl.sync();
+    }
     if (owner && !ACCEL) {
         s.x[eo] = x;
         s.v[eo] = v;
@@ -386,16 +477,27 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, StateView s
     if (!ACCEL && rank == 0 && tid == 0) *since_g = since;
 }
 
-typedef void (*cluster_kernel_t)(Dev, StateView, double*, double, int, int, int, int, int*, int*, double*, int*, int, int64_t,
+typedef void (*cluster_kernel_t)(Dev, RepDev, StateView, double*, double, int, int, int, int, int*, int*, double*, int*, int, int64_t,
                                  int, int, double*, const double*, double*);
 
-static cluster_kernel_t cluster_kernel(int lpa, bool accel = false)
+template <int LPA>
+static cluster_kernel_t cluster_kernel_pots(int pots, bool accel)
+{
+    switch (pots & (NBG_POT_LJ | NBG_POT_EL)) {
+    case NBG_POT_LJ: return accel ? k_cluster_vv<LPA, true, NBG_POT_LJ> : k_cluster_vv<LPA, false, NBG_POT_LJ>;
+    case NBG_POT_EL: return accel ? k_cluster_vv<LPA, true, NBG_POT_EL> : k_cluster_vv<LPA, false, NBG_POT_EL>;
+    default:
+        return accel ? k_cluster_vv<LPA, true, NBG_POT_LJ | NBG_POT_EL> : k_cluster_vv<LPA, false, NBG_POT_LJ | NBG_POT_EL>;
+    }
+}
+
+// (at most 128 atoms per CTA: 8 lanes each at least)
+static cluster_kernel_t cluster_kernel(const nbg_ctx* c, int lpa, bool accel = false)
 {
     switch (lpa) {
-    case 4: return accel ? k_cluster_vv<4, true> : k_cluster_vv<4, false>;
-    case 8: return accel ? k_cluster_vv<8, true> : k_cluster_vv<8, false>;
-    case 16: return accel ? k_cluster_vv<16, true> : k_cluster_vv<16, false>;
-    default: return accel ? k_cluster_vv<32, true> : k_cluster_vv<32, false>;
+    case 8: return cluster_kernel_pots<8>(c->d.pots, accel);
+    case 16: return cluster_kernel_pots<16>(c->d.pots, accel);
+    default: return cluster_kernel_pots<32>(c->d.pots, accel);
     }
 }
 
@@ -416,12 +518,12 @@ bool cluster_plan(nbg_ctx* c)
         const int per = (n + C - 1) / C;
         if (per > 128) continue;  // owner threads: 4 warps x 32 lanes
         int lpa = 32;
-        while (lpa > 4 && per * lpa > CL_THREADS) lpa /= 2;
+        while (lpa > 8 && per * lpa > CL_THREADS) lpa /= 2;
         if (per * lpa > CL_THREADS) continue;
         const size_t bytes = sizeof(float4) * 4 * (size_t)n + sizeof(double) * (3 * (size_t)per + ((3 * per) & 1)) +
                              sizeof(int) * ((size_t)per * cap + per) + sizeof(float) * 6 * (size_t)per;
         if (bytes > 200 * 1024) continue;
-        cluster_kernel_t k = cluster_kernel(lpa), ka = cluster_kernel(lpa, true);
+        cluster_kernel_t k = cluster_kernel(c, lpa), ka = cluster_kernel(c, lpa, true);
         bool attrs_ok = true;
         for (cluster_kernel_t f : {k, ka}) {
             attrs_ok = attrs_ok &&
@@ -463,7 +565,7 @@ bool cluster_plan(nbg_ctx* c)
 int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps, int rebuild_every, int64_t step0,
                       unsigned* status)
 {
-    cluster_kernel_t k = cluster_kernel(c->cluster_lpa);
+    cluster_kernel_t k = cluster_kernel(c, c->cluster_lpa);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -488,7 +590,7 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
     Dev d = c->d;
     d.status = status;
     prof_begin(c);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, s, c->cluster_x, dt, (int)nsteps, rebuild_every,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], s, c->cluster_x, dt, (int)nsteps, rebuild_every,
                                        c->cluster_per, c->cluster_cap, c->cluster_lists, c->cluster_cnt,
                                        c->cluster_xref, c->cluster_since, c->cluster_lists_valid ? 1 : 0, step0,
                                        c->sink_on ? 1 : 0, drop, c->bk, (const double*)nullptr, (double*)nullptr);
@@ -504,7 +606,7 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
 // own lists reused while no atom moved more than skin/2 from their build.
 int launch_cluster_accel(nbg_ctx* c, const double* u, double* dv, unsigned* status)
 {
-    cluster_kernel_t k = cluster_kernel(c->cluster_lpa, true);
+    cluster_kernel_t k = cluster_kernel(c, c->cluster_lpa, true);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -520,7 +622,7 @@ int launch_cluster_accel(nbg_ctx* c, const double* u, double* dv, unsigned* stat
     Dev d = c->d;
     d.status = status;
     prof_begin(c);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->st, c->cluster_x, 0.0, 1, 0, c->cluster_per, c->cluster_cap,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], c->st, c->cluster_x, 0.0, 1, 0, c->cluster_per, c->cluster_cap,
                                        c->cla_lists, c->cla_cnt, c->cla_xref, c->cluster_since,
                                        c->cla_valid ? 1 : 0, (int64_t)0, 0, -2, c->bk, u, dv);
     prof_end(c);

@@ -5,16 +5,19 @@
 // not arithmetic, set its pace. Here the cluster's CTAs (up to 16 SMs) run
 // many steps in one launch:
 //   - CTA r owns atoms [r per, (r+1) per); its threads drift them (FP64, the
-//     reference's velocity-Verlet arithmetic) and split the new positions
-//     into its shared memory, in the buffer of the step's parity; a thread
-//     per peer sends the contiguous range to that CTA's same buffer as two bulk
-//     asynchronous copies (cp.async.bulk, distributed shared memory), which
-//     complete as transaction bytes on the receiver's mbarrier of that parity,
-//     then arrives there (release): the arrival carries the rebuild flag and
-//     the FP64 copies. No barrier of the whole cluster: a CTA waits (bounded)
-//     for its mbarrier alone. With two parity buffers that orders the reuse
-//     too: a peer sends step s+2 after it has received this CTA's step s+1,
-//     which this CTA sends when all its threads are done reading step s;
+//     reference's velocity-Verlet arithmetic) and write the new positions, split
+//     and FP64, to global buffers of the step's parity; a thread per peer then
+//     arrives (release) at that CTA's mbarrier of the parity, after setting
+//     its rebuild flag where an atom moved too far;
+//   - a CTA waits (bounded) for its own mbarrier alone, no barrier of the whole
+//     cluster, and reads all split positions through L2 into shared memory.
+//     (Sent from SM to SM, as bulk copies into the peers' shared memory, the
+//     30 KB per CTA and step at 1000 atoms took 3000 cycles, 10 bytes per
+//     cycle, whether one thread issued the copies or seven warps did. Through
+//     L2 it is about the same, but the threads' work between runs faster.)
+//     With two parity buffers the arrivals order
+//     their reuse too: a CTA writes step s+2 after it has received every
+//     peer's step s+1, which a peer sends when its threads are done with step s;
 //   - each CTA keeps the Verlet lists of its own atoms in shared memory,
 //     rebuilt from the shared positions (all atoms scanned, the FP32 superset
 //     test of the list builders) when any atom moved more than skin/2 since
@@ -34,10 +37,11 @@
 //
 // Cycles per step and CTA at 1000 LJ atoms (63 per CTA, 16 lanes each), before
 // and after the cluster barrier of every step gave way to the arrivals, the
-// constants came from the constant bank and the pair lost its branches: kick
-// and drift 7100 and 4500 (FP64, two warps per SM sub-partition), exchange
-// 5100 and 4000, list build, over its ~9 steps, 4300 and 3300, forces 7200 and 5000;
-// 200 steps 2.24 ms and 1.81.
+// constants came from the constant bank, the pair lost its branches and the
+// build its counts per test: kick and drift 7100 and 3700 (FP64, two warps per
+// SM sub-partition), exchange 5100 and 3900 (three L2 round trips), list
+// build, over its ~9 steps, 4300 and 2150, forces 7200 and 5000; 200 steps
+// 2.24 ms and 1.58.
 //
 // The same kernel with ACCEL evaluates the right-hand side alone (nbg_accel):
 // the positions come from src (pinned host memory read over the CPU-GPU
@@ -56,7 +60,7 @@ namespace cg = cooperative_groups;
 #define CL_THREADS 1024
 #define CL_MAX 16
 
-// mbarrier and bulk-copy helpers (shared-memory addresses as 32-bit
+// mbarrier helpers (shared-memory addresses as 32-bit
 // shared-window offsets; remote ones from mapa)
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -70,11 +74,6 @@ __device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank)
 __device__ __forceinline__ void mbar_init(unsigned a, unsigned count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned a, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(unsigned a, unsigned parity)
@@ -107,18 +106,6 @@ __device__ __forceinline__ bool owners_sync_or(unsigned threads, bool v)
         : "r"((unsigned)v), "r"(threads)
         : "memory");
     return r != 0;
-}
-
-// bytes (a multiple of 16, 16-byte aligned ends) of this CTA's shared memory
-// to another CTA's, completing as transaction bytes on that CTA's mbarrier
-__device__ __forceinline__ void bulk_copy_to_peer(unsigned dst_cluster, unsigned src, unsigned bytes,
-                                                  unsigned mbar_cluster)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            dst_cluster),
-        "r"(src), "r"(bytes), "r"(mbar_cluster)
-        : "memory");
 }
 
 #define CL_WAIT_TRIES (1u << 16)
@@ -176,14 +163,41 @@ __device__ __forceinline__ void cl_pair(const Dev& d, const RepDev& R, int i, in
     p[2] = __fadd_rn(p[2], __fmul_rn(f, dr.z));
 }
 
-// Shared memory (dynamic): split positions [parity][hi, lo][n] (float4), the
+// Shared memory (dynamic): split positions [hi, lo][n] (float4), the
 // own atoms' positions at the last list build [per][3] (double, padded to a 16-byte end), their lists
 // [per][cap], counts [per] (int) and force partials [per][6] (float: h, e per
 // component).
+static size_t cluster_smem(int n, int per, int cap)
+{
+    return sizeof(float4) * 2 * (size_t)n + sizeof(double) * (3 * (size_t)per + ((3 * per) & 1)) +
+           sizeof(int) * ((size_t)per * cap + per) + sizeof(float) * 6 * (size_t)per;
+}
+
+// split_component under cubic boundaries, given the box image img (the floor of
+// p / L) of the last step: while the wrapped position keeps clear of both
+// faces the image is the same and the floor (with its product a sixth of a
+// step's FP64 time per component) is not taken. Images too large for p / L to be
+// that exact are not kept (NaN).
+__device__ __forceinline__ void split_kept_image(const RepDev& R, double p, double& img, float& h, float& l)
+{
+    double w = fma(-R.L, img, p);
+    // L 2^-20 <= w < L (1 - 2^-21), by the high words (positive doubles order like integers)
+    const int hL = __double2hiint(R.L), lo = hL - (20 << 20);
+    if ((unsigned)(__double2hiint(w) - lo) >= (unsigned)(hL - 1 - lo)) {
+        img = floor(p * R.invL);
+        w = fma(-R.L, img, p);
+        if (negative64(w)) w += R.L;
+        if (__double_as_longlong(w) >= __double_as_longlong(R.L)) w -= R.L;
+        if (!(fabs(img) < 1048576.0)) img = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    grid_split(R, w, h, l);
+}
+
 // R: the replica's constants as a kernel argument (operands from the constant
 // bank; through d.reps every use was a load again, as the kernel stores).
 template <int LPA, bool ACCEL, int POTS>
-__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __grid_constant__ RepDev R, StateView s, double* xb, double dt, int nsteps,
+__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __grid_constant__ RepDev R, StateView s, double* xb,
+                                                              float4* xs, double dt, int nsteps,
                                                               int rebuild_every, int per, int cap, int* lst_g,
                                                               int* cnt_g, double* xref_g, int* since_g, int reuse,
                                                               int64_t step0, int save, int drop_step,
@@ -195,13 +209,14 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
     const int C = (int)cl.num_blocks();
     const int n = (int)d.n;
     extern __shared__ float4 cl_pos[];
-    double* xref_s = reinterpret_cast<double*>(cl_pos + 4 * (size_t)n);
+    float4* const ph = cl_pos;
+    float4* const pl = ph + n;
+    double* xref_s = reinterpret_cast<double*>(cl_pos + 2 * (size_t)n);
     int* lst = reinterpret_cast<int*>(xref_s + 3 * (size_t)per + ((3 * per) & 1));  // 16-byte aligned
     int* cnt = lst + (size_t)per * cap;
     float* fsum = reinterpret_cast<float*>(cnt + per);
     __shared__ unsigned flag[2];  // rebuild requests of the step of each parity
-    __shared__ __align__(8) unsigned long long mbar[2];  // other CTAs' positions of each parity arrived
-    __shared__ int abort_s;      // some CTA's wait ran out
+    __shared__ __align__(8) unsigned long long mbar[2];  // the CTAs' positions of each parity are written
     const int tid = threadIdx.x;
     const int a0 = rank * per;
     const int na = max(0, min(n - a0, per));
@@ -231,13 +246,10 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
         bk[2 * seg + eo] = a;
     }
 
-    // the static w parts (charge, atom flags) of every atom in both parities
-    for (int j = tid; j < n; j += CL_THREADS) {
-        const float wh = d.phi[j].w, wl = d.plo[j].w;
-        for (int p = 0; p < 2; ++p) {
-            cl_pos[(2 * p) * (size_t)n + j].w = wh;
-            cl_pos[(2 * p + 1) * (size_t)n + j].w = wl;
-        }
+    // the static w parts (charge, atom flags) of the own atoms in both parities
+    for (int t = tid; t < 4 * na; t += CL_THREADS) {
+        const int j = a0 + (t >> 2);
+        xs[(size_t)(t & 3) * n + j].w = (t & 1) ? d.plo[j].w : d.phi[j].w;
     }
     int since = 0;
     bool built = false;  // a list build ran in this launch (the same in every CTA)
@@ -255,7 +267,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
     }
     if (tid < 2) flag[tid] = 0u;
     if (tid == 0) {
-        abort_s = 0;
         mbar_init(smem_addr(&mbar[0]), C);  // an arrival per CTA
         mbar_init(smem_addr(&mbar[1]), C);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -276,7 +287,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
     // the FP32 sum of squares of a displacement below this is one below
     // (skin/2)^2 in FP64 (the FP32 sum is within 5e-7 of it)
     const float still2 = d.skin_half2 > 1e-30 ? (float)d.skin_half2 * (1.0f - 4e-6f) : 0.0f;
-    int timed_out = -1;  // the step whose wait ran out
+    double img = __longlong_as_double(0x7ff8000000000000ll);  // the component's box image (not known)
 
     for (int st = 0; st <= nsteps; ++st) {
         // kick of the previous step with the forces its groups left in fsum
@@ -305,8 +316,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
         }
         if (st == nsteps) break;  // uniform: every thread leaves after the last kick
         const int par = st & 1;
-        float4* ph = cl_pos + (2 * par) * (size_t)n;
-        float4* pl = ph + n;
+        float4* const P = xs + (size_t)(2 * par) * n;  // split positions of this step
         double* X = xb + (size_t)par * 3 * n;  // FP64 positions of this step
         const unsigned mb = smem_addr(&mbar[par]);
         // drift, split and displacement check of the own atoms
@@ -316,9 +326,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
                 if (!ACCEL) x = drift1(x, v, a, dt, dtsq);
                 X[eo] = x;
                 float h, l;
-                split_component(d, R, x, h, l);
-                reinterpret_cast<float*>(ph + io)[k] = h;
-                reinterpret_cast<float*>(pl + io)[k] = l;
+                split_kept_image(R, x, img, h, l);
+                reinterpret_cast<float*>(P + io)[k] = h;
+                reinterpret_cast<float*>(P + n + io)[k] = l;
                 // (a launch that does not reuse lists builds at step 0, which
                 // sets xref_s)
                 dk = x - xref_s[3 * ko + k];
@@ -330,49 +340,37 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
                 const double dy = __shfl_down_sync(0xffffffffu, dk, 1), dz = __shfl_down_sync(0xffffffffu, dk, 2);
                 moved = moved && !(dk * dk + dy * dy + dz * dz <= d.skin_half2);
             }
-            // the owners' generic writes become visible to the bulk-copy engine
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            // every thread has read the last step's flag; peers write it again
+            // only after this step's arrivals
+            if (tid == 0) flag[par ^ 1] = 0u;
             const bool any_moved = owners_sync_or((unsigned)owners, moved);
-            // the own atoms' split positions (contiguous hi and lo ranges) go to
-            // every other CTA as two bulk copies each, completing on its mbarrier
-            // of this parity; this CTA expects the other (n - na) atoms' 32 bytes
-            if (tid < 32) {
-                // every thread has read the last step's flag; peers write it
-                // again only after the arrivals below
-                if (tid == 0) flag[par ^ 1] = 0u;
-                __syncwarp();
-                if (tid < C) {
-                    if (any_moved) *cl.map_shared_rank(&flag[par], tid) = 1u;
-                    if (tid == rank) {
-                        mbar_arrive_expect_tx(mb, (unsigned)(n - na) * 32u);
-                    } else {
-                        const unsigned rmb = cluster_addr(mb, tid);
-                        // (drop_step: a host-set test of the timeout path; no CTA sends
-                        // that step's positions, so its waits run out with nothing in flight)
-                        if (na > 0 && st != drop_step) {
-                            const unsigned sh = smem_addr(ph + a0), sl = smem_addr(pl + a0), bytes = (unsigned)na * 16u;
-                            bulk_copy_to_peer(cluster_addr(sh, tid), sh, bytes, rmb);
-                            bulk_copy_to_peer(cluster_addr(sl, tid), sl, bytes, rmb);
-                        }
-                        mbar_arrive_peer(rmb);
-                    }
-                }
+            // (drop_step: a host-set test of the timeout path; no CTA arrives for
+            // that step, so every wait runs out)
+            if (tid < C && st != drop_step) {
+                if (any_moved) *cl.map_shared_rank(&flag[par], tid) = 1u;
+                mbar_arrive_peer(cluster_addr(mb, tid));
             }
         }
-        // the other CTAs' positions of this step: the k-th use of mbar[par]
-        // completes phase k. A wait that ran out ends this CTA's loop (and, as
-        // it sends no further step, the others' at their next wait)
-        if (__syncthreads_or(mbar_wait(mb, (unsigned)((st >> 1) & 1)) ? 0 : 1)) {
+        // all positions of this step (the k-th use of mbar[par] completes phase
+        // k). A wait that ran out ends this CTA's loop and, as it arrives for
+        // no further step, the others' at their next wait
+        const bool ok = mbar_wait(mb, (unsigned)((st >> 1) & 1));
+        if (ok) {
+#pragma unroll 2
+            for (int t = tid; t < 2 * n; t += CL_THREADS) cl_pos[t] = __ldcg(P + t);
+        }
+        if (__syncthreads_or(ok ? 0 : 1)) {
             if (tid == 0) status_set(d.status, ST_TIMEOUT);
-            if (tid < C) *cl.map_shared_rank(&abort_s, tid) = 1;
-            timed_out = st;
             break;
         }
         const bool build = (st == 0 && !reuse) || *(volatile unsigned*)&flag[par] != 0u ||
                            (rebuild_every > 0 && since >= rebuild_every);
         if (build) {
-            // lists of the own atoms, entries in j order (ballot-compacted): a
-            // warp tests 32 atoms j at a time against the atoms of its groups
+            // lists of the own atoms, entries in j order: a warp tests 32 atoms j
+            // at a time against the atoms of its groups, 1024 in a row, and
+            // lane t keeps the t-th mask of hits; the masks' entries are then
+            // placed by a prefix sum over the lanes (a count per mask and test
+            // was a third of the build)
             constexpr int A = 32 / LPA;
             const int ga = (tid >> 5) * A, ln = tid & 31;
             if (ga < na) {
@@ -386,20 +384,43 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
                     hz[q] = h.z;
                     c0[q] = 0;
                 }
-                for (int jb = 0; jb < n; jb += 32) {
-                    const int j = jb + ln;
-                    const float4 hj = ph[min(j, n - 1)];
+                for (int j0 = 0; j0 < n; j0 += 1024) {
+                    unsigned hits[A];
+#pragma unroll
+                    for (int q = 0; q < A; ++q) hits[q] = 0u;
+                    const int tests = min(32, (n - j0 + 31) >> 5);
+#pragma unroll 2
+                    for (int t = 0; t < tests; ++t) {
+                        const float4 hj = ph[min(j0 + t * 32 + ln, n - 1)];
+#pragma unroll
+                        for (int q = 0; q < A; ++q) {
+                            float dx = hj.x - hx[q], dy = hj.y - hy[q], dz = hj.z - hz[q];
+                            dx = __fmaf_rn(-__fsub_rn(__fmaf_rn(dx, R.invLf, magic), magic), R.Lh, dx);
+                            dy = __fmaf_rn(-__fsub_rn(__fmaf_rn(dy, R.invLf, magic), magic), R.Lh, dy);
+                            dz = __fmaf_rn(-__fsub_rn(__fmaf_rn(dz, R.invLf, magic), magic), R.Lh, dz);
+                            const unsigned m = __ballot_sync(0xffffffffu, dx * dx + dy * dy + dz * dz < R.rl2);
+                            if (ln == t) hits[q] = m;
+                        }
+                    }
+                    const int jl = j0 + ln * 32;  // the first atom of this lane's masks
 #pragma unroll
                     for (int q = 0; q < A; ++q) {
-                        float dx = hj.x - hx[q], dy = hj.y - hy[q], dz = hj.z - hz[q];
-                        dx = __fmaf_rn(-__fsub_rn(__fmaf_rn(dx, R.invLf, magic), magic), R.Lh, dx);
-                        dy = __fmaf_rn(-__fsub_rn(__fmaf_rn(dy, R.invLf, magic), magic), R.Lh, dy);
-                        dz = __fmaf_rn(-__fsub_rn(__fmaf_rn(dz, R.invLf, magic), magic), R.Lh, dz);
-                        const bool take = j < n && j != a0 + ga + q && dx * dx + dy * dy + dz * dz < R.rl2;
-                        const unsigned m = __ballot_sync(0xffffffffu, take);
-                        const int t = c0[q] + __popc(m & ((1u << ln) - 1u));
-                        if (take && t < cap && ga + q < na) lst[(ga + q) * cap + t] = j;
-                        c0[q] += __popc(m);
+                        unsigned m = hits[q];
+                        const int self = a0 + ga + q - jl, left = n - jl;
+                        if (self >= 0 && self < 32) m &= ~(1u << self);
+                        if (left < 32) m &= left > 0 ? (1u << left) - 1u : 0u;
+                        int sum = __popc(m);
+                        const int own = sum;
+#pragma unroll
+                        for (int o = 1; o < 32; o *= 2) {
+                            const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                            if (ln >= o) sum += up;
+                        }
+                        int at = c0[q] + sum - own;
+                        if (ga + q < na) {
+                            for (; m != 0u && at < cap; m &= m - 1u, ++at) lst[(ga + q) * cap + at] = jl + __ffs(m) - 1;
+                        }
+                        c0[q] += __shfl_sync(0xffffffffu, sum, 31);
                     }
                 }
 #pragma unroll
@@ -445,18 +466,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
         // barrier, no cluster barrier
         __syncthreads();
     }
-    // every CTA has waited for all copies into its shared memory, so after
-    // this barrier no copy reads a CTA's shared memory any more: all may exit.
-    // After a timeout (every CTA sees it past the barrier) copies of the step
-    // that it broke off at and of the next may still be on their way: one more
-    // bounded wait for each
+    // all flags and arrivals are in: no CTA's shared memory is written to any more
     cl.sync();
-    if (abort_s) {
-        if (timed_out >= 0) {
-            for (int q = timed_out; q < timed_out + 2; ++q) mbar_wait(smem_addr(&mbar[q & 1]), (unsigned)((q >> 1) & 1));
-        }
-        cl.sync();
-    }
     if (owner && !ACCEL) {
         s.x[eo] = x;
         s.v[eo] = v;
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
     if (!ACCEL && rank == 0 && tid == 0) *since_g = since;
 }
 
-typedef void (*cluster_kernel_t)(Dev, RepDev, StateView, double*, double, int, int, int, int, int*, int*, double*, int*, int, int64_t,
+typedef void (*cluster_kernel_t)(Dev, RepDev, StateView, double*, float4*, double, int, int, int, int, int*, int*, double*, int*, int, int64_t,
                                  int, int, double*, const double*, double*);
 
 template <int LPA>
@@ -520,9 +531,10 @@ bool cluster_plan(nbg_ctx* c)
         int lpa = 32;
         while (lpa > 8 && per * lpa > CL_THREADS) lpa /= 2;
         if (per * lpa > CL_THREADS) continue;
-        const size_t bytes = sizeof(float4) * 4 * (size_t)n + sizeof(double) * (3 * (size_t)per + ((3 * per) & 1)) +
-                             sizeof(int) * ((size_t)per * cap + per) + sizeof(float) * 6 * (size_t)per;
-        if (bytes > 200 * 1024) continue;
+        const size_t bytes = cluster_smem(n, per, cap);
+        // (two position buffers' worth: with lists longer than this leaves room
+        // for, the step graphs serve the system)
+        if (bytes + sizeof(float4) * 2 * (size_t)n > 200 * 1024) continue;
         cluster_kernel_t k = cluster_kernel(c, lpa), ka = cluster_kernel(c, lpa, true);
         bool attrs_ok = true;
         for (cluster_kernel_t f : {k, ka}) {
@@ -590,7 +602,7 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
     Dev d = c->d;
     d.status = status;
     prof_begin(c);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], s, c->cluster_x, dt, (int)nsteps, rebuild_every,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], s, c->cluster_x, c->cluster_split, dt, (int)nsteps, rebuild_every,
                                        c->cluster_per, c->cluster_cap, c->cluster_lists, c->cluster_cnt,
                                        c->cluster_xref, c->cluster_since, c->cluster_lists_valid ? 1 : 0, step0,
                                        c->sink_on ? 1 : 0, drop, c->bk, (const double*)nullptr, (double*)nullptr);
@@ -622,7 +634,7 @@ int launch_cluster_accel(nbg_ctx* c, const double* u, double* dv, unsigned* stat
     Dev d = c->d;
     d.status = status;
     prof_begin(c);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], c->st, c->cluster_x, 0.0, 1, 0, c->cluster_per, c->cluster_cap,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], c->st, c->cluster_x, c->cluster_split, 0.0, 1, 0, c->cluster_per, c->cluster_cap,
                                        c->cla_lists, c->cla_cnt, c->cla_xref, c->cluster_since,
                                        c->cla_valid ? 1 : 0, (int64_t)0, 0, -2, c->bk, u, dv);
     prof_end(c);

@@ -634,6 +634,7 @@ static int plan_cluster(nbg_ctx* c)
     if (!cluster_plan(c)) return NBG_OK;
     int st;
     if (!c->cluster_x && (st = dalloc(c, &c->cluster_x, 6 * (size_t)c->n))) return st;
+    if (!c->cluster_split && (st = dalloc(c, &c->cluster_split, 4 * (size_t)c->n))) return st;
     for (int** p : {&c->cluster_lists, &c->cluster_cnt, &c->cla_lists, &c->cla_cnt}) {
         if (*p) dfree(c, *p);
         *p = nullptr;

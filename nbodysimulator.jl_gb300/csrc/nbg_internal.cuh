@@ -265,6 +265,7 @@ struct nbg_ctx {
     int cluster_size = 0, cluster_per = 0, cluster_lpa = 0, cluster_cap = 0;
     size_t cluster_bytes = 0;
     double* cluster_x = nullptr;  // FP64 positions of the two step parities [2][3n]
+    float4* cluster_split = nullptr;  // and split ones [2][hi, lo][n]
     // the lists a cluster launch leaves for the next ([CTA][per][cap], counts,
     // steps since the build); valid only while nothing else changed the state
     int* cluster_lists = nullptr;

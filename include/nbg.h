@@ -274,18 +274,17 @@ NBG_API int nbg_force_kernel_time(nbg_ctx* ctx, double* total_ms, int64_t* launc
 /*
  * Small systems (no reference counterpart): one potential system under cubic
  * boundaries without thermostat, up to 2048 atoms, runs velocity Verlet as one
- * persistent launch per chunk of steps over a thread-block cluster (the
- * positions shared in distributed shared memory, one cluster barrier per
- * step) instead of a CUDA graph of kernels. Returns 1 and the cluster's CTAs
+ * persistent cooperative launch per chunk of steps over a group of CTAs (the
+ * positions exchanged through L2 as tagged records) instead of a CUDA graph
+ * of kernels. Returns 1 and the group's CTAs
  * and lanes per atom when the context uses it, 0 otherwise (either pointer
  * may be NULL). The environment variable NBG_NO_CLUSTER, read at creation,
  * keeps such a system on the graph step loop.
  */
 NBG_API int nbg_cluster_shape(nbg_ctx* ctx, int32_t* ctas, int32_t* lanes);
 
-/* The launch floor of that cluster shape (measurement): an empty kernel with
- * the same CTAs, threads, shared memory and cluster, which passes one
- * cluster barrier, timed with CUDA events on the context's stream: 200
+/* The launch floor of that shape (measurement): an empty kernel with
+ * the same CTAs, threads and shared memory, launched the same way, timed with CUDA events on the context's stream: 200
  * launches back to back (*us_per_launch) and 200 one at a time with the host
  * waiting for each (*us_single). NBG_ERR_UNSUPPORTED off the cluster path. */
 NBG_API int nbg_cluster_launch_floor(nbg_ctx* ctx, double* us_single, double* us_per_launch);

@@ -1,23 +1,21 @@
 // k_cluster.cu - velocity Verlet for small systems (up to 2048 atoms) as one
-// persistent launch over a thread-block cluster.
+// persistent cooperative launch.
 //
 // A step of a small system is a handful of microsecond kernels, so launches,
-// not arithmetic, set its pace. Here the cluster's CTAs (up to 16 SMs) run
-// many steps in one launch:
+// not arithmetic, set its pace. Here up to 64 co-resident CTAs run many steps
+// in one launch:
 //   - CTA r owns atoms [r per, (r+1) per); its threads drift them (FP64, the
-//     reference's velocity-Verlet arithmetic) and write the new positions, split
-//     and FP64, to global buffers of the step's parity; a thread per peer then
-//     arrives (release) at that CTA's mbarrier of the parity, after setting
-//     its rebuild flag where an atom moved too far;
-//   - a CTA waits (bounded) for its own mbarrier alone, no barrier of the whole
-//     cluster, and reads all split positions through L2 into shared memory.
-//     (Sent from SM to SM, as bulk copies into the peers' shared memory, the
-//     30 KB per CTA and step at 1000 atoms took 3000 cycles, 10 bytes per
-//     cycle, whether one thread issued the copies or seven warps did. Through
-//     L2 it is about the same, but the threads' work between runs faster.)
-//     With two parity buffers the arrivals order
-//     their reuse too: a CTA writes step s+2 after it has received every
-//     peer's step s+1, which a peer sends when its threads are done with step s;
+//     reference's velocity-Verlet arithmetic) and write each atom's new split
+//     position as two 16-byte records (hi, tag) and (lo, tag) to the global
+//     buffer of the step's parity. The tag is the step's number over all
+//     launches and, as its lowest bit, whether the atom moved too far for the
+//     lists. FP64 positions follow as records of their own;
+//   - every CTA reads all records through L2 into its shared memory, again
+//     (bounded) while a tag is not the step's. 16-byte accesses are single
+//     ones, so a record with the right tag is whole: no barrier, flag or
+//     fence between the CTAs. With two parity buffers their reuse is ordered
+//     too: a CTA writes step s+2 after it has read every step s+1 record,
+//     and a peer writes those when all its threads are done with step s;
 //   - each CTA keeps the Verlet lists of its own atoms in shared memory,
 //     rebuilt from the shared positions (all atoms scanned, the FP32 superset
 //     test of the list builders) when any atom moved more than skin/2 since
@@ -27,21 +25,22 @@
 //     state), else it builds first;
 //   - at its start a launch writes x, v, a_old of its atoms to the backup,
 //     from which the host undoes a launch that timed out or overflowed;
-//   - LPA lanes per atom evaluate the pairs (cl_pair: the exact pair set;
-//     the ambiguous ones read FP64 positions, which the drift also writes to
-//     a global copy of the step's parity, through L2) and join their
+//   - LPA lanes per atom evaluate the pairs (cl_pairs: the exact pair set;
+//     the ambiguous ones read the FP64 records) and join their
 //     partials (compensated FP32) into shared memory; the atom's owner thread,
 //     which keeps its x, v, a in registers for the whole launch, kicks the
 //     velocity at the start of the next step.
-// Every thread of every CTA passes the same cluster barriers (no early exit).
 //
-// Cycles per step and CTA at 1000 LJ atoms (63 per CTA, 16 lanes each), before
-// and after the cluster barrier of every step gave way to the arrivals, the
-// constants came from the constant bank, the pair lost its branches and the
-// build its counts per test: kick and drift 7100 and 3700 (FP64, two warps per
-// SM sub-partition), exchange 5100 and 3900 (three L2 round trips), list
-// build, over its ~9 steps, 4300 and 2150, forces 7200 and 5000; 200 steps
-// 2.24 ms and 1.58.
+// Two exchanges were measured before this one, both in a cluster of 16 CTAs:
+// bulk copies into the peers' shared memory, and global buffers with an arrival
+// (release) at each peer's mbarrier. Either took ~3900 cycles per step at
+// 1000 atoms (10 bytes per cycle from SM to SM; three L2 round trips), and 16
+// SMs left the pairs 5000 cycles, kick and drift (FP64) 3700 and the list
+// build, over its ~9 steps, 2150. The records take 4000 cycles among 63 CTAs
+// (two or three rounds of reads), the rest 1800, 2300 and 850. Step times at
+// 500, 1000 and 2000 atoms: 128 threads per CTA 3.6, 4.4, 6.9 us, 256: 3.4, 4.3,
+// 6.6, 512: 3.8, 4.8, 8.5, 1024: 5.3, 7.6, 14.4. 200 steps of 1000 atoms: 2.24 ms
+// with the cluster's barrier in every step, 1.58 with arrivals, 1.09 now.
 //
 // The same kernel with ACCEL evaluates the right-hand side alone (nbg_accel):
 // the positions come from src (pinned host memory read over the CPU-GPU
@@ -51,116 +50,145 @@
 // calls' positions, and the resident state is not touched.
 #include <algorithm>
 
-#include <cooperative_groups.h>
-
 #include "nbg_internal.cuh"
 
-namespace cg = cooperative_groups;
+#define CL_THREADS 256  // up to 64 CTAs
 
-#define CL_THREADS 1024
-#define CL_MAX 16
-
-// mbarrier helpers (shared-memory addresses as 32-bit
-// shared-window offsets; remote ones from mapa)
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank)
+// A 16-byte record as one access (single-copy atomic), at L2.
+__device__ __forceinline__ ulonglong2 rec_load(const ulonglong2* p)
 {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    ulonglong2 r;
+    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+                 : "=l"(r.x), "=l"(r.y)
+                 : "l"(p)
+                 : "memory");
     return r;
 }
 
-__device__ __forceinline__ void mbar_init(unsigned a, unsigned count)
+__device__ __forceinline__ void rec_store(ulonglong2* p, unsigned long long x, unsigned long long y)
 {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
+    asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x),
+                 "l"(y)
+                 : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(unsigned a, unsigned parity)
+// three floats and their record's tag
+__device__ __forceinline__ void rec_store3(ulonglong2* p, float x, float y, float z, unsigned tag)
 {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    return ok != 0;
+    rec_store(p, (unsigned long long)__float_as_uint(x) | (unsigned long long)__float_as_uint(y) << 32,
+              (unsigned long long)__float_as_uint(z) | (unsigned long long)tag << 32);
 }
 
-// arrival on another CTA's mbarrier: this thread's writes, and those it has
-// seen through a block barrier, are visible to who waits for the phase
-__device__ __forceinline__ void mbar_arrive_peer(unsigned mbar_cluster)
-{
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mbar_cluster) : "memory");
-}
+#define CL_TRIES (1u << 18)  // reads of a record before a launch gives up
 
-// block barrier of the first `threads` threads, with an OR
-__device__ __forceinline__ bool owners_sync_or(unsigned threads, bool v)
-{
-    unsigned r;
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, %2, p;\n"
-        " selp.u32 %0, 1, 0, q;\n}"
-        : "=r"(r)
-        : "r"((unsigned)v), "r"(threads)
-        : "memory");
-    return r != 0;
-}
-
-#define CL_WAIT_TRIES (1u << 16)
-
-__device__ __forceinline__ bool mbar_wait(unsigned a, unsigned parity)
+// The FP64 position of an atom of this step (three records (bits, tag)).
+__device__ __forceinline__ bool rec_position(const ulonglong2* X, unsigned tag, double (&x)[3])
 {
     unsigned tries = 0;
-    while (!mbar_try_wait(a, parity))
-        if (++tries >= CL_WAIT_TRIES) return false;
+    for (int k = 0; k < 3; ++k) {
+        ulonglong2 r = rec_load(X + k);
+        while ((unsigned)r.y != tag) {
+            if (++tries >= CL_TRIES) return false;
+            r = rec_load(X + k);
+        }
+        x[k] = __longlong_as_double((long long)r.x);
+    }
     return true;
 }
 
-// The force on i of listed atom j, in pair_cutoff's arithmetic and
-// classification without its branches (only a pair that FP32 does not decide
-// takes one), added to p. A potential system: every listed pair has both
+// A pair that FP32 does not decide, by the FP64 records (out of line: rare).
+struct ClExact {
+    float x, y, z, r2;
+    int in;  // 1: inside lj_R2, 2: inside el_R2, 4: image not found, 8: a record did not come
+};
+
+__device__ __noinline__ ClExact cl_exact(const ulonglong2* X, unsigned tag, int i, int j, double L, double lj_R2, double el_R2)
+{
+    ClExact o = {0.f, 0.f, 0.f, 1.f, 0};
+    double xi[3], xj[3];
+    if (!rec_position(X + 3 * i, tag, xi) || !rec_position(X + 3 * j, tag, xj)) {
+        o.in = 8;
+        return o;
+    }
+    double x = __dsub_rn(xi[0], xj[0]), y = __dsub_rn(xi[1], xj[1]), z = __dsub_rn(xi[2], xj[2]);
+    const double radius = __dmul_rn(0.5, L);
+    if (!(wrap_cubic64(x, L, radius) && wrap_cubic64(y, L, radius) && wrap_cubic64(z, L, radius))) {
+        o.in = 4;
+        return o;
+    }
+    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+    o.x = (float)x;
+    o.y = (float)y;
+    o.z = (float)z;
+    o.r2 = (float)r2;
+    o.in = (r2 < lj_R2 ? 1 : 0) | (r2 < el_R2 ? 2 : 0);
+    return o;
+}
+
+// The forces on i of M listed atoms j[] (the first m of them), in
+// pair_cutoff's arithmetic and classification, added to p in order. One branch for
+// all, to the pairs that FP32 does not decide: with one per pair a lane's
+// pairs did not overlap, and there are only two warps per SM sub-partition
+// to hide a pair's latency. A potential system: every listed pair has both
 // potentials of POTS.
+#define CL_M 3
 template <int POTS>
-__device__ __forceinline__ void cl_pair(const Dev& d, const RepDev& R, int i, int j, const float4& hi_i, const float4& lo_i,
-                                        const float4& hi_j, const float4& lo_j, float kqi, const double* X, float (&p)[3],
-                                        bool& range_err)
+__device__ __forceinline__ void cl_pairs(const Dev& d, const RepDev& R, int i, const int (&j)[CL_M], int m, const float4& hi_i,
+                                         const float4& lo_i, const float4* ph, const float4* pl, float kqi,
+                                         const ulonglong2* X, unsigned tag, float (&p)[3], bool& range_err)
 {
     constexpr bool LJ = (POTS & NBG_POT_LJ) != 0, EL = (POTS & NBG_POT_EL) != 0;
-    float3 dr = split_diff(hi_i, lo_i, hi_j, lo_j, true, R);
-    float r2 = __fmaf_rn(dr.x, dr.x, __fmaf_rn(dr.y, dr.y, __fmul_rn(dr.z, dr.z)));
-    bool lj = LJ && r2 < R.lj_lo, el = EL && r2 < R.el_lo;
-    if ((LJ && !lj && r2 < R.lj_hi) || (EL && !el && r2 < R.el_hi)) {
-        Dist64 q;
-        if (!distance64<true>(X + 3 * i, X + 3 * j, NBG_BC_CUBIC, R, q)) {
-            range_err = true;
-            return;
+    float3 dr[CL_M];
+    float r2[CL_M], qj[CL_M];
+    bool lj[CL_M], el[CL_M], open[CL_M], any = false;
+#pragma unroll
+    for (int q = 0; q < CL_M; ++q) {
+        const float4 hj = ph[j[q]], lj4 = pl[j[q]];
+        qj[q] = hj.w;
+        dr[q] = split_diff(hi_i, lo_i, hj, lj4, true, R);
+        r2[q] = __fmaf_rn(dr[q].x, dr[q].x, __fmaf_rn(dr[q].y, dr[q].y, __fmul_rn(dr[q].z, dr[q].z)));
+        lj[q] = LJ && r2[q] < R.lj_lo;
+        el[q] = EL && r2[q] < R.el_lo;
+        open[q] = q < m && ((LJ && !lj[q] && r2[q] < R.lj_hi) || (EL && !el[q] && r2[q] < R.el_hi));
+        any |= open[q];
+    }
+    if (any) {
+#pragma unroll
+        for (int q = 0; q < CL_M; ++q) {
+            if (!open[q]) continue;
+            const ClExact e = cl_exact(X, tag, i, j[q], R.L, d.lj_R2, d.el_R2);
+            lj[q] = LJ && (e.in & 1);
+            el[q] = EL && (e.in & 2);
+            dr[q] = make_float3(e.x, e.y, e.z);
+            r2[q] = e.r2;
+            range_err |= (e.in & 4) != 0;
+            if (e.in & 8) status_set(d.status, ST_TIMEOUT);
         }
-        lj = LJ && q.r2 < d.lj_R2;
-        el = EL && q.r2 < d.el_R2;
-        dr = make_float3((float)q.x, (float)q.y, (float)q.z);
-        r2 = (float)q.r2;
     }
-    const float rr = lj || el ? r2 : 1.0f;
-    float f = 0.0f;
-    if (LJ) {
-        const float ri = rcp_ftz(rr);
-        const float s2 = __fmul_rn(d.lj_sig2, ri);
-        const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
-        const float s12 = __fmul_rn(s6, s6);
-        const float g = __fmul_rn(d.lj_eps24, __fmul_rn(__fmaf_rn(2.0f, s12, -s6), ri));
-        f = lj ? g : 0.0f;
+#pragma unroll
+    for (int q = 0; q < CL_M; ++q) {
+        const float rr = lj[q] || el[q] ? r2[q] : 1.0f;
+        float f = 0.0f;
+        if (LJ) {
+            const float ri = rcp_ftz(rr);
+            const float s2 = __fmul_rn(d.lj_sig2, ri);
+            const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+            const float s12 = __fmul_rn(s6, s6);
+            const float g = __fmul_rn(d.lj_eps24, __fmul_rn(__fmaf_rn(2.0f, s12, -s6), ri));
+            f = lj[q] ? g : 0.0f;
+        }
+        if (EL) {
+            const float rb = rsqrt_ftz(rr);
+            const float t = __fmaf_rn(__fmul_rn(rb, rb), rb, -d.el_krf2);
+            const float g = __fmaf_rn(__fmul_rn(kqi, qj[q]), t, f);
+            f = el[q] ? g : f;
+        }
+        if (q < m) {
+            p[0] = __fadd_rn(p[0], __fmul_rn(f, dr[q].x));
+            p[1] = __fadd_rn(p[1], __fmul_rn(f, dr[q].y));
+            p[2] = __fadd_rn(p[2], __fmul_rn(f, dr[q].z));
+        }
     }
-    if (EL) {
-        const float rb = rsqrt_ftz(rr);
-        const float t = __fmaf_rn(__fmul_rn(rb, rb), rb, -d.el_krf2);
-        const float g = __fmaf_rn(__fmul_rn(kqi, hi_j.w), t, f);
-        f = el ? g : f;
-    }
-    p[0] = __fadd_rn(p[0], __fmul_rn(f, dr.x));
-    p[1] = __fadd_rn(p[1], __fmul_rn(f, dr.y));
-    p[2] = __fadd_rn(p[2], __fmul_rn(f, dr.z));
 }
 
 // Shared memory (dynamic): split positions [hi, lo][n] (float4), the
@@ -196,17 +224,15 @@ __device__ __forceinline__ void split_kept_image(const RepDev& R, double p, doub
 // R: the replica's constants as a kernel argument (operands from the constant
 // bank; through d.reps every use was a load again, as the kernel stores).
 template <int LPA, bool ACCEL, int POTS>
-__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __grid_constant__ RepDev R, StateView s, double* xb,
-                                                              float4* xs, double dt, int nsteps,
+__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __grid_constant__ RepDev R, StateView s, ulonglong2* xb,
+                                                              ulonglong2* xs, unsigned seq, double dt, int nsteps,
                                                               int rebuild_every, int per, int cap, int* lst_g,
                                                               int* cnt_g, double* xref_g, int* since_g, int reuse,
                                                               int64_t step0, int save, int drop_step,
                                                               double* __restrict__ bk,
                                                               const double* __restrict__ src, double* __restrict__ dst)
 {
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    const int C = (int)cl.num_blocks();
+    const int rank = blockIdx.x;
     const int n = (int)d.n;
     extern __shared__ float4 cl_pos[];
     float4* const ph = cl_pos;
@@ -215,8 +241,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
     int* lst = reinterpret_cast<int*>(xref_s + 3 * (size_t)per + ((3 * per) & 1));  // 16-byte aligned
     int* cnt = lst + (size_t)per * cap;
     float* fsum = reinterpret_cast<float*>(cnt + per);
-    __shared__ unsigned flag[2];  // rebuild requests of the step of each parity
-    __shared__ __align__(8) unsigned long long mbar[2];  // the CTAs' positions of each parity are written
+    __shared__ int gave_up;  // some record of this step did not come
     const int tid = threadIdx.x;
     const int a0 = rank * per;
     const int na = max(0, min(n - a0, per));
@@ -246,11 +271,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
         bk[2 * seg + eo] = a;
     }
 
-    // the static w parts (charge, atom flags) of the own atoms in both parities
-    for (int t = tid; t < 4 * na; t += CL_THREADS) {
-        const int j = a0 + (t >> 2);
-        xs[(size_t)(t & 3) * n + j].w = (t & 1) ? d.plo[j].w : d.phi[j].w;
-    }
+    // the charges of all atoms
+    if (POTS & NBG_POT_EL)
+        for (int j = tid; j < n; j += CL_THREADS) ph[j].w = d.phi[j].w;
     int since = 0;
     bool built = false;  // a list build ran in this launch (the same in every CTA)
     if (reuse) {
@@ -265,15 +288,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
         for (int t = tid; t < 3 * na; t += CL_THREADS) xref_s[t] = xref_g[3 * (size_t)a0 + t];
         since = *since_g;
     }
-    if (tid < 2) flag[tid] = 0u;
-    if (tid == 0) {
-        mbar_init(smem_addr(&mbar[0]), C);  // an arrival per CTA
-        mbar_init(smem_addr(&mbar[1]), C);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    // every CTA of the cluster is running (and initialised) before any
-    // remote shared-memory access
-    cl.sync();
+    if (tid == 0) gave_up = 0;
+    __syncthreads();
 
     // the frame sink (trajectory saving): state of time index step0 + st;
     // its other fields are read at a save point, `unsaved` steps ahead
@@ -316,54 +332,83 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
         }
         if (st == nsteps) break;  // uniform: every thread leaves after the last kick
         const int par = st & 1;
-        float4* const P = xs + (size_t)(2 * par) * n;  // split positions of this step
-        double* X = xb + (size_t)par * 3 * n;  // FP64 positions of this step
-        const unsigned mb = smem_addr(&mbar[par]);
+        ulonglong2* const P = xs + (size_t)(2 * par) * n;  // split positions of this step
+        ulonglong2* const X = xb + (size_t)par * 3 * n;    // FP64 positions
+        const unsigned tag = (seq + (unsigned)st) << 1;
         // drift, split and displacement check of the own atoms
         if (tid < owners) {
             double dk = 0.0;
+            float h = 0.f, l = 0.f;
             if (owner) {
                 if (!ACCEL) x = drift1(x, v, a, dt, dtsq);
-                X[eo] = x;
-                float h, l;
-                split_kept_image(R, x, img, h, l);
-                reinterpret_cast<float*>(P + io)[k] = h;
-                reinterpret_cast<float*>(P + n + io)[k] = l;
                 // (a launch that does not reuse lists builds at step 0, which
                 // sets xref_s)
                 dk = x - xref_s[3 * ko + k];
+                split_kept_image(R, x, img, h, l);
             }
             const float fk = (float)dk, fk2 = fk * fk;
-            const float f2 = fk2 + __shfl_down_sync(0xffffffffu, fk2, 1) + __shfl_down_sync(0xffffffffu, fk2, 2);
-            bool moved = owner && k == 0 && (st > 0 || reuse) && !(f2 < still2);
+            const int l0 = (tid & 31) - k;  // the atom's first lane
+            const float f2 = __shfl_sync(0xffffffffu, fk2, l0) + __shfl_sync(0xffffffffu, fk2, l0 + 1) +
+                             __shfl_sync(0xffffffffu, fk2, l0 + 2);
+            bool moved = owner && (st > 0 || reuse) && !(f2 < still2);
             if (__any_sync(0xffffffffu, moved)) {
-                const double dy = __shfl_down_sync(0xffffffffu, dk, 1), dz = __shfl_down_sync(0xffffffffu, dk, 2);
-                moved = moved && !(dk * dk + dy * dy + dz * dz <= d.skin_half2);
+                const double dx = __shfl_sync(0xffffffffu, dk, l0), dy = __shfl_sync(0xffffffffu, dk, l0 + 1),
+                             dz = __shfl_sync(0xffffffffu, dk, l0 + 2);
+                moved = moved && !(dx * dx + dy * dy + dz * dz <= d.skin_half2);
             }
-            // every thread has read the last step's flag; peers write it again
-            // only after this step's arrivals
-            if (tid == 0) flag[par ^ 1] = 0u;
-            const bool any_moved = owners_sync_or((unsigned)owners, moved);
-            // (drop_step: a host-set test of the timeout path; no CTA arrives for
-            // that step, so every wait runs out)
-            if (tid < C && st != drop_step) {
-                if (any_moved) *cl.map_shared_rank(&flag[par], tid) = 1u;
-                mbar_arrive_peer(cluster_addr(mb, tid));
+            // lane 0 of the atom writes the hi record, lane 1 the lo record
+            const float hx = __shfl_sync(0xffffffffu, h, l0), hy = __shfl_sync(0xffffffffu, h, l0 + 1),
+                        hz = __shfl_sync(0xffffffffu, h, l0 + 2);
+            const float lx = __shfl_sync(0xffffffffu, l, l0), ly = __shfl_sync(0xffffffffu, l, l0 + 1),
+                        lz = __shfl_sync(0xffffffffu, l, l0 + 2);
+            // (drop_step: a host-set test of the timeout path; no CTA writes
+            // that step's records, so every wait runs out)
+            if (owner && st != drop_step) {
+                if (k < 2) rec_store3(P + k * n + io, k ? lx : hx, k ? ly : hy, k ? lz : hz, tag | (moved ? 1u : 0u));
+                rec_store(X + eo, (unsigned long long)__double_as_longlong(x), tag);
             }
         }
-        // all positions of this step (the k-th use of mbar[par] completes phase
-        // k). A wait that ran out ends this CTA's loop and, as it arrives for
-        // no further step, the others' at their next wait
-        const bool ok = mbar_wait(mb, (unsigned)((st >> 1) & 1));
-        if (ok) {
-#pragma unroll 2
-            for (int t = tid; t < 2 * n; t += CL_THREADS) cl_pos[t] = __ldcg(P + t);
+        // all records of this step, several reads in flight per thread. One that
+        // does not come ends this CTA's loop and, as it writes no further
+        // step, the others' at their next one
+        bool moved = false;
+        {
+            constexpr int B = 8;
+            unsigned tries = 0;
+            for (int t0 = tid; t0 < 2 * n; t0 += B * CL_THREADS) {
+                // (all that are missing are read again together: one after
+                // the other they cost a round trip each)
+                ulonglong2 r[B];
+                unsigned missing = 0u;
+#pragma unroll
+                for (int q = 0; q < B; ++q)
+                    if (t0 + q * CL_THREADS < 2 * n) missing |= 1u << q;
+                while (missing != 0u && tries < CL_TRIES) {
+                    ++tries;
+#pragma unroll
+                    for (int q = 0; q < B; ++q)
+                        if (missing >> q & 1u) r[q] = rec_load(P + t0 + q * CL_THREADS);
+#pragma unroll
+                    for (int q = 0; q < B; ++q) {
+                        if ((missing >> q & 1u) && ((unsigned)(r[q].y >> 32) ^ tag) <= 1u) {
+                            missing &= ~(1u << q);
+                            moved |= ((unsigned)(r[q].y >> 32) & 1u) != 0u;
+                            float* o = reinterpret_cast<float*>(cl_pos + t0 + q * CL_THREADS);
+                            *reinterpret_cast<float2*>(o) =
+                                make_float2(__uint_as_float((unsigned)r[q].x), __uint_as_float((unsigned)(r[q].x >> 32)));
+                            o[2] = __uint_as_float((unsigned)r[q].y);
+                        }
+                    }
+                }
+                if (missing != 0u) gave_up = 1;
+            }
         }
-        if (__syncthreads_or(ok ? 0 : 1)) {
+        const int any_moved = __syncthreads_or(moved ? 1 : 0);
+        if (gave_up) {
             if (tid == 0) status_set(d.status, ST_TIMEOUT);
             break;
         }
-        const bool build = (st == 0 && !reuse) || *(volatile unsigned*)&flag[par] != 0u ||
+        const bool build = (st == 0 && !reuse) || any_moved ||
                            (rebuild_every > 0 && since >= rebuild_every);
         if (build) {
             // lists of the own atoms, entries in j order: a warp tests 32 atoms j
@@ -450,10 +495,11 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
             const int c = active ? cnt[g] : 0;
             float p[3] = {0.f, 0.f, 0.f};
             bool range_err = false;
-#pragma unroll 2
-            for (int k = lane; k < c; k += LPA) {
-                const int j = dbg_index(lst[g * cap + k], d.n, i, d.status);
-                cl_pair<POTS>(d, R, i, j, hi_i, lo_i, ph[j], pl[j], kqi, X, p, range_err);
+            for (int k = lane; k < c; k += CL_M * LPA) {
+                int j[CL_M];
+#pragma unroll
+                for (int q = 0; q < CL_M; ++q) j[q] = dbg_index(lst[g * cap + min(k + q * LPA, c - 1)], d.n, i, d.status);
+                cl_pairs<POTS>(d, R, i, j, (c - k + LPA - 1) / LPA, hi_i, lo_i, ph, pl, kqi, X, tag, p, range_err);
             }
             const LaneSum f = lane_sums3<LPA>(p[0], p[1], p[2], lane);
             if (range_err) status_set(d.status, ST_RANGE);
@@ -462,12 +508,8 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
                 fsum[6 * g + 2 * f.comp + 1] = f.e;
             }
         }
-        // the next kick and drift touch only this CTA's own atoms: a block
-        // barrier, no cluster barrier
         __syncthreads();
     }
-    // all flags and arrivals are in: no CTA's shared memory is written to any more
-    cl.sync();
     if (owner && !ACCEL) {
         s.x[eo] = x;
         s.v[eo] = v;
@@ -488,7 +530,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_vv(Dev d, const __gri
     if (!ACCEL && rank == 0 && tid == 0) *since_g = since;
 }
 
-typedef void (*cluster_kernel_t)(Dev, RepDev, StateView, double*, float4*, double, int, int, int, int, int*, int*, double*, int*, int, int64_t,
+typedef void (*cluster_kernel_t)(Dev, RepDev, StateView, ulonglong2*, ulonglong2*, unsigned, double, int, int, int, int, int*, int*, double*, int*, int, int64_t,
                                  int, int, double*, const double*, double*);
 
 template <int LPA>
@@ -502,7 +544,6 @@ static cluster_kernel_t cluster_kernel_pots(int pots, bool accel)
     }
 }
 
-// (at most 128 atoms per CTA: 8 lanes each at least)
 static cluster_kernel_t cluster_kernel(const nbg_ctx* c, int lpa, bool accel = false)
 {
     switch (lpa) {
@@ -512,9 +553,26 @@ static cluster_kernel_t cluster_kernel(const nbg_ctx* c, int lpa, bool accel = f
     }
 }
 
-// Plan the cluster path for the current list capacity: cluster size (16 where
-// the device allows it, else the portable 8), atoms per CTA, lanes per atom
-// and shared-memory bytes. Returns false when the system does not qualify
+// A cooperative launch of the loop's shape: its CTAs wait for one another.
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    explicit ClusterLaunch(const nbg_ctx* c)
+    {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.gridDim = dim3(c->cluster_size);
+        cfg.blockDim = dim3(CL_THREADS);
+        cfg.dynamicSmemBytes = c->cluster_bytes;
+        cfg.stream = c->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    ClusterLaunch(const ClusterLaunch&) = delete;
+};
+
+// Plan the loop for the current list capacity: CTAs, atoms per CTA, lanes per
+// atom and shared-memory bytes. Returns false when the system does not qualify
 // (one replica of a potential system under cubic boundaries, no
 // thermostat, small enough for the shared-memory copies).
 bool cluster_plan(nbg_ctx* c)
@@ -523,73 +581,40 @@ bool cluster_plan(nbg_ctx* c)
     if (c->cluster_disabled || c->path != PATH_LIST || c->nrep != 1 || c->d.kind != NBG_SYSTEM_POTENTIAL ||
         c->d.bc != NBG_BC_CUBIC || c->d.therm != NBG_THERMO_NULL || c->baoab || c->n < 64 || c->n > 2048)
         return false;
-    // (the cluster lists' rows are whole 16-byte units: cap rounded up to 4)
+    // (the lists' rows are whole 16-byte units: cap rounded up to 4)
     const int n = (int)c->n, cap = (c->d.nbr_cap + 3) & ~3;
-    for (int C = CL_MAX; C >= 8; C /= 2) {
-        const int per = (n + C - 1) / C;
-        if (per > 128) continue;  // owner threads: 4 warps x 32 lanes
-        int lpa = 32;
-        while (lpa > 8 && per * lpa > CL_THREADS) lpa /= 2;
-        if (per * lpa > CL_THREADS) continue;
-        const size_t bytes = cluster_smem(n, per, cap);
-        // (two position buffers' worth: with lists longer than this leaves room
-        // for, the step graphs serve the system)
-        if (bytes + sizeof(float4) * 2 * (size_t)n > 200 * 1024) continue;
-        cluster_kernel_t k = cluster_kernel(c, lpa), ka = cluster_kernel(c, lpa, true);
-        bool attrs_ok = true;
-        for (cluster_kernel_t f : {k, ka}) {
-            attrs_ok = attrs_ok &&
-                       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess &&
-                       (C <= 8 || cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                                      cudaSuccess);
-        }
-        if (!attrs_ok) {
+    // the lanes per atom and the line between this loop and the step graphs
+    // are those of 1024 threads and 200 KB on each of 16 SMs, so that a
+    // system keeps the order of its FP32 sums whatever the CTAs
+    const int part = (n + 15) / 16;
+    const int lpa = part <= 32 ? 32 : part <= 64 ? 16 : 8;
+    if (cluster_smem(n, part, cap) + sizeof(float4) * 2 * (size_t)n > 200 * 1024) return false;
+    const int per = CL_THREADS / lpa, C = (n + per - 1) / per;
+    const size_t bytes = cluster_smem(n, per, cap);
+    for (cluster_kernel_t f : {cluster_kernel(c, lpa), cluster_kernel(c, lpa, true)}) {
+        // (the attribute is the function's, for every context of the process)
+        int blocks = 0;
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, f, CL_THREADS, bytes) != cudaSuccess ||
+            blocks * c->sms < C) {
             cudaGetLastError();
-            continue;
+            return false;
         }
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = C;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(C);
-        cfg.blockDim = dim3(CL_THREADS);
-        cfg.dynamicSmemBytes = bytes;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)k, &cfg) != cudaSuccess || clusters < 1) {
-            cudaGetLastError();
-            continue;
-        }
-        c->cluster_ok = true;
-        c->cluster_size = C;
-        c->cluster_per = per;
-        c->cluster_lpa = lpa;
-        c->cluster_bytes = bytes;
-        c->cluster_cap = cap;
-        return true;
     }
-    return false;
+    c->cluster_ok = true;
+    c->cluster_size = C;
+    c->cluster_per = per;
+    c->cluster_lpa = lpa;
+    c->cluster_bytes = bytes;
+    c->cluster_cap = cap;
+    return true;
 }
 
 int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps, int rebuild_every, int64_t step0,
                       unsigned* status)
 {
     cluster_kernel_t k = cluster_kernel(c, c->cluster_lpa);
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c->cluster_size;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(c->cluster_size);
-    cfg.blockDim = dim3(CL_THREADS);
-    cfg.dynamicSmemBytes = c->cluster_bytes;
-    cfg.stream = c->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    ClusterLaunch L(c);
     // a one-shot test of the timeout path (NBG_TEST_CLUSTER_DROP at context
     // creation): the launch drops the position copies of one step
     int drop = -2;
@@ -602,11 +627,12 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
     Dev d = c->d;
     d.status = status;
     prof_begin(c);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], s, c->cluster_x, c->cluster_split, dt, (int)nsteps, rebuild_every,
+    cudaError_t e = cudaLaunchKernelEx(&L.cfg, k, d, c->reps_h[0], s, c->cluster_x, c->cluster_split, c->cluster_seq, dt, (int)nsteps, rebuild_every,
                                        c->cluster_per, c->cluster_cap, c->cluster_lists, c->cluster_cnt,
                                        c->cluster_xref, c->cluster_since, c->cluster_lists_valid ? 1 : 0, step0,
                                        c->sink_on ? 1 : 0, drop, c->bk, (const double*)nullptr, (double*)nullptr);
     prof_end(c);
+    c->cluster_seq += (unsigned)nsteps;
     if (e != cudaSuccess) return cuda_fail(c, e, "k_cluster_vv launch");
     NBG_LAUNCH_CHECK(c, "k_cluster_vv");
     return NBG_OK;
@@ -619,74 +645,49 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
 int launch_cluster_accel(nbg_ctx* c, const double* u, double* dv, unsigned* status)
 {
     cluster_kernel_t k = cluster_kernel(c, c->cluster_lpa, true);
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c->cluster_size;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(c->cluster_size);
-    cfg.blockDim = dim3(CL_THREADS);
-    cfg.dynamicSmemBytes = c->cluster_bytes;
-    cfg.stream = c->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    ClusterLaunch L(c);
     Dev d = c->d;
     d.status = status;
     prof_begin(c);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k, d, c->reps_h[0], c->st, c->cluster_x, c->cluster_split, 0.0, 1, 0, c->cluster_per, c->cluster_cap,
+    cudaError_t e = cudaLaunchKernelEx(&L.cfg, k, d, c->reps_h[0], c->st, c->cluster_x, c->cluster_split, c->cluster_seq, 0.0, 1, 0, c->cluster_per, c->cluster_cap,
                                        c->cla_lists, c->cla_cnt, c->cla_xref, c->cluster_since,
                                        c->cla_valid ? 1 : 0, (int64_t)0, 0, -2, c->bk, u, dv);
     prof_end(c);
+    ++c->cluster_seq;
     if (e != cudaSuccess) return cuda_fail(c, e, "k_cluster_vv (right-hand side) launch");
     NBG_LAUNCH_CHECK(c, "k_cluster_vv");
     return NBG_OK;
 }
 
-// The launch floor of the cluster loop's shape: a kernel with the same CTAs,
-// threads, shared memory and cluster that only passes one cluster barrier.
-__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_empty(int* sink)
+// The launch floor of the loop's shape: a kernel with the same CTAs, threads,
+// shared memory and launch attribute that does nothing.
+__global__ void __launch_bounds__(CL_THREADS) k_cluster_empty(int* sink)
 {
     extern __shared__ float4 ce_s[];
-    cg::cluster_group cl = cg::this_cluster();
     if (threadIdx.x == 0) ce_s[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-    cl.sync();
+    __syncthreads();
     if (threadIdx.x == 0 && ce_s[0].x != 0.f) *sink = 1;  // never: keeps the store live
 }
 
 int cluster_launch_floor(nbg_ctx* c, double* us_single, double* us_per_launch)
 {
     if (!c->cluster_ok) return NBG_ERR_UNSUPPORTED;
-    if (cudaFuncSetAttribute(k_cluster_empty, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->cluster_bytes) !=
-            cudaSuccess ||
-        (c->cluster_size > 8 &&
-         cudaFuncSetAttribute(k_cluster_empty, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
+    if (cudaFuncSetAttribute(k_cluster_empty, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
         return cuda_fail(c, cudaGetLastError(), "k_cluster_empty attributes");
     int* sink = nullptr;
     if (cudaMalloc(&sink, sizeof(int)) != cudaSuccess) return cuda_fail(c, cudaGetLastError(), "probe sink");
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c->cluster_size;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(c->cluster_size);
-    cfg.blockDim = dim3(CL_THREADS);
-    cfg.dynamicSmemBytes = c->cluster_bytes;
-    cfg.stream = c->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    ClusterLaunch L(c);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaError_t e = cudaSuccess;
-    for (int k = 0; k < 20 && e == cudaSuccess; ++k) e = cudaLaunchKernelEx(&cfg, k_cluster_empty, sink);
+    for (int k = 0; k < 20 && e == cudaSuccess; ++k) e = cudaLaunchKernelEx(&L.cfg, k_cluster_empty, sink);
     const int reps = 200;
     float ms = 0.f, single = 0.f;
     if (e == cudaSuccess) {
         // back to back
         cudaEventRecord(e0, c->stream);
-        for (int k = 0; k < reps && e == cudaSuccess; ++k) e = cudaLaunchKernelEx(&cfg, k_cluster_empty, sink);
+        for (int k = 0; k < reps && e == cudaSuccess; ++k) e = cudaLaunchKernelEx(&L.cfg, k_cluster_empty, sink);
         cudaEventRecord(e1, c->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
@@ -695,7 +696,7 @@ int cluster_launch_floor(nbg_ctx* c, double* us_single, double* us_per_launch)
     for (int k = 0; k < reps && e == cudaSuccess; ++k) {
         float m1 = 0.f;
         cudaEventRecord(e0, c->stream);
-        e = cudaLaunchKernelEx(&cfg, k_cluster_empty, sink);
+        e = cudaLaunchKernelEx(&L.cfg, k_cluster_empty, sink);
         cudaEventRecord(e1, c->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&m1, e0, e1);

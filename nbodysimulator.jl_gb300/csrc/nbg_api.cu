@@ -633,8 +633,12 @@ static int plan_cluster(nbg_ctx* c)
     c->cla_valid = false;
     if (!cluster_plan(c)) return NBG_OK;
     int st;
-    if (!c->cluster_x && (st = dalloc(c, &c->cluster_x, 6 * (size_t)c->n))) return st;
-    if (!c->cluster_split && (st = dalloc(c, &c->cluster_split, 4 * (size_t)c->n))) return st;
+    if (!c->cluster_x) {
+        // (no record carries a step's tag before it is written)
+        if ((st = dalloc(c, &c->cluster_x, 10 * (size_t)c->n))) return st;
+        c->cluster_split = c->cluster_x + 6 * (size_t)c->n;
+        CK(cudaMemsetAsync(c->cluster_x, 0, 10 * sizeof(ulonglong2) * (size_t)c->n, c->stream), "loop records");
+    }
     for (int** p : {&c->cluster_lists, &c->cluster_cnt, &c->cla_lists, &c->cla_cnt}) {
         if (*p) dfree(c, *p);
         *p = nullptr;

@@ -259,13 +259,14 @@ struct nbg_ctx {
     int64_t npad = 0;
     int grav_chunks = 1;
     int grav_variant = 1;     // k_gravity form (bodies per thread, packed FP32x2)
-    // small systems: velocity Verlet in one persistent cluster launch (k_cluster.cu)
+    // small systems: velocity Verlet in one persistent launch of CTAs that wait for one another (k_cluster.cu)
     bool cluster_disabled = false;
     bool cluster_ok = false;
     int cluster_size = 0, cluster_per = 0, cluster_lpa = 0, cluster_cap = 0;
     size_t cluster_bytes = 0;
-    double* cluster_x = nullptr;  // FP64 positions of the two step parities [2][3n]
-    float4* cluster_split = nullptr;  // and split ones [2][hi, lo][n]
+    ulonglong2* cluster_x = nullptr;      // FP64 positions of the two step parities as records [2][3n]
+    ulonglong2* cluster_split = nullptr;  // and split ones [2][hi, lo][n] (the same allocation)
+    unsigned cluster_seq = 1;             // the tag of the next launch's first step
     // the lists a cluster launch leaves for the next ([CTA][per][cap], counts,
     // steps since the build); valid only while nothing else changed the state
     int* cluster_lists = nullptr;
@@ -290,7 +291,7 @@ struct nbg_ctx {
     int* ens_since = nullptr;     // per replica: steps since its list build
     uint4* ens_pref = nullptr;    // per atom: fixed-point position at its replica's last build
     // test of the cluster loop's timeout path: the launch after
-    // cluster_test_skip others drops the position copies of this step (-1:
+    // cluster_test_skip others drops the position records of this step (-1:
     // its last step; -2: none)
     int cluster_test_drop = -2;
     // debug builds: NBG_TEST_PLANT_INDEX=k writes n + k into the first entry

@@ -759,19 +759,21 @@ int launch_step_advance(nbg_ctx* c, int64_t by)
 // pinned staging (host memory the GPU reads directly), stored into the
 // scratch state, packed, and checked for displacement against the positions
 // of the last list build (rebuild flag of the call counter's parity); the
-// status word starts clean.
+// status word starts clean. Without lists the accelerations are cleared instead.
 __global__ void k_accel_import(Dev d, StateView s, const double* __restrict__ hu, const double* __restrict__ hv,
-                               int v_read, StepRef pos)
+                               int v_read, int lists, StepRef pos)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) *d.status = 0u;
-    const int parity = (int)(step_of(pos) & 1);
+    const int parity = lists ? (int)(step_of(pos) & 1) : 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < d.cols; i += (int64_t)gridDim.x * blockDim.x) {
         for (int k = 0; k < 3; ++k) {
             s.x[3 * i + k] = hu[3 * i + k];
             if (v_read) s.v[3 * i + k] = hv[3 * i + k];
+            if (!lists) s.a_new[3 * i + k] = 0.0;
         }
         if (i >= d.n) continue;
         pack_atom(d, i, s.x);
+        if (!lists) continue;
         const double dx = s.x[3 * i] - d.xref[3 * i];
         const double dy = s.x[3 * i + 1] - d.xref[3 * i + 1];
         const double dz = s.x[3 * i + 2] - d.xref[3 * i + 2];
@@ -790,13 +792,14 @@ __global__ void k_accel_export(Dev d, StateView s, double* __restrict__ hdv, dou
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (nh) hv[3 * d.n] = s.v[3 * d.n];
         *hstat = *d.status;
-        *counter += 1;
+        if (counter) *counter += 1;
     }
 }
 
 int launch_accel_import(nbg_ctx* c, const StateView& s, const double* hu, const double* hv, bool v_read, StepRef pos)
 {
-    k_accel_import<<<grid_for(c->cols, 256), 256, 0, c->stream>>>(c->d, s, hu, hv, v_read ? 1 : 0, pos);
+    k_accel_import<<<grid_for(c->cols, 256), 256, 0, c->stream>>>(c->d, s, hu, hv, v_read ? 1 : 0,
+                                                                  c->path == PATH_LIST ? 1 : 0, pos);
     NBG_LAUNCH_CHECK(c, "k_accel_import");
     return NBG_OK;
 }

@@ -895,7 +895,9 @@ __device__ __forceinline__ bool ap_skips(int t, int b, int n, bool water)
 // COOP, for systems of up to AP_COOP_TILES tiles, which are bound by
 // latency: the CTA's 8 warps evaluate 16 bodies j each of one tile into
 // shared memory, and three warps then add a component each in body order
-// (n = 648 water: 11 us against 22 with a tile per warp).
+// (n = 648 water: 11 us against 22 with a tile per warp; 8.2 to 7.7 in a step
+// since the cluster's first barrier orders no memory and ends behind the pairs).
+// 16 warps of 8 bodies were slower from 1000 bodies on (18.5 us against 14.5).
 // Otherwise a warp takes a whole tile and adds as it evaluates (bound by the
 // FP32 pipe: 22 instructions a pair and warp for the bare Coulomb force, 10
 // of them packed; an evaluation of 4000 ions 27 us, 41 with COOP; of 12000,
@@ -905,6 +907,9 @@ __device__ __forceinline__ bool ap_skips(int t, int b, int n, bool water)
 template <bool COOP, bool CUBIC, bool HAS_LJ, bool HAS_EL, bool CUT, bool WATER>
 __global__ void __launch_bounds__(APC_WARPS * 32) k_allpairs_cut(Dev d, StateView s, int C)
 {
+    // every CTA of the cluster runs before its shared memory is written to:
+    // waited for before the first such write (no data goes with this barrier)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;");
     extern __shared__ float apc_sm[];
     auto cluster = cooperative_groups::this_cluster();
     float* const sums = cluster.map_shared_rank(apc_sm, 0);   // [tiles][3][32], the first CTA's
@@ -920,10 +925,10 @@ __global__ void __launch_bounds__(APC_WARPS * 32) k_allpairs_cut(Dev d, StateVie
     const ApOwn own(d.reps[0], hi_i, lo_i, HAS_EL ? (float)(d.el_k_d * d.charge[ii]) : 0.0f);
     ApStage<SUB>& sh = stage[w];
     bool range_err = false;
-    cluster.sync();  // every CTA runs before its shared memory is written to
+    if constexpr (!COOP) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     // the m staged bodies from j0 on; put(k, the AP_G values from slot k on)
     auto eval = [&](auto skip, int j0, int m, auto put) {
-#pragma unroll(COOP ? 4 : 2)
+#pragma unroll 2
         for (int k = 0; k < SUB; k += AP_G) {
             if (k >= m) break;
             float fx[AP_G], fy[AP_G], fz[AP_G];
@@ -952,6 +957,7 @@ __global__ void __launch_bounds__(APC_WARPS * 32) k_allpairs_cut(Dev d, StateVie
             if (ap_skips(t, b, n, WATER)) eval(std::true_type{}, j0, m, put);
             else eval(std::false_type{}, j0, m, put);
             __syncthreads();
+            if (ti == 0) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
             if (w < 3) {
                 const float* v = val + w * AT * 32 + lane;
                 const int mt = min(AT, n - t * AT);

@@ -24,10 +24,10 @@ e2e      : the same steps through the reference-facing drop-in, nbg_accel
            reads back dv.
 roofline : the dominant force kernel's algorithmic FLOP/s (20 flop per pair)
            or bytes against the measured peak. The LJ workload runs as
-           persistent cluster launches of many steps: its line gives the step
-           loop's time per step against the issue floor of the cluster's SMs
-           (warp instructions per step from ncu), and the launch floor of the
-           cluster shape. A batch that runs the persistent ensemble loop is
+           persistent launches of many steps: its line gives the step
+           loop's time per step against the issue floor of its SMs
+           (warp instructions per step from ncu), and the launch floor of its
+           shape. A batch that runs the persistent ensemble loop is
            reported the same way against all SMs; the ensemble tuner times
            the loop's forms and the per-step graphs after 100 untimed steps.
 --workload rdf: the radial distribution function's pair histogram
@@ -804,7 +804,7 @@ def main():
     prof_steps = min(args.steps, 20 if args.workload == "gravity" else 200)
     eng.advance(dt, prof_steps)
     kern_ms, kern_n = eng.force_kernel_time()
-    # small systems run the persistent cluster step loop: one launch per
+    # small systems run the persistent step loop (k_cluster_vv): one launch per
     # chunk of steps, timed whole
     cluster = None if batch else eng.cluster_shape()
     ens = eng.ensemble_form() if batch else None
@@ -915,14 +915,15 @@ def main():
     form = eng.force_form() if kernel_name == "k_force_list" else None
     if form is not None and form[1]:
         # the fixed-point kernel: per-warp list staging up to 16 lanes per atom
-        kernel_name = "k_force_fxw" if form[0] <= 16 and not os.environ.get("NBG_FX_BLOCK") else "k_force_fx"
+        # and a warp per atom at 32
+        kernel_name = "k_force_fx" if os.environ.get("NBG_FX_BLOCK") else "k_force_fxw" if form[0] <= 16 else "k_force_fxr"
     traffic = profile_traffic(f"{kernel_name}:{w['name']}")
     roofline = {"bound": bound, "achieved": achieved, "peak": peak, "unit": unit,
                 "frac": (achieved / peak) if peak else None, "traffic": traffic, "kernel": kernel_name,
                 "kernel_ms": avg_kern, "kernel_launches": kern_n, "peak_source": peak_src}
     if cluster is not None:
-        # a few kB per step stay on chip: the bound is the issue rate of the
-        # cluster's SMs (4 warp instructions per clock each) for the step's
+        # the state stays on chip: the bound is the issue rate of the
+        # loop's SMs (4 warp instructions per clock each) for the step's
         # warp instructions (ncu), at the sampled SM clock
         inst = profile_value(f"k_cluster_vv:{w['name']}", "issue.json")
         mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 2070.0

@@ -324,7 +324,8 @@ __global__ void __launch_bounds__(256) k_kick_T(Dev d, ThermoK K, const double* 
 // sub-partition, and a third of the warps. The Nose-Hoover column is moved by
 // the block after the atoms'; the other blocks read zeta from zc_in, so that
 // it may be moved meanwhile (zc_out). One launch instead of up to four per
-// step (kick, Andersen, frame, drift): 10,976 LJ atoms 45 -> 36 us a step.
+// step (kick, Andersen, frame, drift): 10,976 LJ atoms 45 -> 36 us a step
+// (28 since the list forces take a warp per atom).
 // WATER: 3 molecules a warp (27 lanes), and the bond and angle accelerations
 // (k_bonded's) are added before the kick from the positions the lanes hold:
 // a launch and a pass over a_new less, with 4 FP64 instructions a warp

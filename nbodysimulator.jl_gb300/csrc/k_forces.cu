@@ -900,12 +900,15 @@ __device__ __forceinline__ bool ap_skips(int t, int b, int n, bool water)
 // 16 warps of 8 bodies were slower from 1000 bodies on (18.5 us against 14.5).
 // Otherwise a warp takes a whole tile and adds as it evaluates (bound by the
 // FP32 pipe: 22 instructions a pair and warp for the bare Coulomb force, 10
-// of them packed; an evaluation of 4000 ions 27 us, 41 with COOP; of 12000,
-// 136 us = 0.33 of the FP32 rate at 23 flop a pair).
+// of them packed; an evaluation of 4000 ions 25 us, 41 with COOP; of 12000,
+// 133 us = 0.33 of the FP32 rate at 23 flop a pair). Three blocks per SM are
+// asked for there: the bare Coulomb form then takes 80 registers instead of
+// 73 and overlaps more pairs (5000 ions 35 -> 33 us). The forms with a cutoff
+// or LJ spill at 80 (LJ and charges, 2500 bodies: 32.9 -> 34.7 us).
 #define APC_WARPS 8
 
 template <bool COOP, bool CUBIC, bool HAS_LJ, bool HAS_EL, bool CUT, bool WATER>
-__global__ void __launch_bounds__(APC_WARPS * 32) k_allpairs_cut(Dev d, StateView s, int C)
+__global__ void __launch_bounds__(APC_WARPS * 32, !COOP && !HAS_LJ && !CUT ? 3 : 0) k_allpairs_cut(Dev d, StateView s, int C)
 {
     // every CTA of the cluster runs before its shared memory is written to:
     // waited for before the first such write (no data goes with this barrier)

@@ -1092,7 +1092,7 @@ static int accel_cluster(nbg_ctx* c, double* dv, const double* u)
 // nbg_accel off the lists: the kernels read u (and v) from the pinned staging and write
 // dv and the status word there, so that the launches are queued without a
 // wait in between (with pageable copies and clears a call for 5000 ions took
-// 86 us, now 71, of which the pairs are 35). Up to ACCEL_STAGED_MAX columns (the first call allocates 9
+// 86 us, then 71; the pairs are 33 of it). Up to ACCEL_STAGED_MAX columns (the first call allocates 9
 // doubles of pinned memory each; beyond, the pairs take milliseconds).
 #define ACCEL_STAGED_MAX 16384
 

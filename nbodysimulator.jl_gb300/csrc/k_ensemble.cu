@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
     // buffer's memory, 2 cap per atom (nothing else reads them: every other
     // path builds its own lists first). Entry k of a row lies where lane
     // k % LPA finds its 8 entries of a block of 8 LPA in one 16-byte load,
-    // four packed steps of the force loop (ens_slot).
+    // four packed steps of the force loop (ens_slot). (Row capacities are
+    // whole 16-byte units and hold whole blocks: list_rows.h.)
     uint16_t* const rows = reinterpret_cast<uint16_t*>(d.nbr);
     for (int i = tid; i < n; i += THREADS) {
         pos[i].w = d.pfx[a0 + i].w;

@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "list_rows.h"
 #include "nbg_internal.cuh"
 
 static const char* kVersion = "libnbg 1.0 (sm_103a)";
@@ -524,7 +525,7 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
         if ((st = dalloc(c, &D.xref, 3 * n))) return st;
         if (d0->bc == NBG_BC_CUBIC && (st = dalloc(c, &D.img, 3 * n))) return st;
         int cell_cap = ((2 * max_cell_occ + 16 + 7) / 8) * 8;
-        int nbr_cap = ((int)std::ceil(1.3 * max_nbr + 32) + 7) / 8 * 8;
+        int nbr_cap = list_row_capacity((int)std::ceil(1.3 * max_nbr + 32));
         // lanes per atom of the list force kernel: a group of lanes per atom
         // until the GPU holds ~64 resident lanes per SM-thread slot, then one
         // thread per atom (column-major list); and at least one lane per 32
@@ -930,7 +931,7 @@ static int grow_lists(nbg_ctx* c, unsigned st)
 {
     int cell_cap = c->d.cell_cap, nbr_cap = c->d.nbr_cap;
     if (st & ST_CELL_OVERFLOW) cell_cap *= 2;
-    if (st & ST_NBR_OVERFLOW) nbr_cap = nbr_cap + nbr_cap / 2 + 32;
+    if (st & ST_NBR_OVERFLOW) nbr_cap = list_grown_capacity(nbr_cap);
     // the per-cell sort stages a cell in 48 KB of shared memory
     if (cell_cap > 12288)
         return fail(c, NBG_ERR_CAPACITY, "more than 12288 atoms in one cell: the configuration has collapsed");

@@ -755,7 +755,8 @@ struct ApOwn {
 // m of them real), in pair_cutoff's arithmetic and classification, two
 // bodies per packed instruction. One branch for the group, to the pairs that
 // FP32 does not decide: a branch per pair kept a lane's pairs from
-// overlapping. Exactly zero for a pair outside both cutoffs.
+// overlapping. Exactly zero for a pair outside both cutoffs, but NaN (the sum
+// is then reported) where a difference is not finite.
 // CUT: some cutoff is finite. SKIP: the group may hold i itself, its
 // molecule, or slots past the last body.
 #define AP_G 4
@@ -817,7 +818,7 @@ __device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApS
         lj_in[q] = lj_pair && r < (CUT ? o.lj_lo : INFINITY);
         el_in[q] = el_pair && r < (CUT ? o.el_lo : INFINITY);
         if (CUT) any |= (lj_pair && !lj_in[q] && r < o.lj_hi) || (el_pair && !el_in[q] && r < o.el_hi);
-        any |= !(r < INFINITY);
+        if (SKIP) any |= !(r < INFINITY);  // (a slot past the last body holds anything)
     }
     if (any) {
 #pragma unroll
@@ -835,7 +836,7 @@ __device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApS
                 at(r2, q) = e.r2;
                 range_err |= e.range_err;
             }
-            if (!(at(r2, q) < INFINITY) && !lj_in[q] && !el_in[q]) {
+            if (SKIP && !(r < INFINITY) && (q >= m || j0 + q == i)) {
                 at(dx, q) = at(dy, q) = at(dz, q) = 0.f;
                 at(r2, q) = 1.0f;
             }
@@ -845,7 +846,7 @@ __device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApS
     for (int h = 0; h < AP_G / 2; ++h) {
         float2 f = make_float2(0.f, 0.f);
         // (without cutoffs and skipped bodies every pair is in, but for those
-        // the branch above set to a difference of zero)
+        // with an r^2 past FP32's range: their factors are zero by themselves)
         constexpr bool ALL = !CUT && !SKIP && !WATER;
         const bool in0 = lj_in[2 * h] || el_in[2 * h], in1 = lj_in[2 * h + 1] || el_in[2 * h + 1];
         const float2 rr = make_float2(ALL || in0 ? r2[h].x : 1.f, ALL || in1 ? r2[h].y : 1.f);

@@ -747,13 +747,19 @@ __device__ __forceinline__ PairOut pair_cutoff(const Dev& d, const RepDev& R, co
 }
 
 // w rounded to the hi grid of 2^-k (w + M with M = 1.5 * 2^(52-k): the sum's
-// unit is the grid's) and the remainder; the grid's integer comes from the
-// sum's low word.
+// unit is the grid's) and the remainder. While |w| is below 2^31 grid units
+// (512 boxes and more) the sum's words differ from M's by the grid's integer,
+// which is the low word. Otherwise (a wrap that lost its meaning 2^60 boxes
+// out, or a position that is not finite) hi is the plain rounding: such an
+// atom is far from every other one, not at the place its low word names.
 __device__ __forceinline__ void grid_split(const RepDev& R, double w, float& h, float& l)
 {
     const double t = __dadd_rn(w, R.qmagic);
-    h = (float)__double2loint(t) * R.qinv;
-    l = (float)(w - __dsub_rn(t, R.qmagic));
+    const double g = __dsub_rn(t, R.qmagic);
+    const int q = __double2loint(t);
+    h = (float)q * R.qinv;
+    if (__double2hiint(t) - __double2hiint(R.qmagic) != q >> 31) h = (float)g;
+    l = (float)(w - g);
 }
 
 // Split a position component into (hi, lo) floats (see the layout note above).

@@ -43,10 +43,11 @@ __device__ __forceinline__ bool nearest_image(double& d, double L, double invL)
     return (h == 0x43380000 || h == 0x4337ffff) && k >= -MINIMAGE_MAX_ITERS && k <= MINIMAGE_MAX_ITERS;
 }
 
-// x < y for non-negative doubles (NaN compares as large)
+// x < y for non-negative doubles; a NaN of either sign compares as large (as
+// unsigned words: a negative one has the top bit)
 __device__ __forceinline__ bool below(double x, double y)
 {
-    return __double_as_longlong(x) < __double_as_longlong(y);
+    return (unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(y);
 }
 
 // Sums over the block of up to 3 values per thread, by warps and then in

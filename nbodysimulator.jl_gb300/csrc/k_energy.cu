@@ -217,6 +217,12 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_energy_list(Dev d, const doub
         const int cnt = min(d.nbr_count[i], d.nbr_cap);
         const uint4 qi = d.pfx ? d.pfx[i] : make_uint4(0u, 0u, 0u, 0u);
         const long long* im = reinterpret_cast<const long long*>(d.img) + 3 * i;
+        // an atom over half the minimum-image cap of boxes out (or lost): its
+        // row is not screened, for its fixed-point position may mean nothing,
+        // and every listed pair has to stay within the cap
+        bool far = false;
+        if (d.pfx)
+            for (int c = 0; c < 3; ++c) far |= (im[c] & 0x7fffffffffffffffll) > 0x40e0000000000000ll;  // |image| > 2^15
         for (int k0 = 0; k0 < cnt; k0 += 32) {
             const int k = k0 + lane;
             int j = 0;
@@ -224,9 +230,14 @@ __global__ void __launch_bounds__(EL_WARPS * 32) k_energy_list(Dev d, const doub
             if (k < cnt) {
                 j = dbg_index(d.nbr[(int64_t)k * d.nbr_kstride + i * d.nbr_istride], d.n, (int)i, d.status);
                 const bool lj = lj_i && (!water || fx_oxygen(j));
-                if (j > (int)i && (lj || (has_el && !el_excluded(d.kind, i, j)))) {
-                    cls = lj ? 3 : 1;
-                    if (d.pfx) {
+                if ((j > (int)i || far) && (lj || (has_el && !el_excluded(d.kind, i, j)))) {
+                    if (j > (int)i) {
+                        cls = lj ? 3 : 1;
+                    } else {  // (the pair's sums are with the row of j)
+                        Dist64 o;
+                        range_err |= !distance64(X + 3 * (int64_t)j, X + 3 * i, NBG_BC_CUBIC, R, o);
+                    }
+                    if (d.pfx && !far) {
                         const uint4 qj = d.pfx[j];
                         float fx, fy, fz;
                         if (fx_r2(qi, qj, fx, fy, fz) >= reach) cls = -1;

@@ -1593,6 +1593,7 @@ static int settle(nbg_ctx* c)
     }
     if (w & (ST_NONFINITE | ST_RANGE | ST_INDEX)) return status_error(c, w);
     if (w & (ST_CELL_OVERFLOW | ST_NBR_OVERFLOW)) {
+        if (c->pend_fresh) c->accel_valid = false;  // (its lists overflowed too)
         if ((st = grow_lists(c, w))) return st;
         if ((st = backup_state(c, true))) return st;
         c->step = c->pend_step0;
@@ -1640,7 +1641,10 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
     // neither cleared nor read in this call
     const bool hw_ok = can_overflow && !em && c->accel_valid && (c->cluster_ok || c->ens_ok);
     if (!hw_ok && (st = clear_status(c))) return st;
-    if (!em && !c->accel_valid) {
+    // fresh: this call computed the first acceleration, and no chunk has
+    // shown yet that the lists it came from held every pair
+    bool fresh = !em && !c->accel_valid;
+    if (fresh) {
         if ((st = init_accel(c))) return st;
     } else if (em) {
         if ((st = launch_pack(c, c->st))) return st;
@@ -1714,6 +1718,7 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
             c->pend_dt = dt;
             c->pend_steps = k;
             c->pend_step0 = step0;
+            c->pend_fresh = fresh;
             return NBG_OK;
         }
         unsigned w = 0;
@@ -1731,6 +1736,7 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
         }
         if (w & ST_FATAL) return status_error(c, w);
         if (w & (ST_CELL_OVERFLOW | ST_NBR_OVERFLOW)) {
+            if (fresh) c->accel_valid = false;  // (its lists overflowed too)
             if (++retries > 6) return fail(c, NBG_ERR_CAPACITY, "list capacity could not be grown enough");
             if ((st = grow_lists(c, w))) return st;
             if ((st = backup_state(c, true))) return st;
@@ -1740,10 +1746,11 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
             c->ens_lists_valid = false;
             c->T_valid = false;
             if ((st = clear_status(c))) return st;
-            if ((st = launch_pack(c, c->st))) return st;
+            if ((st = fresh ? init_accel(c) : launch_pack(c, c->st))) return st;
             continue;
         }
         if ((st = status_error(c, w))) return st;
+        fresh = false;
         done += k;
     }
     return NBG_OK;
@@ -2623,7 +2630,15 @@ extern "C" int nbg_ensemble_tune(nbg_ctx* c, int32_t steps, int32_t* form, doubl
         c->ens_tuned_off = false;
         if (!ensemble_plan(c)) return fail(c, NBG_ERR_UNSUPPORTED, "the batch no longer fits the ensemble loop");
     }
-    if (!c->accel_valid && (st = init_accel(c))) return st;
+    for (int attempt = 0; !c->accel_valid; ++attempt) {
+        if ((st = clear_status(c)) || (st = init_accel(c))) return st;
+        unsigned w = 0;
+        if ((st = read_status(c, &w))) return st;
+        if (attempt < 6 && (w & (ST_CELL_OVERFLOW | ST_NBR_OVERFLOW))) {  // lists that lack pairs: larger ones
+            c->accel_valid = false;
+            if ((st = grow_lists(c, w))) return st;
+        }
+    }
     if ((st = ensure_backup(c))) return st;
     if ((st = backup_state(c, false))) return st;
     const double dt = c->baoab_dt > 0.0 ? c->baoab_dt : 0.005;

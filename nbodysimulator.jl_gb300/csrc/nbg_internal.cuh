@@ -242,6 +242,7 @@ struct nbg_ctx {
     bool pending = false;
     double pend_dt = 0.0;
     int64_t pend_steps = 0, pend_step0 = 0;
+    bool pend_fresh = false;  // that call also computed the first acceleration
     // the status of a chunk reaches the host through a pinned, mapped word:
     // a chunk run as one launch (cluster or ensemble loop, chunk_hw) sets its
     // bits there directly, any other deferred chunk copies the device word

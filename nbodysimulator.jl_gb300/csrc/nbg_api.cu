@@ -1278,19 +1278,14 @@ static int ensure_backup(nbg_ctx* c)
     return c->bk ? NBG_OK : dalloc(c, &c->bk, 12 * (size_t)c->cols);
 }
 
-// x, v, a_old of the resident state to the backup (one copy), or the n atoms'
-// rows of each back (one strided copy: the cluster loop writes the backup of
-// its atoms itself, not the padding)
+// x, v, a_old of the resident state to the backup, or back: all columns, the
+// Nose-Hoover one too (the small-system loop writes the backup of its atoms
+// itself; its systems have no other column)
 static int backup_state(nbg_ctx* c, bool restore)
 {
-    const size_t seg = 3 * sizeof(double) * (size_t)c->cols;
-    if (restore) {
-        CK(cudaMemcpy2DAsync(c->st.x, seg, c->bk, seg, 3 * sizeof(double) * (size_t)c->n, 3,
-                             cudaMemcpyDeviceToDevice, c->stream),
-           "restore");
-    } else {
-        CK(cudaMemcpyAsync(c->bk, c->st.x, 3 * seg, cudaMemcpyDeviceToDevice, c->stream), "backup");
-    }
+    const size_t bytes = 3 * state_bytes(c);
+    if (restore) CK(cudaMemcpyAsync(c->st.x, c->bk, bytes, cudaMemcpyDeviceToDevice, c->stream), "restore");
+    else CK(cudaMemcpyAsync(c->bk, c->st.x, bytes, cudaMemcpyDeviceToDevice, c->stream), "backup");
     return NBG_OK;
 }
 

@@ -78,3 +78,17 @@ def test_first_steps_of_a_batch_after_regrowth(gpu, oracle, monkeypatch, how):
         s = slice(off, off + int(d.n))
         _check(d, ui, vi, u1[s], v1[s], *oracle.run(d, ui, vi, DT, 3))
         off += int(d.n)
+
+
+# the chunk that overflowed has moved the thermostat's column too
+@pytest.mark.parametrize("steps", [1, 5, 40])
+def test_nosehoover_column_after_regrowth(gpu, oracle, steps):
+    d, keep, u, v = _droplet(14, 45.0, thermostat=nbg.NoseHooverThermostat(0.7, 0.05))
+    u, v = np.concatenate([u, np.zeros((1, 3))]), np.concatenate([v, np.zeros((1, 3))])
+    ur, vr = oracle.run(d, u, v, DT, steps)
+    eng = nbg.Engine(d, 0)
+    u1, v1, _, _, _ = eng.run(u, v, DT, steps, 0, save_trajectory=False)
+    eng.close()
+    _check(d, u, v, u1[:-1], v1[:-1], ur[:-1], vr[:-1])
+    assert abs(u1[-1, 0] - ur[-1, 0]) <= 1e-5 * abs(ur[-1, 0])
+    assert abs(v1[-1, 0] - vr[-1, 0]) <= 1e-5 * abs(vr[-1, 0])

@@ -517,10 +517,7 @@ bool ensemble_plan(nbg_ctx* c)
     c->ens_smem = sizeof(uint4) * (size_t)nmax + sizeof(int) * (2 * (size_t)cmax + 1) +
                   2 * sizeof(uint16_t) * (size_t)nmax;
     ens_kernel_t k = ens_kernel(c);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->ens_smem) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    if (!allow_shared((const void*)k, c->device, c->ens_smem)) return false;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, c->ens_threads, c->ens_smem) != cudaSuccess || occ < 1) {
         cudaGetLastError();

@@ -549,11 +549,7 @@ static int fx_prepare_form(nbg_ctx* c)
     const int nbox_cap = (c->d.nbr_cap + 31) / 32;
     const size_t smem = 2 * (size_t)nbox_cap * (FX_THREADS / LPA) * 128 + 1024;
     auto kern = k_force_fx<LPA, POT>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return NBG_ERR_UNSUPPORTED;  // the list rows are too long for shared memory
-    }
+    if (!allow_shared((const void*)kern, c->device, smem)) return NBG_ERR_UNSUPPORTED;  // the list rows are too long
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, FX_THREADS, smem);
     if (occ < 1) return NBG_ERR_UNSUPPORTED;

@@ -655,6 +655,24 @@ static int plan_cluster(nbg_ctx* c)
     return NBG_OK;
 }
 
+bool allow_shared(const void* kernel, int device, size_t bytes)
+{
+    cudaFuncAttributes fa{};
+    int most = 0;
+    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    most -= (int)fa.sharedSizeBytes;
+    if (most < 0 || bytes > (size_t)most) return false;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 void prof_begin(nbg_ctx* c)
 {
     if (!c->profiling) return;

@@ -478,6 +478,12 @@ int launch_ml_batch_grad(nbg_ctx* c, const float* theta, const float* X, const f
 void prof_begin(nbg_ctx* c);
 void prof_end(nbg_ctx* c);
 
+// Opt a kernel in to dynamic shared memory; false where `bytes` do not fit.
+// The attribute is the function's, for every context of the process: it is
+// set to all the kernel can have, so that a later context with less to stage
+// takes nothing away from an earlier one.
+bool allow_shared(const void* kernel, int device, size_t bytes);
+
 // record a CUDA error on the context; returns NBG_ERR_CUDA
 int cuda_fail(nbg_ctx* c, cudaError_t e, const char* what);
 

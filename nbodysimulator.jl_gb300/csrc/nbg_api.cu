@@ -1517,12 +1517,13 @@ static int capture_graph(nbg_ctx* c, double dt)
         c->T_valid = true;
     }
     const bool fuse_vv = !is_em(c) && !c->baoab && c->nrep == 1 && c->path != PATH_GRAVITY;
-    if (fuse_vv && !c->vv_buf) {
-        int st0 = dalloc(c, &c->vv_buf, 4);
-        if (st0) return st0;
-        CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking), "side stream");
-        CK(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming), "fork event");
-        CK(cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming), "join event");
+    if (fuse_vv) {
+        // (each by itself: a call may have failed between them)
+        int st0 = NBG_OK;
+        if (!c->vv_buf && (st0 = dalloc(c, &c->vv_buf, 4))) return st0;
+        if (!c->side) CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking), "side stream");
+        if (!c->fork_ev) CK(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming), "fork event");
+        if (!c->join_ev) CK(cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming), "join event");
     }
     const int64_t launches0 = c->launches;
     const int64_t ssb0 = c->steps_since_build;
@@ -1540,10 +1541,18 @@ static int capture_graph(nbg_ctx* c, double dt)
         st = fuse ? step_baoab_fused(c, dt, StepRef{k, c->d.step_dev}, k == 0, k == G - 1)
                   : step_any(c, dt, StepRef{k, c->d.step_dev});
     if (st == NBG_OK) st = launch_step_advance(c, G);
+    if (st != NBG_OK && fuse_vv) {
+        // the thermostat's branch may be open: joined, so that the capture ends
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c->side, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive &&
+            cudaEventRecord(c->join_ev, c->side) == cudaSuccess)
+            cudaStreamWaitEvent(c->stream, c->join_ev, 0);
+    }
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     c->steps_since_build = ssb0;  // capture only recorded the steps
     c->T_valid = (c->d.therm == NBG_THERMO_BERENDSEN || c->d.therm == NBG_THERMO_NOSEHOOVER) && c->nrep == 1;
     if (st != NBG_OK) {
+        cudaGetLastError();  // (the capture's own error is not the next launch's)
         if (g) cudaGraphDestroy(g);
         return st;
     }

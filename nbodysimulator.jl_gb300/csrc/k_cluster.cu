@@ -217,8 +217,10 @@ __device__ __forceinline__ void split_kept_image(const RepDev& R, double p, doub
         if (negative64(w)) w += R.L;
         if (__double_as_longlong(w) >= __double_as_longlong(R.L)) w -= R.L;
         if (!(fabs(img) < 1048576.0)) img = __longlong_as_double(0x7ff8000000000000ll);
+        grid_split(R, w, h, l);
+    } else {
+        grid_split<true>(R, w, h, l);
     }
-    grid_split(R, w, h, l);
 }
 
 // R: the replica's constants as a kernel argument (operands from the constant

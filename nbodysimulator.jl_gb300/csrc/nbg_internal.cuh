@@ -759,13 +759,16 @@ __device__ __forceinline__ PairOut pair_cutoff(const Dev& d, const RepDev& R, co
 // which is the low word. Otherwise (a wrap that lost its meaning 2^60 boxes
 // out, or a position that is not finite) hi is the plain rounding: such an
 // atom is far from every other one, not at the place its low word names.
+// INSIDE: |w| is known to be below that (the check is 1 % of a step of the
+// small-system loop).
+template <bool INSIDE = false>
 __device__ __forceinline__ void grid_split(const RepDev& R, double w, float& h, float& l)
 {
     const double t = __dadd_rn(w, R.qmagic);
     const double g = __dsub_rn(t, R.qmagic);
     const int q = __double2loint(t);
     h = (float)q * R.qinv;
-    if (__double2hiint(t) - __double2hiint(R.qmagic) != q >> 31) h = (float)g;
+    if (!INSIDE && __double2hiint(t) - __double2hiint(R.qmagic) != q >> 31) h = (float)g;
     l = (float)(w - g);
 }
 

@@ -689,8 +689,10 @@ int gravity_plan_chunks(nbg_ctx* c, int64_t npad) { return plan_gravity(c, npad)
 #define AT 128        // j-tile: FP32 partials are summed in order over one tile
 #define AP_WARPS 10   // general form: j-tiles in flight per block, at most (48 KB of stages and sums)
 #define AP_SUB 32     // general form: bodies of a tile staged at a time per warp
-#define AP_COOP_TILES 16      // a tile per CTA up to 2048 bodies, then a tile per warp (an evaluation of
-                              // 1000 / 2000 / 3000 ions 12.5 / 18.6 / 31 us per CTA, 14.6 / 18.6 / 25 per warp)
+#define AP_COOP_TILES 16      // a tile per CTA up to 2048 bodies, then a tile per warp (kernel time, us, at 1000 /
+                              // 1500 / 2000 / 2500 bodies: ions 8.3 / 12.3 / 15.1 / 19.8 per CTA, 11.3 / 12.5 /
+                              // 12.5 / 15.6 per warp; LJ and charges in a cube 11.9 / 16.4 / 21.2 / 28.6 and
+                              // 22 / 22 / 21 / 28)
 #define AP_CLUSTER_TILES 256  // most tiles whose sums a CTA holds (96 KB)
 
 // A pair that FP32 leaves open, decided (and its difference taken) in the
@@ -767,6 +769,10 @@ __device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApS
                                          const double* X, float (&fx)[AP_G], float (&fy)[AP_G], float (&fz)[AP_G],
                                          bool& range_err)
 {
+    // an r^2 that is not below infinity takes the branch where a slot may hold
+    // anything; and with both potentials, whose forms then keep their
+    // registers (12,000 bodies 346 -> 336 us; one potential is 5 % faster without)
+    constexpr bool LOST = SKIP || (CUT && HAS_LJ && HAS_EL);
     float2 dx[AP_G / 2], dy[AP_G / 2], dz[AP_G / 2], r2[AP_G / 2], qj[AP_G / 2], fl[AP_G / 2];
     bool lj_in[AP_G], el_in[AP_G], any = false;
     auto at = [](float2* v, int q) -> float& { return (q & 1) ? v[q >> 1].y : v[q >> 1].x; };
@@ -818,7 +824,7 @@ __device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApS
         lj_in[q] = lj_pair && r < (CUT ? o.lj_lo : INFINITY);
         el_in[q] = el_pair && r < (CUT ? o.el_lo : INFINITY);
         if (CUT) any |= (lj_pair && !lj_in[q] && r < o.lj_hi) || (el_pair && !el_in[q] && r < o.el_hi);
-        if (SKIP) any |= !(r < INFINITY);  // (a slot past the last body holds anything)
+        if (LOST) any |= !(r < INFINITY);
     }
     if (any) {
 #pragma unroll
@@ -836,9 +842,9 @@ __device__ __forceinline__ void ap_pairs(const Dev& d, const ApOwn& o, const ApS
                 at(r2, q) = e.r2;
                 range_err |= e.range_err;
             }
-            if (SKIP && !(r < INFINITY) && (q >= m || j0 + q == i)) {
-                at(dx, q) = at(dy, q) = at(dz, q) = 0.f;
+            if (LOST && !(at(r2, q) < INFINITY) && !lj_in[q] && !el_in[q]) {
                 at(r2, q) = 1.0f;
+                if (SKIP && (q >= m || j0 + q == i)) at(dx, q) = at(dy, q) = at(dz, q) = 0.f;
             }
         }
     }
@@ -901,15 +907,18 @@ __device__ __forceinline__ bool ap_skips(int t, int b, int n, bool water)
 // 16 warps of 8 bodies were slower from 1000 bodies on (18.5 us against 14.5).
 // Otherwise a warp takes a whole tile and adds as it evaluates (bound by the
 // FP32 pipe: 22 instructions a pair and warp for the bare Coulomb force, 10
-// of them packed; an evaluation of 4000 ions 25 us, 41 with COOP; of 12000,
-// 133 us = 0.33 of the FP32 rate at 23 flop a pair). Three blocks per SM are
-// asked for there: the bare Coulomb form then takes 80 registers instead of
-// 73 and overlaps more pairs (5000 ions 35 -> 33 us). The forms with a cutoff
-// or LJ spill at 80 (LJ and charges, 2500 bodies: 32.9 -> 34.7 us).
+// of them packed; an evaluation of 4000 ions 23 us, 35 with COOP; of 12000,
+// 126 us = 0.35 of the FP32 rate at 23 flop a pair). Three blocks per SM are
+// asked for where 80 registers were measured to be better or as good at all
+// of these sizes: the bare Coulomb form (5000 ions 35 -> 33 us when it was
+// bounded) and LJ under cubic boundaries (7000 bodies 97 -> 88 us, 12000 232
+// -> 221). With both potentials the bound is mixed (spills): 2500 bodies
+// 28.0 -> 30.9 us, 7000 130 -> 123, 12000 346 -> 298.
 #define APC_WARPS 8
 
 template <bool COOP, bool CUBIC, bool HAS_LJ, bool HAS_EL, bool CUT, bool WATER>
-__global__ void __launch_bounds__(APC_WARPS * 32, !COOP && !HAS_LJ && !CUT ? 3 : 0) k_allpairs_cut(Dev d, StateView s, int C)
+__global__ void __launch_bounds__(APC_WARPS * 32, !COOP && (HAS_EL ? !HAS_LJ && !CUT : CUBIC) ? 3 : 0)
+    k_allpairs_cut(Dev d, StateView s, int C)
 {
     // every CTA of the cluster runs before its shared memory is written to:
     // waited for before the first such write (no data goes with this barrier)

@@ -264,7 +264,7 @@ NBG_API int nbg_pair_list(nbg_ctx* ctx, const double* u, int32_t which, int32_t*
  * Profiling support (no reference counterpart). With profiling on, CUDA
  * events bracket every launch of the context's dominant force kernel
  * (gravity all-pairs, Verlet-list pair forces or the all-pairs kernel; for a
- * context on the cluster step loop, the whole multi-step cluster launch);
+ * context on the small-system loop, the whole multi-step launch);
  * nbg_force_kernel_time returns their summed duration and count since the
  * last reset and resets them.
  */

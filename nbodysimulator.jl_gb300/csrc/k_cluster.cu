@@ -1,5 +1,6 @@
 // k_cluster.cu - velocity Verlet for small systems (up to 2048 atoms) as one
-// persistent cooperative launch.
+// persistent cooperative launch. ("Cluster" in the names is this group of
+// CTAs; it is not a thread-block cluster.)
 //
 // A step of a small system is a handful of microsecond kernels, so launches,
 // not arithmetic, set its pace. Here up to 64 co-resident CTAs run many steps
@@ -618,7 +619,7 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
     cluster_kernel_t k = cluster_kernel(c, c->cluster_lpa);
     ClusterLaunch L(c);
     // a one-shot test of the timeout path (NBG_TEST_CLUSTER_DROP at context
-    // creation): the launch drops the position copies of one step
+    // creation): the launch drops the position records of one step
     int drop = -2;
     if (c->cluster_test_drop != -2 && c->cluster_test_skip > 0) {
         --c->cluster_test_skip;
@@ -640,7 +641,7 @@ int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps,
     return NBG_OK;
 }
 
-// The right-hand side of a small system (nbg_accel) as one cluster launch:
+// The right-hand side of a small system (nbg_accel) as one launch:
 // positions from u, accelerations to dv (device addresses: pinned host
 // memory mapped into the device's space, or device memory), the launch's
 // own lists reused while no atom moved more than skin/2 from their build.
@@ -707,7 +708,7 @@ int cluster_launch_floor(nbg_ctx* c, double* us_single, double* us_per_launch)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(sink);
-    if (e != cudaSuccess) return cuda_fail(c, e, "cluster launch floor");
+    if (e != cudaSuccess) return cuda_fail(c, e, "launch floor of the small-system loop");
     if (us_per_launch) *us_per_launch = 1e3 * ms / reps;
     if (us_single) *us_single = 1e3 * single / reps;
     return NBG_OK;

@@ -14,11 +14,11 @@
 //     rebuild_every steps passed): a counting sort of the atoms into cells in
 //     shared memory, each cell's atoms in index order, then every atom's
 //     Verlet-list row from the stencil cells (FP32 superset test on the
-//     fixed-point differences), written to the global list;
+//     fixed-point differences), written to the list buffer as 16-bit indices;
 //   - the pair forces of each atom from its list row, gathering neighbours
 //     from shared memory (fx_pair2: the fixed-point kernels' classification
 //     and arithmetic, so the pair set is the reference's), joined over the
-//     atom's lanes, and the velocity update by the group's first lane.
+//     atom's lanes, and the velocity update by a lane per component.
 // The Philox noise is keyed (seed, atom, step) as in the step-graph kernels;
 // the lists and each replica's steps since its build carry over to the next
 // launch unless another path moved the state.
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ensemble(Dev d, StateView s, Ens
             ++since;
         }
         // forces from the list rows (neighbours from shared memory), then
-        // the velocity update of the atom by its group's first lane
+        // the velocity update of the atom by a lane per component
         const bool lj_atoms = POT != FX_EL;
         const float lj_lo = R.fx_lj_lo, lj_hi = R.fx_lj_hi, el_lo = R.fx_el_lo, el_hi = R.fx_el_hi;
         const float sig2h = R.fx_sig2_hi, sig2l = R.fx_sig2_lo, krf = R.fx_krf;

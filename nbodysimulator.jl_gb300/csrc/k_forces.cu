@@ -15,10 +15,14 @@
 //                    are apart by at least 1/16 of their largest |r| uses the
 //                    plain difference: its error, 2^-24 of the coordinates,
 //                    is then below 2^-19 of |r_ij|.
-//  k_allpairs        every other potential on small / unbounded systems: 32
-//                    bodies a block, a warp per 128-body j-tile, the pair
-//                    arithmetic of the split-form list kernels plus gravity
-//                    and the magnetic dipole term.
+//  k_allpairs_cut    LJ and electrostatics on small / unbounded systems under
+//                    infinite or cubic boundaries: a cluster of CTAs per 32
+//                    bodies, the 128-body j-tiles shared out over its CTAs,
+//                    their sums folded in tile order by the first one; two
+//                    bodies j per packed instruction.
+//  k_allpairs        every other form off the lists (mixed potentials, general
+//                    periodic boxes, dipoles, more than 32,768 bodies): 32
+//                    bodies a block, a warp per 128-body j-tile.
 //  k_force_list      cutoff LJ + reaction-field electrostatics over a Verlet
 //                    list (one thread per atom, coalesced column-major list).
 //  k_bonded          SPC/Fw harmonic bonds and H-O-H angles, one thread per

@@ -572,10 +572,9 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
     }
     if (getenv("NBG_NO_GRAPHS")) c->use_graphs = false;  // direct launches, for comparisons
     if (getenv("NBG_NO_CLUSTER")) c->cluster_disabled = true;  // the graph step loop for small systems too
-    // a test of the cluster loop's bounded waits: one launch (the first, or
-    // the one after ":k" more) drops the position copies of one step ("last"
-    // or a step index), so that the receivers' waits run out with no copy in
-    // flight
+    // a test of the small-system loop's bounded waits: one launch (the first,
+    // or the one after ":k" more) writes no position records of one step
+    // ("last" or a step index), so that the readers' waits run out
     if (const char* td = getenv("NBG_TEST_CLUSTER_DROP")) {
         c->cluster_test_drop = strncmp(td, "last", 4) == 0 ? -1 : std::max(0, atoi(td));
         if (const char* k = strchr(td, ':')) c->cluster_test_skip = std::max(0, atoi(k + 1));
@@ -625,8 +624,8 @@ static int build_context(nbg_ctx* c, const nbg_system_desc* descs, int nrep)
     return NBG_OK;
 }
 
-// The persistent cluster step loop for small systems (k_cluster.cu), if the
-// system qualifies at the current list capacity; its FP64 position copies.
+// The persistent step loop for small systems (k_cluster.cu), if the system
+// qualifies at the current list capacity; its records and lists.
 static int plan_cluster(nbg_ctx* c)
 {
     c->cluster_lists_valid = false;
@@ -1072,10 +1071,10 @@ static void* mapped_address(const void* p, size_t bytes)
     return a0.devicePointer;
 }
 
-// nbg_accel of a small system (the cluster path): one launch reads u and
+// nbg_accel of a small system (k_cluster.cu): one launch reads u and
 // writes dv in place when they are page-locked host buffers, else through
 // the pinned staging; the status word comes back through the mapped word.
-// Returns 1 when the cluster path no longer applies (lists grew past it).
+// Returns 1 when that loop no longer applies (lists grew past it).
 static int accel_cluster(nbg_ctx* c, double* dv, const double* u)
 {
     int st;
@@ -1111,8 +1110,10 @@ static int accel_cluster(nbg_ctx* c, double* dv, const double* u)
 // nbg_accel off the lists: the kernels read u (and v) from the pinned staging and write
 // dv and the status word there, so that the launches are queued without a
 // wait in between (with pageable copies and clears a call for 5000 ions took
-// 86 us, then 71; the pairs are 33 of it). Up to ACCEL_STAGED_MAX columns (the first call allocates 9
-// doubles of pinned memory each; beyond, the pairs take milliseconds).
+// 86 us, then 71; the pairs are 33 of it). Up to ACCEL_STAGED_MAX columns: the
+// first call allocates 9 doubles of pinned memory each, and what it saves is
+// soon small beside the pairs (16,000 ions 288 us a call, 17,000, with copies,
+// 323).
 #define ACCEL_STAGED_MAX 16384
 
 static int accel_staged(nbg_ctx* c, double* dv, double* v, const double* u, bool v_read, double* stage)
@@ -1145,7 +1146,7 @@ extern "C" int nbg_accel(nbg_ctx* c, double* dv, double* v, const double* u, dou
     // only the Berendsen and Nose-Hoover terms of the right-hand side read v
     const bool v_read = c->d.therm == NBG_THERMO_BERENDSEN || c->d.therm == NBG_THERMO_NOSEHOOVER;
     if (c->path == PATH_LIST && c->cluster_ok) {
-        // (no thermostat term: the cluster path serves plain systems only)
+        // (no thermostat term: the small-system loop serves plain systems only)
         const int st = accel_cluster(c, dv, u);
         if (st != 1) return st;
     }
@@ -1658,7 +1659,7 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
     const bool em = is_em(c);
     const bool can_overflow = c->path == PATH_LIST;
     if (can_overflow && ((st = ensure_backup(c)) || (st = ensure_hw(c)))) return st;
-    // chunks run as one launch (cluster or ensemble loop) on a state whose
+    // chunks run as one launch (small-system or replica loop) on a state whose
     // acceleration is known report to the host word: the device word is
     // neither cleared nor read in this call
     const bool hw_ok = can_overflow && !em && c->accel_valid && (c->cluster_ok || c->ens_ok);
@@ -1683,7 +1684,7 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
         // from the one-launch loops to graphs reads a clean word)
         c->chunk_hw = hw_ok && (c->cluster_ok || c->ens_ok);
         if (c->chunk_hw) *(volatile unsigned*)c->hw = 0u;  // no launch that sets it is in flight
-        // the cluster loop writes the backup of its atoms itself
+        // the small-system loop writes the backup of its atoms itself
         if (can_overflow && !(c->chunk_hw && c->cluster_ok) && (st = backup_state(c, false))) return st;
         int64_t s = 0;
         bool counter_set = false;
@@ -1699,7 +1700,7 @@ static int advance_impl(nbg_ctx* c, double dt, int64_t nsteps, bool defer)
                 continue;
             }
             if (c->cluster_ok) {
-                // the whole chunk in one persistent cluster launch (its lists
+                // the whole chunk in one persistent launch (its lists
                 // live in shared memory: the global ones are rebuilt later)
                 if ((st = launch_cluster_vv(c, c->st, dt, k - s, c->desc.rebuild_every, c->step,
                                              c->chunk_hw ? c->hw_d : c->d.status)))

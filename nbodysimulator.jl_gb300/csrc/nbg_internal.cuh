@@ -244,7 +244,7 @@ struct nbg_ctx {
     int64_t pend_steps = 0, pend_step0 = 0;
     bool pend_fresh = false;  // that call also computed the first acceleration
     // the status of a chunk reaches the host through a pinned, mapped word:
-    // a chunk run as one launch (cluster or ensemble loop, chunk_hw) sets its
+    // a chunk run as one launch (small-system or replica loop, chunk_hw) sets its
     // bits there directly, any other deferred chunk copies the device word
     // there; pend_ev follows the chunk, so settling waits for the chunk
     // alone, not for work queued on the stream after it
@@ -256,7 +256,7 @@ struct nbg_ctx {
     int64_t steps_since_build = 0;
     int64_t list_builds = 0;
     int64_t launches = 0;
-    // gravity path: bodies padded to npad (multiple of the 256-body tile)
+    // gravity path: bodies padded to npad (multiple of the largest i-block, 512)
     int64_t npad = 0;
     int grav_chunks = 1;
     int grav_variant = 1;     // k_gravity form (bodies per thread, packed FP32x2)
@@ -268,14 +268,14 @@ struct nbg_ctx {
     ulonglong2* cluster_x = nullptr;      // FP64 positions of the two step parities as records [2][3n]
     ulonglong2* cluster_split = nullptr;  // and split ones [2][hi, lo][n] (the same allocation)
     unsigned cluster_seq = 1;             // the tag of the next launch's first step
-    // the lists a cluster launch leaves for the next ([CTA][per][cap], counts,
+    // the lists such a launch leaves for the next ([CTA][per][cap], counts,
     // steps since the build); valid only while nothing else changed the state
     int* cluster_lists = nullptr;
     int* cluster_cnt = nullptr;
-    double* cluster_xref = nullptr;  // [3n] positions at the cluster lists' build
+    double* cluster_xref = nullptr;  // [3n] positions at those lists' build
     int* cluster_since = nullptr;
     bool cluster_lists_valid = false;
-    // nbg_accel's cluster launches keep lists of their own (same shapes),
+    // nbg_accel's launches of it keep lists of their own (same shapes),
     // valid for any positions within skin/2 of cla_xref
     int* cla_lists = nullptr;
     int* cla_cnt = nullptr;
@@ -291,7 +291,7 @@ struct nbg_ctx {
     int* ens_order = nullptr;     // replicas, largest first (CTA b runs replica order[b])
     int* ens_since = nullptr;     // per replica: steps since its list build
     uint4* ens_pref = nullptr;    // per atom: fixed-point position at its replica's last build
-    // test of the cluster loop's timeout path: the launch after
+    // test of the small-system loop's timeout path: the launch after
     // cluster_test_skip others drops the position records of this step (-1:
     // its last step; -2: none)
     int cluster_test_drop = -2;
@@ -411,7 +411,7 @@ int launch_gravity(nbg_ctx* c, const StateView& s);
 int launch_gravity_step(nbg_ctx* c, const StateView& s, double dt, StepRef sr, bool first, bool last);
 bool cluster_plan(nbg_ctx* c);
 // step0: the time index of the state at the launch (for the frame sink)
-// (status: the word the launch sets its bits in; the cluster loop also
+// (status: the word the launch sets its bits in; the small-system loop also
 // writes x, v, a_old of its atoms to the backup before its first step)
 int launch_cluster_vv(nbg_ctx* c, const StateView& s, double dt, int64_t nsteps, int rebuild_every, int64_t step0,
                       unsigned* status);
